@@ -69,7 +69,7 @@ BASE_SOURCES = ("core", "tma_desc")
 # residual streams (sequential and parallel blocks), state-space and gated recurrences, attention, rotary and
 # latent-attention kernels, expert routing, argmax and expert sum.  Each
 # registered architecture names its own subset (executor.registry.Architecture.sources).
-LAYERED_SOURCES = ("gemm_dense", "gemm_simt", "gemm_rows_mma", "residual_stream", "parallel_stream", "ssm_scan",
+LAYERED_SOURCES = ("gemm_dense", "gemm_pair", "gemm_simt", "gemm_rows_mma", "residual_stream", "parallel_stream", "ssm_scan",
                    "decay_attention_mma", "gated_recurrence", "gated_linear_attention", "mlstm", "hyper_stream", "tanh_norm_stream",
                    "attention_sink",
                    "rotary_heads", "latent_attention", "moe_routing", "elementwise")

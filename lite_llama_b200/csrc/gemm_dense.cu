@@ -3,6 +3,7 @@
 // lite_llama/models/base.py:489) and the int8 x int8 GEMM of SmoothQuant-W8A8
 // (lite_llama/kernels/quantization/w8a8.py:75-130).  See gemm_tc.cuh for the tile design.
 #include "gemm_tc.cuh"
+#include "gemm_pair.cuh"
 #include <type_traits>
 
 namespace gemm {
@@ -268,6 +269,8 @@ extern "C" int b2l_linear(void* y, const void* x, const void* w, const void* bia
   B2L_REQUIRE(k % 8 == 0 && x_row_stride % 8 == 0 && w_row_stride % 8 == 0,
               "linear: K and the row strides must be multiples of 8 elements (TMA 16-byte rule); k=%lld", (long long)k);
   if (m == 0) return B2L_OK;
+  const PairGemm pg{y, y_row_stride, bias, nullptr, nullptr, m, n, k, x_row_stride, w_row_stride, x, w};
+  if (pair_gemm_wanted(0, pg)) return pair_gemm(0, dtype, pg, (cudaStream_t)stream);
   SplitPlan pl = make_plan(m, n, k, 64, 0, 1024, 4);
   DenseParams p;
   p.y = y; p.ldy = y_row_stride; p.bias = bias; p.a_scale = nullptr; p.b_scale = nullptr;
@@ -301,6 +304,9 @@ extern "C" int b2l_w8a8_gemm(void* y, const void* xq, const void* wq, const void
   B2L_REQUIRE(k % 16 == 0 && xq_row_stride % 16 == 0 && wq_row_stride % 16 == 0,
               "w8a8_gemm: K and the row strides must be multiples of 16 bytes; k=%lld", (long long)k);
   if (m == 0) return B2L_OK;
+  const PairGemm pg{y, y_row_stride, bias_f32, (const float*)a_scale, (const float*)b_scale, m, n, k, xq_row_stride,
+                    wq_row_stride, xq, wq};
+  if (pair_gemm_wanted(1, pg)) return pair_gemm(1, out_dtype, pg, (cudaStream_t)stream);
   SplitPlan pl = make_plan(m, n, k, 128, 0, 1024, 4);
   DenseParams p;
   p.y = y; p.ldy = y_row_stride; p.bias = bias_f32; p.a_scale = (const float*)a_scale; p.b_scale = (const float*)b_scale;

@@ -925,7 +925,7 @@ def random_gufotar_tensors(cfg: LayeredConfig, seed: int = 0) -> dict[str, torch
 
 
 register(Architecture("Gufotar", parse_gufotar_config, map_gufotar_weights, LayeredDecoder, ragged_steps=True,
-                      sources=("gemm_dense", "gemm_simt", "residual_stream", "ssm_scan", "attention_sink", "elementwise")))
+                      sources=("gemm_dense", "gemm_pair", "gemm_simt", "residual_stream", "ssm_scan", "attention_sink", "elementwise")))
 
 
 # ---------------------------------------------------------------------------------------------- Pesivik plumbing #
@@ -1060,7 +1060,7 @@ def random_pesivik_tensors(cfg: LayeredConfig, seed: int = 0) -> dict[str, torch
     return out
 
 
-_PESIVIK_SOURCES = ("gemm_dense", "gemm_simt", "gemm_rows_mma", "residual_stream", "attention_sink", "latent_attention",
+_PESIVIK_SOURCES = ("gemm_dense", "gemm_pair", "gemm_simt", "gemm_rows_mma", "residual_stream", "attention_sink", "latent_attention",
                     "moe_routing", "elementwise")
 register(Architecture("Pesivik", parse_pesivik_config, map_pesivik_weights, LayeredDecoder, ragged_steps=True,
                       sources=_PESIVIK_SOURCES))
@@ -1235,7 +1235,7 @@ def random_tisosun_tensors(cfg: LayeredConfig, seed: int = 0) -> dict[str, torch
     return out
 
 
-_TISOSUN_SOURCES = ("gemm_dense", "gemm_simt", "gemm_rows_mma", "residual_stream", "parallel_stream", "gated_recurrence",
+_TISOSUN_SOURCES = ("gemm_dense", "gemm_pair", "gemm_simt", "gemm_rows_mma", "residual_stream", "parallel_stream", "gated_recurrence",
                     "rotary_heads", "ssm_scan", "decay_attention_mma", "attention_sink", "elementwise")
 register(Architecture("Tisosun", parse_tisosun_config, map_tisosun_weights, LayeredDecoder, ragged_steps=True,
                       sources=_TISOSUN_SOURCES))
@@ -1414,7 +1414,7 @@ def random_gofezen_tensors(cfg: LayeredConfig, seed: int = 0) -> dict[str, torch
     return out
 
 
-_GOFEZEN_SOURCES = ("gemm_dense", "gemm_simt", "gemm_rows_mma", "residual_stream", "parallel_stream", "ssm_scan",
+_GOFEZEN_SOURCES = ("gemm_dense", "gemm_pair", "gemm_simt", "gemm_rows_mma", "residual_stream", "parallel_stream", "ssm_scan",
                     "gated_linear_attention", "rotary_heads", "attention_sink", "moe_routing", "elementwise")
 register(Architecture("Gofezen", parse_gofezen_config, map_gofezen_weights, LayeredDecoder, ragged_steps=True,
                       sources=_GOFEZEN_SOURCES))
@@ -1594,7 +1594,7 @@ def random_torutar_tensors(cfg: LayeredConfig, seed: int = 0) -> dict[str, torch
     return out
 
 
-_TORUTAR_SOURCES = ("gemm_dense", "gemm_simt", "gemm_rows_mma", "residual_stream", "hyper_stream", "ssm_scan", "mlstm",
+_TORUTAR_SOURCES = ("gemm_dense", "gemm_pair", "gemm_simt", "gemm_rows_mma", "residual_stream", "hyper_stream", "ssm_scan", "mlstm",
                     "gated_linear_attention", "rotary_heads", "latent_attention", "attention_sink", "moe_routing",
                     "elementwise")
 register(Architecture("Torutar", parse_torutar_config, map_torutar_weights, LayeredDecoder, ragged_steps=True,
@@ -1797,7 +1797,7 @@ def random_povilorn_tensors(cfg: LayeredConfig, seed: int = 0) -> dict[str, torc
     return out
 
 
-_POVILORN_SOURCES = ("gemm_dense", "gemm_simt", "gemm_rows_mma", "gated_linear_attention", "tanh_norm_stream", "rotary_heads",
+_POVILORN_SOURCES = ("gemm_dense", "gemm_pair", "gemm_simt", "gemm_rows_mma", "gated_linear_attention", "tanh_norm_stream", "rotary_heads",
                      "latent_attention", "attention_sink", "moe_routing", "elementwise")
 register(Architecture("Povilorn", parse_povilorn_config, map_povilorn_weights, LayeredDecoder, ragged_steps=True,
                       sources=_POVILORN_SOURCES))
