@@ -29,6 +29,8 @@
 // per-segment global scale loads, single-lane role loops and serial barrier polling each capped it at
 // 5-20 % of HBM peak before the current structure.
 #include "gemm_tc.cuh"
+#include "dequant.cuh"
+#include "gemm_quant_pair.cuh"
 #include <type_traits>
 #include <stdlib.h>
 
@@ -46,8 +48,6 @@ constexpr int kMaxRawStages = 8;
 // operand ring depth: 6 stages (three raw blocks of int4) when they fit next to the four accumulator buffers
 __host__ __device__ constexpr int op_stages_for(int bt) { return 4 * bt + 6 * 64 <= 512 ? 6 : 4; }
 constexpr int kTabPitch = 129;            // floats per scale-table column (128 weight rows + 1: conflict-free both ways)
-
-enum QuantKind { Q_INT4 = 0, Q_FP8 = 1, Q_INT8 = 2 };
 
 struct QuantParams {
   void* y; int64_t ldy;
@@ -195,69 +195,6 @@ template <int QK, int BT> __host__ __device__ constexpr int raw_stage_bytes() {
   return kABytes + raw_sub<QK>() * BT * kStageKBytes;
 }
 
-// ---- dequantisers: packed weights -> fp16 pairs in K order (one 32-bit TMEM column per pair) ----
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t mask, uint32_t orv) {
-  uint32_t r;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(mask), "r"(orv));  // (a & mask) | orv
-  return r;
-}
-// one int32 word (8 nibbles) -> 4 half2 {n0,n1} {n2,n3} {n4,n5} {n6,n7}
-__device__ __forceinline__ void dequant_int4_word(uint32_t w, __half2 add, uint32_t* out) {
-  // byte j holds nibbles (2j, 2j+1).  Replicate the byte into both halves, keep nibble 2j in the low
-  // half's mantissa and nibble 2j+1 (still shifted left by 4) in the high half's, OR in the fp16
-  // exponent of 1024: low = 1024 + n0, high = 1024 + 16*n1; one HFMA2 maps both back to exact integers.
-  const __half2 mul = __halves2half2(__float2half(1.0f), __float2half(0.0625f));
-  // add = {-(1024 + z), -(64 + z)}: an integer zero point z is subtracted in the same (exact) HFMA2
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint32_t rep = __byte_perm(w, w, 0x1111 * j);
-    const uint32_t h = lop3_and_or(rep, 0x00F0000Fu, 0x64006400u);
-    const __half2 v = __hfma2(*reinterpret_cast<const __half2*>(&h), mul, add);
-    out[j] = *reinterpret_cast<const uint32_t*>(&v);
-  }
-}
-__device__ __forceinline__ uint32_t cvt_e4m3x2_f16x2(uint16_t v) {
-  uint32_t r;
-  asm("cvt.rn.f16x2.e4m3x2 %0, %1;" : "=r"(r) : "h"(v));
-  return r;
-}
-// one 32-bit word (4 bytes) -> 2 half2
-__device__ __forceinline__ void dequant_w8_word(uint32_t w, bool fp8, uint32_t* out) {
-  if (fp8) {
-    out[0] = cvt_e4m3x2_f16x2((uint16_t)(w & 0xFFFFu));
-    out[1] = cvt_e4m3x2_f16x2((uint16_t)(w >> 16));
-  } else {
-    // b -> u = b + 128 (xor 0x80), fp16(0x6400 | u) = 1024 + u, minus 1152 = b   (all exact)
-    const __half2 off = __float2half2_rn(-1152.0f);
-    const uint32_t u = w ^ 0x80808080u;
-    const uint32_t h0 = __byte_perm(u, 0x64646464u, 0x4140u);   // [0x64, byte1, 0x64, byte0]
-    const uint32_t h1 = __byte_perm(u, 0x64646464u, 0x4342u);
-    const __half2 v0 = __hadd2(*reinterpret_cast<const __half2*>(&h0), off);
-    const __half2 v1 = __hadd2(*reinterpret_cast<const __half2*>(&h1), off);
-    out[0] = *reinterpret_cast<const uint32_t*>(&v0);
-    out[1] = *reinterpret_cast<const uint32_t*>(&v1);
-  }
-}
-
-// registers -> TMEM: lane of the warp writes its own TMEM lane, 32 consecutive 32-bit columns
-__device__ __forceinline__ void tmem_st_32x32b_x32(uint32_t taddr, const uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
-        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
-        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
-        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
-               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
-}
-__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // D[tmem] (+)= A[tmem] * B[smem desc]   (A: 128 lanes x 8 columns = 128 x 16 fp16, K-major)
 __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
                                             uint32_t accumulate) {
@@ -268,16 +205,9 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// the swiglu kernel's SiLU (csrc/elementwise.cu), so the fused epilogue rounds like the unfused path
-__device__ __forceinline__ float silu_q(float x) { return __fdividef(x, 1.0f + __expf(-x)); }
 __device__ __forceinline__ float lds_f32(const float* p) {
   float v;
   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(smem_u32(p)));
-  return v;
-}
-__device__ __forceinline__ uint4 lds_128(const void* p) {
-  uint4 v;
-  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_u32(p)));
   return v;
 }
 __device__ __forceinline__ int ld_acquire_smem(const int* p) {
@@ -1124,26 +1054,8 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 #pragma unroll
               for (int j = 0; j < 8; ++j) { vals[4 * j] = ws[j]; vals[4 * j + 1] = ws[j] ^ 1u; vals[4 * j + 2] = ws[j] ^ 2u; vals[4 * j + 3] = ws[j] ^ 3u; }
             } else if (LAYOUT == 1) {
-              // packed word: nibble positions hold K indices [0,2,4,6,1,3,5,7] -> each LOP3 yields a K-consecutive
-              // pair; low-nibble pairs are 1024 + n, high-nibble pairs 1024 + 16 n (5 ALU-pipe instructions per
-              // word instead of 8)
-              const __half2 one = __float2half2_rn(1.0f), sixteenth = __float2half2_rn(0.0625f);
 #pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const uint32_t w8 = ws[j] >> 8;
-                const uint32_t h0 = lop3_and_or(ws[j], 0x000F000Fu, 0x64006400u);
-                const uint32_t h1 = lop3_and_or(ws[j], 0x00F000F0u, 0x64006400u);
-                const uint32_t h2 = lop3_and_or(w8, 0x000F000Fu, 0x64006400u);
-                const uint32_t h3 = lop3_and_or(w8, 0x00F000F0u, 0x64006400u);
-                const __half2 v0 = __hfma2(*reinterpret_cast<const __half2*>(&h0), one, add_lo[sub]);
-                const __half2 v1 = __hfma2(*reinterpret_cast<const __half2*>(&h1), sixteenth, add_hi[sub]);
-                const __half2 v2 = __hfma2(*reinterpret_cast<const __half2*>(&h2), one, add_lo[sub]);
-                const __half2 v3 = __hfma2(*reinterpret_cast<const __half2*>(&h3), sixteenth, add_hi[sub]);
-                vals[4 * j] = *reinterpret_cast<const uint32_t*>(&v0);
-                vals[4 * j + 1] = *reinterpret_cast<const uint32_t*>(&v1);
-                vals[4 * j + 2] = *reinterpret_cast<const uint32_t*>(&v2);
-                vals[4 * j + 3] = *reinterpret_cast<const uint32_t*>(&v3);
-              }
+              for (int j = 0; j < 8; ++j) dequant_int4_packed(ws[j], add_lo[sub], add_hi[sub], vals + 4 * j);
             } else {
 #pragma unroll
               for (int j = 0; j < 8; ++j) dequant_int4_word(ws[j], add_lo[sub], vals + 4 * j);
@@ -1664,7 +1576,16 @@ extern "C" int b2l_w4a16_matmul_packed(void* y, const void* x, const void* qweig
               "w4a16_matmul_packed: row strides must be 16-byte multiples (K a multiple of 32)");
   B2L_REQUIRE((uintptr_t)scales_packed % 16 == 0 && (uintptr_t)zeros_packed % 16 == 0,
               "w4a16_matmul_packed: tables must be 16-byte aligned");
+  B2L_REQUIRE(epilogue == 0 || epilogue == 1, "w4a16_matmul_packed: epilogue %d (0 = none, 1 = swiglu over interleaved rows)", epilogue);
+  B2L_REQUIRE(epilogue == 0 || n % 2 == 0, "w4a16_matmul_packed: the swiglu epilogue needs an even number of rows");
   if (m == 0) return B2L_OK;
+  if (zeros_foldable && quant_pair_wanted(Q_INT4, m, n, k, group_size)) {
+    QuantPairParams q;
+    q.y = y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
+    q.scales = (const float*)scales_packed; q.s_stride_n = q.s_stride_k = 0; q.zeros = (const float*)zeros_packed; q.group_n = 1;
+    return quant_pair_gemm(Q_INT4, q, x, x_row_stride, qweight_packed, qw_row_stride * 4, m, n, k, group_size, epilogue,
+                           (cudaStream_t)stream);
+  }
   QuantParams p; SplitPlan pl; CUtensorMap tw, tx;
   int rc = quant_common(Q_INT4, p, pl, y, x, qweight_packed, m, n, k, x_row_stride, qw_row_stride, y_row_stride,
                         workspace, workspace_bytes, counters, num_counters, &tw, &tx, "w4a16_matmul_packed", group_size);
@@ -1673,8 +1594,6 @@ extern "C" int b2l_w4a16_matmul_packed(void* y, const void* x, const void* qweig
   p.scales = (const float*)scales_packed; p.zeros = (const float*)zeros_packed; p.s_stride_n = 0; p.s_stride_k = 0;
   p.group_n = 1; p.group_k = group_size;
   p.zeros_foldable = zeros_foldable ? 1 : 0;
-  B2L_REQUIRE(epilogue == 0 || epilogue == 1, "w4a16_matmul_packed: epilogue %d (0 = none, 1 = swiglu over interleaved rows)", epilogue);
-  B2L_REQUIRE(epilogue == 0 || n % 2 == 0, "w4a16_matmul_packed: the swiglu epilogue needs an even number of rows");
   p.swiglu = epilogue;
   return launch_q<Q_INT4>(tw, tx, p, pl, (cudaStream_t)stream, 1);
 }
@@ -1744,9 +1663,16 @@ extern "C" int b2l_w8a16_matmul(void* y, const void* x, const void* qweight, int
               (long long)group_k);
   B2L_REQUIRE(x_row_stride % 8 == 0 && qw_row_stride % 16 == 0, "w8a16_matmul: row strides must be 16-byte multiples");
   if (m == 0) return B2L_OK;
-  QuantParams p; SplitPlan pl; CUtensorMap tw, tx;
   const int qk = weight_is_fp8 ? Q_FP8 : Q_INT8;
   const int seg_len = seg_len_for(qk, k, group_k);
+  if (quant_pair_wanted(qk, m, n, k, seg_len)) {
+    QuantPairParams q;
+    q.y = y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
+    q.scales = (const float*)scales; q.s_stride_n = s_row_stride; q.s_stride_k = s_col_stride; q.zeros = nullptr;
+    q.group_n = (int)(group_n > n ? n : group_n);
+    return quant_pair_gemm(qk, q, x, x_row_stride, qweight, qw_row_stride, m, n, k, seg_len, 0, (cudaStream_t)stream);
+  }
+  QuantParams p; SplitPlan pl; CUtensorMap tw, tx;
   int rc = quant_common(qk, p, pl, y, x, qweight, m, n, k, x_row_stride, qw_row_stride, y_row_stride, workspace,
                         workspace_bytes, counters, num_counters, &tw, &tx, "w8a16_matmul", seg_len);
   if (rc != B2L_OK) return rc;

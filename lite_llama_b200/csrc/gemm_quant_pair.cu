@@ -1,0 +1,405 @@
+// Weight-only quantised GEMMs of prompt-sized batches on CTA pairs: W4A16 on the load-time repacked layout and W8A16
+// (entries: gemm_quant.cu; formats and reference lines there).
+//
+// Bound: the tensor pipe, if the conversion of the weights keeps out of its way.  The streaming kernel (gemm_quant.cu)
+// converts every weight tile once per 64 tokens; 128 weights x 128 k cost each scheduler ~190 issue slots to convert and
+// 64 tokens of MMAs last 256 cycles, so its hand-offs were the critical path (430 - 500 TF/s).  Here the tile is 256
+// weight rows x 128 tokens on a pair of SMs:
+//   * 128 rows x 128 k feed 512 cycles of MMAs per SM: conversion (two groups of four warps, each its own half of the
+//     operand stages) plus the drain of one accumulator segment take ~60 % of the issue slots;
+//   * cta_group::2: each SM stages 64 of the 128 tokens, 48 bytes per clock and SM from L2 for int4 weights;
+//   * the operand stays in tensor memory (4 stages of 128 k = 256 columns) beside two accumulator segments of 128 columns;
+//   * the grid is persistent, rings run on across tiles.
+// Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of
+// the accumulator per scale group, acc = fma(scale, segment, acc) in fp32 in ascending k.
+#include "gemm_tc.cuh"
+#include "gemm_quant_pair.cuh"
+#include "pair.cuh"
+#include "dequant.cuh"
+
+namespace gemm {
+
+constexpr int kQpThreads = 16 * 32;
+constexpr int kQpWStages = 6, kQpXStages = 6, kQpOpStages = 4;
+constexpr int kQpTokens = 128;                              // per pair tile; each CTA stages half
+constexpr int kQpStepK = 128;                               // k per operand stage
+constexpr int kQpXSub = kQpTokens / 2 * kStageKBytes;       // 64 tokens x 64 k
+constexpr int kQpXBytes = 2 * kQpXSub;
+constexpr int kQpSmem = 1024 + 1024 + kQpWStages * kABytes + kQpXStages * kQpXBytes;
+constexpr int kQpBand = 16;
+constexpr int kQpAccCols = 128, kQpOpCol0 = 2 * kQpAccCols;
+constexpr int kQpEpi0 = 8, kQpWProd = 12, kQpXProd = 13, kQpMma = 14;   // eight conversion, four epilogue warps
+
+struct __align__(8) QpControl {
+  uint64_t w_full[kQpWStages];      // own: a raw weight block has landed
+  uint64_t w_empty[kQpWStages];     // own: its words have been converted (4 warp arrivals per operand stage in it)
+  uint64_t x_full[kQpXStages];      // leader: both CTAs' token halves have landed
+  uint64_t x_empty[kQpXStages];     // both: the MMAs that read them have retired
+  uint64_t op_full[kQpOpStages];    // leader: both CTAs' converted rows are in tensor memory (8 warp arrivals)
+  uint64_t op_empty[kQpOpStages];   // both
+  uint64_t acc_full[2];             // both: a segment is complete
+  uint64_t acc_empty[2];            // leader: both CTAs' epilogue warps have read it (8 warp arrivals)
+  uint32_t tmem_base;
+};
+static_assert(sizeof(QpControl) <= 1024, "control block too large");
+
+__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+// two IEEE fused multiply-adds in one instruction
+__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm volatile("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// tokens of a tile rounded up to what cta_group::2 takes as N
+__device__ __forceinline__ int qp_tile_n(int rows_left) {
+  const int n = (rows_left + 31) & ~31;
+  return n < kQpTokens ? n : kQpTokens;
+}
+
+template <int QK, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kQpThreads, 1)
+gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                       const QuantPairParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  QpControl* ctl = reinterpret_cast<QpControl*>(smem);
+  uint8_t* w_ring = smem + 1024;
+  uint8_t* x_ring = w_ring + kQpWStages * kABytes;
+  constexpr int kStepsPerRaw = QK == Q_INT4 ? 2 : 1;       // a raw block is 128 rows x 128 bytes
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = pair_rank();
+  const int pairs = gridDim.x >> 1, pair = blockIdx.x >> 1;
+  const int tiles = p.m_tiles * p.n_tiles;
+  const int steps = p.steps;                               // operand stages per tile
+  if (threadIdx.x == kQpWProd * 32) {
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+    for (int s = 0; s < kQpWStages; ++s) {
+      mbar_init(&ctl->w_full[s], 1);
+      mbar_init(&ctl->w_empty[s], 4 * kStepsPerRaw);
+    }
+    for (int s = 0; s < kQpXStages; ++s) {
+      mbar_init(&ctl->x_full[s], 1);
+      mbar_init(&ctl->x_empty[s], 1);
+    }
+    for (int s = 0; s < kQpOpStages; ++s) {
+      mbar_init(&ctl->op_full[s], 8);
+      mbar_init(&ctl->op_empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&ctl->acc_full[s], 1);
+      mbar_init(&ctl->acc_empty[s], 8);
+    }
+    mbar_fence_init();
+  }
+  if (warp == kQpMma) {
+    tmem_alloc_pair(&ctl->tmem_base, 512);
+    tmem_relinquish_pair();
+    pdl_launch_dependents();        // after the allocation (gemm_dense.cu)
+  }
+  tc_fence_before();
+  pair_sync();
+  tc_fence_after();
+  const uint32_t tmem_base = ctl->tmem_base;
+
+  // registers per lane: four warpgroups x 128 at launch = 2 x 104 + 240 + 64
+  if (warp >= kQpWProd) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    if (warp == kQpWProd) {
+      // ===================== raw weight blocks of this CTA's 128 rows =====================
+      PipeState ws(kQpWStages);
+      const int raws = (steps + kStepsPerRaw - 1) / kStepsPerRaw;
+      for (int t = pair; t < tiles; t += pairs) {
+        const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+        const int row = pt.n * 2 * kBlockW + (int)rank * kBlockW;
+        for (int rb = 0; rb < raws; ++rb) {
+          mbar_wait(&ctl->w_empty[ws.stage], ws.phase ^ 1);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(&ctl->w_full[ws.stage], kABytes);
+            tma_load_2d_hint(w_ring + (size_t)ws.stage * kABytes, &tmap_w, rb * (QK == Q_INT4 ? 32 : 128), row,
+                             &ctl->w_full[ws.stage], kEvictNormal);
+          }
+          __syncwarp();
+          ws.advance();
+        }
+      }
+    } else if (warp == kQpXProd) {
+      // ===================== activations: this CTA's half of the tile's tokens =====================
+      pdl_wait_prior();
+      PipeState xs(kQpXStages);
+      for (int t = pair; t < tiles; t += pairs) {
+        const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+        const int m0 = pt.m * kQpTokens;
+        const int row = m0 + (int)rank * (qp_tile_n(p.M - m0) / 2);
+        for (int s = 0; s < steps; ++s) {
+          mbar_wait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
+          if (elect_one()) {
+            if (rank == 0) mbar_arrive_expect_tx(&ctl->x_full[xs.stage], 2 * kQpXBytes);
+            uint8_t* dst = x_ring + (size_t)xs.stage * kQpXBytes;
+            const uint32_t bar = leader_addr(&ctl->x_full[xs.stage]);
+            tma_load_2d_pair(dst, &tmap_x, s * kQpStepK, row, bar, kEvictNormal);
+            tma_load_2d_pair(dst + kQpXSub, &tmap_x, s * kQpStepK + 64, row, bar, kEvictNormal);
+          }
+          __syncwarp();
+          xs.advance();
+        }
+      }
+      // every stage handed back: no commit is still on its way to this CTA's barriers when it leaves
+      for (int s = 0; s < kQpXStages; ++s) {
+        mbar_wait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
+        xs.advance();
+      }
+    } else if (warp == kQpMma && rank == 0) {
+      // ===================== MMA issuer (leader) =====================
+      const uint64_t x_desc0 = umma_desc_sw128_kmajor(smem_u32(x_ring));
+      PipeState xs(kQpXStages), os(kQpOpStages);
+      int seg = 0;
+      for (int t = pair; t < tiles; t += pairs) {
+        const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+        const uint32_t idesc = umma_idesc(1u, 0u, 0u, 0u, 0u, 2 * kBlockW, (uint32_t)qp_tile_n(p.M - pt.m * kQpTokens));
+        int in_seg = 0;
+        for (int s = 0; s < steps; ++s) {
+          const int buf = seg & 1;
+          if (in_seg == 0) mbar_wait(&ctl->acc_empty[buf], ((seg >> 1) & 1) ^ 1);
+          mbar_wait(&ctl->x_full[xs.stage], xs.phase);
+          mbar_wait(&ctl->op_full[os.stage], os.phase);
+          tc_fence_after();
+          const bool last = in_seg + 1 == p.seg_steps || s + 1 == steps;
+          if (elect_one()) {
+            const uint32_t a = tmem_base + kQpOpCol0 + os.stage * 64;
+            const uint64_t b = x_desc0 + (uint64_t)((xs.stage * kQpXBytes) >> 4);
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              umma_pair_ts(tmem_base + buf * kQpAccCols, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)),
+                           idesc, (in_seg | k) != 0 ? 1u : 0u);
+            tc_commit_pair(&ctl->op_empty[os.stage]);
+            tc_commit_pair(&ctl->x_empty[xs.stage]);
+            if (last) tc_commit_pair(&ctl->acc_full[buf]);
+          }
+          __syncwarp();
+          if (last) { ++seg; in_seg = 0; } else { ++in_seg; }
+          xs.advance();
+          os.advance();
+        }
+      }
+    }
+  } else if (warp >= kQpEpi0) {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
+    // ===================== epilogue: one thread per weight row =====================
+    const int quad = warp & 3;
+    const int row = quad * 32 + lane;
+    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const uint32_t empty0 = leader_addr(&ctl->acc_empty[0]), empty1 = leader_addr(&ctl->acc_empty[1]);
+    const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
+    pdl_wait_prior();               // y may still be read upstream
+    int seg = 0;
+    for (int t = pair; t < tiles; t += pairs) {
+      const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+      const int n_tile = pt.n * 2 + (int)rank;
+      const int n = n_tile * kBlockW + row;
+      const bool n_ok = n < p.N;
+      // scale of group g: packed int4 tables are [tile][group][128], 8-bit tables strided by scale block
+      const float* sp = p.scales;
+      int64_t s_step;
+      if (QK == Q_INT4) {
+        sp += ((int64_t)(n_ok ? n_tile : 0) * nseg) * kBlockW + row;
+        s_step = kBlockW;
+      } else {
+        sp += (int64_t)((n_ok ? n : 0) / p.group_n) * p.s_stride_n;
+        s_step = p.s_stride_k;
+      }
+      uint64_t acc[kQpTokens / 2];
+#pragma unroll
+      for (int j = 0; j < kQpTokens / 2; ++j) acc[j] = 0ull;
+      float sc = __ldg(sp);
+      for (int g = 0; g < nseg; ++g, ++seg) {
+        const int buf = seg & 1;
+        const uint64_t s2 = pack_f32x2(sc, sc);
+        if (g + 1 < nseg) sc = __ldg(sp + (int64_t)(g + 1) * s_step);
+        mbar_wait(&ctl->acc_full[buf], (seg >> 1) & 1);
+        tc_fence_after();
+#pragma unroll
+        for (int c = 0; c < kQpTokens; c += 64) {
+          uint32_t v[64];
+          tmem_ld_32x32b_x32(taddr + buf * kQpAccCols + c, *reinterpret_cast<uint32_t(*)[32]>(v));
+          tmem_ld_32x32b_x32(taddr + buf * kQpAccCols + c + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
+          tc_wait_ld();
+          if (c + 64 == kQpTokens) {          // in registers: the segment's buffer may be refilled
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(buf ? empty1 : empty0);
+          }
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const uint64_t pv = pack_f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+            acc[c / 2 + j] = fma_f32x2(s2, pv, acc[c / 2 + j]);
+          }
+        }
+      }
+      // ---- the tile's results: a warp writes 32 consecutive outputs of one token at a time ----
+      float bv = 0.f;
+      if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
+                                             : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
+      const int m0 = pt.m * kQpTokens;
+      const int rows = p.M - m0;
+      __half* y = reinterpret_cast<__half*>(p.y);
+      if (EPI == 0) {
+        __half* yp = y + (int64_t)m0 * p.ldy + n;
+        if (n_ok) {
+#pragma unroll
+          for (int j = 0; j < kQpTokens / 2; ++j) {
+            float a, b;
+            unpack_f32x2(acc[j], a, b);
+            if (2 * j < rows) yp[0] = __float2half_rn(a + bv);
+            if (2 * j + 1 < rows) yp[p.ldy] = __float2half_rn(b + bv);
+            yp += 2 * p.ldy;
+          }
+        }
+      } else {
+        // SiLU(gate) * up over (gate_i, up_i) row pairs, both rounded to fp16 first (gemm_quant.cu).  Of two tokens the
+        // even lane forms the first result and the odd lane the second: one exchange for both.
+        const bool odd = lane & 1;
+        __half* yp = y + (int64_t)(m0 + (odd ? 1 : 0)) * p.ldy + (n >> 1);
+#pragma unroll
+        for (int j = 0; j < kQpTokens / 2; ++j) {
+          float a, b;
+          unpack_f32x2(acc[j], a, b);
+          a = __half2float(__float2half_rn(a + bv));
+          b = __half2float(__float2half_rn(b + bv));
+          const float other = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
+          const float gate = odd ? other : a, up = odd ? b : other;
+          if (n_ok && 2 * j + (odd ? 1 : 0) < rows) *yp = __float2half_rn(silu_q(gate) * up);
+          yp += 2 * p.ldy;
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    // ===================== conversion: one thread per weight row, the two groups take alternate operand stages ==========
+    // Stage i of the CTA's running count belongs to group i & 1, so every op_empty barrier is waited on by one group
+    // that has seen all of its phases.
+    const int group = warp >> 2, quad = warp & 3;
+    const int row = quad * 32 + lane, rx = row & 7;
+    const uint32_t dst0 = tmem_base + ((uint32_t)(quad * 32) << 16) + kQpOpCol0;
+    const uint32_t full0 = leader_addr(&ctl->op_full[group]), full1 = leader_addr(&ctl->op_full[group + 2]);
+    int i0 = 0;                                             // running stage count at the tile's first step
+    int raw0 = 0;                                           // running raw-block count
+    int use = 0;                                            // stages this group has filled
+    const int raws = (steps + kStepsPerRaw - 1) / kStepsPerRaw;
+    for (int t = pair; t < tiles; t += pairs) {
+      const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+      const int n_tile = pt.n * 2 + (int)rank;
+      const float* zp = nullptr;
+      int k = (group - i0) & 1;                             // first step of this tile that is this group's
+      float z = 0.f;
+      if (QK == Q_INT4) {
+        const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
+        zp = p.zeros + ((int64_t)(n_tile * kBlockW < p.N ? n_tile : 0) * nseg) * kBlockW + row;
+        if (k < steps) z = __ldg(zp + (int64_t)(k / p.seg_steps) * kBlockW);
+      }
+      for (; k < steps; k += 2) {
+        __half2 add_lo, add_hi;
+        if (QK == Q_INT4) {
+          add_lo = __float2half2_rn(-1024.f - z);
+          add_hi = __float2half2_rn(-64.f - z);
+          if (k + 2 < steps) z = __ldg(zp + (int64_t)((k + 2) / p.seg_steps) * kBlockW);
+        }
+        const int raw = raw0 + (QK == Q_INT4 ? k >> 1 : k);
+        const int rs = raw % kQpWStages;
+        mbar_wait(&ctl->w_full[rs], (raw / kQpWStages) & 1);
+        const uint8_t* src = w_ring + (size_t)rs * kABytes + row * 128;
+        constexpr int kChunks = QK == Q_INT4 ? 4 : 8;       // 16-byte chunks of the row per stage
+        const int c0 = QK == Q_INT4 ? (k & 1) * 4 : 0;
+        uint4 w[kChunks];
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) w[c] = lds_128(src + (((c0 + c) ^ rx) << 4));
+        const int stage = group + 2 * (use & 1);
+        mbar_wait(&ctl->op_empty[stage], ((use >> 1) & 1) ^ 1);
+        tc_fence_after();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          uint32_t vals[32];
+#pragma unroll
+          for (int c = 0; c < kChunks / 2; ++c) {
+            const uint4 q = w[h * (kChunks / 2) + c];
+            const uint32_t ws[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (QK == Q_INT4) dequant_int4_packed(ws[j], add_lo, add_hi, vals + (QK == Q_INT4 ? 16 * c + 4 * j : 0));
+              else dequant_w8_word(ws[j], QK == Q_FP8, vals + (QK == Q_INT4 ? 0 : 8 * c + 2 * j));
+            }
+          }
+          tmem_st_32x32b_x32(dst0 + stage * 64 + h * 32, vals);
+        }
+        // the raw words have all been converted: the block may be refilled (an odd last step speaks for both halves)
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&ctl->w_empty[rs]);
+          if (QK == Q_INT4 && k + 1 == steps && (k & 1) == 0) mbar_arrive(&ctl->w_empty[rs]);
+        }
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(use & 1 ? full1 : full0);
+        ++use;
+      }
+      i0 += steps;
+      raw0 += raws;
+    }
+  }
+
+  tc_fence_before();
+  pair_sync();                      // the peer's MMAs, commits and arrivals are over
+  if (warp == kQpMma) tmem_dealloc_pair(tmem_base, 512);
+}
+
+template <int QK, int EPI>
+static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
+  auto kern = gemm_quant_pair_kernel<QK, EPI>;
+  static int configured[64] = {0};
+  B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, kQpSmem, configured));
+  b2l_launch(kern, dim3((unsigned)grid), dim3(kQpThreads), (size_t)kQpSmem, st, tw, tx, p);
+  B2L_LAUNCH_CHECK();
+  return B2L_OK;
+}
+
+bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k) {
+  // segments of whole operand stages, or one segment over all of K
+  if (group_k % kQpStepK != 0 && group_k < K) return false;
+  if (qk == Q_INT4 && K % kQpStepK != 0) return false;      // the packed tables are read per 128 k
+  const int64_t m_tiles = cdiv64(M, kQpTokens), n_tiles = cdiv64(N, 2 * kBlockW);
+  return M > 64 && m_tiles * n_tiles >= 40;
+}
+
+int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, const void* w, int64_t w_stride_bytes,
+                    int64_t M, int64_t N, int64_t K, int64_t group_k, int swiglu, cudaStream_t st) {
+  const int pairs = b2l_num_sms() / 2;
+  p.M = (int)M; p.N = (int)N;
+  p.steps = (int)cdiv64(K, kQpStepK);
+  p.seg_steps = group_k >= K ? p.steps : (int)(group_k / kQpStepK);
+  p.m_tiles = (int)cdiv64(M, kQpTokens);
+  p.n_tiles = (int)cdiv64(N, 2 * kBlockW);
+  const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
+  const int grid = 2 * (int)(tiles < pairs ? tiles : pairs);
+  CUtensorMap tw, tx;
+  int rc;
+  if (qk == Q_INT4) rc = b2l_make_tmap_2d(&tw, w, TMA_I32, (uint64_t)N, (uint64_t)(K / 8), (uint64_t)w_stride_bytes, kBlockW, 32, true);
+  else rc = b2l_make_tmap_2d(&tw, w, TMA_U8, (uint64_t)N, (uint64_t)K, (uint64_t)w_stride_bytes, kBlockW, 128, true);
+  if (rc != B2L_OK) return rc;
+  rc = b2l_make_tmap_2d(&tx, x, TMA_F16, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, kQpTokens / 2, 64, true);
+  if (rc != B2L_OK) return rc;
+  if (qk == Q_INT4) return swiglu ? launch_qp<Q_INT4, 1>(tw, tx, p, grid, st) : launch_qp<Q_INT4, 0>(tw, tx, p, grid, st);
+  if (qk == Q_FP8) return launch_qp<Q_FP8, 0>(tw, tx, p, grid, st);
+  return launch_qp<Q_INT8, 0>(tw, tx, p, grid, st);
+}
+
+}  // namespace gemm
