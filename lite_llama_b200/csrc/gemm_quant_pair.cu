@@ -372,12 +372,21 @@ static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPa
   return B2L_OK;
 }
 
+// Where the pair kernel is the faster one (both kernels measured over 72 - 4096 tokens and seven projection shapes).  A
+// wave of pair tiles takes about 1.35 times a wave of the streaming kernel's 128 x 64 tiles (6144 x 4096, one wave each:
+// 23.5 against 17.5 us) and covers four of them per pair, so the waves decide: int4, us, streaming -> pair:
+//   28672 x 4096, 72 tokens 72 -> 46, 4096 tokens 1854 -> 982; 4096 x 4096, 320 tokens 33 -> 23, but 192 tokens 17 -> 22.
+// One segment over all of k (a scale per output row) leaves the streaming kernel a single MMA warp; there the pair
+// kernel wins as soon as it has 16 tiles (int8, 896 x 4864, 512 tokens 27 -> 19; 320 tokens, 12 tiles: level).
 bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k) {
   // segments of whole operand stages, or one segment over all of K
   if (group_k % kQpStepK != 0 && group_k < K) return false;
   if (qk == Q_INT4 && K % kQpStepK != 0) return false;      // the packed tables are read per 128 k
-  const int64_t m_tiles = cdiv64(M, kQpTokens), n_tiles = cdiv64(N, 2 * kBlockW);
-  return M > 64 && m_tiles * n_tiles >= 40;
+  if (M <= 64) return false;
+  const int64_t sms = b2l_num_sms();
+  const int64_t tiles = cdiv64(M, kQpTokens) * cdiv64(N, 2 * kBlockW);
+  if (group_k >= K) return tiles >= 16;
+  return 4 * cdiv64(cdiv64(M, 64) * cdiv64(N, kBlockW), sms) >= 5 * cdiv64(tiles, sms / 2);
 }
 
 int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, const void* w, int64_t w_stride_bytes,

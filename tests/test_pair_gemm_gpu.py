@@ -56,3 +56,59 @@ def test_linear_forms_the_pair_kernel_does_not_take():
     assert rel(K().linear(x, w), x.double() @ w.double().T) < REL[torch.bfloat16]
     xs, ws = x[:, 64:320], w[:10240, 128:384]
     assert rel(K().linear(xs, ws), xs.double() @ ws.double().T) < REL[torch.bfloat16]
+
+
+# ---- quantised weights (csrc/gemm_quant_pair.cu): 256-row x 128-token tiles, 128 k per operand stage ----
+# m: one token over / under a tile, 64-token edge of the dispatch; n: rows past the last tile; k: an odd number of stages
+# (half a raw block is left over), one and several stages per scale group
+QUANT_EDGES = [(65, 10240, 128), (127, 10140, 384), (129, 5128, 640), (500, 2600, 256), (1000, 1300, 896)]
+
+
+def int4_case(n, k, group, m):
+    q = torch.randint(-(2**31), 2**31 - 1, (n, k // 8), device="cuda", dtype=torch.int64).to(torch.int32)
+    s = torch.rand(n, k // group, device="cuda") * 4e-3 + 1e-3
+    z = torch.randint(0, 16, (n, k // group), device="cuda").float()
+    codes = torch.stack([(q >> (4 * j)) & 15 for j in range(8)], -1).view(n, k // group, group).double()
+    w = ((codes - z.double()[..., None]) * s.double()[..., None]).view(n, k)
+    return q, s, z, w, torch.randn(m, k, device="cuda", dtype=torch.float16)
+
+
+@pytest.mark.parametrize("m,n,k", QUANT_EDGES)
+@pytest.mark.parametrize("group", [128, 256])
+@pytest.mark.parametrize("bias", [None, torch.float16, torch.float32])
+def test_int4_pair_tiles(m, n, k, group, bias):
+    if k % group:
+        pytest.skip("groups divide k")
+    q, s, z, w, x = int4_case(n, k, group, m)
+    b = None if bias is None else torch.randn(n, device="cuda", dtype=bias)
+    got = K().w4a16_matmul_packed(x, K().w4a16_pack(q, s, z, group_size=group), bias=b)
+    assert rel(got, x.double() @ w.T + (0.0 if b is None else b.double())) < REL[torch.float16]
+
+
+@pytest.mark.parametrize("m,n,k", QUANT_EDGES)
+def test_int4_pair_swiglu_is_gemm_then_swiglu(m, n, k):
+    from lite_llama_b200.kernels.quantization import interleave_gate_up
+
+    q, s, z, _, x = int4_case(n, k, 128, m)
+    wide = K().w4a16_matmul_packed(x, K().w4a16_pack(q, s, z, group_size=128))
+    want = K().swiglu_forward(wide[:, : n // 2], wide[:, n // 2 :])
+    packed = K().w4a16_pack(interleave_gate_up(q), interleave_gate_up(s), interleave_gate_up(z), group_size=128)
+    assert torch.equal(K().w4a16_matmul_packed(x, packed, swiglu=True), want)
+
+
+@pytest.mark.parametrize("m,n,k", QUANT_EDGES + [(300, 5000, 400)])       # 400: the last stage is partly past k
+@pytest.mark.parametrize("fmt", ["fp8_block", "fp8_channel", "int8_channel", "int8_group_n"])
+def test_w8_pair_tiles(m, n, k, fmt):
+    x = torch.randn(m, k, device="cuda", dtype=torch.float16)
+    if fmt.startswith("fp8"):
+        q = (torch.randn(n, k, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+        w = q.view(torch.float8_e4m3fn).double()
+    else:
+        q = torch.randint(-127, 128, (n, k), device="cuda", dtype=torch.int8)
+        w = q.double()
+    gn, gk = {"fp8_block": (128, 128), "int8_group_n": (48, k)}.get(fmt, (1, k))
+    s = torch.rand((n + gn - 1) // gn, (k + gk - 1) // gk, device="cuda") * 1e-3
+    w = w * s.double().repeat_interleave(gn, 0)[:n].repeat_interleave(gk, 1)[:, :k]
+    b = torch.randn(n, device="cuda")
+    got = K().w8a16_matmul(x, q, s, group_n=gn, group_k=gk, bias=b)
+    assert rel(got, x.double() @ w.T + b.double()) < REL[torch.float16]
