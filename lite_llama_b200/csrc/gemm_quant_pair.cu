@@ -9,7 +9,12 @@
 //     operand stages) plus the drain of one accumulator segment take ~60 % of the issue slots;
 //   * cta_group::2: each SM stages 64 of the 128 tokens, 48 bytes per clock and SM from L2 for int4 weights;
 //   * the operand stays in tensor memory (4 stages of 128 k = 256 columns) beside two accumulator segments of 128 columns;
+//   * a segment's buffer is handed back as soon as its 128 columns are in the registers of eight epilogue warps, before the
+//     multiply-adds: with four warps that read it in two turns the MMAs waited for the drain (977 us against 900);
 //   * the grid is persistent, rings run on across tiles.
+// Measured, 28672 x 4096 at 4096 tokens (streaming kernel -> this one): int4 1853 -> 900 us (1.07 PFLOP/s), fp8 in 128 x 128
+// blocks 1748 -> 867 us, int8 per channel 3124 -> 754 us (no drain before the end of k: 1.28 PFLOP/s).  A third accumulator
+// at the cost of two operand stages: int4 878, fp8 901 us.
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of
 // the accumulator per scale group, acc = fma(scale, segment, acc) in fp32 in ascending k.
 #include "gemm_tc.cuh"
@@ -19,7 +24,7 @@
 
 namespace gemm {
 
-constexpr int kQpThreads = 16 * 32;
+constexpr int kQpThreads = 20 * 32;
 constexpr int kQpWStages = 6, kQpXStages = 6, kQpOpStages = 4;
 constexpr int kQpTokens = 128;                              // per pair tile; each CTA stages half
 constexpr int kQpStepK = 128;                               // k per operand stage
@@ -27,8 +32,9 @@ constexpr int kQpXSub = kQpTokens / 2 * kStageKBytes;       // 64 tokens x 64 k
 constexpr int kQpXBytes = 2 * kQpXSub;
 constexpr int kQpSmem = 1024 + 1024 + kQpWStages * kABytes + kQpXStages * kQpXBytes;
 constexpr int kQpBand = 16;
+constexpr int kQpHalf = kQpTokens / 2;                      // tokens per epilogue warp
 constexpr int kQpAccCols = 128, kQpOpCol0 = 2 * kQpAccCols;
-constexpr int kQpEpi0 = 8, kQpWProd = 12, kQpXProd = 13, kQpMma = 14;   // eight conversion, four epilogue warps
+constexpr int kQpEpi0 = 8, kQpWProd = 16, kQpXProd = 17, kQpMma = 18;   // eight conversion, eight epilogue warps
 
 struct __align__(8) QpControl {
   uint64_t w_full[kQpWStages];      // own: a raw weight block has landed
@@ -38,7 +44,7 @@ struct __align__(8) QpControl {
   uint64_t op_full[kQpOpStages];    // leader: both CTAs' converted rows are in tensor memory (8 warp arrivals)
   uint64_t op_empty[kQpOpStages];   // both
   uint64_t acc_full[2];             // both: a segment is complete
-  uint64_t acc_empty[2];            // leader: both CTAs' epilogue warps have read it (8 warp arrivals)
+  uint64_t acc_empty[2];            // leader: both CTAs' epilogue warps have read it (16 warp arrivals)
   uint32_t tmem_base;
 };
 static_assert(sizeof(QpControl) <= 1024, "control block too large");
@@ -97,7 +103,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
     for (int s = 0; s < 2; ++s) {
       mbar_init(&ctl->acc_full[s], 1);
-      mbar_init(&ctl->acc_empty[s], 8);
+      mbar_init(&ctl->acc_empty[s], 16);
     }
     mbar_fence_init();
   }
@@ -111,9 +117,9 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
 
-  // registers per lane: four warpgroups x 128 at launch = 2 x 104 + 240 + 64
+  // registers per lane: five warpgroups x 96 at launch = 2 x 80 + 2 x 136 + 48
   if (warp >= kQpWProd) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
     if (warp == kQpWProd) {
       // ===================== raw weight blocks of this CTA's 128 rows =====================
       PipeState ws(kQpWStages);
@@ -193,11 +199,11 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       }
     }
   } else if (warp >= kQpEpi0) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 240;");
-    // ===================== epilogue: one thread per weight row =====================
-    const int quad = warp & 3;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
+    // ===================== epilogue: one thread per weight row and token half =====================
+    const int quad = warp & 3, half = (warp - kQpEpi0) >> 2;
     const int row = quad * 32 + lane;
-    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + half * kQpHalf;
     const uint32_t empty0 = leader_addr(&ctl->acc_empty[0]), empty1 = leader_addr(&ctl->acc_empty[1]);
     const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
     pdl_wait_prior();               // y may still be read upstream
@@ -217,9 +223,9 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         sp += (int64_t)((n_ok ? n : 0) / p.group_n) * p.s_stride_n;
         s_step = p.s_stride_k;
       }
-      uint64_t acc[kQpTokens / 2];
+      uint64_t acc[kQpHalf / 2];
 #pragma unroll
-      for (int j = 0; j < kQpTokens / 2; ++j) acc[j] = 0ull;
+      for (int j = 0; j < kQpHalf / 2; ++j) acc[j] = 0ull;
       float sc = __ldg(sp);
       for (int g = 0; g < nseg; ++g, ++seg) {
         const int buf = seg & 1;
@@ -227,36 +233,31 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         if (g + 1 < nseg) sc = __ldg(sp + (int64_t)(g + 1) * s_step);
         mbar_wait(&ctl->acc_full[buf], (seg >> 1) & 1);
         tc_fence_after();
+        uint32_t v[kQpHalf];
+        tmem_ld_32x32b_x32(taddr + buf * kQpAccCols, *reinterpret_cast<uint32_t(*)[32]>(v));
+        tmem_ld_32x32b_x32(taddr + buf * kQpAccCols + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(buf ? empty1 : empty0);     // in registers: the segment's buffer may be refilled
 #pragma unroll
-        for (int c = 0; c < kQpTokens; c += 64) {
-          uint32_t v[64];
-          tmem_ld_32x32b_x32(taddr + buf * kQpAccCols + c, *reinterpret_cast<uint32_t(*)[32]>(v));
-          tmem_ld_32x32b_x32(taddr + buf * kQpAccCols + c + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
-          tc_wait_ld();
-          if (c + 64 == kQpTokens) {          // in registers: the segment's buffer may be refilled
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(buf ? empty1 : empty0);
-          }
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const uint64_t pv = pack_f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-            acc[c / 2 + j] = fma_f32x2(s2, pv, acc[c / 2 + j]);
-          }
+        for (int j = 0; j < kQpHalf / 2; ++j) {
+          const uint64_t pv = pack_f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
+          acc[j] = fma_f32x2(s2, pv, acc[j]);
         }
       }
       // ---- the tile's results: a warp writes 32 consecutive outputs of one token at a time ----
       float bv = 0.f;
       if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
-      const int m0 = pt.m * kQpTokens;
+      const int m0 = pt.m * kQpTokens + half * kQpHalf;
       const int rows = p.M - m0;
       __half* y = reinterpret_cast<__half*>(p.y);
       if (EPI == 0) {
         __half* yp = y + (int64_t)m0 * p.ldy + n;
         if (n_ok) {
 #pragma unroll
-          for (int j = 0; j < kQpTokens / 2; ++j) {
+          for (int j = 0; j < kQpHalf / 2; ++j) {
             float a, b;
             unpack_f32x2(acc[j], a, b);
             if (2 * j < rows) yp[0] = __float2half_rn(a + bv);
@@ -270,7 +271,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const bool odd = lane & 1;
         __half* yp = y + (int64_t)(m0 + (odd ? 1 : 0)) * p.ldy + (n >> 1);
 #pragma unroll
-        for (int j = 0; j < kQpTokens / 2; ++j) {
+        for (int j = 0; j < kQpHalf / 2; ++j) {
           float a, b;
           unpack_f32x2(acc[j], a, b);
           a = __half2float(__float2half_rn(a + bv));
@@ -283,7 +284,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       }
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     // ===================== conversion: one thread per weight row, the two groups take alternate operand stages ==========
     // Stage i of the CTA's running count belongs to group i & 1, so every op_empty barrier is waited on by one group
     // that has seen all of its phases.
@@ -317,21 +318,20 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const int rs = raw % kQpWStages;
         mbar_wait(&ctl->w_full[rs], (raw / kQpWStages) & 1);
         const uint8_t* src = w_ring + (size_t)rs * kABytes + row * 128;
-        constexpr int kChunks = QK == Q_INT4 ? 4 : 8;       // 16-byte chunks of the row per stage
-        const int c0 = QK == Q_INT4 ? (k & 1) * 4 : 0;
-        uint4 w[kChunks];
-#pragma unroll
-        for (int c = 0; c < kChunks; ++c) w[c] = lds_128(src + (((c0 + c) ^ rx) << 4));
         const int stage = group + 2 * (use & 1);
         mbar_wait(&ctl->op_empty[stage], ((use >> 1) & 1) ^ 1);
         tc_fence_after();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
+          constexpr int kChunks = QK == Q_INT4 ? 2 : 4;     // 16-byte chunks of the row per 64 k
+          const int c0 = (QK == Q_INT4 ? (k & 1) * 4 : 0) + h * kChunks;
+          uint4 w[kChunks];
+#pragma unroll
+          for (int c = 0; c < kChunks; ++c) w[c] = lds_128(src + (((c0 + c) ^ rx) << 4));
           uint32_t vals[32];
 #pragma unroll
-          for (int c = 0; c < kChunks / 2; ++c) {
-            const uint4 q = w[h * (kChunks / 2) + c];
-            const uint32_t ws[4] = {q.x, q.y, q.z, q.w};
+          for (int c = 0; c < kChunks; ++c) {
+            const uint32_t ws[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               if (QK == Q_INT4) dequant_int4_packed(ws[j], add_lo, add_hi, vals + (QK == Q_INT4 ? 16 * c + 4 * j : 0));
