@@ -64,13 +64,36 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
   return r;
 }
 
+// What a tile is: `mode` plain = one weight matrix; grouped = experts, one entry of the tile table per 128 rows of an
+// expert's run of the sorted activations (moe_sort, moe_routing.cu), the entries' output tiles next to one another so that
+// the pairs in flight share the activations and an expert's second entry finds the weights in L2.
+enum { QP_PLAIN = 0, QP_GATE_UP = 1, QP_DOWN = 2 };
+struct QpTile { int n, m0, rows, expert; };
+template <int MODE>
+__device__ __forceinline__ int qp_tiles(const QuantPairParams& p) {
+  return MODE == QP_PLAIN ? p.m_tiles * p.n_tiles : __ldg(p.table) * p.n_tiles;
+}
+template <int MODE>
+__device__ __forceinline__ QpTile qp_tile(const QuantPairParams& p, int t) {
+  QpTile o;
+  if (MODE == QP_PLAIN) {
+    const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+    o.n = pt.n; o.m0 = pt.m * kQpTokens; o.rows = p.M - o.m0; o.expert = 0;
+  } else {
+    const int e = t / p.n_tiles;
+    o.n = t - e * p.n_tiles;
+    o.expert = __ldg(p.table + 1 + 3 * e); o.m0 = __ldg(p.table + 2 + 3 * e); o.rows = __ldg(p.table + 3 + 3 * e);
+  }
+  return o;
+}
+
 // tokens of a tile rounded up to what cta_group::2 takes as N
 __device__ __forceinline__ int qp_tile_n(int rows_left) {
   const int n = (rows_left + 31) & ~31;
   return n < kQpTokens ? n : kQpTokens;
 }
 
-template <int QK, int EPI>
+template <int QK, int EPI, int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kQpThreads, 1)
 gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                        const QuantPairParams p) {
@@ -84,7 +107,8 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = pair_rank();
   const int pairs = gridDim.x >> 1, pair = blockIdx.x >> 1;
-  const int tiles = p.m_tiles * p.n_tiles;
+  if (MODE != QP_PLAIN) pdl_wait_prior();                  // the tile table is an earlier kernel's output
+  const int tiles = qp_tiles<MODE>(p);
   const int steps = p.steps;                               // operand stages per tile
   if (threadIdx.x == kQpWProd * 32) {
     tma_prefetch_desc(&tmap_w);
@@ -125,14 +149,24 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       PipeState ws(kQpWStages);
       const int raws = (steps + kStepsPerRaw - 1) / kStepsPerRaw;
       for (int t = pair; t < tiles; t += pairs) {
-        const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
-        const int row = pt.n * 2 * kBlockW + (int)rank * kBlockW;
+        const QpTile pt = qp_tile<MODE>(p, t);
+        const int row = MODE == QP_GATE_UP ? pt.expert * p.N + pt.n * kBlockW + (int)rank * (kBlockW / 2)
+                                           : pt.expert * p.N + pt.n * 2 * kBlockW + (int)rank * kBlockW;
         for (int rb = 0; rb < raws; ++rb) {
           mbar_wait(&ctl->w_empty[ws.stage], ws.phase ^ 1);
           if (elect_one()) {
             mbar_arrive_expect_tx(&ctl->w_full[ws.stage], kABytes);
-            tma_load_2d_hint(w_ring + (size_t)ws.stage * kABytes, &tmap_w, rb * (QK == Q_INT4 ? 32 : 128), row,
-                             &ctl->w_full[ws.stage], kEvictNormal);
+            uint8_t* dst = w_ring + (size_t)ws.stage * kABytes;
+            const int col = rb * (QK == Q_INT4 ? 32 : 128);
+            if (MODE == QP_GATE_UP) {
+              // 16 gate rows, the 16 up rows of the same outputs, 16 gate rows ...: a warp then holds both
+#pragma unroll
+              for (int b = 0; b < 8; ++b)
+                tma_load_2d_hint(dst + b * 16 * kStageKBytes, &tmap_w, col, row + (b & 1) * (p.N / 2) + (b >> 1) * 16,
+                                 &ctl->w_full[ws.stage], kEvictNormal);
+            } else {
+              tma_load_2d_hint(dst, &tmap_w, col, row, &ctl->w_full[ws.stage], kEvictNormal);
+            }
           }
           __syncwarp();
           ws.advance();
@@ -143,17 +177,26 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       pdl_wait_prior();
       PipeState xs(kQpXStages);
       for (int t = pair; t < tiles; t += pairs) {
-        const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
-        const int m0 = pt.m * kQpTokens;
-        const int row = m0 + (int)rank * (qp_tile_n(p.M - m0) / 2);
+        const QpTile pt = qp_tile<MODE>(p, t);
+        const int half = qp_tile_n(pt.rows) / 2;            // rows of this CTA that the MMAs read
+        const int row = pt.m0 + (int)rank * half;
         for (int s = 0; s < steps; ++s) {
           mbar_wait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
           if (elect_one()) {
-            if (rank == 0) mbar_arrive_expect_tx(&ctl->x_full[xs.stage], 2 * kQpXBytes);
             uint8_t* dst = x_ring + (size_t)xs.stage * kQpXBytes;
             const uint32_t bar = leader_addr(&ctl->x_full[xs.stage]);
-            tma_load_2d_pair(dst, &tmap_x, s * kQpStepK, row, bar, kEvictNormal);
-            tma_load_2d_pair(dst + kQpXSub, &tmap_x, s * kQpStepK + 64, row, bar, kEvictNormal);
+            if (MODE == QP_PLAIN) {
+              if (rank == 0) mbar_arrive_expect_tx(&ctl->x_full[xs.stage], 2 * kQpXBytes);
+              tma_load_2d_pair(dst, &tmap_x, s * kQpStepK, row, bar, kEvictNormal);
+              tma_load_2d_pair(dst + kQpXSub, &tmap_x, s * kQpStepK + 64, row, bar, kEvictNormal);
+            } else {
+              // an expert may have two rows: only the 16-row boxes that are read
+              if (rank == 0) mbar_arrive_expect_tx(&ctl->x_full[xs.stage], 2 * 2 * half * kStageKBytes);
+              for (int r = 0; r < half; r += 16) {
+                tma_load_2d_pair(dst + r * kStageKBytes, &tmap_x, s * kQpStepK, row + r, bar, kEvictNormal);
+                tma_load_2d_pair(dst + kQpXSub + r * kStageKBytes, &tmap_x, s * kQpStepK + 64, row + r, bar, kEvictNormal);
+              }
+            }
           }
           __syncwarp();
           xs.advance();
@@ -170,8 +213,8 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       PipeState xs(kQpXStages), os(kQpOpStages);
       int seg = 0;
       for (int t = pair; t < tiles; t += pairs) {
-        const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
-        const uint32_t idesc = umma_idesc(1u, 0u, 0u, 0u, 0u, 2 * kBlockW, (uint32_t)qp_tile_n(p.M - pt.m * kQpTokens));
+        const QpTile pt = qp_tile<MODE>(p, t);
+        const uint32_t idesc = umma_idesc(1u, 0u, 0u, 0u, 0u, 2 * kBlockW, (uint32_t)qp_tile_n(pt.rows));
         int in_seg = 0;
         for (int s = 0; s < steps; ++s) {
           const int buf = seg & 1;
@@ -209,10 +252,12 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     pdl_wait_prior();               // y may still be read upstream
     int seg = 0;
     for (int t = pair; t < tiles; t += pairs) {
-      const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
+      const QpTile pt = qp_tile<MODE>(p, t);
       const int n_tile = pt.n * 2 + (int)rank;
-      const int n = n_tile * kBlockW + row;
-      const bool n_ok = n < p.N;
+      // weight row of this thread, and for the gate / up rows the output that the pair (lane, lane + 16) forms
+      const int out = pt.n * kBlockW + (int)rank * (kBlockW / 2) + quad * 16 + (lane & 15);
+      const int n = MODE == QP_GATE_UP ? out + (lane >> 4) * (p.N / 2) : n_tile * kBlockW + row;
+      const bool n_ok = MODE == QP_GATE_UP ? out < p.N / 2 : n < p.N;
       // scale of group g: packed int4 tables are [tile][group][128], 8-bit tables strided by scale block
       const float* sp = p.scales;
       int64_t s_step;
@@ -220,7 +265,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         sp += ((int64_t)(n_ok ? n_tile : 0) * nseg) * kBlockW + row;
         s_step = kBlockW;
       } else {
-        sp += (int64_t)((n_ok ? n : 0) / p.group_n) * p.s_stride_n;
+        sp += (int64_t)pt.expert * p.s_stride_e + (int64_t)((n_ok ? n : 0) / p.group_n) * p.s_stride_n;
         s_step = p.s_stride_k;
       }
       uint64_t acc[kQpHalf / 2];
@@ -250,9 +295,47 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       float bv = 0.f;
       if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
-      const int m0 = pt.m * kQpTokens + half * kQpHalf;
-      const int rows = p.M - m0;
+      const int m0 = pt.m0 + half * kQpHalf;
+      const int rows = pt.rows - half * kQpHalf;
       __half* y = reinterpret_cast<__half*>(p.y);
+      if (MODE == QP_GATE_UP) {
+        // like the fused activation below, with the pair 16 lanes apart
+        const bool high = lane >> 4;
+        __half* yp = y + (int64_t)(m0 + (high ? 1 : 0)) * p.ldy + out;
+#pragma unroll
+        for (int j = 0; j < kQpHalf / 2; ++j) {
+          float a, b;
+          unpack_f32x2(acc[j], a, b);
+          a = __half2float(__float2half_rn(a));
+          b = __half2float(__float2half_rn(b));
+          const float other = __shfl_xor_sync(0xffffffffu, high ? a : b, 16);
+          const float gate = high ? other : a, up = high ? b : other;
+          if (n_ok && 2 * j + (high ? 1 : 0) < rows) *yp = __float2half_rn(silu_q(gate) * up);
+          yp += 2 * p.ldy;
+        }
+        continue;
+      }
+      if (MODE == QP_DOWN) {
+        // rows go back to their slots, times the routing weight in fp32 before the rounding (fused_moe.py:201-205);
+        // lane l keeps the slots and weights of rows l and l + 32 of this half
+        int slot[2];
+        float wt[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const bool in = 32 * q + lane < rows;
+          slot[q] = in ? __ldg(p.order + m0 + 32 * q + lane) : 0;
+          wt[q] = in ? __half2float(p.row_weights[slot[q]]) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < kQpHalf; ++j) {
+          float v[2];
+          unpack_f32x2(acc[j / 2], v[0], v[1]);
+          const int to = __shfl_sync(0xffffffffu, slot[j / 32], j % 32);
+          const float w = __shfl_sync(0xffffffffu, wt[j / 32], j % 32);
+          if (n_ok && j < rows) y[(int64_t)to * p.ldy + n] = __float2half_rn(v[j & 1] * w);
+        }
+        continue;
+      }
       if (EPI == 0) {
         __half* yp = y + (int64_t)m0 * p.ldy + n;
         if (n_ok) {
@@ -297,13 +380,12 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     int use = 0;                                            // stages this group has filled
     const int raws = (steps + kStepsPerRaw - 1) / kStepsPerRaw;
     for (int t = pair; t < tiles; t += pairs) {
-      const PairTile pt = pair_tile(t, p.m_tiles, p.n_tiles, kQpBand);
-      const int n_tile = pt.n * 2 + (int)rank;
       const float* zp = nullptr;
       int k = (group - i0) & 1;                             // first step of this tile that is this group's
       float z = 0.f;
       if (QK == Q_INT4) {
         const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
+        const int n_tile = qp_tile<MODE>(p, t).n * 2 + (int)rank;
         zp = p.zeros + ((int64_t)(n_tile * kBlockW < p.N ? n_tile : 0) * nseg) * kBlockW + row;
         if (k < steps) z = __ldg(zp + (int64_t)(k / p.seg_steps) * kBlockW);
       }
@@ -362,9 +444,9 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (warp == kQpMma) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int QK, int EPI>
+template <int QK, int EPI, int MODE = QP_PLAIN>
 static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
-  auto kern = gemm_quant_pair_kernel<QK, EPI>;
+  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE>;
   static int configured[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, kQpSmem, configured));
   b2l_launch(kern, dim3((unsigned)grid), dim3(kQpThreads), (size_t)kQpSmem, st, tw, tx, p);
@@ -411,4 +493,58 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
   return launch_qp<Q_INT8, 0>(tw, tx, p, grid, st);
 }
 
+// Row boxes of the tensor map of W in the grouped modes: 16 (gate | up interleaved) or a CTA's 128 rows.
+template <int MODE>
+static int grouped(int qk, const MoePairGemm& g, cudaStream_t st) {
+  const int pairs = b2l_num_sms() / 2;
+  QuantPairParams p;
+  p.y = g.y; p.ldy = g.ldy; p.bias = nullptr; p.bias_is_f32 = 0;
+  p.scales = g.scales; p.s_stride_e = g.s_stride_e; p.s_stride_n = g.s_stride_n; p.s_stride_k = g.s_stride_k;
+  p.zeros = nullptr;
+  p.group_n = (int)(g.group_n > g.N ? g.N : g.group_n);
+  p.table = g.table; p.order = g.order; p.row_weights = (const __half*)g.row_weights;
+  p.M = (int)g.rows; p.N = (int)g.N;
+  p.steps = (int)cdiv64(g.K, kQpStepK);
+  p.seg_steps = g.group_k >= g.K ? p.steps : (int)(g.group_k / kQpStepK);
+  p.m_tiles = 0;
+  p.n_tiles = (int)cdiv64(g.N, 2 * kBlockW);
+  const int64_t most = (int64_t)g.max_tiles * p.n_tiles;
+  const int grid = 2 * (int)(most < pairs ? most : pairs);
+  CUtensorMap tw, tx;
+  int rc = b2l_make_tmap_2d(&tw, g.w, TMA_U8, (uint64_t)g.experts * g.N, (uint64_t)g.K, (uint64_t)g.w_row_stride,
+                            MODE == QP_GATE_UP ? 16 : kBlockW, 128, true);
+  if (rc != B2L_OK) return rc;
+  rc = b2l_make_tmap_2d(&tx, g.x, TMA_F16, (uint64_t)g.rows, (uint64_t)g.K, (uint64_t)g.ldx * 2, 16, 64, true);
+  if (rc != B2L_OK) return rc;
+  return qk == Q_FP8 ? launch_qp<Q_FP8, 0, MODE>(tw, tx, p, grid, st) : launch_qp<Q_INT8, 0, MODE>(tw, tx, p, grid, st);
+}
+static int moe_pair_gate_up(int qk, const MoePairGemm& g, cudaStream_t st) { return grouped<QP_GATE_UP>(qk, g, st); }
+static int moe_pair_down(int qk, const MoePairGemm& g, cudaStream_t st) { return grouped<QP_DOWN>(qk, g, st); }
+
 }  // namespace gemm
+
+// The products of a routed layer with 8-bit experts over rows sorted by expert; `table` and `order` are b2l_moe_sort's with
+// 128-row tiles.  gate_up: y[r, i] = silu(gate_i) * up_i for the sorted row r, w [E, n, k] with the gate rows first;
+// down: y[slot, :] = topk_weights[slot] * (x[r] . w), slot = order[r].
+extern "C" int b2l_moe_pair_gemm(void* y, const void* x, const void* w, int weight_is_fp8, const void* scales,
+                                 const void* topk_weights, const void* order, const void* table, int64_t max_tiles,
+                                 int64_t rows, int num_experts, int64_t n, int64_t k, int64_t x_row_stride,
+                                 int64_t w_row_stride, int64_t y_row_stride, int64_t group_n, int64_t group_k,
+                                 int64_t s_stride_e, int64_t s_stride_n, int64_t s_stride_k, int down, void* stream) {
+  using namespace gemm;
+  B2L_REQUIRE(y && x && w && scales && table && (!down || (topk_weights && order)), "moe_pair_gemm: null pointer");
+  B2L_REQUIRE(num_experts >= 1 && n > 0 && k > 0 && rows >= 0 && max_tiles >= 0 && (int64_t)num_experts * n < (1ll << 31),
+              "moe_pair_gemm: bad shape");
+  B2L_REQUIRE(k % 16 == 0 && x_row_stride % 8 == 0 && w_row_stride % 16 == 0, "moe_pair_gemm: rows must be 16-byte multiples");
+  B2L_REQUIRE(group_n >= 1 && group_k >= 1 && (group_k >= k || group_k % kQpStepK == 0),
+              "moe_pair_gemm: group_k (%lld) must be a multiple of %d unless it covers K", (long long)group_k, kQpStepK);
+  B2L_REQUIRE(down || n % 2 == 0, "moe_pair_gemm: gate|up needs an even number of rows");
+  if (rows == 0 || max_tiles == 0) return B2L_OK;
+  MoePairGemm g;
+  g.y = y; g.ldy = y_row_stride; g.x = x; g.ldx = x_row_stride; g.w = w; g.w_row_stride = w_row_stride;
+  g.scales = (const float*)scales; g.s_stride_e = s_stride_e; g.s_stride_n = s_stride_n; g.s_stride_k = s_stride_k;
+  g.group_n = group_n; g.group_k = group_k; g.experts = num_experts; g.rows = rows; g.N = n; g.K = k;
+  g.table = (const int32_t*)table; g.max_tiles = max_tiles; g.order = (const int32_t*)order; g.row_weights = topk_weights;
+  const int qk = weight_is_fp8 ? Q_FP8 : Q_INT8;
+  return down ? moe_pair_down(qk, g, (cudaStream_t)stream) : moe_pair_gate_up(qk, g, (cudaStream_t)stream);
+}

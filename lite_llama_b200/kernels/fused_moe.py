@@ -87,6 +87,54 @@ def _moe_gemm(a, w, c, scale, kind, topk_weights, sorted_ids, expert_ids, num_po
     )
 
 
+_PAIR_TILE = 128      # rows of a tile of the pair GEMMs (csrc/gemm_quant_pair.cu)
+
+
+def _pair_gemm_takes(kind: int, hidden: int, intermediate: int, group_k: int, w1: torch.Tensor, w2: torch.Tensor) -> bool:
+    """8-bit experts whose scale groups are whole operand stages of 128 (or cover k), in 16-byte rows."""
+    return kind != _KIND_F16 and hidden % 16 == 0 and intermediate % 16 == 0 and \
+        (group_k % 128 == 0 or group_k >= max(hidden, intermediate)) and \
+        all(w.stride(-1) == 1 and w.stride(1) % 16 == 0 and w.data_ptr() % 16 == 0 for w in (w1, w2))
+
+
+def _fused_moe_pair(x, w1, w2, flat_weights, topk_ids, w1_scale, w2_scale, kind, group_n, group_k):
+    """Rows gathered into one run per expert, both products as persistent grouped GEMMs on CTA pairs with the activation in
+    the first one's epilogue.  Every rounding of :func:`fused_moe` stays where it is."""
+    tokens, hidden = x.shape
+    num_experts, two_inter, _ = w1.shape
+    top_k = topk_ids.shape[1]
+    slots = tokens * top_k
+    ids = topk_ids.reshape(-1)
+    if ids.dtype not in (torch.int32, torch.int64):
+        ids = ids.to(torch.int64)
+    ids = ids.contiguous()
+    L, dev, st = lib(), x.device, stream_handle()
+    max_tiles = L.b2l_moe_sort_max_tiles(slots, _PAIR_TILE, num_experts)
+    order = torch.empty(slots + 1, dtype=torch.int32, device=dev)
+    table = torch.empty(1 + 3 * max_tiles, dtype=torch.int32, device=dev)
+    check(L.b2l_moe_sort(order.data_ptr(), table.data_ptr(), ids.data_ptr(), index_width(ids, "topk_ids"), slots, _PAIR_TILE,
+                         num_experts, st))
+    rows = torch.empty((slots, hidden), dtype=x.dtype, device=dev)
+    check(L.b2l_moe_gather(rows.data_ptr(), x.data_ptr(), order.data_ptr(), slots, top_k, hidden, x.stride(0), st))
+
+    def product(y, a, w, scale, down):
+        n, k = w.shape[1:]
+        if w.stride(0) != n * w.stride(1):
+            w = w.contiguous()
+        if scale.dtype != torch.float32:
+            scale = scale.float()
+        check(L.b2l_moe_pair_gemm(y.data_ptr(), a.data_ptr(), w.data_ptr(), 1 if kind == _KIND_FP8 else 0, scale.data_ptr(),
+                                  flat_weights.data_ptr(), order.data_ptr(), table.data_ptr(), max_tiles, slots, num_experts,
+                                  n, k, a.stride(0), w.stride(1), y.stride(0), int(group_n or 1), int(group_k or k),
+                                  *scale.stride(), down, st))
+
+    act = torch.empty((slots, two_inter // 2), dtype=x.dtype, device=dev)
+    product(act, rows, w1, w1_scale, 0)
+    expanded = torch.empty((slots, hidden), dtype=x.dtype, device=dev)
+    product(expanded, act, w2, w2_scale, 1)
+    return expanded
+
+
 @torch.no_grad()
 def fused_moe(
     hidden_states: torch.Tensor,
@@ -126,23 +174,23 @@ def fused_moe(
         raise ValueError("fp16 expert weights must match the activation dtype")
     x = hidden_states if hidden_states.stride(-1) == 1 and hidden_states.stride(0) % 8 == 0 else hidden_states.contiguous()
     flat_weights = topk_weights.reshape(-1).to(dtype).contiguous()
-    block = _block_size(num_tokens, top_k, num_experts)
-    sorted_ids, expert_ids, num_post = moe_align_block_size(topk_ids, block, num_experts)
-
-    gate_up = torch.empty((num_tokens * top_k, two_inter), device=device, dtype=dtype)
-    _moe_gemm(x, w1, gate_up, w1_scale, kind, None, sorted_ids, expert_ids, num_post, top_k, block, group_n, group_k)
-
-    act = torch.empty((num_tokens * top_k, intermediate), device=device, dtype=dtype)
-    check(
-        lib().b2l_swiglu(
-            act.data_ptr(), gate_up.data_ptr(), gate_up[:, intermediate:].data_ptr(), num_tokens * top_k, intermediate,
-            gate_up.stride(0), gate_up.stride(0), act.stride(0), dtype_code(act, "act"), stream_handle(),
+    if _pair_gemm_takes(kind, hidden, intermediate, group_k, w1, w2) and x.data_ptr() % 16 == 0:
+        expanded = _fused_moe_pair(x, w1, w2, flat_weights, topk_ids, w1_scale, w2_scale, kind, group_n, group_k)
+    else:
+        block = _block_size(num_tokens, top_k, num_experts)
+        sorted_ids, expert_ids, num_post = moe_align_block_size(topk_ids, block, num_experts)
+        gate_up = torch.empty((num_tokens * top_k, two_inter), device=device, dtype=dtype)
+        _moe_gemm(x, w1, gate_up, w1_scale, kind, None, sorted_ids, expert_ids, num_post, top_k, block, group_n, group_k)
+        act = torch.empty((num_tokens * top_k, intermediate), device=device, dtype=dtype)
+        check(
+            lib().b2l_swiglu(
+                act.data_ptr(), gate_up.data_ptr(), gate_up[:, intermediate:].data_ptr(), num_tokens * top_k, intermediate,
+                gate_up.stride(0), gate_up.stride(0), act.stride(0), dtype_code(act, "act"), stream_handle(),
+            )
         )
-    )
-
-    expanded = torch.empty((num_tokens * top_k, hidden), device=device, dtype=dtype)
-    _moe_gemm(act, w2, expanded, w2_scale, kind, flat_weights, sorted_ids, expert_ids, num_post, 1, block, group_n,
-              group_k)
+        expanded = torch.empty((num_tokens * top_k, hidden), device=device, dtype=dtype)
+        _moe_gemm(act, w2, expanded, w2_scale, kind, flat_weights, sorted_ids, expert_ids, num_post, 1, block, group_n,
+                  group_k)
 
     out = torch.empty((num_tokens, hidden), device=device, dtype=dtype)
     check(lib().b2l_moe_sum(out.data_ptr(), expanded.data_ptr(), None, num_tokens, hidden, top_k,

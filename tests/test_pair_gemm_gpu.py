@@ -112,3 +112,62 @@ def test_w8_pair_tiles(m, n, k, fmt):
     b = torch.randn(n, device="cuda")
     got = K().w8a16_matmul(x, q, s, group_n=gn, group_k=gk, bias=b)
     assert rel(got, x.double() @ w.T + b.double()) < REL[torch.float16]
+
+
+# ---- routed experts (b2l_moe_sort / b2l_moe_gather / b2l_moe_pair_gemm) ----
+@pytest.mark.parametrize("fmt", ["fp8", "int8"])
+@pytest.mark.parametrize("hidden,inter,gn,gk", [(256, 128, 128, 128), (400, 208, 16, 512), (1024, 320, 64, 128)])
+def test_experts_with_runs_around_the_tile(fmt, hidden, inter, gn, gk):
+    """Runs of 0, 1, 16, 17, 32, 33, 127, 128, 129 and 300 rows; outputs and intermediate columns past the last tile."""
+    runs = [0, 1, 16, 17, 32, 33, 127, 128, 129, 300]
+    E, top_k = len(runs), 1
+    ids = torch.cat([torch.full((n,), e) for e, n in enumerate(runs)])
+    ids = ids[torch.randperm(ids.numel())].view(-1, top_k).cuda()
+    T = ids.shape[0]
+    x = torch.randn(T, hidden, device="cuda", dtype=torch.float16)
+
+    def weight(n, k):
+        if fmt == "fp8":
+            q = (torch.randn(E, n, k, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn)
+            raw, q = q.view(torch.uint8), q.double()
+        else:
+            raw = torch.randint(-127, 128, (E, n, k), device="cuda", dtype=torch.int8)
+            q = raw.double()
+        s = torch.rand(E, -(-n // gn), -(-k // gk), device="cuda") * 5e-4
+        return raw, s, q * s.double().repeat_interleave(gn, 1)[:, :n].repeat_interleave(gk, 2)[:, :, :k]
+
+    w1, s1, d1 = weight(2 * inter, hidden)
+    w2, s2, d2 = weight(hidden, inter)
+    tw = torch.rand(T, top_k, device="cuda").half()
+    got = K().fused_moe(x, w1, w2, tw, ids, w1_scale=s1, w2_scale=s2, group_n=gn, group_k=gk)
+    want = torch.empty(T, hidden, dtype=torch.float64, device="cuda")
+    for e in range(E):
+        t = (ids[:, 0] == e).nonzero()[:, 0]
+        g, u = (x[t].double() @ d1[e].T).half().double().chunk(2, -1)
+        a = (torch.nn.functional.silu(g) * u).half().double()
+        want[t] = (a @ d2[e].T) * tw[t].double()
+    assert rel(got, want) < 2 * REL[torch.float16]        # two roundings to 16 bits between the products, one at the end
+
+
+@pytest.mark.parametrize("slots,experts,width", [(1, 1, torch.int32), (255, 3, torch.int64), (4000, 130, torch.int32),
+                                                 (700, 2048, torch.int64)])
+def test_moe_sort_lists_every_valid_slot_once(slots, experts, width):
+    from lite_llama_b200 import _lib
+
+    L = _lib.load()
+    ids = torch.randint(-1, experts + 1, (slots,), device="cuda", dtype=width)       # -1 and `experts` belong to nobody
+    most = L.b2l_moe_sort_max_tiles(slots, 128, experts)
+    order = torch.full((slots + 1,), -7, dtype=torch.int32, device="cuda")
+    table = torch.full((1 + 3 * most,), -7, dtype=torch.int32, device="cuda")
+    _lib.check(L.b2l_moe_sort(order.data_ptr(), table.data_ptr(), ids.data_ptr(), ids.element_size(), slots, 128, experts,
+                              torch.cuda.current_stream().cuda_stream))
+    order, table, ids = order.tolist(), table.tolist(), ids.tolist()
+    valid = [i for i, e in enumerate(ids) if 0 <= e < experts]
+    assert order[slots] == len(valid) and sorted(order[: len(valid)]) == valid
+    assert table[0] <= most
+    row = 0
+    for t in range(table[0]):
+        e, first, rows = table[1 + 3 * t : 4 + 3 * t]
+        assert first == row and 1 <= rows <= 128 and all(ids[s] == e for s in order[first : first + rows])
+        row += rows
+    assert row == len(valid)
