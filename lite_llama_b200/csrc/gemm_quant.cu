@@ -31,6 +31,7 @@
 #include "gemm_tc.cuh"
 #include "dequant.cuh"
 #include "gemm_quant_pair.cuh"
+#include "gemm_quant_decode.cuh"
 #include <type_traits>
 #include <stdlib.h>
 
@@ -1546,6 +1547,10 @@ extern "C" int b2l_w4a16_matmul(void* y, const void* x, const void* qweight, con
   B2L_REQUIRE(x_row_stride % 8 == 0 && qw_row_stride % 4 == 0,
               "w4a16_matmul: row strides must be 16-byte multiples (K a multiple of 32)");
   if (m == 0) return B2L_OK;
+  if (quant_decode_wanted(m, k, group_size) && (uintptr_t)x % 16 == 0 && (uintptr_t)qweight % 16 == 0)
+    return quant_decode_gemm(0, y, y_row_stride, x, x_row_stride, qweight, qw_row_stride, (const float*)scales,
+                             (const float*)zeros, s_row_stride, s_col_stride, bias, bias_is_f32, m, n, k, group_size, 0,
+                             0, (cudaStream_t)stream);
   QuantParams p; SplitPlan pl; CUtensorMap tw, tx;
   int rc = quant_common(Q_INT4, p, pl, y, x, qweight, m, n, k, x_row_stride, qw_row_stride, y_row_stride, workspace,
                         workspace_bytes, counters, num_counters, &tw, &tx, "w4a16_matmul", group_size);
@@ -1579,6 +1584,10 @@ extern "C" int b2l_w4a16_matmul_packed(void* y, const void* x, const void* qweig
   B2L_REQUIRE(epilogue == 0 || epilogue == 1, "w4a16_matmul_packed: epilogue %d (0 = none, 1 = swiglu over interleaved rows)", epilogue);
   B2L_REQUIRE(epilogue == 0 || n % 2 == 0, "w4a16_matmul_packed: the swiglu epilogue needs an even number of rows");
   if (m == 0) return B2L_OK;
+  if (quant_decode_wanted(m, k, group_size) && (uintptr_t)x % 16 == 0 && (uintptr_t)qweight_packed % 16 == 0)
+    return quant_decode_gemm(1, y, y_row_stride, x, x_row_stride, qweight_packed, qw_row_stride, (const float*)scales_packed,
+                             (const float*)zeros_packed, 0, 0, bias, bias_is_f32, m, n, k, group_size, epilogue,
+                             zeros_foldable, (cudaStream_t)stream);
   if (zeros_foldable && quant_pair_wanted(Q_INT4, m, n, k, group_size)) {
     QuantPairParams q;
     q.y = y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
