@@ -102,6 +102,7 @@ class _Declared:
         fn = self._lib.__dict__.get(name)
         if fn is None:
             raise UndeclaredSymbol(f"{HEADER_PATH.name} declares no {name}: the binding would call it without a prototype")
+        self.__dict__[name] = fn                  # found without this function from now on
         return fn
 
 

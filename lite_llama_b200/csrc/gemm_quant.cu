@@ -1360,8 +1360,9 @@ static inline SplitPlan quant_plan(int qk, int64_t M, int64_t N, int64_t K, int 
         // most CTAs that can share one tile: a tile's nrb_tile blocks cut by ranges of >= floor(total/ctas) blocks
         int slots = 1;
         for (int t = 0; t < pl.n_tiles; ++t) {
-          const int64_t lo = (((int64_t)t * nrb_tile + 1) * ctas - 1) / total;
-          const int64_t hi = (((int64_t)(t + 1) * nrb_tile) * ctas - 1) / total;
+          // 32 bits hold total * (ctas + 1), see above (this loop runs on every call: 2 us for 224 tiles in 64 bits)
+          const unsigned lo = (((unsigned)t * nrb_tile + 1) * ctas - 1) / (unsigned)total;
+          const unsigned hi = (((unsigned)(t + 1) * nrb_tile) * ctas - 1) / (unsigned)total;
           if ((int)(hi - lo + 1) > slots) slots = (int)(hi - lo + 1);
         }
         pl.sk_slots = slots;

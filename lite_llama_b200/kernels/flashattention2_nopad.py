@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, dtype_code, index_width, lib, require_cuda, stream_handle
+from ._common import check, dtype_code, index_width, lib, no_grad, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def flash_attention2_no_pad(q, k, v, sm_scale, b_start_loc, b_seq_len, max_seq_len):
     """``q [T, Hq, D]``, ``k``/``v`` ``[T, Hkv, D]``; ``sm_scale`` already multiplied by log2(e).
 

@@ -6,14 +6,14 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, dtype_code, float_code, index_width, lib, ptr, require_cuda, stream_handle
+from ._common import check, dtype_code, float_code, index_width, lib, no_grad, ptr, require_cuda, stream_handle
 
 _KIND_F16, _KIND_FP8, _KIND_INT8 = 0, 1, 2
 SCORES = {"sigmoid": 0, "softmax": 1}
 GROUP_SCORES = {"top2": 0, "max": 1}
 
 
-@torch.no_grad()
+@no_grad
 def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: int):
     """Sort token slots by expert and pad each expert's run to ``block_size``.
 
@@ -135,7 +135,7 @@ def _fused_moe_pair(x, w1, w2, flat_weights, topk_ids, w1_scale, w2_scale, kind,
     return expanded
 
 
-@torch.no_grad()
+@no_grad
 def fused_moe(
     hidden_states: torch.Tensor,
     w1: torch.Tensor,
@@ -198,7 +198,7 @@ def fused_moe(
     return out
 
 
-@torch.no_grad()
+@no_grad
 def route_topk(router_logits: torch.Tensor, top_k: int, renormalize: bool = True):
     """``(weights [T, k] in the logits dtype, ids [T, k] int64)``: fp32 softmax over all experts,
     top-k, optional renormalisation (lite_llama/models/qwen3_moe.py:94-100), one kernel."""
@@ -217,7 +217,7 @@ def route_topk(router_logits: torch.Tensor, top_k: int, renormalize: bool = True
     return w, ids
 
 
-@torch.no_grad()
+@no_grad
 def route_sigmoid_groups(x: torch.Tensor, router_w: torch.Tensor, bias: torch.Tensor | None, top_k: int,
                          groups: int = 1, keep: int = 1, renormalize: bool = True, scores: str = "sigmoid",
                          scale: float = 1.0, group_score: str = "top2"):
@@ -263,7 +263,7 @@ def _swiglu_into(mid: torch.Tensor, wide: torch.Tensor, ff: int, in_scale: torch
                                   float_code(mid, "mid"), stream_handle()))
 
 
-@torch.no_grad()
+@no_grad
 def grouped_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, weights: torch.Tensor,
                     ids: torch.Tensor, addend: torch.Tensor | None = None, activation: str = "gelu",
                     gated: bool = False, weight_on_input: bool = False, limit: float = 0.0,

@@ -5,13 +5,13 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, counters, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, counters, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 GATED_UNITS = {"silu": 0, "clamped": 1, "gelu_tanh": 2}
 GATED_LINEAR_MODES = {"forget_gate": 0, "delta_rule": 1}
 
 
-@torch.no_grad()
+@no_grad
 def gated_linear_scan(mode: str, state: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, seq_start,
                       seq_ctx, seq_slot, heads: int, qk_heads: int, dim: int, vdim: int, c0: torch.Tensor,
                       c1: torch.Tensor | None = None, p0: torch.Tensor | None = None, p1: torch.Tensor | None = None,
@@ -50,7 +50,7 @@ def mlstm_head_floats(dim: int, vdim: int) -> int:
     return -(-(dim * vdim + dim + 1) // 4) * 4
 
 
-@torch.no_grad()
+@no_grad
 def mlstm(state: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, zi: torch.Tensor, zf: torch.Tensor,
           bias_i: torch.Tensor, bias_f: torch.Tensor, batch, heads: int, dim: int, vdim: int, gate_cap: float,
           q_scale: float) -> torch.Tensor:
@@ -88,7 +88,7 @@ def mlstm(state: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor
     return y
 
 
-@torch.no_grad()
+@no_grad
 def head_norm_gate(y: torch.Tensor, weight: torch.Tensor, heads: int, eps: float,
                    gate: torch.Tensor | None = None, gate_form: str = "silu") -> torch.Tensor:
     """``unit_rms(y[t, h, :]) * weight * silu(gate[t, h, :])`` per head (``gate=None``: no gate; ``gate_form="sigmoid"``:
@@ -108,7 +108,7 @@ def head_norm_gate(y: torch.Tensor, weight: torch.Tensor, heads: int, eps: float
     return out
 
 
-@torch.no_grad()
+@no_grad
 def head_mix(wide: torch.Tensor, mix: torch.Tensor, heads: int, kv_heads: int, per_call: int, vdim: int) -> torch.Tensor:
     """``out[t, h, :] = sum_g mix[h, g] * wide[t, g, kv(h), :]`` for ``wide [tokens, calls, heads, per_call, vdim]``
     (contiguous), where ``wide[t, c // per_call, g, c % per_call]`` is query head g's softmax weights applied to kv head
@@ -124,7 +124,7 @@ def head_mix(wide: torch.Tensor, mix: torch.Tensor, heads: int, kv_heads: int, p
     return out
 
 
-@torch.no_grad()
+@no_grad
 def swiglu_scaled(gate: torch.Tensor, up: torch.Tensor, in_scale: torch.Tensor | None = None,
                   out_logit: torch.Tensor | None = None, form: str = "silu", limit: float = 0.0,
                   alpha: float = 1.702) -> torch.Tensor:

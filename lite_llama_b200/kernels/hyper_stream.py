@@ -6,7 +6,7 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 MAX_STREAMS = 8
 
@@ -24,7 +24,7 @@ def _conv_args(conv, h: torch.Tensor):
     return (weight.data_ptr(), ptr(tail), hc.data_ptr(), seq_ctx.data_ptr(), seq_slot.data_ptr(), weight.shape[1]), hc
 
 
-@torch.no_grad()
+@no_grad
 def stream_embed(tokens: torch.Tensor, embed: torch.Tensor, embed_weight: torch.Tensor, streams: int, read_in: torch.Tensor,
                  weight: torch.Tensor, eps: float, conv=None):
     """All streams = ``unit_rms(embed[token]) * embed_weight``; then a read ``h = unit_rms(sum_s read_in[s] x_s) * weight``.
@@ -43,7 +43,7 @@ def stream_embed(tokens: torch.Tensor, embed: torch.Tensor, embed_weight: torch.
     return x, h, hc
 
 
-@torch.no_grad()
+@no_grad
 def stream_mix(x: torch.Tensor, y: torch.Tensor, coef: torch.Tensor, read_in: torch.Tensor, weight: torch.Tensor, eps: float,
                addend: torch.Tensor | None = None, gate: torch.Tensor | None = None, gate_bias: torch.Tensor | None = None,
                rows: torch.Tensor | None = None, conv=None):

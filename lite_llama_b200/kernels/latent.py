@@ -7,11 +7,11 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 from .rotary_heads import PAIRINGS
 
 
-@torch.no_grad()
+@no_grad
 def rope_table(positions: torch.Tensor, rot_dims: int, rot_base: float) -> torch.Tensor | None:
     """fp32 ``[T, rot_dims]`` = per token ``[cos | sin]`` of ``position * base^(-2i / rot_dims)`` (angles in fp64); one
     table per step serves every layer with these rotary constants.  ``None`` when nothing rotates."""
@@ -24,7 +24,7 @@ def rope_table(positions: torch.Tensor, rot_dims: int, rot_base: float) -> torch
     return out
 
 
-@torch.no_grad()
+@no_grad
 def latent_prepare(proj: torch.Tensor, pool: torch.Tensor, kv_rows: torch.Tensor, cos_sin: torch.Tensor | None,
                    q_norm: torch.Tensor | None, kv_norm: torch.Tensor, q_rank: int, kv_rank: int, rot_dim: int,
                    rot_dims: int, eps: float, pairing: str = "halves") -> None:
@@ -40,7 +40,7 @@ def latent_prepare(proj: torch.Tensor, pool: torch.Tensor, kv_rows: torch.Tensor
                                    stream_handle()))
 
 
-@torch.no_grad()
+@no_grad
 def rope_heads(dst: torch.Tensor, dst_head_stride: int, src: torch.Tensor, src_head_stride: int,
                cos_sin: torch.Tensor | None, heads: int, width: int, rot_dims: int, pairing: str = "halves") -> None:
     """``dst[t, h, :width] = src[t, h, :width]`` with the first ``rot_dims`` entries rotated by the token's
@@ -52,7 +52,7 @@ def rope_heads(dst: torch.Tensor, dst_head_stride: int, src: torch.Tensor, src_h
                                float_code(src, "src"), stream_handle()))
 
 
-@torch.no_grad()
+@no_grad
 def head_linear(out: torch.Tensor, out_head_stride: int, x: torch.Tensor, x_head_stride: int, w: torch.Tensor,
                 gate: torch.Tensor | None = None, gate_elements: bool = False) -> None:
     """``out[t, h, :n] = w[h] @ x[t, h, :k]`` for ``w [heads, n, k]``; optional ``gate [T, >= heads]``:

@@ -8,10 +8,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, counters, dtype_code, float_code, lib, ptr, require_cuda, stream_handle, workspace
+from ._common import as_rows, check, counters, dtype_code, float_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, workspace
 
 
-@torch.no_grad()
+@no_grad
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """``[..., K] @ [N, K].T -> [..., N]`` in ``x``'s dtype, fp32 accumulation."""
     require_cuda(x, weight, bias)
@@ -25,12 +25,11 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
     if weight.stride(-1) != 1:
         weight = weight.contiguous()
-    leading = x.shape[:-1]
-    a = x.reshape(-1, k)
+    a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
         a = a.contiguous()
     m = a.shape[0]
-    out = torch.empty((m, n), dtype=x.dtype, device=x.device)
+    out = x.new_empty((m, n))
     if bias is not None:
         bias = bias.to(x.dtype).contiguous()
     L = lib()
@@ -43,10 +42,10 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
             out.stride(0), ptr(ws), nbytes, cnt.data_ptr(), cnt.numel(), code, stream_handle(),
         )
     )
-    return out.reshape(*leading, n)
+    return unrows(out, x)
 
 
-@torch.no_grad()
+@no_grad
 def linear_simt(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """The same product on the CUDA cores: fp32 accumulation in ascending k, any shape, fp16 / bf16 / TRUE fp32
     (no reduced-precision tensor mode).  A row's result does not depend on the other rows of the batch."""
@@ -59,8 +58,7 @@ def linear_simt(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
     if weight.stride(-1) != 1:
         weight = weight.contiguous()
-    leading = x.shape[:-1]
-    a = x.reshape(-1, k)
+    a = as_rows(x)
     if a.stride(-1) != 1:
         a = a.contiguous()
     out = torch.empty((a.shape[0], n), dtype=x.dtype, device=x.device)
@@ -68,4 +66,4 @@ def linear_simt(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None
         bias = bias.to(x.dtype).contiguous()
     check(lib().b2l_gemm_simt(out.data_ptr(), a.data_ptr(), weight.data_ptr(), ptr(bias), a.shape[0], n, k,
                               a.stride(0), weight.stride(0), out.stride(0), code, stream_handle()))
-    return out.reshape(*leading, n)
+    return unrows(out, x)

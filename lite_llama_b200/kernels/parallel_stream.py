@@ -8,10 +8,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def embed_rmsnorm(tokens: torch.Tensor, embed: torch.Tensor, weight: torch.Tensor | None, eps: float,
                   weight_offset: float = 1.0, scale: float = 1.0, out: torch.Tensor | None = None) -> torch.Tensor:
     """fp32 ``unit_rms(scale * embed[tokens]) * (weight_offset + weight)`` (``weight=None``: the unit-RMS rows),
@@ -30,7 +30,7 @@ def embed_rmsnorm(tokens: torch.Tensor, embed: torch.Tensor, weight: torch.Tenso
     return out
 
 
-@torch.no_grad()
+@no_grad
 def depth_mix_norms(stack: torch.Tensor, count: int, coef: torch.Tensor | None, w1: torch.Tensor | None,
                     w2: torch.Tensor | None, eps: float, weight_offset: float = 1.0, out: torch.Tensor | None = None,
                     dtype: torch.dtype | None = None):
@@ -59,7 +59,7 @@ def depth_mix_norms(stack: torch.Tensor, count: int, coef: torch.Tensor | None, 
     return out, h1, h2
 
 
-@torch.no_grad()
+@no_grad
 def branch_sum_residual(residual: torch.Tensor, a: torch.Tensor, a_weight: torch.Tensor | None = None,
                         b: torch.Tensor | None = None, b_weight: torch.Tensor | None = None,
                         c: torch.Tensor | None = None, eps: float = 0.0, scale: float = 1.0,
@@ -91,7 +91,7 @@ def branch_sum_residual(residual: torch.Tensor, a: torch.Tensor, a_weight: torch
     return act
 
 
-@torch.no_grad()
+@no_grad
 def gelu_mul_gather(z: torch.Tensor, tokens: torch.Tensor, table: torch.Tensor, col0: int) -> torch.Tensor:
     """``gelu_tanh(z[t, d]) * table[tokens[t], col0 + d]`` for ``z [tokens, dim]``."""
     require_cuda(z, tokens, table)

@@ -4,12 +4,12 @@ from __future__ import annotations
 
 import torch
 
-from .._common import check, counters, lib, ptr, require_cuda, stream_handle, zeroed_workspace
+from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, zeroed_workspace
 
 _Q_INT4 = 0
 
 
-@torch.no_grad()
+@no_grad
 def w4a16_matmul(
     x: torch.Tensor,
     qweight: torch.Tensor,
@@ -39,12 +39,11 @@ def w4a16_matmul(
         scales = scales.contiguous()
     if qweight.stride(-1) != 1:
         qweight = qweight.contiguous()
-    leading = x.shape[:-1]
-    a = x.reshape(-1, k)
+    a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
         a = a.contiguous()
     m = a.shape[0]
-    out = torch.empty((m, n), dtype=x.dtype, device=x.device)
+    out = x.new_empty((m, n))
     bias_f32 = 0
     if bias is not None:
         if bias.dtype == torch.float32:
@@ -54,7 +53,7 @@ def w4a16_matmul(
             bias_f32 = 1
         bias = bias.contiguous()
     L = lib()
-    nbytes = L.b2l_quant_gemm_workspace_bytes(_Q_INT4, m, n, k, int(group_size))
+    nbytes = quant_gemm_workspace_bytes(_Q_INT4, m, n, k, int(group_size), current_device())
     ws = zeroed_workspace(nbytes, x.device)
     cnt = counters(x.device)
     check(
@@ -64,7 +63,7 @@ def w4a16_matmul(
             out.stride(0), ptr(ws), nbytes, cnt.data_ptr(), cnt.numel(), stream_handle(),
         )
     )
-    return out.reshape(*leading, n)
+    return unrows(out, x)
 
 
 class PackedW4:
@@ -82,7 +81,7 @@ class PackedW4:
         return sum(t.numel() * t.element_size() for t in (self.qweight, self.scales, self.zeros))
 
 
-@torch.no_grad()
+@no_grad
 def w4a16_pack(qweight: torch.Tensor, scales: torch.Tensor, zeros: torch.Tensor, *, group_size: int = 128) -> PackedW4:
     """Repack reference-layout ``(qweight [N, K/8] int32, scales/zeros [N, K/g] fp32)`` for
     :func:`w4a16_matmul_packed`. Load-time only (it synchronises once to classify the zero points)."""
@@ -112,7 +111,7 @@ def w4a16_pack(qweight: torch.Tensor, scales: torch.Tensor, zeros: torch.Tensor,
     return PackedW4(qp, sp, zp, n, k, int(group_size), foldable)
 
 
-@torch.no_grad()
+@no_grad
 def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor | None = None,
                         swiglu: bool = False) -> torch.Tensor:
     """:func:`w4a16_matmul` on a :class:`PackedW4` (same result, bit for bit in the integer unpack).
@@ -126,13 +125,12 @@ def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor
     n, k = packed.n, packed.k
     if x.shape[-1] != k:
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
-    leading = x.shape[:-1]
-    a = x.reshape(-1, k)
+    a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
         a = a.contiguous()
     m = a.shape[0]
     n_out = n // 2 if swiglu else n
-    out = torch.empty((m, n_out), dtype=x.dtype, device=x.device)
+    out = x.new_empty((m, n_out))
     bias_f32 = 0
     if bias is not None:
         if bias.dtype == torch.float32:
@@ -142,7 +140,7 @@ def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor
             bias_f32 = 1
         bias = bias.contiguous()
     L = lib()
-    nbytes = L.b2l_quant_gemm_workspace_bytes(_Q_INT4, m, n, k, packed.group_size)
+    nbytes = quant_gemm_workspace_bytes(_Q_INT4, m, n, k, packed.group_size, current_device())
     ws = zeroed_workspace(nbytes, x.device)
     cnt = counters(x.device)
     check(
@@ -153,7 +151,7 @@ def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor
             stream_handle(),
         )
     )
-    return out.reshape(*leading, n_out)
+    return unrows(out, x)
 
 
 def interleave_gate_up(t: torch.Tensor) -> torch.Tensor:

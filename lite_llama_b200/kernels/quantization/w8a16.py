@@ -4,12 +4,12 @@ from __future__ import annotations
 
 import torch
 
-from .._common import check, counters, lib, ptr, require_cuda, stream_handle, zeroed_workspace
+from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, zeroed_workspace
 
 _Q_FP8, _Q_INT8 = 1, 2
 
 
-@torch.no_grad()
+@no_grad
 def w8a16_matmul(
     x: torch.Tensor,
     qweight: torch.Tensor,
@@ -38,12 +38,11 @@ def w8a16_matmul(
         scales = scales.float()
     if scales.dim() == 1:
         scales = scales.unsqueeze(-1)
-    leading = x.shape[:-1]
-    a = x.reshape(-1, k)
+    a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
         a = a.contiguous()
     m = a.shape[0]
-    out = torch.empty((m, n), dtype=x.dtype, device=x.device)
+    out = x.new_empty((m, n))
     bias_f32 = 0
     if bias is not None:
         if bias.dtype == torch.float32:
@@ -54,7 +53,7 @@ def w8a16_matmul(
         bias = bias.contiguous()
     L = lib()
     kind = _Q_FP8 if is_fp8 else _Q_INT8
-    nbytes = L.b2l_quant_gemm_workspace_bytes(kind, m, n, k, int(group_k))
+    nbytes = quant_gemm_workspace_bytes(kind, m, n, k, int(group_k), current_device())
     ws = zeroed_workspace(nbytes, x.device)
     cnt = counters(x.device)
     check(
@@ -64,4 +63,4 @@ def w8a16_matmul(
             scales.stride(1), out.stride(0), ptr(ws), nbytes, cnt.data_ptr(), cnt.numel(), stream_handle(),
         )
     )
-    return out.reshape(*leading, n)
+    return unrows(out, x)

@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from .._common import check, counters, dtype_code, lib, ptr, require_cuda, stream_handle, workspace
+from .._common import as_rows, check, counters, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, workspace
 
 
-@torch.no_grad()
+@no_grad
 def quantize_activations_int8(a: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     """Per-token dynamic int8 quantisation: ``scale = absmax/127``, ``q = trunc(x / scale)``
     (reference kernel: w8a8.py:35-68). Returns ``(q [M, K] int8, scales [M] fp32)``."""
@@ -24,7 +24,7 @@ def quantize_activations_int8(a: torch.Tensor) -> tuple[torch.Tensor, torch.Tens
     return q, s
 
 
-@torch.no_grad()
+@no_grad
 def smoothquant_matmul_prequant(
     qa: torch.Tensor,
     a_scales: torch.Tensor,
@@ -50,8 +50,10 @@ def smoothquant_matmul_prequant(
         raise ValueError(f"K ({k}) must be a multiple of 16 for the int8 tensor-core path")
     if weight_scales.dim() > 1:
         weight_scales = weight_scales.squeeze(-1)
-    weight_scales = weight_scales.float().contiguous()
-    a_scales = a_scales.float().contiguous()
+    if weight_scales.dtype != torch.float32 or not weight_scales.is_contiguous():
+        weight_scales = weight_scales.float().contiguous()
+    if a_scales.dtype != torch.float32 or not a_scales.is_contiguous():
+        a_scales = a_scales.float().contiguous()
     if qweight.stride(-1) != 1 or qweight.stride(0) % 16 != 0:
         qweight = qweight.contiguous()
     if bias is not None:
@@ -71,7 +73,7 @@ def smoothquant_matmul_prequant(
     return out
 
 
-@torch.no_grad()
+@no_grad
 def smoothquant_matmul(
     x: torch.Tensor,
     qweight: torch.Tensor,
@@ -90,10 +92,9 @@ def smoothquant_matmul(
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
     if k % 16 != 0:
         raise ValueError(f"K ({k}) must be a multiple of 16 for the int8 tensor-core path")
-    leading = x.shape[:-1]
-    a = x.reshape(-1, k)
+    a = as_rows(x)
     if a.stride(-1) != 1:
         a = a.contiguous()
     qa, a_scales = quantize_activations_int8(a)
     out = smoothquant_matmul_prequant(qa, a_scales, qweight, weight_scales, bias=bias, out_dtype=x.dtype)
-    return out.reshape(*leading, n)
+    return unrows(out, x)

@@ -6,13 +6,13 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
 NORM_KINDS = {"rms": 0, "layer": 1}
 
 
-@torch.no_grad()
+@no_grad
 def embed_positions(tokens: torch.Tensor, positions: torch.Tensor, embed: torch.Tensor,
                     pos_table: torch.Tensor | None, want_act: bool = True, scale: float = 1.0):
     """``residual[t] = scale * embed[tokens[t]] + pos_table[positions[t]]`` in fp32; also returns the copy in
@@ -30,7 +30,7 @@ def embed_positions(tokens: torch.Tensor, positions: torch.Tensor, embed: torch.
     return resid, act
 
 
-@torch.no_grad()
+@no_grad
 def post_norm_residual(residual: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: float,
                        weight_offset: float = 1.0, want_act: bool = True, kind: str = "rms",
                        layer_scale: torch.Tensor | None = None, next_weight: torch.Tensor | None = None,
@@ -56,7 +56,7 @@ def post_norm_residual(residual: torch.Tensor, y: torch.Tensor, weight: torch.Te
     return act
 
 
-@torch.no_grad()
+@no_grad
 def rmsnorm_from_f32(residual: torch.Tensor, weight: torch.Tensor, eps: float, weight_offset: float = 1.0,
                      rows: torch.Tensor | None = None, kind: str = "rms") -> torch.Tensor:
     """Norm (``kind``: "rms" or "layer") of (selected rows of) the fp32 residual, written in ``weight``'s dtype."""
@@ -74,7 +74,7 @@ def rmsnorm_from_f32(residual: torch.Tensor, weight: torch.Tensor, eps: float, w
     return out
 
 
-@torch.no_grad()
+@no_grad
 def relu_squared(x: torch.Tensor) -> torch.Tensor:
     require_cuda(x)
     x = x if x.is_contiguous() else x.contiguous()
@@ -83,7 +83,7 @@ def relu_squared(x: torch.Tensor) -> torch.Tensor:
     return out
 
 
-@torch.no_grad()
+@no_grad
 def gelu(x: torch.Tensor, approximate: str = "none") -> torch.Tensor:
     """Exact (erf) GELU, or the tanh form with ``approximate="tanh"``; evaluated in fp32."""
     require_cuda(x)
@@ -94,7 +94,7 @@ def gelu(x: torch.Tensor, approximate: str = "none") -> torch.Tensor:
     return out
 
 
-@torch.no_grad()
+@no_grad
 def softcap_to_f32(x: torch.Tensor, cap: float, scale: float = 1.0) -> torch.Tensor:
     """``cap * tanh(scale * x / cap)`` as fp32 (``cap <= 0``: ``scale * x``): the logits a scaled, soft-capped head
     hands out."""

@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, dtype_code, index_width, lib, require_cuda, stream_handle
+from ._common import check, dtype_code, index_width, lib, no_grad, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def rope_emb_forward(q, k, cos, sin, batch_size, seq_len):
     """Rotate ``q [B*S, Hq, D]`` and ``k [B*S, Hkv, D]`` by ``cos/sin [B, S, D]`` (first D/2 read).
 
@@ -35,7 +35,7 @@ def rope_emb_forward(q, k, cos, sin, batch_size, seq_len):
     return q, k
 
 
-@torch.no_grad()
+@no_grad
 def rope_emb_inplace(q, k, cos, sin, batch_size, seq_len):
     """Stride-aware variant used by the host layer: rotates ``q``/``k`` where they lie (e.g. the q and
     k column blocks of one fused QKV projection output), so no ``.contiguous()`` copy of ``k`` is made
@@ -58,7 +58,7 @@ def rope_emb_inplace(q, k, cos, sin, batch_size, seq_len):
     return q, k
 
 
-@torch.no_grad()
+@no_grad
 def rope_kv_write(q, k, v, cos, sin, select_index, kv_buffer, batch_size, seq_len):
     """RoPE on ``q``/``k`` (in place, where they lie) + the K|V cache write in one launch: what the reference does
     with ``rope_emb_forward`` -> ``torch.cat([xk, xv])`` -> ``update_kv_buffer`` (models/base.py:76-79,228).

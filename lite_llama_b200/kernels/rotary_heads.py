@@ -9,7 +9,7 @@ import math
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 PAIRINGS = {"neighbours": 0, "halves": 1}
 
@@ -38,7 +38,7 @@ def rotary_frequencies(dims: int, base: float, factor: float = 1.0, original: fl
     return out, 0.1 * math.log(factor) + 1.0
 
 
-@torch.no_grad()
+@no_grad
 def rope_table_freqs(positions: torch.Tensor, freqs: torch.Tensor, magnitude: float = 1.0) -> torch.Tensor:
     """fp32 ``[T, 2 * len(freqs)]`` = per token ``magnitude * [cos | sin]`` of ``position * freqs[i]``; the frequencies
     are an fp64 tensor and the angles are formed and evaluated in fp64."""
@@ -52,7 +52,7 @@ def rope_table_freqs(positions: torch.Tensor, freqs: torch.Tensor, magnitude: fl
     return out
 
 
-@torch.no_grad()
+@no_grad
 def head_norm_rope_prepare(qkv: torch.Tensor, kv_pool: torch.Tensor | None, kv_rows: torch.Tensor,
                            cos_sin: torch.Tensor | None, q_norm: torch.Tensor | None, k_norm: torch.Tensor | None,
                            heads: int, kv_heads: int, head_dim: int, v_head_dim: int, rot_dims: int, eps: float,

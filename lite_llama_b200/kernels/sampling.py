@@ -5,10 +5,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def argmax_rows(logits: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     """``logits [rows, n]`` (last dim contiguous) -> int64 ``[rows]``; ties resolve to the lowest index."""
     require_cuda(logits, out)

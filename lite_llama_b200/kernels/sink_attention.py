@@ -6,10 +6,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle, workspace
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle, workspace
 
 
-@torch.no_grad()
+@no_grad
 def attn_prepare(qkv: torch.Tensor, kv_pool: torch.Tensor, kv_rows: torch.Tensor, positions: torch.Tensor,
                  q_cols: int, k_cols: int, v_cols: int, q_norm: torch.Tensor | None, k_norm: torch.Tensor | None,
                  eps: float, gain_coef: float = 0.0, gain_every: float = 0.0, v_first_in: torch.Tensor | None = None,
@@ -28,7 +28,7 @@ def key_factor_column(k_cols: int) -> int:
     return -(-k_cols // 2) * 2
 
 
-@torch.no_grad()
+@no_grad
 def norm_query_keep_key(qk: torch.Tensor, kv_pool: torch.Tensor, kv_rows: torch.Tensor, positions: torch.Tensor,
                         q_cols: int, k_cols: int, query_weight: torch.Tensor, eps: float, gain_coef: float = 0.0,
                         gain_every: float = 0.0) -> None:
@@ -48,7 +48,7 @@ def norm_query_keep_key(qk: torch.Tensor, kv_pool: torch.Tensor, kv_rows: torch.
                                         float_code(qk, "qk"), stream_handle()))
 
 
-@torch.no_grad()
+@no_grad
 def sink_attention(out: torch.Tensor, q: torch.Tensor, kv_pool: torch.Tensor, table: torch.Tensor, seq_start, seq_ctx,
                    seq_slot, seq_list: torch.Tensor | None, num_seqs: int, max_q_len: int, sink: torch.Tensor | None,
                    heads: int, kv_heads: int, head_dim: int, v_head_dim: int, scale: float, softcap: float,
@@ -86,7 +86,7 @@ def sink_attention(out: torch.Tensor, q: torch.Tensor, kv_pool: torch.Tensor, ta
 MIXED_HEAD_MAX_KEYS = 32768      # the weights of one head and sequence stay in a CTA's shared memory
 
 
-@torch.no_grad()
+@no_grad
 def mixed_head_attention(out: torch.Tensor, q: torch.Tensor, kv_pool: torch.Tensor, table: torch.Tensor, seq_start,
                          seq_ctx, seq_slot, seq_list: torch.Tensor | None, num_seqs: int, mix: torch.Tensor, heads: int,
                          kv_heads: int, head_dim: int, v_head_dim: int, scale: float, softcap: float, max_keys: int,

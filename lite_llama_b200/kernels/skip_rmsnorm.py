@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, dtype_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def skip_rmsnorm(X, residual, weight, eps=1e-5):
     """``(Y, residual)``: ``residual += X`` in place, ``Y = rmsnorm(residual) * weight``.
 
@@ -18,7 +18,10 @@ def skip_rmsnorm(X, residual, weight, eps=1e-5):
     require_cuda(X, residual, weight)
     orig_shape = X.shape
     n = orig_shape[-1]
-    x2 = X.contiguous().view(-1, n)
+    # matrices go through as they are (unless the results would inherit a requires_grad)
+    flat = len(orig_shape) == 2 and not X.requires_grad and X.is_contiguous() and \
+        (residual is None or (residual.shape == orig_shape and not residual.requires_grad and residual.is_contiguous()))
+    x2 = X if flat else X.contiguous().view(-1, n)
     code = dtype_code(x2, "X")
     if weight.dtype != x2.dtype:
         raise ValueError(f"weight dtype {weight.dtype} must match X dtype {x2.dtype}")
@@ -28,13 +31,16 @@ def skip_rmsnorm(X, residual, weight, eps=1e-5):
     if residual is not None:
         if residual.dtype != x2.dtype:
             raise ValueError(f"residual dtype {residual.dtype} must match X dtype {x2.dtype}")
-        r2 = residual.contiguous().view(-1, n)  # aliases the caller's residual when it is contiguous
+        # aliases the caller's residual when it is contiguous
+        r2 = residual if flat else residual.contiguous().view(-1, n)
     check(
         lib().b2l_skip_rmsnorm(
             y.data_ptr(), x2.data_ptr(), ptr(r2), w.data_ptr(), x2.shape[0], n, x2.stride(0),
             r2.stride(0) if r2 is not None else 0, y.stride(0), float(eps), code, stream_handle(),
         )
     )
+    if flat:
+        return y, (x2 if r2 is None else r2)
     if r2 is not None:
         return y.view(orig_shape), r2.view(orig_shape)
     return y.view(orig_shape), x2.view(orig_shape)
@@ -45,7 +51,7 @@ def can_fuse_int8_quant(n: int) -> bool:
     return n % 8 == 0 and n <= 16384
 
 
-@torch.no_grad()
+@no_grad
 def skip_rmsnorm_quant_int8(X, residual, weight, eps=1e-5):
     """``skip_rmsnorm`` whose output goes straight into a SmoothQuant GEMM: returns ``(q int8 [rows, n],
     scales fp32 [rows], residual)`` -- the per-token dynamic quantisation of the (fp16-rounded) norm output
@@ -54,7 +60,10 @@ def skip_rmsnorm_quant_int8(X, residual, weight, eps=1e-5):
     require_cuda(X, residual, weight)
     orig_shape = X.shape
     n = orig_shape[-1]
-    x2 = X.contiguous().view(-1, n)
+    # matrices go through as they are (unless the results would inherit a requires_grad)
+    flat = len(orig_shape) == 2 and not X.requires_grad and X.is_contiguous() and \
+        (residual is None or (residual.shape == orig_shape and not residual.requires_grad and residual.is_contiguous()))
+    x2 = X if flat else X.contiguous().view(-1, n)
     code = dtype_code(x2, "X")
     if weight.dtype != x2.dtype:
         raise ValueError(f"weight dtype {weight.dtype} must match X dtype {x2.dtype}")

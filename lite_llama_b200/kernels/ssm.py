@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def causal_conv_silu(proj: torch.Tensor, col: int, channels: int, weight: torch.Tensor, bias: torch.Tensor | None,
                      tail: torch.Tensor | None, seq_start: torch.Tensor, seq_ctx: torch.Tensor, seq_slot: torch.Tensor,
                      activation: bool = True, residual: bool = False):
@@ -25,7 +25,7 @@ def causal_conv_silu(proj: torch.Tensor, col: int, channels: int, weight: torch.
     return out
 
 
-@torch.no_grad()
+@no_grad
 def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, d_skip, state: torch.Tensor,
              seq_start, seq_ctx, seq_slot, heads: int, groups: int, state_size: int, head_dim: int,
              fixed_decay: torch.Tensor | None = None, silu_inputs: bool = False) -> torch.Tensor:
@@ -49,7 +49,7 @@ def ssm_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias, a_log, d_skip, st
     return y
 
 
-@torch.no_grad()
+@no_grad
 def gated_group_norm(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, groups: int, eps: float) -> torch.Tensor:
     """``unit_rms(y * silu(z)) * weight`` with the statistic taken in ``groups`` equal parts; ``y`` fp32, ``z`` a
     column view of the projection, output in ``weight``'s dtype."""
@@ -64,7 +64,7 @@ def gated_group_norm(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, gro
 DECAY_ATTENTION_CHUNK = 64
 
 
-@torch.no_grad()
+@no_grad
 def decay_attention(x: torch.Tensor, state: torch.Tensor, decay: torch.Tensor, seq_start, seq_ctx, seq_slot, heads: int,
                     state_size: int, head_dim: int, longest: int) -> torch.Tensor:
     """Decayed linear attention ``S <- decay_h S + k v^T``, ``y = S^T q`` on SiLU'd ``x = [v | k | q]`` columns (a view
@@ -88,7 +88,7 @@ def decay_attention(x: torch.Tensor, state: torch.Tensor, decay: torch.Tensor, s
                     fixed_decay=decay, silu_inputs=True)
 
 
-@torch.no_grad()
+@no_grad
 def norm_sigmoid_gate(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """``unit_rms(y) * weight * sigmoid(z)`` over whole rows: the gate acts AFTER the norm (``gated_group_norm`` gates
     first).  ``y`` fp32, ``z`` a column view of a projection, output in ``weight``'s dtype."""
@@ -105,7 +105,7 @@ def norm_sigmoid_gate(y: torch.Tensor, z: torch.Tensor, weight: torch.Tensor, ep
 GATED_SCAN_MODES = {"mingru": 0, "rglru": 1}
 
 
-@torch.no_grad()
+@no_grad
 def gated_scan(mode: str, state: torch.Tensor, p0: torch.Tensor, p1: torch.Tensor, p2: torch.Tensor, seq_start, seq_ctx,
                seq_slot, p3: torch.Tensor | None = None, bias_r: torch.Tensor | None = None,
                bias_i: torch.Tensor | None = None, lam: torch.Tensor | None = None,

@@ -7,10 +7,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, float_code, lib, ptr, require_cuda, stream_handle
+from ._common import check, float_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def tanh_norm_stream(residual: torch.Tensor, norm: tuple[torch.Tensor, torch.Tensor, torch.Tensor] | None = None, *,
                      y: torch.Tensor | None = None, routed: tuple[torch.Tensor, torch.Tensor, int, torch.Tensor] | None = None,
                      addend: torch.Tensor | None = None, embedding: tuple[torch.Tensor, torch.Tensor, float] | None = None,

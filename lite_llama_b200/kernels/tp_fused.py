@@ -12,11 +12,11 @@ from __future__ import annotations
 import torch
 
 from ..distributed import all_reduce_tp, get_tp_comm, get_tp_world_size
-from ._common import check, dtype_code, lib, require_cuda, stream_handle
+from ._common import check, dtype_code, lib, no_grad, require_cuda, stream_handle
 from .skip_rmsnorm import skip_rmsnorm
 
 
-@torch.no_grad()
+@no_grad
 def allreduce_skip_rmsnorm(partial: torch.Tensor, residual: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5):
     if get_tp_world_size() <= 1:
         return skip_rmsnorm(partial, residual, weight, eps)
@@ -45,7 +45,7 @@ def allreduce_skip_rmsnorm(partial: torch.Tensor, residual: torch.Tensor, weight
     return y.view(partial.shape), r2.view(residual.shape)
 
 
-@torch.no_grad()
+@no_grad
 def allreduce_nvlink(partial: torch.Tensor) -> torch.Tensor:
     """Plain SUM all-reduce through the same kernel (used by tests and the bench's latency probe)."""
     comm = get_tp_comm()

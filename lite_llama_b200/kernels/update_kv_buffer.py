@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, index_width, lib, require_cuda, stream_handle
+from ._common import check, index_width, lib, no_grad, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def update_kv_buffer(KV_Values, Select_Index, KV_Buffer):
     """``KV_Buffer[Select_Index[i]] = KV_Values[i]`` for ``[tokens, 2*Hkv, D]`` rows."""
     require_cuda(KV_Values, Select_Index, KV_Buffer)
@@ -27,7 +27,7 @@ def update_kv_buffer(KV_Values, Select_Index, KV_Buffer):
     )
 
 
-@torch.no_grad()
+@no_grad
 def update_kv_buffer_split(K_Values, V_Values, Select_Index, KV_Buffer):
     """Same scatter from separate K and V row tensors (no ``torch.cat``; lite_llama/models/base.py:76)."""
     require_cuda(K_Values, V_Values, Select_Index, KV_Buffer)

@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, index_width, lib, require_cuda, stream_handle
+from ._common import check, index_width, lib, no_grad, require_cuda, stream_handle
 
 
-@torch.no_grad()
+@no_grad
 def update_kv_index(req_to_token_indexs, b_req_idx, b_seq_len, select_index):
     require_cuda(req_to_token_indexs, b_req_idx, b_seq_len, select_index)
     assert (
