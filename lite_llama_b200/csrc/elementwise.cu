@@ -594,18 +594,74 @@ __global__ void __launch_bounds__(256) quantize_act_int8_kernel(int8_t* __restri
   if (threadIdx.x == 0) scales[row] = scale;
 }
 
+// The same on 16-byte rows of up to VPT * 4096 elements: one pass, the row stays in registers between the maximum and the
+// division.  Bound: the division's instructions, then HBM.  256 rows of 18944: 20.4 us in the scalar kernel (two-byte loads,
+// twice; eight warps for 37 KB) -> see the launch below.
+template <typename T, int VPT>
+__global__ void __launch_bounds__(512) quantize_act_int8_vec_kernel(int8_t* __restrict__ q, float* __restrict__ scales,
+                                                                    const T* __restrict__ x, int64_t k, int64_t x_stride,
+                                                                    int64_t q_stride) {
+  pdl_prologue();
+  const int64_t row = blockIdx.x;
+  const T* xr = x + row * x_stride;
+  int8_t* qr = q + row * q_stride;
+  const int chunks = (int)(k / 8);
+  uint4 v[VPT];
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = threadIdx.x + i * 512;
+    v[i] = c < chunks ? ldg_128(xr + (int64_t)c * 8) : make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const T* e = reinterpret_cast<const T*>(&v[i]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(to_f32(e[j])));
+  }
+  __shared__ float red[16];
+  amax = warp_reduce_max(amax);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  float m = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) m = fmaxf(m, red[i]);
+  float scale = m / 127.0f;
+  scale = scale > 0.f ? scale : 1.0f;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    const int c = threadIdx.x + i * 512;
+    if (c < chunks) {
+      const T* e = reinterpret_cast<const T*>(&v[i]);
+      union { int8_t b[8]; uint2 u; } o;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) o.b[j] = (int8_t)__float2int_rz(to_f32(e[j]) / scale);
+      *reinterpret_cast<uint2*>(qr + (int64_t)c * 8) = o.u;
+    }
+  }
+  if (threadIdx.x == 0) scales[row] = scale;
+}
+
+template <typename T>
+static void launch_quantize(int8_t* q, float* scales, const T* x, int64_t m, int64_t k, int64_t xs, int64_t qs, cudaStream_t st) {
+  const bool vec = k % 8 == 0 && xs % 8 == 0 && qs % 8 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)q % 8 == 0;
+  if (vec && k >= 2048 && k <= 2 * 4096)
+    b2l_launch(quantize_act_int8_vec_kernel<T, 2>, dim3((unsigned)m), dim3(512), (size_t)0, st, q, scales, x, k, xs, qs);
+  else if (vec && k >= 2048 && k <= 8 * 4096)
+    b2l_launch(quantize_act_int8_vec_kernel<T, 8>, dim3((unsigned)m), dim3(512), (size_t)0, st, q, scales, x, k, xs, qs);
+  else
+    b2l_launch(quantize_act_int8_kernel<T>, dim3((unsigned)m), dim3(k >= 2048 ? 256 : 128), (size_t)0, st, q, scales, x, k, xs, qs);
+}
+
 extern "C" int b2l_quantize_activations_int8(void* q, void* scales, const void* x, int64_t m, int64_t k,
                                              int64_t x_row_stride, int64_t q_row_stride, int dtype, void* stream) {
   B2L_REQUIRE(q && scales && x, "quantize_activations_int8: null pointer");
   if (m == 0) return B2L_OK;
   cudaStream_t st = (cudaStream_t)stream;
-  const int threads = k >= 2048 ? 256 : 128;
   if (dtype == B2L_F16)
-    b2l_launch(quantize_act_int8_kernel<__half>, dim3((unsigned)m), dim3(threads), (size_t)(0), st, (int8_t*)q, (float*)scales, (const __half*)x, k,
-                                                                     x_row_stride, q_row_stride);
+    launch_quantize((int8_t*)q, (float*)scales, (const __half*)x, m, k, x_row_stride, q_row_stride, st);
   else if (dtype == B2L_BF16)
-    b2l_launch(quantize_act_int8_kernel<__nv_bfloat16>, dim3((unsigned)m), dim3(threads), (size_t)(0), st, 
-        (int8_t*)q, (float*)scales, (const __nv_bfloat16*)x, k, x_row_stride, q_row_stride);
+    launch_quantize((int8_t*)q, (float*)scales, (const __nv_bfloat16*)x, m, k, x_row_stride, q_row_stride, st);
   else
     B2L_UNSUPPORTED("quantize_activations_int8: dtype %d", dtype);
   B2L_LAUNCH_CHECK();
@@ -769,12 +825,66 @@ __global__ void moe_sum_kernel(T* __restrict__ out, const T* __restrict__ in, co
   }
 }
 
+// The same on 16-byte rows, 8 columns per thread (16-bit types): all of a token's rows are requested before the first sum.
+// Bound: HBM / L2 bandwidth.  2000 tokens x 8 rows of 2048: 31.5 us with one column per thread.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_sum_vec_kernel(T* __restrict__ out, const T* __restrict__ in,
+                                                          const T* __restrict__ addend, int64_t items, int64_t chunks, int top_k) {
+  pdl_prologue();
+  const int64_t it = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (it >= items) return;
+  const int64_t m = it / chunks, c = it - m * chunks;
+  const uint4* base = reinterpret_cast<const uint4*>(in) + m * top_k * chunks + c;
+  float acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+  for (int i0 = 0; i0 < top_k; i0 += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) if (i0 + i < top_k) v[i] = __ldcg(base + (int64_t)(i0 + i) * chunks);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (i0 + i < top_k) {
+        const T* e = reinterpret_cast<const T*>(&v[i]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] += to_f32(e[j]);
+      }
+    }
+  }
+  if (addend) {
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(addend) + it);
+    const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] += to_f32(e[j]);
+  }
+  uint4 o;
+  T* oe = reinterpret_cast<T*>(&o);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) oe[j] = from_f32<T>(acc[j]);
+  reinterpret_cast<uint4*>(out)[it] = o;
+}
+
 extern "C" int b2l_moe_sum(void* out, const void* in, const void* addend, int64_t tokens, int64_t n, int top_k,
                            int dtype, void* stream) {
   B2L_REQUIRE(out && in, "moe_sum: null pointer");
   if (tokens == 0 || n == 0) return B2L_OK;
   dim3 grid((unsigned)cdiv64(n, 256), (unsigned)(tokens > 65535 ? 65535 : tokens));
   cudaStream_t st = (cudaStream_t)stream;
+  if (dtype != B2L_F32 && n % 8 == 0 && ((uintptr_t)out | (uintptr_t)in | (uintptr_t)addend) % 16 == 0 &&
+      cdiv64(tokens * (n / 8), 256) < (1ll << 31)) {
+    const int64_t items = tokens * (n / 8);
+    const dim3 blocks((unsigned)cdiv64(items, 256));
+    if (dtype == B2L_F16)
+      b2l_launch(moe_sum_vec_kernel<__half>, blocks, dim3(256), (size_t)0, st, (__half*)out, (const __half*)in,
+                 (const __half*)addend, items, n / 8, top_k);
+    else if (dtype == B2L_BF16)
+      b2l_launch(moe_sum_vec_kernel<__nv_bfloat16>, blocks, dim3(256), (size_t)0, st, (__nv_bfloat16*)out,
+                 (const __nv_bfloat16*)in, (const __nv_bfloat16*)addend, items, n / 8, top_k);
+    else
+      B2L_UNSUPPORTED("moe_sum: dtype %d", dtype);
+    B2L_LAUNCH_CHECK();
+    return B2L_OK;
+  }
   B2L_DISPATCH_FLOAT(dtype, "moe_sum", {
     b2l_launch(moe_sum_kernel<T>, dim3(grid), dim3(256), (size_t)(0), st, (T*)out, (const T*)in, (const T*)addend,
                tokens, n, top_k);

@@ -171,3 +171,38 @@ def test_moe_sort_lists_every_valid_slot_once(slots, experts, width):
         assert first == row and 1 <= rows <= 128 and all(ids[s] == e for s in order[first : first + rows])
         row += rows
     assert row == len(valid)
+
+
+# ---- the 16-byte forms of two element-wise kernels against the forms for any alignment ----
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("m,k", [(1, 2048), (3, 8192), (2, 8200), (5, 18944), (2, 32768), (2, 32776)])
+def test_quantiser_in_vectors_equals_the_scalar_one(m, k, dtype):
+    x = torch.randn(m, k + 8, device="cuda", dtype=dtype)
+    x[0, 3], x[-1, :8] = 30.0, 0.0
+    q, s = K().quantize_activations_int8(x[:, :k])                    # 16-byte rows
+    q2, s2 = K().quantize_activations_int8(x[:, 1 : k + 1])           # the same kernel family on unaligned rows ...
+    xs = torch.empty(m, k + 9, device="cuda", dtype=dtype)
+    xs[:, 1 : k + 1] = x[:, :k]
+    q3, s3 = K().quantize_activations_int8(xs[:, 1 : k + 1])          # ... and on the same values, unaligned
+    assert torch.equal(q, q3) and torch.equal(s, s3)
+    assert q2.shape == q.shape and s2.shape == s.shape
+    want = (x[:, :k].float().abs().amax(-1) / 127.0)
+    assert torch.equal(s, torch.where(want > 0, want, torch.ones_like(want)))
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens,n,top_k", [(1, 8, 1), (3, 2048, 8), (70, 264, 9), (5, 100, 8)])
+@pytest.mark.parametrize("addend", [False, True])
+def test_expert_sum_in_vectors(tokens, n, top_k, addend, dtype):
+    from lite_llama_b200 import _lib
+
+    L = _lib.load()
+    x = torch.randn(tokens, top_k, n, device="cuda", dtype=dtype)
+    add = torch.randn(tokens, n, device="cuda", dtype=dtype) if addend else None
+    out = torch.empty(tokens, n, device="cuda", dtype=dtype)
+    _lib.check(L.b2l_moe_sum(out.data_ptr(), x.data_ptr(), add.data_ptr() if addend else None, tokens, n, top_k,
+                             0 if dtype == torch.float16 else 1, torch.cuda.current_stream().cuda_stream))
+    acc = torch.zeros(tokens, n, device="cuda")
+    for k in range(top_k):
+        acc = acc + x[:, k].float()
+    assert torch.equal(out, (acc + add.float() if addend else acc).to(dtype))
