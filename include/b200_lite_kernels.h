@@ -228,7 +228,7 @@ int b2l_moe_gemm(void* c, const void* a, const void* w, int weight_kind, const v
  * b2l_moe_sort: order int32 [num_slots + 1] = slot of every sorted row, then the number of rows that belong to an expert;
  * table int32 [1 + 3 * b2l_moe_sort_max_tiles] = {tiles, {expert, first row, rows} per tile of tile_rows}.
  * b2l_moe_gather: out[r, :] = x[order[r] / top_k, :] (16-bit elements).
- * b2l_moe_pair_gemm (tile_rows 128): down 0: y[r, i] = silu(gate_i) * up_i, W [E, n, k] with n / 2 gate rows first;
+ * b2l_moe_pair_gemm (tile_rows 64 or 128, as sorted): down 0: y[r, i] = silu(gate_i) * up_i, W [E, n, k] with n / 2 gate rows first;
  * down 1: y[order[r], :] = topk_weights[order[r]] * (x[r] . W).  group_k: a multiple of 128, or >= k. */
 int64_t b2l_moe_sort_max_tiles(int64_t num_slots, int tile_rows, int num_experts);
 int b2l_moe_sort(void* order, void* table, const void* topk_ids, int id_width, int64_t num_slots, int tile_rows,
@@ -236,8 +236,8 @@ int b2l_moe_sort(void* order, void* table, const void* topk_ids, int id_width, i
 int b2l_moe_gather(void* out, const void* x, const void* order, int64_t num_slots, int top_k, int64_t k,
                    int64_t x_row_stride, void* stream);
 int b2l_moe_pair_gemm(void* y, const void* x, const void* w, int weight_is_fp8, const void* scales,
-                      const void* topk_weights, const void* order, const void* table, int64_t max_tiles, int64_t rows,
-                      int num_experts, int64_t n, int64_t k, int64_t x_row_stride, int64_t w_row_stride,
+                      const void* topk_weights, const void* order, const void* table, int64_t max_tiles, int tile_rows,
+                      int64_t rows, int num_experts, int64_t n, int64_t k, int64_t x_row_stride, int64_t w_row_stride,
                       int64_t y_row_stride, int64_t group_n, int64_t group_k, int64_t s_stride_e, int64_t s_stride_n,
                       int64_t s_stride_k, int down, void* stream);
 int b2l_moe_sum(void* out, const void* in, const void* addend, int64_t tokens, int64_t n, int top_k, int dtype,

@@ -25,15 +25,17 @@
 namespace gemm {
 
 constexpr int kQpThreads = 20 * 32;
-constexpr int kQpWStages = 6, kQpXStages = 6, kQpOpStages = 4;
+constexpr int kQpWStages = 6, kQpXStages = 6, kQpMaxOp = 6;
 constexpr int kQpTokens = 128;                              // per pair tile; each CTA stages half
+// Operand stages that fit beside the two accumulator segments of a tile of NT tokens.  With few tokens the MMAs are short and
+// the trip conversion -> leader -> MMA -> both CTAs is what a stage waits for: three stages per conversion group instead of
+// two.
+__host__ __device__ constexpr int qp_op_stages(int nt) { return nt == kQpTokens ? 4 : 6; }
 constexpr int kQpStepK = 128;                               // k per operand stage
 constexpr int kQpXSub = kQpTokens / 2 * kStageKBytes;       // 64 tokens x 64 k
 constexpr int kQpXBytes = 2 * kQpXSub;
 constexpr int kQpSmem = 1024 + 1024 + kQpWStages * kABytes + kQpXStages * kQpXBytes;
 constexpr int kQpBand = 16;
-constexpr int kQpHalf = kQpTokens / 2;                      // tokens per epilogue warp
-constexpr int kQpAccCols = 128, kQpOpCol0 = 2 * kQpAccCols;
 constexpr int kQpEpi0 = 8, kQpWProd = 16, kQpXProd = 17, kQpMma = 18;   // eight conversion, eight epilogue warps
 
 struct __align__(8) QpControl {
@@ -41,8 +43,8 @@ struct __align__(8) QpControl {
   uint64_t w_empty[kQpWStages];     // own: its words have been converted (4 warp arrivals per operand stage in it)
   uint64_t x_full[kQpXStages];      // leader: both CTAs' token halves have landed
   uint64_t x_empty[kQpXStages];     // both: the MMAs that read them have retired
-  uint64_t op_full[kQpOpStages];    // leader: both CTAs' converted rows are in tensor memory (8 warp arrivals)
-  uint64_t op_empty[kQpOpStages];   // both
+  uint64_t op_full[kQpMaxOp];    // leader: both CTAs' converted rows are in tensor memory (8 warp arrivals)
+  uint64_t op_empty[kQpMaxOp];   // both
   uint64_t acc_full[2];             // both: a segment is complete
   uint64_t acc_empty[2];            // leader: both CTAs' epilogue warps have read it (16 warp arrivals)
   uint32_t tmem_base;
@@ -88,12 +90,13 @@ __device__ __forceinline__ QpTile qp_tile(const QuantPairParams& p, int t) {
 }
 
 // tokens of a tile rounded up to what cta_group::2 takes as N
+template <int NT>
 __device__ __forceinline__ int qp_tile_n(int rows_left) {
   const int n = (rows_left + 31) & ~31;
-  return n < kQpTokens ? n : kQpTokens;
+  return n < NT ? n : NT;
 }
 
-template <int QK, int EPI, int MODE>
+template <int QK, int EPI, int MODE, int NT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kQpThreads, 1)
 gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                        const QuantPairParams p) {
@@ -102,6 +105,9 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   QpControl* ctl = reinterpret_cast<QpControl*>(smem);
   uint8_t* w_ring = smem + 1024;
   uint8_t* x_ring = w_ring + kQpWStages * kABytes;
+  constexpr int kHalf = NT / 2;                            // tokens per epilogue warp
+  constexpr int kAccCols = NT, kOpCol0 = 2 * NT, kOpStages = qp_op_stages(NT);
+  static_assert(MODE != QP_PLAIN || NT == kQpTokens, "plain tiles are 128 tokens");
   constexpr int kStepsPerRaw = QK == Q_INT4 ? 2 : 1;       // a raw block is 128 rows x 128 bytes
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -121,7 +127,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       mbar_init(&ctl->x_full[s], 1);
       mbar_init(&ctl->x_empty[s], 1);
     }
-    for (int s = 0; s < kQpOpStages; ++s) {
+    for (int s = 0; s < kOpStages; ++s) {
       mbar_init(&ctl->op_full[s], 8);
       mbar_init(&ctl->op_empty[s], 1);
     }
@@ -178,7 +184,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       PipeState xs(kQpXStages);
       for (int t = pair; t < tiles; t += pairs) {
         const QpTile pt = qp_tile<MODE>(p, t);
-        const int half = qp_tile_n(pt.rows) / 2;            // rows of this CTA that the MMAs read
+        const int half = qp_tile_n<NT>(pt.rows) / 2;            // rows of this CTA that the MMAs read
         const int row = pt.m0 + (int)rank * half;
         for (int s = 0; s < steps; ++s) {
           mbar_wait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
@@ -210,11 +216,11 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     } else if (warp == kQpMma && rank == 0) {
       // ===================== MMA issuer (leader) =====================
       const uint64_t x_desc0 = umma_desc_sw128_kmajor(smem_u32(x_ring));
-      PipeState xs(kQpXStages), os(kQpOpStages);
+      PipeState xs(kQpXStages), os(kOpStages);
       int seg = 0;
       for (int t = pair; t < tiles; t += pairs) {
         const QpTile pt = qp_tile<MODE>(p, t);
-        const uint32_t idesc = umma_idesc(1u, 0u, 0u, 0u, 0u, 2 * kBlockW, (uint32_t)qp_tile_n(pt.rows));
+        const uint32_t idesc = umma_idesc(1u, 0u, 0u, 0u, 0u, 2 * kBlockW, (uint32_t)qp_tile_n<NT>(pt.rows));
         int in_seg = 0;
         for (int s = 0; s < steps; ++s) {
           const int buf = seg & 1;
@@ -224,11 +230,11 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           tc_fence_after();
           const bool last = in_seg + 1 == p.seg_steps || s + 1 == steps;
           if (elect_one()) {
-            const uint32_t a = tmem_base + kQpOpCol0 + os.stage * 64;
+            const uint32_t a = tmem_base + kOpCol0 + os.stage * 64;
             const uint64_t b = x_desc0 + (uint64_t)((xs.stage * kQpXBytes) >> 4);
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              umma_pair_ts(tmem_base + buf * kQpAccCols, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)),
+              umma_pair_ts(tmem_base + buf * kAccCols, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)),
                            idesc, (in_seg | k) != 0 ? 1u : 0u);
             tc_commit_pair(&ctl->op_empty[os.stage]);
             tc_commit_pair(&ctl->x_empty[xs.stage]);
@@ -246,7 +252,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     // ===================== epilogue: one thread per weight row and token half =====================
     const int quad = warp & 3, half = (warp - kQpEpi0) >> 2;
     const int row = quad * 32 + lane;
-    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + half * kQpHalf;
+    const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + half * kHalf;
     const uint32_t empty0 = leader_addr(&ctl->acc_empty[0]), empty1 = leader_addr(&ctl->acc_empty[1]);
     const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
     pdl_wait_prior();               // y may still be read upstream
@@ -268,9 +274,9 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         sp += (int64_t)pt.expert * p.s_stride_e + (int64_t)((n_ok ? n : 0) / p.group_n) * p.s_stride_n;
         s_step = p.s_stride_k;
       }
-      uint64_t acc[kQpHalf / 2];
+      uint64_t acc[kHalf / 2];
 #pragma unroll
-      for (int j = 0; j < kQpHalf / 2; ++j) acc[j] = 0ull;
+      for (int j = 0; j < kHalf / 2; ++j) acc[j] = 0ull;
       float sc = __ldg(sp);
       for (int g = 0; g < nseg; ++g, ++seg) {
         const int buf = seg & 1;
@@ -278,15 +284,15 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         if (g + 1 < nseg) sc = __ldg(sp + (int64_t)(g + 1) * s_step);
         mbar_wait(&ctl->acc_full[buf], (seg >> 1) & 1);
         tc_fence_after();
-        uint32_t v[kQpHalf];
-        tmem_ld_32x32b_x32(taddr + buf * kQpAccCols, *reinterpret_cast<uint32_t(*)[32]>(v));
-        tmem_ld_32x32b_x32(taddr + buf * kQpAccCols + 32, *reinterpret_cast<uint32_t(*)[32]>(v + 32));
+        uint32_t v[kHalf];
+        tmem_ld_32x32b_x32(taddr + buf * kAccCols, *reinterpret_cast<uint32_t(*)[32]>(v));
+        if (kHalf == 64) tmem_ld_32x32b_x32(taddr + buf * kAccCols + 32, *reinterpret_cast<uint32_t(*)[32]>(v + (kHalf - 32)));
         tc_wait_ld();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(buf ? empty1 : empty0);     // in registers: the segment's buffer may be refilled
 #pragma unroll
-        for (int j = 0; j < kQpHalf / 2; ++j) {
+        for (int j = 0; j < kHalf / 2; ++j) {
           const uint64_t pv = pack_f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
           acc[j] = fma_f32x2(s2, pv, acc[j]);
         }
@@ -295,15 +301,15 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       float bv = 0.f;
       if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
-      const int m0 = pt.m0 + half * kQpHalf;
-      const int rows = pt.rows - half * kQpHalf;
+      const int m0 = pt.m0 + half * kHalf;
+      const int rows = pt.rows - half * kHalf;
       __half* y = reinterpret_cast<__half*>(p.y);
       if (MODE == QP_GATE_UP) {
         // like the fused activation below, with the pair 16 lanes apart
         const bool high = lane >> 4;
         __half* yp = y + (int64_t)(m0 + (high ? 1 : 0)) * p.ldy + out;
 #pragma unroll
-        for (int j = 0; j < kQpHalf / 2; ++j) {
+        for (int j = 0; j < kHalf / 2; ++j) {
           float a, b;
           unpack_f32x2(acc[j], a, b);
           a = __half2float(__float2half_rn(a));
@@ -327,7 +333,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           wt[q] = in ? __half2float(p.row_weights[slot[q]]) : 0.f;
         }
 #pragma unroll
-        for (int j = 0; j < kQpHalf; ++j) {
+        for (int j = 0; j < kHalf; ++j) {
           float v[2];
           unpack_f32x2(acc[j / 2], v[0], v[1]);
           const int to = __shfl_sync(0xffffffffu, slot[j / 32], j % 32);
@@ -340,7 +346,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         __half* yp = y + (int64_t)m0 * p.ldy + n;
         if (n_ok) {
 #pragma unroll
-          for (int j = 0; j < kQpHalf / 2; ++j) {
+          for (int j = 0; j < kHalf / 2; ++j) {
             float a, b;
             unpack_f32x2(acc[j], a, b);
             if (2 * j < rows) yp[0] = __float2half_rn(a + bv);
@@ -354,7 +360,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const bool odd = lane & 1;
         __half* yp = y + (int64_t)(m0 + (odd ? 1 : 0)) * p.ldy + (n >> 1);
 #pragma unroll
-        for (int j = 0; j < kQpHalf / 2; ++j) {
+        for (int j = 0; j < kHalf / 2; ++j) {
           float a, b;
           unpack_f32x2(acc[j], a, b);
           a = __half2float(__float2half_rn(a + bv));
@@ -373,11 +379,13 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     // that has seen all of its phases.
     const int group = warp >> 2, quad = warp & 3;
     const int row = quad * 32 + lane, rx = row & 7;
-    const uint32_t dst0 = tmem_base + ((uint32_t)(quad * 32) << 16) + kQpOpCol0;
-    const uint32_t full0 = leader_addr(&ctl->op_full[group]), full1 = leader_addr(&ctl->op_full[group + 2]);
+    const uint32_t dst0 = tmem_base + ((uint32_t)(quad * 32) << 16) + kOpCol0;
+    constexpr int kOwn = kOpStages / 2;                     // stages of this group: group, group + 2, ...
+    const uint32_t full0 = leader_addr(&ctl->op_full[group]);
+    int own = 0;
+    uint32_t own_phase = 0;
     int i0 = 0;                                             // running stage count at the tile's first step
     int raw0 = 0;                                           // running raw-block count
-    int use = 0;                                            // stages this group has filled
     const int raws = (steps + kStepsPerRaw - 1) / kStepsPerRaw;
     for (int t = pair; t < tiles; t += pairs) {
       const float* zp = nullptr;
@@ -400,8 +408,8 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const int rs = raw % kQpWStages;
         mbar_wait(&ctl->w_full[rs], (raw / kQpWStages) & 1);
         const uint8_t* src = w_ring + (size_t)rs * kABytes + row * 128;
-        const int stage = group + 2 * (use & 1);
-        mbar_wait(&ctl->op_empty[stage], ((use >> 1) & 1) ^ 1);
+        const int stage = group + 2 * own;
+        mbar_wait(&ctl->op_empty[stage], own_phase ^ 1);
         tc_fence_after();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -431,8 +439,8 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(use & 1 ? full1 : full0);
-        ++use;
+        if (lane == 0) mbar_arrive_cluster(full0 + own * 16);   // barriers are 8 bytes apart
+        if (++own == kOwn) { own = 0; own_phase ^= 1; }
       }
       i0 += steps;
       raw0 += raws;
@@ -444,9 +452,9 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (warp == kQpMma) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int QK, int EPI, int MODE = QP_PLAIN>
+template <int QK, int EPI, int MODE = QP_PLAIN, int NT = kQpTokens>
 static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
-  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE>;
+  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE, NT>;
   static int configured[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, kQpSmem, configured));
   b2l_launch(kern, dim3((unsigned)grid), dim3(kQpThreads), (size_t)kQpSmem, st, tw, tx, p);
@@ -516,6 +524,7 @@ static int grouped(int qk, const MoePairGemm& g, cudaStream_t st) {
   if (rc != B2L_OK) return rc;
   rc = b2l_make_tmap_2d(&tx, g.x, TMA_F16, (uint64_t)g.rows, (uint64_t)g.K, (uint64_t)g.ldx * 2, 16, 64, true);
   if (rc != B2L_OK) return rc;
+  if (g.tile_rows == 64) return qk == Q_FP8 ? launch_qp<Q_FP8, 0, MODE, 64>(tw, tx, p, grid, st) : launch_qp<Q_INT8, 0, MODE, 64>(tw, tx, p, grid, st);
   return qk == Q_FP8 ? launch_qp<Q_FP8, 0, MODE>(tw, tx, p, grid, st) : launch_qp<Q_INT8, 0, MODE>(tw, tx, p, grid, st);
 }
 static int moe_pair_gate_up(int qk, const MoePairGemm& g, cudaStream_t st) { return grouped<QP_GATE_UP>(qk, g, st); }
@@ -524,11 +533,11 @@ static int moe_pair_down(int qk, const MoePairGemm& g, cudaStream_t st) { return
 }  // namespace gemm
 
 // The products of a routed layer with 8-bit experts over rows sorted by expert; `table` and `order` are b2l_moe_sort's with
-// 128-row tiles.  gate_up: y[r, i] = silu(gate_i) * up_i for the sorted row r, w [E, n, k] with the gate rows first;
+// the same tile_rows.  gate_up: y[r, i] = silu(gate_i) * up_i for the sorted row r, w [E, n, k] with the gate rows first;
 // down: y[slot, :] = topk_weights[slot] * (x[r] . w), slot = order[r].
 extern "C" int b2l_moe_pair_gemm(void* y, const void* x, const void* w, int weight_is_fp8, const void* scales,
                                  const void* topk_weights, const void* order, const void* table, int64_t max_tiles,
-                                 int64_t rows, int num_experts, int64_t n, int64_t k, int64_t x_row_stride,
+                                 int tile_rows, int64_t rows, int num_experts, int64_t n, int64_t k, int64_t x_row_stride,
                                  int64_t w_row_stride, int64_t y_row_stride, int64_t group_n, int64_t group_k,
                                  int64_t s_stride_e, int64_t s_stride_n, int64_t s_stride_k, int down, void* stream) {
   using namespace gemm;
@@ -538,13 +547,14 @@ extern "C" int b2l_moe_pair_gemm(void* y, const void* x, const void* w, int weig
   B2L_REQUIRE(k % 16 == 0 && x_row_stride % 8 == 0 && w_row_stride % 16 == 0, "moe_pair_gemm: rows must be 16-byte multiples");
   B2L_REQUIRE(group_n >= 1 && group_k >= 1 && (group_k >= k || group_k % kQpStepK == 0),
               "moe_pair_gemm: group_k (%lld) must be a multiple of %d unless it covers K", (long long)group_k, kQpStepK);
+  B2L_REQUIRE(tile_rows == 64 || tile_rows == 128, "moe_pair_gemm: tile_rows %d (64 or 128)", tile_rows);
   B2L_REQUIRE(down || n % 2 == 0, "moe_pair_gemm: gate|up needs an even number of rows");
   if (rows == 0 || max_tiles == 0) return B2L_OK;
   MoePairGemm g;
   g.y = y; g.ldy = y_row_stride; g.x = x; g.ldx = x_row_stride; g.w = w; g.w_row_stride = w_row_stride;
   g.scales = (const float*)scales; g.s_stride_e = s_stride_e; g.s_stride_n = s_stride_n; g.s_stride_k = s_stride_k;
   g.group_n = group_n; g.group_k = group_k; g.experts = num_experts; g.rows = rows; g.N = n; g.K = k;
-  g.table = (const int32_t*)table; g.max_tiles = max_tiles; g.order = (const int32_t*)order; g.row_weights = topk_weights;
+  g.table = (const int32_t*)table; g.max_tiles = max_tiles; g.tile_rows = tile_rows; g.order = (const int32_t*)order; g.row_weights = topk_weights;
   const int qk = weight_is_fp8 ? Q_FP8 : Q_INT8;
   return down ? moe_pair_down(qk, g, (cudaStream_t)stream) : moe_pair_gate_up(qk, g, (cudaStream_t)stream);
 }

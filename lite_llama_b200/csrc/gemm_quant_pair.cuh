@@ -31,7 +31,7 @@ struct MoePairGemm {
   const float* scales; int64_t s_stride_e, s_stride_n, s_stride_k;
   int64_t group_n, group_k;
   int64_t experts, rows, N, K;
-  const int32_t* table; int64_t max_tiles;
+  const int32_t* table; int64_t max_tiles; int tile_rows;
   const int32_t* order; const void* row_weights;     // down only
 };
 

@@ -87,7 +87,10 @@ def _moe_gemm(a, w, c, scale, kind, topk_weights, sorted_ids, expert_ids, num_po
     )
 
 
-_PAIR_TILE = 128      # rows of a tile of the pair GEMMs (csrc/gemm_quant_pair.cu)
+def _pair_tile(slots: int, num_experts: int) -> int:
+    """Rows of a tile of the pair GEMMs (csrc/gemm_quant_pair.cu): 64 leave room for more conversion stages, 128 convert an
+    expert's weights once for twice the rows.  The line is where an expert's run rarely exceeds 64 rows."""
+    return 64 if slots <= 32 * num_experts else 128
 
 
 def _pair_gemm_takes(kind: int, hidden: int, intermediate: int, group_k: int, w1: torch.Tensor, w2: torch.Tensor) -> bool:
@@ -109,10 +112,11 @@ def _fused_moe_pair(x, w1, w2, flat_weights, topk_ids, w1_scale, w2_scale, kind,
         ids = ids.to(torch.int64)
     ids = ids.contiguous()
     L, dev, st = lib(), x.device, stream_handle()
-    max_tiles = L.b2l_moe_sort_max_tiles(slots, _PAIR_TILE, num_experts)
+    tile = _pair_tile(slots, num_experts)
+    max_tiles = L.b2l_moe_sort_max_tiles(slots, tile, num_experts)
     order = torch.empty(slots + 1, dtype=torch.int32, device=dev)
     table = torch.empty(1 + 3 * max_tiles, dtype=torch.int32, device=dev)
-    check(L.b2l_moe_sort(order.data_ptr(), table.data_ptr(), ids.data_ptr(), index_width(ids, "topk_ids"), slots, _PAIR_TILE,
+    check(L.b2l_moe_sort(order.data_ptr(), table.data_ptr(), ids.data_ptr(), index_width(ids, "topk_ids"), slots, tile,
                          num_experts, st))
     rows = torch.empty((slots, hidden), dtype=x.dtype, device=dev)
     check(L.b2l_moe_gather(rows.data_ptr(), x.data_ptr(), order.data_ptr(), slots, top_k, hidden, x.stride(0), st))
@@ -124,8 +128,8 @@ def _fused_moe_pair(x, w1, w2, flat_weights, topk_ids, w1_scale, w2_scale, kind,
         if scale.dtype != torch.float32:
             scale = scale.float()
         check(L.b2l_moe_pair_gemm(y.data_ptr(), a.data_ptr(), w.data_ptr(), 1 if kind == _KIND_FP8 else 0, scale.data_ptr(),
-                                  flat_weights.data_ptr(), order.data_ptr(), table.data_ptr(), max_tiles, slots, num_experts,
-                                  n, k, a.stride(0), w.stride(1), y.stride(0), int(group_n or 1), int(group_k or k),
+                                  flat_weights.data_ptr(), order.data_ptr(), table.data_ptr(), max_tiles, tile, slots,
+                                  num_experts, n, k, a.stride(0), w.stride(1), y.stride(0), int(group_n or 1), int(group_k or k),
                                   *scale.stride(), down, st))
 
     act = torch.empty((slots, two_inter // 2), dtype=x.dtype, device=dev)
