@@ -208,7 +208,8 @@ int b2l_w8a8_gemm(void* y, const void* xq, const void* wq, const void* a_scale, 
 /* fused_moe(hidden_states, w1, w2, topk_weights, topk_ids, *, w1_scale, w2_scale, group_n, group_k)
  * -- lite_llama/kernels/fused_moe.py:352-438 -- is moe_align_block_size (:45-99), grouped GEMM1
  * (b2l_moe_gemm), silu_and_mul (b2l_swiglu on the two halves, :296-313), grouped GEMM2 with the routing
- * weight folded in (b2l_moe_gemm, :201-205) and moe_sum (:316-333).
+ * weight folded in (b2l_moe_gemm, :201-205) and moe_sum (:316-333).  8-bit experts in scale groups of 128: b2l_moe_sort,
+ * b2l_moe_gather, b2l_moe_pair_gemm twice, moe_sum.
  *
  * moe_align_block_size(topk_ids, block_size, num_experts): sorted_token_ids int32
  * [num_slots + E*(block-1)] (sentinel = num_slots), expert_ids int32 [ceil(that / block)],

@@ -6,6 +6,10 @@
 //   int4 : qweight int32 [N, K/8], nibble j of word i = K index 8i+j; scales, zeros fp32 [N, K/g]
 //   8-bit: qweight uint8(e4m3)/int8 [N, K]; scales fp32 [ceil(N/gn), ceil(K/gk)]
 //
+// Up to 8 tokens of int4 run in gemm_quant_decode.cu, prompt-sized batches (and 8-bit weights with one scale per output row
+// at any size with enough tiles) in gemm_quant_pair.cu; this file streams the weights for what lies between, for fine scale
+// groups and for int4 zero points that are not whole numbers.
+//
 // Pipeline per CTA (tile orientation: gemm_tc.cuh -- 128 weight rows on the TMEM lanes, tokens on UMMA N):
 //   TMA producer     raw quantised weight tile (128 rows x 128 BYTES, 128B-swizzled) + the matching
 //                    activation sub-tiles -> deep shared-memory ring (HBM latency hiding)

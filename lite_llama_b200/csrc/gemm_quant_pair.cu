@@ -107,7 +107,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   uint8_t* x_ring = w_ring + kQpWStages * kABytes;
   constexpr int kHalf = NT / 2;                            // tokens per epilogue warp
   constexpr int kAccCols = NT, kOpCol0 = 2 * NT, kOpStages = qp_op_stages(NT);
-  static_assert(MODE != QP_PLAIN || NT == kQpTokens, "plain tiles are 128 tokens");
+  // (plain mode with NT 64 is launched for up to 64 tokens only: one row of tiles)
   constexpr int kStepsPerRaw = QK == Q_INT4 ? 2 : 1;       // a raw block is 128 rows x 128 bytes
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -467,15 +467,18 @@ static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPa
 // 23.5 against 17.5 us) and covers four of them per pair, so the waves decide: int4, us, streaming -> pair:
 //   28672 x 4096, 72 tokens 72 -> 46, 4096 tokens 1854 -> 982; 4096 x 4096, 320 tokens 33 -> 23, but 192 tokens 17 -> 22.
 // One segment over all of k (a scale per output row) leaves the streaming kernel a single MMA warp; there the pair
-// kernel wins as soon as it has 16 tiles (int8, 896 x 4864, 512 tokens 27 -> 19; 320 tokens, 12 tiles: level).
+// kernel wins as soon as it has 16 tiles (int8, 896 x 4864, 512 tokens 27 -> 19; 320 tokens, 12 tiles: level).  That holds
+// for decode batches too (tiles of 64 tokens, six conversion stages; int8, 32 tokens: 28672 x 4096 82 -> 28, 6144 x 4096
+// 18.7 -> 14.5, 4096 x 4096 16.1 -> 14.5) unless k is long and few pairs have work, where the split of k wins (4096 x 14336,
+// 16 tiles: 37 against 45).
 bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k) {
   // segments of whole operand stages, or one segment over all of K
   if (group_k % kQpStepK != 0 && group_k < K) return false;
   if (qk == Q_INT4 && K % kQpStepK != 0) return false;      // the packed tables are read per 128 k
-  if (M <= 64) return false;
   const int64_t sms = b2l_num_sms();
   const int64_t tiles = cdiv64(M, kQpTokens) * cdiv64(N, 2 * kBlockW);
-  if (group_k >= K) return tiles >= 16;
+  if (group_k >= K) return M > 64 ? tiles >= 16 : qk != Q_INT4 && (tiles >= 40 || (tiles >= 16 && K <= 4096));
+  if (M <= 64) return false;
   return 4 * cdiv64(cdiv64(M, 64) * cdiv64(N, kBlockW), sms) >= 5 * cdiv64(tiles, sms / 2);
 }
 
@@ -497,6 +500,8 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
   rc = b2l_make_tmap_2d(&tx, x, TMA_F16, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, kQpTokens / 2, 64, true);
   if (rc != B2L_OK) return rc;
   if (qk == Q_INT4) return swiglu ? launch_qp<Q_INT4, 1>(tw, tx, p, grid, st) : launch_qp<Q_INT4, 0>(tw, tx, p, grid, st);
+  if (M <= 64)
+    return qk == Q_FP8 ? launch_qp<Q_FP8, 0, QP_PLAIN, 64>(tw, tx, p, grid, st) : launch_qp<Q_INT8, 0, QP_PLAIN, 64>(tw, tx, p, grid, st);
   if (qk == Q_FP8) return launch_qp<Q_FP8, 0>(tw, tx, p, grid, st);
   return launch_qp<Q_INT8, 0>(tw, tx, p, grid, st);
 }

@@ -6,6 +6,9 @@
 // Expert weights are fp16 [E, N, K] or 8-bit (uint8 e4m3 / int8) with one fp32 scale per
 // (group_n x group_k) block, the same layout w8a16 uses (fused_moe.py:188-197).
 //
+// 8-bit experts whose scale groups are multiples of 128 (or cover K) run in gemm_quant_pair.cu (b2l_moe_pair_gemm); this
+// kernel serves fp16 experts and finer groups (sub-block tensor-parallel shards).
+//
 // Same swap-AB tile as the dense/quantised GEMMs (gemm_tc.cuh): 128 weight rows of one expert on the
 // TMEM lanes, the block's BT token slots on the UMMA N dimension.  Differences:
 //   * the activation rows of a block are scattered (gathered through sorted_token_ids), so the eight

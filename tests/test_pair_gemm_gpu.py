@@ -114,6 +114,22 @@ def test_w8_pair_tiles(m, n, k, fmt):
     assert rel(got, x.double() @ w.T + b.double()) < REL[torch.float16]
 
 
+@pytest.mark.parametrize("m", [1, 31, 33, 64])
+@pytest.mark.parametrize("n,k", [(10140, 528), (4096, 4096)])
+@pytest.mark.parametrize("fp8", [True, False])
+def test_w8_per_channel_decode_tiles(m, n, k, fp8):
+    x = torch.randn(m, k, device="cuda", dtype=torch.float16)
+    if fp8:
+        q = (torch.randn(n, k, device="cuda") * 60).clamp(-448, 448).to(torch.float8_e4m3fn).view(torch.uint8)
+        w = q.view(torch.float8_e4m3fn).double()
+    else:
+        q = torch.randint(-127, 128, (n, k), device="cuda", dtype=torch.int8)
+        w = q.double()
+    s = torch.rand(n, 1, device="cuda") * 1e-3
+    got = K().w8a16_matmul(x, q, s, group_n=1, group_k=k)
+    assert rel(got, x.double() @ (w * s.double()).T) < REL[torch.float16]
+
+
 # ---- routed experts (b2l_moe_sort / b2l_moe_gather / b2l_moe_pair_gemm) ----
 @pytest.mark.parametrize("fmt", ["fp8", "int8"])
 @pytest.mark.parametrize("hidden,inter,gn,gk", [(256, 128, 128, 128), (400, 208, 16, 512), (1024, 320, 64, 128)])
