@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle
+from ._common import check, dtype_code, is_rows, lib, no_grad, ptr, require_cuda, stream_handle
 
 
 @no_grad
@@ -19,8 +19,9 @@ def skip_rmsnorm(X, residual, weight, eps=1e-5):
     orig_shape = X.shape
     n = orig_shape[-1]
     # matrices go through as they are (unless the results would inherit a requires_grad)
-    flat = len(orig_shape) == 2 and not X.requires_grad and X.is_contiguous() and \
-        (residual is None or (residual.shape == orig_shape and not residual.requires_grad and residual.is_contiguous()))
+    flat = is_rows(X) and not X.requires_grad and X.is_contiguous() and \
+        (residual is None or (residual.shape == orig_shape and is_rows(residual) and not residual.requires_grad and
+                              residual.is_contiguous()))
     x2 = X if flat else X.contiguous().view(-1, n)
     code = dtype_code(x2, "X")
     if weight.dtype != x2.dtype:
@@ -61,8 +62,9 @@ def skip_rmsnorm_quant_int8(X, residual, weight, eps=1e-5):
     orig_shape = X.shape
     n = orig_shape[-1]
     # matrices go through as they are (unless the results would inherit a requires_grad)
-    flat = len(orig_shape) == 2 and not X.requires_grad and X.is_contiguous() and \
-        (residual is None or (residual.shape == orig_shape and not residual.requires_grad and residual.is_contiguous()))
+    flat = is_rows(X) and not X.requires_grad and X.is_contiguous() and \
+        (residual is None or (residual.shape == orig_shape and is_rows(residual) and not residual.requires_grad and
+                              residual.is_contiguous()))
     x2 = X if flat else X.contiguous().view(-1, n)
     code = dtype_code(x2, "X")
     if weight.dtype != x2.dtype:
