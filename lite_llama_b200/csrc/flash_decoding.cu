@@ -297,7 +297,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
 }
 
 // Stage 2: log-sum-exp merge of the per-split partials (reference: flashdecoding.py:224-313).
-template <typename T, int D, bool MANY>   // MANY: more than 8 splits
+template <typename T, int D, bool MANY>   // MANY: some row may have more than 8 splits
 __global__ void flash_decode_combine_kernel(const DecodeParams p) {
   pdl_prologue();
   const int b = blockIdx.x, head = blockIdx.y;
@@ -305,7 +305,7 @@ __global__ void flash_decode_combine_kernel(const DecodeParams p) {
   int nsp = (int)((seq_len + p.chunk - 1) / p.chunk);
   nsp = nsp < p.splits ? nsp : p.splits;
   const int64_t off = ((int64_t)b * p.Hq + head) * p.splits;
-  if (!MANY) {
+  if (!MANY || nsp <= 8) {
     float M = -INFINITY;
     for (int s = 0; s < nsp; ++s) M = fmaxf(M, p.ws_lse[off + s]);
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -375,13 +375,12 @@ Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
   pl.smem = stages * stage + 128;
   const int64_t pairs = batch * (Hkv / HB);
   const int64_t tiles = max_len > 0 ? (max_len + kTT - 1) / kTT : 1;
-  // One wave of the CTAs that share an SM (two with rows of several KB), if that leaves every row at least three splits: more and shorter ones pay the
-  // start of the ring and a partial row each (32 sequences of up to 2000 tokens, 8 kv heads of 128: 25 splits 54.0 us, 9
-  // splits 46 us; 64 of 1000, 4 kv heads: 31.5 -> 25.7).  With more rows than that, six waves even out ragged lengths.
-  int resident = smem_cap / (pl.smem + 1024);
-  resident = resident < 2 ? 2 : resident > 6 ? 6 : resident;
-  const int64_t wave = (int64_t)resident * b2l_num_sms(), most = 6LL * b2l_num_sms();
-  int64_t splits = wave / pairs >= 3 ? wave / pairs : (most + pairs - 1) / pairs;
+  // Six CTAs per SM over all splits of the longest possible length.  max_len is only a bound: the lengths are device data, one
+  // long sequence may stand among short ones, and a captured graph's bucket may be twice the longest.  One wave of larger
+  // splits is faster where every length is near max_len (32 sequences of 1000 - 2000 tokens, 8 kv heads of 128: 25 splits
+  // 54 us, 9 splits 47 us) and slower where it is not: sequences shorter than a split then occupy one CTA each.
+  const int64_t target = 6LL * b2l_num_sms();
+  int64_t splits = (target + pairs - 1) / pairs;
   const int64_t max_splits = (tiles + 3) / 4;   // at least 4 tiles (64 tokens) per split
   if (splits > max_splits) splits = max_splits;
   if (splits < 1) splits = 1;
