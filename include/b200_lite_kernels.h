@@ -58,6 +58,10 @@ int64_t b2l_launch_count(void);
  * overlap it; see csrc/common.cuh).  Returns the previous setting.  Also: environment B2L_PDL=0 at load.
  * No reference counterpart: the reference launches every Triton kernel fully serialised. */
 int b2l_set_pdl(int enabled);
+/* The GEMMs (b2l_linear, b2l_w8a8_gemm, b2l_w4a16_matmul*, b2l_w8a16_matmul) request weights, scales and zero points before
+ * the previous kernel of the stream has finished.  Whoever writes those tensors on the stream right before such a call
+ * enqueues this in between (one empty kernel); b2l_w4a16_pack_* do it themselves. */
+int b2l_weights_written(void* stream);
 /* Device-side hang watchdog (csrc/common.cuh): every barrier wait of the warp-specialised kernels traps after
  * B2L_HANG_MS milliseconds (environment, default 4000, 0 = off) instead of parking for ever, after writing a
  * host-pinned record.  out16 receives: [0] 0xB2D00DED when a record exists, [1] FNV-1a hash of the source file's

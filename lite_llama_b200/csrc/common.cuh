@@ -48,6 +48,7 @@ void b2l_set_error(const char* fmt, ...);
 
 // every kernel launch of this library goes through B2L_LAUNCH_CHECK: count them (bench.py reports it)
 void b2l_count_launch();
+extern "C" int b2l_weights_written(void* stream);   // core.cu
 
 #define B2L_LAUNCH_CHECK()                                                          \
   do {                                                                              \
@@ -454,6 +455,7 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, f
 //     kernel has completed and flushed; since that kernel waited for ITS predecessor before finishing,
 //     completion is transitive over the whole stream.  Every kernel must therefore execute the wait on
 //     every path.  Without the launch attribute both instructions are no-ops.
+// Weights that a call itself converts or copies are NOT static: b2l_weights_written() (core.cu) goes in between.
 __device__ __forceinline__ void pdl_wait_prior() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // for kernels whose first instruction already reads the previous kernel's output

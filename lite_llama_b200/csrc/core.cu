@@ -33,6 +33,16 @@ extern "C" int b2l_set_pdl(int enabled) {
   return old;
 }
 
+// Under programmatic dependent launch the GEMMs read weights before they wait for the previous kernel (common.cuh).  A kernel
+// without the launch attribute starts only when everything before it has completed and is visible, and nothing that
+// follows starts before it ends: behind it, freshly written weights are as static as any.
+__global__ void weights_written_kernel() {}
+extern "C" int b2l_weights_written(void* stream) {
+  weights_written_kernel<<<1, 32, 0, (cudaStream_t)stream>>>();
+  B2L_LAUNCH_CHECK();
+  return B2L_OK;
+}
+
 extern "C" const char* b2l_last_error(void) { return g_err; }
 extern "C" int b2l_version(void) { return 100; }
 

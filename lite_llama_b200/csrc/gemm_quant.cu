@@ -1651,7 +1651,7 @@ extern "C" int b2l_w4a16_pack_qweight(void* out, const void* in, int64_t n, int6
   b2l_launch(w4_pack_qweight_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, (uint32_t*)out,
              (const uint32_t*)in, n, k8, in_row_stride, out_row_stride);
   B2L_LAUNCH_CHECK();
-  return B2L_OK;
+  return b2l_weights_written(stream);   // the GEMMs read weights ahead of the previous kernel's end
 }
 extern "C" int b2l_w4a16_pack_table(void* out, const void* in, int64_t n, int64_t groups, int64_t row_stride,
                                     int64_t col_stride, void* stream) {
@@ -1662,7 +1662,7 @@ extern "C" int b2l_w4a16_pack_table(void* out, const void* in, int64_t n, int64_
   b2l_launch(w4_pack_table_kernel, dim3(blocks), dim3(256), 0, (cudaStream_t)stream, (float*)out, (const float*)in, n,
              groups, row_stride, col_stride, tiles);
   B2L_LAUNCH_CHECK();
-  return B2L_OK;
+  return b2l_weights_written(stream);
 }
 
 extern "C" int b2l_w8a16_matmul(void* y, const void* x, const void* qweight, int weight_is_fp8, const void* scales,

@@ -86,6 +86,12 @@ def unrows(y: torch.Tensor, like: torch.Tensor) -> torch.Tensor:
     return y if like.dim() == 2 else y.view(*like.shape[:-1], y.shape[-1])
 
 
+def weights_written() -> None:
+    """Between the conversion or copy of a weight-side tensor and a GEMM that reads it: the GEMMs request their weights before
+    the previous kernel has finished (csrc/common.cuh, programmatic dependent launch)."""
+    check(lib().b2l_weights_written(stream_handle()))
+
+
 @functools.lru_cache(maxsize=4096)
 def quant_gemm_workspace_bytes(kind: int, m: int, n: int, k: int, group: int, device: int) -> int:
     """Workspace of a quantised GEMM: a function of the sizes and the device's SM count."""

@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from ._common import as_rows, check, counters, dtype_code, float_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, workspace
+from ._common import as_rows, check, counters, dtype_code, float_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, weights_written, workspace
 
 
 @no_grad
@@ -25,6 +25,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
     if weight.stride(-1) != 1:
         weight = weight.contiguous()
+        weights_written()
     a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
         a = a.contiguous()

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, zeroed_workspace
+from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
 
 _Q_INT4 = 0
 
@@ -32,6 +32,7 @@ def w4a16_matmul(
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
     if k % group_size != 0:
         raise ValueError(f"K ({k}) must be a multiple of group_size ({group_size})")
+    given = qweight, scales, zeros
     if scales.dtype != torch.float32 or zeros.dtype != torch.float32:
         scales, zeros = scales.float(), zeros.float()
     if zeros.stride() != scales.stride():
@@ -39,6 +40,8 @@ def w4a16_matmul(
         scales = scales.contiguous()
     if qweight.stride(-1) != 1:
         qweight = qweight.contiguous()
+    if qweight is not given[0] or scales is not given[1] or zeros is not given[2]:
+        weights_written()
     a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
         a = a.contiguous()

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, zeroed_workspace
+from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
 
 _Q_FP8, _Q_INT8 = 1, 2
 
@@ -36,6 +36,7 @@ def w8a16_matmul(
         raise ValueError(f"group_k ({group_k}) must be a multiple of 128 unless it covers K")
     if scales.dtype != torch.float32:
         scales = scales.float()
+        weights_written()
     if scales.dim() == 1:
         scales = scales.unsqueeze(-1)
     a = as_rows(x)

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .._common import as_rows, check, counters, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, workspace
+from .._common import as_rows, check, counters, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, weights_written, workspace
 
 
 @no_grad
@@ -56,6 +56,7 @@ def smoothquant_matmul_prequant(
         a_scales = a_scales.float().contiguous()
     if qweight.stride(-1) != 1 or qweight.stride(0) % 16 != 0:
         qweight = qweight.contiguous()
+        weights_written()
     if bias is not None:
         bias = bias.float().contiguous()
     out = torch.empty((m, n), dtype=out_dtype, device=qa.device)
