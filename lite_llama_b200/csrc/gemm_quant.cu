@@ -78,19 +78,8 @@ struct QuantParams {
   int aligned;                             // no segment spans two raw blocks (two MMA warps may alternate blocks)
   int zeros_foldable;                      // packed layout: the packer verified that every zero point is an integer in [0, 1023]
   int swiglu;                              // epilogue: rows are (gate_i, up_i) pairs; y[m, i] = silu(gate) * up (N/2 columns)
-  long long* timeline;                     // debug: [16][256] clock64 stamps of CTA (0,0,0), or null
-  int debug;                               // debug experiments (timing only, results are wrong): see DBG_*
+  long long* timeline;                     // B2L_TLITE builds: [CTA][32] clock64 stamps, or null
 };
-// DBG_RAW_OPERAND: skip the int4 -> fp16 arithmetic (operand = raw bits): how much of the time is the ALU pipe?
-// DBG_PAIR_K4: extract nibble pairs (k, k+4) with one LOP3 + HFMA2 each (5 ALU-pipe instructions per word instead
-// of 8) WITHOUT permuting the activations -- prices a pre-shuffled activation layout.  DBG_NO_STREAMK: host side.
-// DBG_SKIP_DRAIN: only the last segment of a piece is read back from TMEM (prices a scale-folded operand).
-enum { DBG_FORCE_XSUM = 8, DBG_RAW_OPERAND = 16, DBG_PAIR_K4 = 32, DBG_NO_STREAMK = 64, DBG_SKIP_DRAIN = 128,
-       DBG_FEW_MMA = 256 /* issue 1 of every 4 MMAs */, DBG_NO_STTM = 512 /* skip the TMEM operand store */,
-       DBG_WAIT_SPIN = 1024 /* mbarrier.test_wait polling */, DBG_WAIT_SHORT = 2048 /* try_wait without the long suspend hint */,
-       DBG_NO_XLOAD = 4096 /* activation tiles are never fetched */, DBG_HALF_RING = 8192 /* half the weight ring depth */,
-       DBG_LEGACY_OPRING = 16384 /* round-1 operand-ring indexing (phase-aliasing hang repro; results may be wrong) */,
-       DBG_FORCE = 32768 /* no experiment: just run the DBG instantiation (prices its code size) */ };
 // Wait flavour of the hand-off barriers (0: try_wait with the long suspend hint, 1: test_wait polling, 2: try_wait
 // with the default suspend window).  B2L_QWAIT_MODE covers every wait, B2L_QWAIT_LAT_MODE the latency-critical
 // ones (operand stage full / free, accumulator full): A/B builds, see tools/build_variants.py.
@@ -105,35 +94,22 @@ enum { DBG_FORCE_XSUM = 8, DBG_RAW_OPERAND = 16, DBG_PAIR_K4 = 32, DBG_NO_STREAM
 #define B2L_DQ_ORDER 0
 #endif
 template <int MODE>
-__device__ __forceinline__ void qwait_at(uint64_t* bar, uint32_t parity, int debug, int line) {
+__device__ __forceinline__ void qwait_at(uint64_t* bar, uint32_t parity, int line) {
   constexpr unsigned int fh = b2l_file_hash(__FILE__);
-  if ((debug & DBG_WAIT_SPIN) || MODE == 1) mbar_wait_spin_at(bar, parity, fh, line);
-  else if ((debug & DBG_WAIT_SHORT) || MODE == 2) mbar_wait_short_at(bar, parity, fh, line);
+  if (MODE == 1) mbar_wait_spin_at(bar, parity, fh, line);
+  else if (MODE == 2) mbar_wait_short_at(bar, parity, fh, line);
   else mbar_wait_at(bar, parity, fh, line);
 }
-#define qwait(bar, parity, debug) qwait_at<B2L_QWAIT_MODE>((bar), (parity), (debug), __LINE__)
-#define qwait_lat(bar, parity, debug) qwait_at<B2L_QWAIT_LAT_MODE>((bar), (parity), (debug), __LINE__)
-constexpr int kTlCta = 4096;    // timeline: [1024][3] per-CTA {globaltimer at entry, at exit, SM id}
-constexpr int kTlSub = 3072 + 32;   // timeline: [96][5] per-sub-block stamps of dequant warp 0
-constexpr int kTlMisc = 3072;   // timeline: start-up / shutdown stamps of CTA (0,0,0), see tools/timeline.py
-
-// B2L_TLITE (A/B builds only, tools/build_variants.py): a handful of clock stamps per CTA in the PRODUCT instantiation
-// (the DBG instantiation's own bookkeeping makes it ~50 % slower, so its timeline misplaces the critical path)
+#define qwait(bar, parity) qwait_at<B2L_QWAIT_MODE>((bar), (parity), __LINE__)
+#define qwait_lat(bar, parity) qwait_at<B2L_QWAIT_LAT_MODE>((bar), (parity), __LINE__)
+// B2L_TLITE (A/B builds only, tools/build_variants.py): a handful of clock stamps per CTA
 #ifdef B2L_TLITE
 #define LT(i) do { if (p.timeline) p.timeline[(size_t)blockIdx.x * 32 + (i)] = clock64(); } while (0)
 #else
 #define LT(i) do {} while (0)
 #endif
 
-// role rows of the debug timeline
-enum { TL_PROD = 0, TL_MMA_READY = 1, TL_MMA_ISSUED = 2, TL_DQ_START = 3, TL_DQ_DONE = 4, TL_EPI_START = 5, TL_EPI_DONE = 6 };
-#define TL_STAMP(role, idx)                                                                   \
-  do {                                                                                        \
-    if (tl && (idx) < 256 && lane == 0) tl[(role) * 256 + (idx)] = clock64();                 \
-  } while (0)
-
-static long long* g_timeline = nullptr;   // set through b2l_debug_set_timeline (tools/timeline.py)
-static int g_debug = 0;                   // b2l_debug_set_flags
+static long long* g_timeline = nullptr;   // set through b2l_debug_set_timeline (tools/tlite.py)
 
 struct __align__(8) QControl {
   uint64_t w_full[kMaxRawStages];
@@ -240,21 +216,15 @@ __device__ __forceinline__ void st_release_smem(int* p, int v) {
 // Operand-ring slot of operand stage `sp` (0 .. SUBST-1) of raw block `rb`.  The ring is split into two halves of
 // NST/2 stages: even raw blocks (dequant warps 0-3, MMA warp 0) cycle through the first half, odd raw blocks
 // (dequant warps 4-7, MMA warp 1) through the second.  Every op_full / op_empty barrier is then produced and
-// waited on by ONE dequant group and ONE MMA warp which both see every one of its phases in order.  (Round 1
-// indexed the ring as (2*rb + sp) % 6: a stage alternated between the two groups, so a waiter skipped every
-// other phase of "its" barrier and a parity wait could be satisfied by the completion of the phase BEFORE the
-// one it needed whenever one group ran a raw block ahead of the other -- stale operands, extra arrivals and,
-// eventually, a dead-locked pipeline: the intermittent decode hangs at 16- and 32-token tiles.)
+// waited on by ONE dequant group and ONE MMA warp which both see every one of its phases in order.  (With the
+// ring indexed as (2*rb + sp) % 6 a stage alternates between the two groups, so a waiter skips every
+// other phase of "its" barrier and a parity wait can be satisfied by the completion of the phase BEFORE the
+// one it needs whenever one group runs a raw block ahead of the other -- stale operands, extra arrivals and,
+// eventually, a dead-locked pipeline at 16- and 32-token tiles.)
 template <int NST, int SUBST>
-__device__ __forceinline__ void op_slot(int rb, int sp, int& stage, uint32_t& parity, int debug) {
+__device__ __forceinline__ void op_slot(int rb, int sp, int& stage, uint32_t& parity) {
   constexpr int H = NST / 2;
   static_assert(NST % 2 == 0 && H >= 1, "operand ring must split into two halves");
-  if (debug & DBG_LEGACY_OPRING) {            // round-1 indexing, kept in the DBG instantiation to reproduce the hang
-    const int gst = rb * SUBST + sp;
-    stage = gst % NST;
-    parity = (uint32_t)(gst / NST) & 1u;
-    return;
-  }
   const int u = (rb >> 1) * SUBST + sp;       // running operand-stage count of this raw block's group
   const int q = u / H;
   stage = (rb & 1) * H + (u - q * H);
@@ -263,7 +233,7 @@ __device__ __forceinline__ void op_slot(int rb, int sp, int& stage, uint32_t& pa
 
 template <int QK, int BT, int NST, int SPS>
 __device__ __forceinline__ void issue_block(QControl* ctl, uint32_t tmem_base, uint32_t a_base, uint64_t bdesc0,
-                                            int seg0, int rb, uint64_t* x_empty, int debug) {
+                                            int seg0, int rb, uint64_t* x_empty) {
   constexpr int RW = raw_sub<QK>();
   constexpr int NB = 4;
   constexpr int kXBytes = BT * kStageKBytes;
@@ -271,12 +241,12 @@ __device__ __forceinline__ void issue_block(QControl* ctl, uint32_t tmem_base, u
 #pragma unroll
   for (int sp = 0; sp < RW / 2; ++sp) {
     int ostage; uint32_t oparity;
-    op_slot<NST, RW / 2>(rb, sp, ostage, oparity, debug);
+    op_slot<NST, RW / 2>(rb, sp, ostage, oparity);
     // segments touched by this stage: sub-blocks 2sp and 2sp+1
     const int segA = seg0 + (2 * sp) / SPS, segB = seg0 + (2 * sp + 1) / SPS;
-    if ((2 * sp) % SPS == 0) qwait(&ctl->acc_empty[segA & (NB - 1)], ((segA / NB) & 1) ^ 1, debug);
-    if (SPS == 1) qwait(&ctl->acc_empty[segB & (NB - 1)], ((segB / NB) & 1) ^ 1, debug);
-    qwait_lat(&ctl->op_full[ostage], oparity, debug);
+    if ((2 * sp) % SPS == 0) qwait(&ctl->acc_empty[segA & (NB - 1)], ((segA / NB) & 1) ^ 1);
+    if (SPS == 1) qwait(&ctl->acc_empty[segB & (NB - 1)], ((segB / NB) & 1) ^ 1);
+    qwait_lat(&ctl->op_full[ostage], oparity);
     tc_fence_after();
     if (elect_one()) {
       const uint32_t a_addr = a_base + ostage * 64;
@@ -288,8 +258,7 @@ __device__ __forceinline__ void issue_block(QControl* ctl, uint32_t tmem_base, u
         const uint64_t bd = bdesc0 + (uint64_t)((sub * kXBytes) >> 4);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-          if (!(debug & DBG_FEW_MMA) || j == 3)
-            umma_f16_ts(d, a_addr + h * 32 + j * 8, bd + 2 * j, idesc, (sub % SPS != 0 || j > 0) ? 1u : 0u);
+          umma_f16_ts(d, a_addr + h * 32 + j * 8, bd + 2 * j, idesc, (sub % SPS != 0 || j > 0) ? 1u : 0u);
         if (sub % SPS == SPS - 1) tc_commit(&ctl->acc_full[sseg & (NB - 1)]);
       }
       tc_commit(&ctl->op_empty[ostage]);
@@ -304,7 +273,7 @@ __device__ __forceinline__ void issue_block(QControl* ctl, uint32_t tmem_base, u
 // rows] so that a CTA's share is one contiguous bulk copy per piece).
 // EPI: 0 = store the projection; 1 = SiLU(gate) * up over row-interleaved gate|up weights (its own instantiation: the
 // activation code unrolled over the token tile grew the kernel by ~10 % and that alone slowed every GEMM, profiles/).
-template <int QK, int BT, bool DBG, int LAYOUT, int EPI = 0>
+template <int QK, int BT, int LAYOUT, int EPI = 0>
 __global__ void __launch_bounds__(kQuantThreads, 1)
 gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                   const QuantParams p) {
@@ -312,10 +281,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   constexpr int OPS = op_stages_for(BT);
   constexpr int kOpStages = OPS;
   constexpr int TP = LAYOUT == 1 ? kBlockW : kTabPitch;   // floats per table column
-  // the debug experiments and the timeline stamps only exist in the DBG instantiation (selected by the host when a
-  // debug flag or a timeline buffer is set): the product kernel carries none of their code
-  const int debug = DBG ? p.debug : 0;
-  long long* const timeline = DBG ? p.timeline : nullptr;
   // first thing: the TMA unit starts fetching the weight descriptor while the CTA works out its range (the first
   // weight request otherwise waits for the descriptor AND for the data: two dependent trips to memory)
   if (threadIdx.x == kWarpWProd * 32) tma_prefetch_desc(&tmap_w);
@@ -353,7 +318,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m_tile = blockIdx.y;
-  long long* tl = (timeline && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) ? timeline : nullptr;
   const int seg_len = p.group_k;                  // K elements per scale group (multiple of 16)
   // ---- this CTA's work: pieces (tile, raw-block range); see struct Piece ----
   WorkRange wr;
@@ -387,7 +351,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   // two MMA warps (alternate raw blocks) when no segment spans two raw blocks, else warp 1 alone
   const int mma_warps = p.aligned ? 2 : 1;
 
-  if (tl && threadIdx.x == 0) tl[kTlMisc + 0] = clock64();
 #ifdef B2L_TLITE
   if (threadIdx.x == 0) {
     LT(0);
@@ -400,23 +363,13 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     }
   }
 #endif
-  // every CTA: wall-clock (globaltimer, ns) at entry and exit + its SM id -> who is the straggler, and what is the
-  // real SM clock (CTA 0 also stamps clock64 at both ends)
-  if (timeline && threadIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && blockIdx.x < 1024) {
-    unsigned long long gt; unsigned smid;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-    timeline[kTlCta + 3 * blockIdx.x] = (long long)gt;
-    timeline[kTlCta + 3 * blockIdx.x + 2] = (long long)smid;
-  }
-
   // weight producer state (warp kWarpWProd): the first ring-full of TMA loads is issued BEFORE the set-up barrier
   PipeState ws(p.w_stages);
   int w_pi = 0, w_lin = 0;
   Piece w_pc = wr.piece(0);
   int w_rb = w_pc.rb_lo;
   auto w_issue = [&](bool wait) {
-    if (wait) qwait(&ctl->w_empty[ws.stage], ws.phase ^ 1, debug);
+    if (wait) qwait(&ctl->w_empty[ws.stage], ws.phase ^ 1);
     if (elect_one()) {
       mbar_arrive_expect_tx(&ctl->w_full[ws.stage], kABytes);     // OOB parts are zero-filled but still counted
       const int kb = w_rb * RW;                                      // first 64-element k-block of this raw block
@@ -424,14 +377,13 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
                        w_pc.n_tile * kBlockW, &ctl->w_full[ws.stage], kEvictFirst);
     }
     __syncwarp();
-    TL_STAMP(TL_PROD, w_lin);
     ws.advance();
     ++w_lin;
     if (++w_rb == w_pc.rb_hi && w_lin < nrb) { w_pc = wr.piece(++w_pi); w_rb = w_pc.rb_lo; }
   };
 
   // int4: this thread saw a zero point that cannot be folded (or the group size rules folding out altogether)
-  int bad_zero = (QK == Q_INT4 && (p.force_xsum || (debug & DBG_FORCE_XSUM) || (LAYOUT == 1 && !p.zeros_foldable))) ? 1 : 0;
+  int bad_zero = (QK == Q_INT4 && (p.force_xsum || (LAYOUT == 1 && !p.zeros_foldable))) ? 1 : 0;
   constexpr int kFillWarps = kWarpEpi0 + 4;
   if (LAYOUT == 0 && warp < kFillWarps) {
     // ---- warps 0..11 (idle until the first weights land): stage the scale / zero-point table ----
@@ -513,7 +465,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         }
       }
     }
-    if (tl && warp == kWarpEpi0 && lane == 0) tl[kTlMisc + 7] = clock64();
   }
 
   if (LAYOUT == 1 && warp == kWarpXProd && lane == 0) {
@@ -567,7 +518,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       mbar_fence_init();
       fence_proxy_async_smem();
       LT(26);
-      if (tl) tl[kTlMisc + 8] = clock64();
     }
     __syncwarp();
     // Weights are static: under programmatic dependent launch this stream starts while the previous kernel is
@@ -603,15 +553,12 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     // could take the SM's TMEM columns and park in griddepcontrol.wait for this grid, while this CTA blocks in
     // tcgen05.alloc (dead-lock).  No other warp triggers, so the CTA counts as triggered only from here on.
     pdl_launch_dependents();
-    if (tl && lane == 0) tl[kTlMisc + 9] = clock64();
   }
-  if (tl && threadIdx.x == 0) tl[kTlMisc + 10] = clock64();
   tc_fence_before();
   // the set-up barrier also publishes the table and ORs the "zero point cannot be folded" flags of the fill threads
   const bool cta_need_xsum = __syncthreads_or(bad_zero) != 0;
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  if (tl && threadIdx.x == 0) tl[kTlMisc + 1] = clock64();
   if (threadIdx.x == 0) LT(2);
 
   if (warp == kWarpWProd) {
@@ -625,10 +572,8 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int pi = 0; pi < wr.npieces; ++pi) {
       const Piece pc = wr.piece(pi);
       for (int rb = pc.rb_lo; rb < pc.rb_hi; ++rb) {
-        qwait(&ctl->x_empty[xs.stage], xs.phase ^ 1, debug);
-        if (debug & DBG_NO_XLOAD) {
-          if (elect_one()) mbar_arrive(&ctl->x_full[xs.stage]);
-        } else if (elect_one()) {
+        qwait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
+        if (elect_one()) {
           mbar_arrive_expect_tx(&ctl->x_full[xs.stage], kXStage);
           const int kb = rb * RW;
 #pragma unroll
@@ -657,10 +602,8 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       uint32_t rphase = (mma_idx / p.x_stages) & 1;
       for (int rb = mma_idx; rb < nrb; rb += mma_warps) {
         const int gsub0 = rb * RW;                                       // first operand sub-block of this raw block
-        TL_STAMP(7, rb);
-        qwait(&ctl->x_full[rstage], rphase, debug);                         // activation sub-tiles (TMA)
+        qwait(&ctl->x_full[rstage], rphase);                         // activation sub-tiles (TMA)
         tc_fence_after();
-        TL_STAMP(TL_MMA_READY, rb);
         if (rb == 0 && lane == 0) LT(4);
         int steps_here = steps_total - rb * (RW * 4);
         if (steps_here > RW * 4) steps_here = RW * 4;
@@ -674,23 +617,23 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         if (mma_warps == 2 && steps_here == RW * 4) {
           // aligned mode: the raw block holds 1 or 2 whole segments
           if (seg_steps == RW * 4)
-            issue_block<QK, BT, OPS, RW>(ctl, tmem_base, a_base, bdesc0, seg, rb, &ctl->x_empty[rstage], debug);
+            issue_block<QK, BT, OPS, RW>(ctl, tmem_base, a_base, bdesc0, seg, rb, &ctl->x_empty[rstage]);
           else
-            issue_block<QK, BT, OPS, RW / 2>(ctl, tmem_base, a_base, bdesc0, seg, rb, &ctl->x_empty[rstage], debug);
+            issue_block<QK, BT, OPS, RW / 2>(ctl, tmem_base, a_base, bdesc0, seg, rb, &ctl->x_empty[rstage]);
         } else if (elect_one()) {
 #pragma unroll
           for (int st = 0; st < RW * 4; ++st) {
             if (st < steps_here) {
               const int buf = seg % NB;
               int ostage; uint32_t oparity;                      // operand stage = two sub-blocks
-              op_slot<kOpStages, RW / 2>(rb, st >> 3, ostage, oparity, debug);
+              op_slot<kOpStages, RW / 2>(rb, st >> 3, ostage, oparity);
               if ((st & 7) == 0) {
-                qwait_lat(&ctl->op_full[ostage], oparity, debug);   // dequantised stage
+                qwait_lat(&ctl->op_full[ostage], oparity);   // dequantised stage
                 tc_fence_after();
               }
               if (!seg_open) {
                 // accumulator buffer `buf` must have been drained (segment seg-NB) by all four epilogue warps
-                qwait(&ctl->acc_empty[buf], ((seg / NB) & 1) ^ 1, debug);
+                qwait(&ctl->acc_empty[buf], ((seg / NB) & 1) ^ 1);
                 tc_fence_after();
               }
               const uint64_t bdesc = bdesc0 + (uint64_t)(((st >> 2) * kXBytes) >> 4) + 2 * (st & 3);
@@ -712,7 +655,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           tc_commit(&ctl->x_empty[rstage]);
         }
         __syncwarp();
-        TL_STAMP(TL_MMA_ISSUED, rb);
         if (rb == 0 && lane == 0) LT(5);
         if (rb + mma_warps >= nrb && lane == 0) LT(6 + mma_idx);
         rstage += mma_warps;
@@ -753,7 +695,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     }
     if (LAYOUT == 1) mbar_wait(&ctl->tab_full, 0);
     if (need_xsum) pdl_wait_prior();   // the fallback reads the activations (the previous kernel's output) from global
-    if (tl && warp == kWarpEpi0 && lane == 0) tl[kTlMisc + 3] = clock64();
     constexpr int PARTS = 128 / BT;
     const int xs_m = epi_tid / PARTS, xs_part = epi_tid % PARTS;
     T* y = reinterpret_cast<T*>(p.y);
@@ -821,17 +762,9 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         const float sc = lds_f32(scale_tab + tcol * TP + epi_tid);        // rows past N hold zeros
         float zp = 0.f;
         if (QK == Q_INT4 && need_xsum) zp = lds_f32(zero_tab + tcol * TP + epi_tid);
-        qwait_lat(&ctl->acc_full[buf], (seg / NB) & 1, debug);
+        qwait_lat(&ctl->acc_full[buf], (seg / NB) & 1);
         tc_fence_after();
-        if (warp == kWarpEpi0) TL_STAMP(TL_EPI_START, seg);
         if (warp == kWarpEpi0 && lane == 0 && seg == 0) LT(12);
-        if ((debug & DBG_SKIP_DRAIN) && k_next < k_lim) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&ctl->acc_empty[buf]);
-          k_pos = k_next; k_group_end += seg_len; ++tcol; ++seg;
-          continue;
-        }
         const uint32_t ta = taddr + buf * BT;
         constexpr int CH = BT < 32 ? BT : 32;                  // columns drained per tcgen05.wait::ld
         const float4* xs4 = reinterpret_cast<const float4*>(xs_smem + (seg & 1) * BT);
@@ -862,7 +795,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
             for (int j = 0; j < CH; ++j) acc[c0 + j] = fmaf(sc, __uint_as_float(pv[j]), acc[c0 + j]);
           }
         }
-        if (warp == kWarpEpi0) TL_STAMP(TL_EPI_DONE, seg);
         k_pos = k_next;
         k_group_end += seg_len;
         ++tcol;
@@ -870,7 +802,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
 
       // ---- the piece is complete: write the tile, or hand the partial sum to the tile's last finisher ----
-      if (tl && warp == kWarpEpi0 && lane == 0 && pi == wr.npieces - 1) tl[kTlMisc + 5] = clock64();
       if (warp == kWarpEpi0 && lane == 0 && pi == wr.npieces - 1) LT(13);
       pdl_wait_prior();              // output / workspace buffers may still be in use by the previous kernel
       auto store_final = [&]() {
@@ -990,7 +921,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     const int g_last = (k_begin + steps_total * 16 - 1) / seg_len - k_begin / seg_len;
     if (QK == Q_INT4) fold_zero = !cta_need_xsum;
     if (LAYOUT == 1) mbar_wait(&ctl->tab_full, 0);
-    if (tl && warp == 0 && lane == 0) tl[kTlMisc + 4] = clock64();
     // ring position of this group's next raw block, advanced by 2 per iteration (ring depths are even, so no
     // integer division -- it cost ~30 ALU-pipe instructions per raw block on the pipe that bounds this kernel)
     int rstage = half;
@@ -1019,7 +949,7 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           }
         }
       }
-      qwait(&ctl->w_full[rstage], rphase, debug);
+      qwait(&ctl->w_full[rstage], rphase);
       const uint8_t* rawrow = w_ring + (size_t)rstage * kABytes + row * 128;
       uint4 raw[8];                                          // the row's 128 raw bytes (8 swizzled 16-byte chunks)
 #pragma unroll
@@ -1027,10 +957,9 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       // The weight stage is handed back to the TMA producer at the END of this block, not here: at this point the
       // loads have been issued, not returned, and nothing that follows depends on them until the conversion --
       // a refill that found its weights in L2 could land in the stage first (rows are written in order, so the
-      // lowest rows of a tile were the ones hit).  Found in round 2 by tests/test_kernels_gpu.py::
+      // lowest rows of a tile were the ones hit).  Found by tests/test_kernels_gpu.py::
       // test_w4a16_streamk_back_to_back_launches_are_isolated at 33-64 tokens: ~10 % of the launches over a long-K
       // shape had one or a few output columns off by one scale group's contribution (tools/nondet_probe.py).
-      if (quad == 0) TL_STAMP(TL_DQ_START, rb);
       if (warp == 0 && lane == 0 && rb == 0) LT(8);
       // one operand sub-stage per 64-element sub-block; the "sub-block ready" arrive of sub-block s is issued
       // after the conversion of s+1, so tcgen05.wait::st never waits for a store that was just issued
@@ -1039,26 +968,18 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       for (int sub = 0; sub < RW; ++sub) {
         const int gsub = rb * RW + sub;
         constexpr int CPS = 8 / RW;                            // 16-byte chunks of the row per sub-block
-        // DBG: five clock stamps per sub-block of warp 0 (loop top, operand stage free, converted, previous store
-        // retired + announced, store issued): tools/timeline.py prints the phase lengths
-        long long* const tls = (DBG && tl && warp == 0 && lane == 0 && gsub < 96) ? tl + kTlSub + gsub * 5 : nullptr;
-        if (tls) tls[0] = clock64();
         if (gsub < nsub_total) {                               // sub-blocks past the k-range have no MMA step
           int ostage; uint32_t oparity;                        // operand stage = sub-blocks (2i, 2i+1); rb * RW is even
-          op_slot<kOpStages, RW / 2>(rb, sub >> 1, ostage, oparity, debug);
+          op_slot<kOpStages, RW / 2>(rb, sub >> 1, ostage, oparity);
           if (B2L_DQ_ORDER == 0 && (sub & 1) == 0) {
-            qwait_lat(&ctl->op_empty[ostage], oparity ^ 1, debug);
+            qwait_lat(&ctl->op_empty[ostage], oparity ^ 1);
             tc_fence_after();
           }
-          if (tls) tls[1] = clock64();
           uint32_t vals[32];
           if (QK == Q_INT4) {
             const uint4 w0 = raw[sub * CPS], w1 = raw[sub * CPS + CPS - 1];
             const uint32_t ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-            if (debug & DBG_RAW_OPERAND) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) { vals[4 * j] = ws[j]; vals[4 * j + 1] = ws[j] ^ 1u; vals[4 * j + 2] = ws[j] ^ 2u; vals[4 * j + 3] = ws[j] ^ 3u; }
-            } else if (LAYOUT == 1) {
+            if (LAYOUT == 1) {
 #pragma unroll
               for (int j = 0; j < 8; ++j) dequant_int4_packed(ws[j], add_lo[sub], add_hi[sub], vals + 4 * j);
             } else {
@@ -1074,11 +995,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
               for (int j = 0; j < 4; ++j) dequant_w8_word(ws[j], QK == Q_FP8, vals + 8 * c + 2 * j);
             }
           }
-          if (tls) {
-            long long t;
-            asm volatile("mov.u64 %0, %%clock64;" : "=l"(t) : "r"(vals[0]), "r"(vals[15]), "r"(vals[31]) : "memory");
-            tls[2] = t;
-          }
           // the previous stage is announced after the conversion of this stage's first half: by then its
           // tcgen05.st have retired and tcgen05.wait::st does not wait
           if ((sub & 1) == 0 && pending >= 0) {
@@ -1091,13 +1007,10 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           // the operand stage is only needed for the store: waiting for it here, after the conversion and after the
           // previous stage has been announced, keeps a late stage from delaying either
           if (B2L_DQ_ORDER == 1 && (sub & 1) == 0) {
-            qwait_lat(&ctl->op_empty[ostage], oparity ^ 1, debug);
+            qwait_lat(&ctl->op_empty[ostage], oparity ^ 1);
             tc_fence_after();
           }
-          if (tls) tls[3] = clock64();
-          if (!(debug & DBG_NO_STTM)) tmem_st_32x32b_x32(lane_base + kAColBase + ostage * 64 + (sub & 1) * 32, vals);
-          else asm volatile("" ::"r"(vals[0] ^ vals[7] ^ vals[13] ^ vals[31]));
-          if (tls) tls[4] = clock64();
+          tmem_st_32x32b_x32(lane_base + kAColBase + ostage * 64 + (sub & 1) * 32, vals);
           if ((sub & 1) == 1 || gsub == nsub_total - 1) pending = ostage;
         }
       }
@@ -1110,7 +1023,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       // every raw word has been converted: the stage can be refilled
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl->w_empty[rstage]);
-      if (quad == 0) TL_STAMP(TL_DQ_DONE, rb);
       if (warp == 0 && lane == 0 && rb == 0) LT(9);
       if (quad == 0 && lane == 0 && rb + 2 >= nrb) LT(10 + half);
       rstage += 2;
@@ -1267,12 +1179,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       }
     }
   }
-  if (tl && threadIdx.x == 0) tl[kTlMisc + 6] = clock64();
-  if (timeline && threadIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && blockIdx.x < 1024) {
-    unsigned long long gt;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(gt));
-    timeline[kTlCta + 3 * blockIdx.x + 1] = (long long)gt;
-  }
 #ifdef B2L_TLITE
   if (threadIdx.x == 0 && p.timeline) {
     LT(20);
@@ -1350,7 +1256,7 @@ static inline SplitPlan quant_plan(int qk, int64_t M, int64_t N, int64_t K, int 
   {
     const int raw_k = qk == Q_INT4 ? 256 : 128;
     const bool aligned = raw_k % seg_len == 0 && raw_k / seg_len <= 2;     // same rule as QuantParams::aligned
-    if (streamk_enabled() && !(g_debug & DBG_NO_STREAMK) && aligned && K % raw_k == 0 && pl.m_tiles == 1 &&
+    if (streamk_enabled() && aligned && K % raw_k == 0 && pl.m_tiles == 1 &&
         (int64_t)pl.n_tiles * (K / raw_k) < (1 << 22)) {        // the kernel's range arithmetic is 32-bit: total * (ctas + 1)
       const int nrb_tile = (int)(K / raw_k);
       const int64_t total = (int64_t)pl.n_tiles * nrb_tile;
@@ -1403,10 +1309,10 @@ static inline int env_int(const char* name, int dflt) {
   return e && e[0] ? atoi(e) : dflt;
 }
 
-template <int QK, int BT, bool DBG, int LAYOUT, int EPI = 0>
+template <int QK, int BT, int LAYOUT, int EPI = 0>
 static int launch_q_inst(const CUtensorMap& tw, const CUtensorMap& tx, const QuantParams& p, const SplitPlan& pl,
                          cudaStream_t st) {
-  auto kern = gemm_quant_kernel<QK, BT, DBG, LAYOUT, EPI>;
+  auto kern = gemm_quant_kernel<QK, BT, LAYOUT, EPI>;
   static int configured_smem[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, pl.smem_bytes, configured_smem));
   dim3 grid((unsigned)pl.n_tiles, (unsigned)pl.m_tiles, (unsigned)pl.splits);
@@ -1419,21 +1325,11 @@ static int launch_q_inst(const CUtensorMap& tw, const CUtensorMap& tx, const Qua
 template <int QK, int BT>
 static int launch_q_bt(const CUtensorMap& tw, const CUtensorMap& tx, const QuantParams& p, const SplitPlan& pl,
                        cudaStream_t st, int layout) {
-#ifdef B2L_TLITE
-  const bool dbg = p.debug != 0;
-#else
-  const bool dbg = p.debug != 0 || p.timeline != nullptr;
-#endif
   if constexpr (QK == Q_INT4) {
-    if (layout == 1) {
-      if (p.swiglu) {
-        B2L_REQUIRE(!dbg, "w4a16_matmul_packed: the swiglu epilogue has no debug instantiation");
-        return launch_q_inst<QK, BT, false, 1, 1>(tw, tx, p, pl, st);
-      }
-      return dbg ? launch_q_inst<QK, BT, true, 1>(tw, tx, p, pl, st) : launch_q_inst<QK, BT, false, 1>(tw, tx, p, pl, st);
-    }
+    if (layout == 1)
+      return p.swiglu ? launch_q_inst<QK, BT, 1, 1>(tw, tx, p, pl, st) : launch_q_inst<QK, BT, 1>(tw, tx, p, pl, st);
   }
-  return dbg ? launch_q_inst<QK, BT, true, 0>(tw, tx, p, pl, st) : launch_q_inst<QK, BT, false, 0>(tw, tx, p, pl, st);
+  return launch_q_inst<QK, BT, 0>(tw, tx, p, pl, st);
 }
 
 template <int QK>
@@ -1455,9 +1351,7 @@ static int quant_common(int qk, QuantParams& p, SplitPlan& pl, void* y, const vo
   p.sk_ctas = pl.sk_ctas; p.sk_slots = pl.sk_slots; p.nrb_tile = pl.nrb_tile; p.n_tiles = pl.n_tiles;
   p.y = y; p.ldy = y_row_stride; p.M = (int)m; p.N = (int)n; p.K = (int)k;
   p.splits = pl.splits; p.kb_per_split = pl.kb_per_split; p.num_kb = pl.num_kb; p.w_stages = pl.stages; p.x_stages = pl.x_stages;
-  if ((g_debug & DBG_HALF_RING) && p.w_stages >= 4) p.w_stages = (p.w_stages / 2) & ~1;
   p.timeline = g_timeline;
-  p.debug = g_debug;
   p.swiglu = 0;
   p.zeros_foldable = 0;
   p.x = x; p.ldx = x_row_stride;
@@ -1504,18 +1398,11 @@ static inline int seg_len_for(int kind, int64_t k, int64_t group_k) {
   return (int)((gk + 15) / 16 * 16);
 }
 
-// Debug hook: device buffer of 8*256 int64 receiving clock64 stamps from CTA (0,0,0) of the next quantised
-// GEMM launches (null disables).  Not part of the product path.
+// B2L_TLITE builds: device buffer of 32 int64 per CTA for the clock stamps of the next launches (null disables).
 extern "C" int b2l_debug_set_timeline(void* device_buffer) {
   gemm::g_timeline = (long long*)device_buffer;
   return B2L_OK;
 }
-// DBG_* experiments: any non-zero flag runs the DBG instantiation of the kernel
-extern "C" int b2l_debug_set_flags(int flags) {
-  gemm::g_debug = flags & 0xFFFF;
-  return B2L_OK;
-}
-
 extern "C" int64_t b2l_quant_gemm_workspace_bytes(int kind, int64_t m, int64_t n, int64_t k, int64_t group_k) {
   if (m <= 0 || n <= 0 || k <= 0 || group_k <= 0) return 0;
   SplitPlan pl = quant_plan(kind, m, n, k, seg_len_for(kind, k, group_k));

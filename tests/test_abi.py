@@ -74,3 +74,14 @@ def test_shims_refuse_cpu_tensors():
         w4a16_matmul(x.float(), torch.zeros(8, 8, dtype=torch.int32), torch.ones(8, 1), torch.zeros(8, 1))
     with pytest.raises(ValueError, match="qweight must be int32"):
         w4a16_matmul(x, torch.zeros(8, 8, dtype=torch.int8), torch.ones(8, 1), torch.zeros(8, 1))
+
+
+def test_no_process_wide_switch_changes_what_a_remembered_workspace_was_for():
+    """The shims remember a quantised GEMM's workspace by its sizes alone; the plan behind it has no debug switch."""
+    from lite_llama_b200.kernels._common import quant_gemm_workspace_bytes
+
+    lib = _lib.load()
+    assert not hasattr(lib.cdll, "b2l_debug_set_flags")
+    for kind, m, n, k, group in [(0, 7, 28672, 4096, 128), (0, 32, 4096, 14336, 128), (1, 64, 6144, 4096, 128), (2, 3, 896, 4864, 4864)]:
+        for _ in range(2):
+            assert quant_gemm_workspace_bytes(kind, m, n, k, group, 0) == lib.b2l_quant_gemm_workspace_bytes(kind, m, n, k, group)

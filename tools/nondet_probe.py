@@ -9,7 +9,6 @@ ap = argparse.ArgumentParser()
 ap.add_argument("--m", type=int, default=36); ap.add_argument("--n", type=int, default=4096); ap.add_argument("--k", type=int, default=14336)
 ap.add_argument("--reps", type=int, default=200); ap.add_argument("--packed", type=int, default=1)
 ap.add_argument("--const-zp", type=int, default=0); ap.add_argument("--const-sc", type=int, default=0); ap.add_argument("--const-x", type=int, default=0)
-ap.add_argument("--flags", type=int, default=0, help="b2l_debug_set_flags (DBG instantiation; timing-only flags change the values but must stay deterministic)")
 a = ap.parse_args()
 torch.manual_seed(7)
 x = torch.randn(a.m, a.k, device="cuda", dtype=torch.float16) * 0.5
@@ -20,18 +19,13 @@ if a.const_zp: zp.fill_(8.0)
 if a.const_sc: sc.fill_(0.005)
 if a.const_x: x.fill_(0.25)
 pk = K.w4a16_pack(qw, sc, zp, group_size=128)
-if a.flags:
-    import ctypes
-    from lite_llama_b200 import _lib
-    L = _lib.load().cdll; L.b2l_debug_set_flags.argtypes = [ctypes.c_int]; L.b2l_debug_set_flags.restype = ctypes.c_int
-    L.b2l_debug_set_flags(a.flags)
 outs = []
 for _ in range(a.reps):
     y = K.w4a16_matmul_packed(x, pk) if a.packed else K.w4a16_matmul(x, qw, sc, zp, group_size=128)
     torch.cuda.synchronize()
     outs.append(y.clone())
 keys = collections.Counter(o.cpu().numpy().tobytes() for o in outs)
-print(f"m={a.m} n={a.n} k={a.k} packed={a.packed} flags={a.flags} const zp/sc/x={a.const_zp}{a.const_sc}{a.const_x}: {len(keys)} distinct results in {a.reps} launches; counts {sorted(keys.values(), reverse=True)[:6]}")
+print(f"m={a.m} n={a.n} k={a.k} packed={a.packed} const zp/sc/x={a.const_zp}{a.const_sc}{a.const_x}: {len(keys)} distinct results in {a.reps} launches; counts {sorted(keys.values(), reverse=True)[:6]}")
 ref = max(outs, key=lambda o: keys[o.cpu().numpy().tobytes()])
 shown = 0
 for i, o in enumerate(outs):

@@ -1,12 +1,11 @@
-"""A/B timing of the W4A16 GEMM at the Llama-3-8B projection shapes under the library's debug flags
-(b2l_debug_set_flags; gemm_quant.cu: DBG_*). Per-launch microseconds from a CUDA graph of `reps` launches over
-distinct weight tensors (working set >> L2), like bench.py's kernel breakdown. Timing-only flags give wrong results
-on purpose; they price an idea before it is built."""
+"""Timing of the W4A16 GEMM at the Llama-3-8B projection shapes, on the reference's tensors (base) and on the load-time
+repack (packed). Per-launch microseconds from a CUDA graph of `reps` launches over distinct weight tensors (working set >>
+L2), like bench.py's kernel breakdown. Up to 8 tokens that is csrc/gemm_quant_decode.cu, packed prompts run in
+csrc/gemm_quant_pair.cu, what lies between in csrc/gemm_quant.cu."""
 
 from __future__ import annotations
 
 import argparse
-import ctypes
 import json
 import sys
 from pathlib import Path
@@ -15,10 +14,8 @@ import torch
 
 sys.path.insert(0, str(Path(__file__).resolve().parent.parent))
 import lite_llama_b200.kernels as K  # noqa: E402
-from lite_llama_b200 import _lib  # noqa: E402
 
 SHAPES = {"qkv": (6144, 4096), "o": (4096, 4096), "gate_up": (28672, 4096), "down": (4096, 14336)}
-FLAGS = {"ops8": 65536, "segwait": 131072, "ops8+segwait": 196608, "dbg_inst": 32768, "noX": 4096, "halfring": 8192, "skipall": 144+768, "skipall+noX": 144+768+4096, "skipall+halfring": 144+768+8192, "spin": 1024, "short": 2048, "A+few_mma+no_sttm+spin": 144+768+1024, "A+few_mma+no_sttm+short": 144+768+2048, "no_streamk+spin": 64+1024, "no_streamk+short": 64+2048, "A": 144, "A+few_mma": 144 + 256, "A+no_sttm": 144 + 512, "A+few_mma+no_sttm": 144 + 768, "few_mma": 256, "no_sttm": 512, "skip_drain": 128, "skip_drain+raw": 144, "skip_drain+pair_k4": 160, "base": 0, "raw_operand": 16, "pair_k4": 32, "no_streamk": 64, "no_streamk+pair_k4": 96, "no_streamk+raw": 80}
 
 
 def main():
@@ -26,11 +23,8 @@ def main():
     ap.add_argument("--m", type=int, default=32)
     ap.add_argument("--reps", type=int, default=8)
     ap.add_argument("--shapes", default="qkv,o,gate_up,down")
-    ap.add_argument("--flags", default="base,no_streamk,pair_k4,raw_operand,no_streamk+pair_k4,no_streamk+raw")
+    ap.add_argument("--flags", default="base,packed", help="which layouts")
     a = ap.parse_args()
-    lib = _lib.load().cdll          # debug symbols are not part of the declared ABI
-    lib.b2l_debug_set_flags.argtypes = [ctypes.c_int]
-    lib.b2l_debug_set_flags.restype = ctypes.c_int
     dev = "cuda"
     ap2 = [x for x in a.shapes.split(",")]
     for name, (n, k) in SHAPES.items():
@@ -47,8 +41,7 @@ def main():
         row = {"shape": name, "m": a.m, "n": n, "k": k}
         packed = [K.w4a16_pack(qw, sc, zp, group_size=128) for qw, sc, zp in ws]
         for fname in a.flags.split(","):
-            use_packed = fname.startswith("packed")
-            lib.b2l_debug_set_flags(FLAGS[fname[7:] if fname.startswith("packed+") else ("base" if use_packed else fname)])
+            use_packed = fname == "packed"
 
             def fn():
                 if use_packed:
@@ -82,7 +75,6 @@ def main():
             row[fname] = round(us, 2)
             row[fname + "_gbs"] = round(nbytes / us / 1e3, 0)
             del g
-        lib.b2l_debug_set_flags(0)
         print(json.dumps(row), flush=True)
 
 
