@@ -1,6 +1,6 @@
 """A/B builds of the quantised GEMM: compiles csrc/gemm_quant.cu with -D knobs and links each against the other
 objects of the regular build into tools/variants/lib_<name>.so (git-ignored, travels to the GPU box).
-tools/run_variants.sh swaps each one in for libb200lite.so on the box and runs the probe. Not part of the product."""
+Copy one over libb200lite.so to run a probe on it. Not part of the product."""
 from __future__ import annotations
 
 import subprocess

@@ -1,11 +1,11 @@
 """Condense what a GPU pass left in gpurun_out/ into small text files under profiles/ (tracked).
 
-    python tools/keep_profiles.py r1b        # prefix for this round/pass
+    python tools/keep_profiles.py r1b        # file prefix
 
 * launches.csv (ncu --metrics gpu__time_duration.sum over `bench.py --steps 2 --warmup 1`): one decode step's
   launch list aggregated per kernel, with each kernel's SHARE of the step (per-launch times under ncu are
   cold-cache and serialised, so only shares are comparable with bench.py's live numbers).
-* *.ncu-rep (--set full captures): the handful of metrics DESIGN.md quotes (duration, DRAM bytes, throughput %,
+* *.ncu-rep (--set full captures): a handful of metrics (duration, DRAM bytes, throughput %,
   pipe utilisation, issue-slot use, stall reasons) per capture.
 * bench*.json: copied verbatim.
 """
