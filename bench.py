@@ -8,8 +8,6 @@ random-initialised with the named architecture's shapes (no checkpoints offline)
 synthetic token ids; a 128-token prefill fills the KV cache, then W warm-up and K timed decode steps
 run with contexts growing from 129. Every rank holds a full replica (data parallel, no collective:
 the path shards by independent sequences), so scaling is weak and `value` is the sum over ranks.
-
-JSON keys follow the driver contract; see DESIGN.md "Measurement" for what each figure means.
 """
 
 from __future__ import annotations
@@ -55,7 +53,7 @@ def parse_args():
                          "row-parallel projection; strong scaling, same global batch); dp = N independent replicas "
                          "(weak scaling, no collective)")
     ap.add_argument("--no-cpu-baseline", action="store_true")
-    ap.add_argument("--no-hf-baseline", action="store_true", help="skip the HF-transformers-on-CPU row (configs[0])")
+    ap.add_argument("--no-hf-baseline", action="store_true", help="skip the HF-transformers-on-CPU row")
     ap.add_argument("--watchdog-s", type=int, default=600, help="give up (exit 3) after this many seconds; 0 = never")
     ap.add_argument("--no-breakdown", action="store_true")
     ap.add_argument("--no-dp-line", action="store_true", help="N > 1, tp: skip the extra replica (weak-scaling) measurement")
@@ -68,8 +66,8 @@ def workload_config(args, world):
     return {
         "workload": f"{args.model} {'W4A16 g128' if args.quant == 'int4' else args.quant} greedy decode, "
                     f"batch {args.batch}{'' if tp else '/GPU'}, prompt {args.prompt_len} -> {args.steps} new tokens "
-                    + ("(BASELINE.json configs[2]; the metric's named config)"
-                       if (args.model, args.quant) == ("llama-3-8b", "int4") else "(a BASELINE.json side configuration)"),
+                    + ("(the headline configuration)"
+                       if (args.model, args.quant) == ("llama-3-8b", "int4") else "(a side configuration)"),
         "model": args.model, "quant": args.quant, "per_gpu_batch": args.batch,
         "global_batch": args.batch if tp else args.batch * world,
         "prompt_len": args.prompt_len, "parallelism": (f"tp{world}" if tp else f"dp{world}") if world > 1 else "single",
@@ -515,7 +513,7 @@ def main() -> None:
     kv_bytes_step = B * mean_ctx * 2 * runner.num_kv_heads * cfg.head_dim * 2 * cfg.num_layers
     step_bytes = weight_bytes + kv_bytes_step
     if cfg.num_experts > 0:
-        # routed experts: expected number of DISTINCT experts a batch of B tokens touches per layer (SURVEY s8d)
+        # routed experts: expected number of DISTINCT experts a batch of B tokens touches per layer
         touched = cfg.num_experts * (1.0 - (1.0 - cfg.num_experts_per_tok / cfg.num_experts) ** B)
         step_bytes += touched * runner.model.w.moe_expert_bytes() * cfg.num_layers
     line = {
@@ -564,7 +562,7 @@ def main() -> None:
         except Exception as ex:
             line["cpu_baseline"] = {"error": repr(ex)[:300]}
     if not args.no_cpu_baseline and not args.no_hf_baseline and world == 1:
-        # BASELINE.json configs[0]: HF transformers on the host cores (Qwen2.5-0.5B, greedy, one prompt) -- a reported
+        # HF transformers on the host cores (Qwen2.5-0.5B, greedy, one prompt) -- a reported
         # baseline row in the same run (tools/bench_hf_baseline.py), not what the GPU number is compared against
         try:
             sys.path.insert(0, str(ROOT / "tools"))

@@ -1,21 +1,21 @@
 /*
  * b200_lite_kernels.h -- C ABI of libb200lite.so, the B200 (sm_100a) kernel layer that stands in
- * for `lite_llama.kernels` (reference: /root/reference/lite_llama/kernels/__init__.py:11-39).
+ * for `lite_llama.kernels` (reference: lite_llama/kernels/__init__.py:11-39).
  *
  * The reference has no FFI: its boundary is Python name binding (`from ..kernels import ...`,
  * lite_llama/models/base.py:31-38, lite_llama/executor/model_runner.py:22,
  * lite_llama/models/quantization/methods/*.py).  Each entry point below is what a ctypes binding
  * for one of those names calls; lite_llama_b200/kernels/ holds that binding with the reference's
- * exact Python signatures, INTEGRATION.md shows how to bind them inside the unmodified reference.
+ * exact Python signatures and can be bound inside the unmodified reference (lite_llama_b200.integration).
  *
  * Conventions
  *   - every pointer is a DEVICE pointer unless stated otherwise; the caller owns all memory;
  *   - no entry point allocates, synchronises or touches the default stream: work is enqueued on
  *     `stream` (a cudaStream_t) and is CUDA-graph capturable;
  *   - strides are in ELEMENTS of the tensor's dtype; the innermost dimension must be contiguous;
- *   - `dtype`: B2L_F16 / B2L_BF16 activation dtype (the reference is fp16-only, SURVEY.md s0.2);
+ *   - `dtype`: B2L_F16 / B2L_BF16 activation dtype (the reference is fp16-only);
  *   - `*_width`: 4 or 8, byte width of an index vector (callers pass int32 or int64 vectors for
- *     b_seq_len / b_req_idx / b_start_loc, SURVEY.md s0.7);
+ *     b_seq_len / b_req_idx / b_start_loc);
  *   - return 0 on success, negative on error (B2L_ERR_*); b2l_last_error() returns a thread-local
  *     message.  The Python shim turns non-zero returns into ValueError, mirroring the reference's
  *     error behaviour (e.g. kernels/quantization/w4a16.py:174-184);

@@ -103,7 +103,7 @@ __device__ __forceinline__ void stg_128(void* p, const uint4& v) {
 }
 
 // Index loads that accept both int32 and int64 device vectors
-// (reference callers pass either: SURVEY.md §0.7).
+// (reference callers pass either).
 __device__ __forceinline__ int64_t load_index(const void* p, int64_t i, int width) {
   return width == 8 ? reinterpret_cast<const int64_t*>(p)[i]
                     : (int64_t)reinterpret_cast<const int32_t*>(p)[i];
@@ -487,7 +487,7 @@ static inline void b2l_hang_arm(cudaStream_t st) {
 }
 
 // cudaFuncAttributeMaxDynamicSharedMemorySize is a per-DEVICE attribute: remember the largest value set per device
-// (a process that drives several GPUs must set it on each; round-1 ADVICE).  `cache` is a function-local static array.
+// (a process that drives several GPUs must set it on each).  `cache` is a function-local static array.
 template <typename Kern>
 static inline cudaError_t b2l_ensure_dynamic_smem(Kern kern, int bytes, int (&cache)[64]) {
   int dev = 0;

@@ -3,7 +3,7 @@
 // and the two small MoE glue ops. All are HBM-bound: 128-bit accesses, one pass.
 //
 // Reference semantics (cited per op) are reproduced including their rounding
-// points, see SURVEY.md §7 "bit-level parity traps".
+// points.
 #include "common.cuh"
 
 // --------------------------------------------------------------------------- //
@@ -325,7 +325,7 @@ extern "C" int b2l_rope_emb(void* q, void* k, const void* cos, const void* sin, 
 }
 
 // --------------------------------------------------------------------------- //
-// rope + KV-cache write in one launch (SURVEY s8f.1): the reference rotates q and k (rope_emb.py:86-134), then
+// rope + KV-cache write in one launch: the reference rotates q and k (rope_emb.py:86-134), then
 // concatenates k|v and scatters the rows into the pool (models/base.py:76-79, update_kv_buffer.py:55-89) -- three
 // launches and two copies per layer.  Here one CTA per token rotates q in place, rotates k in place AND stores the
 // rotated row into the pool, and copies v into the pool.  Same arithmetic as rope_kernel (bit-identical results).

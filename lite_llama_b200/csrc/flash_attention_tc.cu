@@ -336,7 +336,7 @@ fa_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Prompts of at most 128 tokens (the BASELINE prefill shape: 32 x 128): every (sequence, head) is ONE 128 x 128 tile,
+// Prompts of at most 128 tokens (a batch of 32 x 128 tokens): every (sequence, head) is ONE 128 x 128 tile,
 // so the multi-tile pipeline above is all set-up.  This variant keeps the whole score row in registers (one TMEM read,
 // no running output), needs 96 KiB of shared memory and 256 TMEM columns, and is compiled for two resident CTAs per
 // SM: the loads of one CTA overlap the tensor-core and softmax work of the other.

@@ -5,7 +5,7 @@
 //   table[b_req_idx[b], 0 .. b_seq_len[b]-1]            (flashdecoding.py:66-69)
 // K/V are strided views of one [max_tokens, 2*Hkv, D] pool (models/base.py:119-123).
 //
-// B200 design (DESIGN.md "flash_decoding"):
+// B200 design:
 //  * one CTA per (split, kv-head block, batch row) streams WHOLE TOKEN ROWS: in the fused pool a
 //    token's K heads and V heads are one contiguous 2*Hkv*D*2-byte run (4 KiB for Llama-3-8B), so a
 //    single 1-D bulk async copy (cp.async.bulk, the TMA engine) per token brings in

@@ -5,7 +5,7 @@
 // lite_llama/distributed/parallel_state.py:208-213, lite_llama/models/qwen3_moe.py:110), and every one of those
 // all-reduces is immediately followed by the fused residual-add + RMSNorm of the next block
 // (lite_llama/models/base.py:307,312,486; lite_llama/kernels/skip_rmsnorm.py:192-234).  At decode the message is
-// 8 KiB per token -- 256 KiB at batch 32 -- so the collective is pure latency (SURVEY s5): a ring/tree with
+// 8 KiB per token -- 256 KiB at batch 32 -- so the collective is pure latency: a ring/tree with
 // several hops and a separate kernel for the norm costs more than the bytes.
 //
 // Here the two are ONE kernel over peer memory (one process per GPU, buffers exchanged once through CUDA IPC):

@@ -139,7 +139,7 @@ def make_moe_weights(cfg: ModelConfig, router, gate, up, down, method: str, tp: 
 def random_weights(cfg: ModelConfig, method: str = "fp16", device: str = "cuda", seed: int = 0,
                    dtype: torch.dtype = torch.float16, group_size: int = 128,
                    draw_device: str | None = None) -> DecoderWeights:
-    """Seeded random-init weights of ``cfg``'s shapes (``randn * 0.02``, norm weights 1; SURVEY.md s8d),
+    """Seeded random-init weights of ``cfg``'s shapes (``randn * 0.02``, norm weights 1),
     quantised per projection with ``method``. Every rank draws the full matrices and keeps its shard,
     so TP=N computes the same function as TP=1. ``lm_head`` stays fp16 under every scheme
     (lite_llama/models/base.py:366,425-429)."""

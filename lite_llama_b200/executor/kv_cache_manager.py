@@ -1,7 +1,7 @@
 """Token-granular KV pool and its reference-counted row allocator.
 
 Keeps the layout and the allocator surface the reference fixes as part of its executor API
-(lite_llama/executor/kv_cache_manager.py:136-372, SURVEY.md s0.5): one tensor per layer,
+(lite_llama/executor/kv_cache_manager.py:136-372): one tensor per layer,
 ``[max_tokens, 2 * num_kv_heads, head_dim]`` with the K heads first; ``kv_mem_use_state[i]`` is the
 reference count of row ``i`` (free at zero) and ``can_use_mem_size`` the number of free rows.
 

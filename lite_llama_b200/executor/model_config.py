@@ -1,7 +1,7 @@
 """Model geometry for the decoder families the reference serves (LLaMA / Qwen2 / Qwen3 dense).
 
 The reference wraps HF ``AutoConfig`` (lite_llama/models/config.py:48-218); no checkpoints or network
-exist in this environment, so the public HF geometries are written down here (SURVEY.md s8).
+exist in this environment, so the public HF geometries are written down here.
 """
 
 from __future__ import annotations

@@ -30,8 +30,8 @@ from .ragged_batch import RaggedBatch
 from .slot_batch import SlotBatch
 from .state_manager import RecurrentStateManager
 
-# executor/cuda_graph.py:27 stops at 128; 256 added so that a 256-wide continuous batch (BASELINE configs[3]) stays
-# on the graph path (SURVEY s8f.4)
+# executor/cuda_graph.py:27 stops at 128; 256 added so that a 256-wide continuous batch stays
+# on the graph path
 DEFAULT_BATCH_SIZES = (1, 2, 4, 8, 16, 32, 64, 128, 256)
 DEFAULT_SEQ_LEN_BUCKETS = (256, 512, 1024, 2048, 4096)       # executor/cuda_graph.py:28
 

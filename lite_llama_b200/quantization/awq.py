@@ -1,4 +1,4 @@
-"""Load-time ingestion of real 4-bit checkpoints (SURVEY s8f.3): AutoAWQ "GEMM" tensors and AutoGPTQ tensors ->
+"""Load-time ingestion of real 4-bit checkpoints: AutoAWQ "GEMM" tensors and AutoGPTQ tensors ->
 the reference's W4A16 layout (lite_llama/kernels/quantization/w4a16.py:9-12: ``qweight int32 [N, K/8]`` with nibble j
 of word i = input channel 8i + j, ``scales`` / ``zeros`` fp32 ``[N, K/g]``), which ``w4a16_matmul`` consumes as is and
 ``w4a16_pack`` turns into the kernel-native layout.

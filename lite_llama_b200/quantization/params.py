@@ -83,7 +83,7 @@ def reblock_scales(scales: torch.Tensor, block: int, new_block: int, dim: int) -
     ``block``): every sub-block inherits its parent's scale, so ``code * scale`` is unchanged. This is what lets a
     tensor-parallel shard start in the middle of a 128-wide checkpoint block (Qwen3-30B-A3B: 768 / 4 = 192 expert
     columns per rank) -- the reference requires shards to hold whole scale blocks (models/linear.py:164-177) and
-    therefore loads this model at TP = 2 only (SURVEY s0.9)."""
+    therefore loads this model at TP = 2 only."""
     if block % new_block != 0:
         raise ValueError(f"new block {new_block} must divide {block}")
     return scales.repeat_interleave(block // new_block, dim=dim)

@@ -4,8 +4,8 @@ TEST INFRASTRUCTURE ONLY. Nothing under ``lite_llama_b200/`` imports this packag
 ``__graft_entry__.smoke()`` and the ``cpu_baseline`` / ``--impl reference`` legs of ``bench.py`` do,
 and only as the checker (or the timed CPU baseline), never as the product path.
 
-Every function restates one reference operator and cites the file:line it follows (paths relative
-to /root/reference). Parity is PINNED: ``tests/golden/`` holds outputs of the reference's own
+Every function restates one reference operator and cites the file:line it follows (paths within its
+project). Parity is PINNED: ``tests/golden/`` holds outputs of the reference's own
 Triton kernels (run here through Triton's CPU interpreter by ``oracle/make_golden.py``) and of its
 CPU-runnable helpers (quantisers, ``moe_align_block_size``, ``tests/reference.py``); the oracle is
 checked against every one of them in ``tests/test_oracle_golden.py``.

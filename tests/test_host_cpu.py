@@ -175,7 +175,7 @@ def test_fp8_block_quantiser_and_sub_block_tensor_parallel_shards():
     equals the oracle's; refining the scale grid (reblock_scales) leaves every dequantised value unchanged; and a
     tensor-parallel shard that starts inside a 128-block (768 / 4 = 192 columns per rank) dequantises to the same
     values as the matching slice of the full matrix -- the case the reference refuses to load
-    (lite_llama/models/linear.py:164-177, SURVEY s0.9)."""
+    (lite_llama/models/linear.py:164-177)."""
     from lite_llama_b200.quantization.params import quantize_fp8_blockwise, reblock_scales
     from oracle import ops
 

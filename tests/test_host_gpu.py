@@ -206,8 +206,8 @@ def test_programmatic_dependent_launch_is_bit_identical():
 
 def test_one_llama3_8b_shape_layer_matches_the_cpu_restatement():
     """Real projection shapes (hidden 4096, 32/8 heads of 128, intermediate 14336, W4A16 g128), one layer, small
-    vocabulary: prefill of a ragged batch then two decode steps -- at batch 3 and at the batch-1 shape that stalled in
-    round 1 -- against oracle/model.py with the same weights."""
+    vocabulary: prefill of a ragged batch then two decode steps -- at batch 3 and at batch 1 --
+    against oracle/model.py with the same weights."""
     from lite_llama_b200.executor import PRESETS, ModelRunner
 
     cfg = PRESETS["llama-3-8b"].with_(num_layers=1, vocab_size=2048, max_seq_len=64)

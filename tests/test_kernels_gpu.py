@@ -72,7 +72,7 @@ def test_skip_rmsnorm_matches_oracle(shape, dtype):
 
 def test_skip_rmsnorm_wide_unaligned_rows_with_residual():
     """Rows wider than 4096 whose length is not a multiple of 8 take the two-pass warp kernel, residual included
-    (round-1 ADVICE: that combination used to be rejected)."""
+    (that combination used to be rejected)."""
     x = torch.randn(3, 4100 + 3, device="cuda", dtype=torch.float16)
     res = torch.randn_like(x)
     w = torch.randn(x.shape[-1], device="cuda", dtype=torch.float16)
@@ -293,7 +293,7 @@ def test_flash_decoding_uniform_values():
 
 
 def test_flash_decoding_llama3_shape_long_context():
-    # BASELINE shape: B=32, Hq=32, Hkv=8, D=128; ragged contexts up to 2048
+    # headline shape: B=32, Hq=32, Hkv=8, D=128; ragged contexts up to 2048
     torch.manual_seed(1)
     B, hq, hkv, d, ctx = 8, 32, 8, 128, 2048
     pool_rows = B * ctx
@@ -440,7 +440,7 @@ def test_flash_attention_tc_gqa_dtypes_d128(hq, hkv, dtype):
 
 
 def test_flash_attention_tc_matches_the_mma_sync_kernel_on_the_llama_prefill_shape():
-    """BASELINE prefill: 32 sequences x 128 tokens, Llama-3-8B heads, q/k/v as views of one fused-qkv buffer in the
+    """Headline prefill: 32 sequences x 128 tokens, Llama-3-8B heads, q/k/v as views of one fused-qkv buffer in the
     padded-rectangle layout; the tcgen05 kernel against the oracle and against the mma.sync kernel (B2L_FA_TC=0 path
     is exercised by the head_dim 32/64 cases above)."""
     B, S, hq, hkv, d = 32, 128, 32, 8, 128
@@ -931,7 +931,7 @@ def test_w8a16_stream_k_block_scales(m, n, k):
 @pytest.mark.parametrize("n,k", [(6144, 4096), (4096, 4096), (28672, 4096), (4096, 14336)])
 @pytest.mark.parametrize("m", [1, 32])
 def test_w4a16_llama3_8b_projection_shapes(m, n, k):
-    # full BASELINE shapes: compared on the GPU with an fp32 matmul over the dequantised weights (same formula as
+    # full headline shapes: compared on the GPU with an fp32 matmul over the dequantised weights (same formula as
     # oracle/ops.py:w4a16_matmul, which takes minutes at this size on the CPU)
     gs = 128
     torch.manual_seed(1)
@@ -948,7 +948,7 @@ def test_w4a16_llama3_8b_projection_shapes(m, n, k):
 
 
 # --------------------------------------------------------------------------- #
-# batch-1 Llama-3-8B geometry, op by op (the decode step that stalled lives at these shapes)
+# batch-1 Llama-3-8B geometry, op by op (a decode step that once stalled lives at these shapes)
 # --------------------------------------------------------------------------- #
 def test_bs1_llama_geometry_every_op_of_the_layer():
     torch.manual_seed(0)

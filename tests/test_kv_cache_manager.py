@@ -1,5 +1,5 @@
 """KVCacheManager and SlotBatch: the reference's own test list for the allocator
-(/root/reference/tests/executor/test_kv_cache_manager.py:47-215: initial state, scattered / contiguous allocation,
+(tests/executor/test_kv_cache_manager.py:47-215: initial state, scattered / contiguous allocation,
 refusal without side effects, reference counts, bump fast path and when it must switch off) restated against this
 package's implementation, plus the slot layout the continuous-batching engine drives
 (lite_llama/executor/slot_batch.py:56-220). Runs on CPU tensors (pure host logic + torch indexing)."""

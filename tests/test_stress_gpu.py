@@ -1,4 +1,4 @@
-"""Graph-replay stress of the captured decode step at Llama-3-8B geometry (round-1 VERDICT item 1: intermittent
+"""Graph-replay stress of the captured decode step at Llama-3-8B geometry (intermittent
 device hangs that the ~12-replay model tests could not see).  Each case runs tools/stress_decode.py in its own
 process (a trapped kernel kills the CUDA context): 4 real-shape W4A16 layers + lm_head, the whole greedy step as one
 CUDA graph, replayed 2000 times with the token stream compared against a first pass.  The device-side hang
@@ -55,5 +55,5 @@ def test_two_processes_share_the_gpu():
 
 
 def test_full_depth_batch1_smoke():
-    """All 32 layers at batch 1 (the configuration that stalled in round 1), 300 replays."""
+    """All 32 layers at batch 1 (the configuration that once stalled), 300 replays."""
     _run(["--batch", "1", "--layers", "32", "--replays", "300"], timeout=400)
