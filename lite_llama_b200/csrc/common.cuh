@@ -221,10 +221,14 @@ __device__ __forceinline__ unsigned long long b2l_globaltimer() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// noreturn: nothing is live across the call, so a barrier wait does not force the caller's registers into the
-// callee-saved half (ptxas could not allocate a thread with 128 accumulators and a returning call in its wait loops).
-[[noreturn]] static __device__ __noinline__ void b2l_hang_trap(uint32_t bar_addr, uint32_t parity, unsigned int file_hash, int line,
-                                           unsigned long long waited_ns) {
+// A source that defines B2L_HANG_NORETURN before this header tells the compiler that the call does not come back: nothing is
+// live across it, so a barrier wait does not force the caller's registers into the callee-saved half (ptxas could not
+// allocate a thread with 128 accumulators and a returning call in its wait loops).
+#ifdef B2L_HANG_NORETURN
+[[noreturn]]
+#endif
+static __device__ __noinline__ void b2l_hang_trap(uint32_t bar_addr, uint32_t parity, unsigned int file_hash, int line,
+                                                  unsigned long long waited_ns) {
   unsigned int* rec = b2l_hang_ctl.rec;
   if (rec != nullptr && atomicCAS(&b2l_hang_ctl.taken, 0, 1) == 0) {
     rec[1] = file_hash; rec[2] = (unsigned)line;
@@ -242,7 +246,9 @@ __device__ __forceinline__ unsigned long long b2l_globaltimer() {
     }
   }
   __trap();
+#ifdef B2L_HANG_NORETURN
   __builtin_unreachable();
+#endif
 }
 // mode 0: try_wait + long suspend hint, 1: test_wait polling, 2: try_wait with the default suspend window
 template <int MODE>
