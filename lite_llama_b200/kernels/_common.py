@@ -70,15 +70,15 @@ def no_grad(fn):
     return call
 
 
-def is_rows(t: torch.Tensor) -> bool:
-    """Whether ``t`` is a matrix whose row stride can be handed on.  That of a one-row matrix may be anything (the width of
-    the matrix it was sliced from, or 1), and ``contiguous`` leaves it; ``reshape`` makes it the row's length."""
-    return t.dim() == 2 and t.size(1) > 0 and (t.size(0) > 1 or t.stride(0) == t.size(1))
-
-
 def as_rows(t: torch.Tensor) -> torch.Tensor:
     """``t`` with its leading dimensions joined (``t`` itself if it is a matrix already)."""
-    return t if is_rows(t) else t.reshape(-1, t.shape[-1])
+    return t if t.dim() == 2 and t.size(1) else t.reshape(-1, t.shape[-1])
+
+
+def own_rows(t: torch.Tensor) -> torch.Tensor:
+    """The matrix ``t`` with rows that follow one another.  ``contiguous`` alone leaves the row stride of a one-row matrix,
+    which may be anything (the width of the matrix it was sliced from, or 1); ``view`` makes it the row's length."""
+    return t.contiguous().view(-1, t.size(1))
 
 
 def unrows(y: torch.Tensor, like: torch.Tensor) -> torch.Tensor:

@@ -8,7 +8,7 @@ from __future__ import annotations
 
 import torch
 
-from ._common import as_rows, check, counters, dtype_code, float_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, weights_written, workspace
+from ._common import as_rows, check, counters, dtype_code, float_code, lib, no_grad, own_rows, ptr, require_cuda, stream_handle, unrows, weights_written, workspace
 
 
 @no_grad
@@ -28,7 +28,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = No
         weights_written()
     a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
-        a = a.contiguous()
+        a = own_rows(a)
     m = a.shape[0]
     out = x.new_empty((m, n))
     if bias is not None:

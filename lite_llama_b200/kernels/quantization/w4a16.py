@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
+from .._common import as_rows, check, counters, current_device, lib, no_grad, own_rows, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
 
 _Q_INT4 = 0
 
@@ -44,7 +44,7 @@ def w4a16_matmul(
         weights_written()
     a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
-        a = a.contiguous()
+        a = own_rows(a)
     m = a.shape[0]
     out = x.new_empty((m, n))
     bias_f32 = 0
@@ -130,7 +130,7 @@ def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor
         raise ValueError(f"x has {x.shape[-1]} cols but weight expects {k}")
     a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
-        a = a.contiguous()
+        a = own_rows(a)
     m = a.shape[0]
     n_out = n // 2 if swiglu else n
     out = x.new_empty((m, n_out))

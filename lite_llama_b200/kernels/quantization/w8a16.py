@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from .._common import as_rows, check, counters, current_device, lib, no_grad, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
+from .._common import as_rows, check, counters, current_device, lib, no_grad, own_rows, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
 
 _Q_FP8, _Q_INT8 = 1, 2
 
@@ -41,7 +41,7 @@ def w8a16_matmul(
         scales = scales.unsqueeze(-1)
     a = as_rows(x)
     if a.stride(-1) != 1 or a.stride(0) % 8 != 0 or a.data_ptr() % 16 != 0:
-        a = a.contiguous()
+        a = own_rows(a)
     m = a.shape[0]
     out = x.new_empty((m, n))
     bias_f32 = 0

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from ._common import check, dtype_code, is_rows, lib, no_grad, ptr, require_cuda, stream_handle
+from ._common import check, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
 @no_grad
@@ -18,10 +18,10 @@ def skip_rmsnorm(X, residual, weight, eps=1e-5):
     require_cuda(X, residual, weight)
     orig_shape = X.shape
     n = orig_shape[-1]
-    # matrices go through as they are (unless the results would inherit a requires_grad)
-    flat = is_rows(X) and not X.requires_grad and X.is_contiguous() and \
-        (residual is None or (residual.shape == orig_shape and is_rows(residual) and not residual.requires_grad and
-                              residual.is_contiguous()))
+    # matrices go through as they are (unless the results would inherit a requires_grad); all rows follow one another, whatever
+    # stride a single one claims
+    flat = len(orig_shape) == 2 and not X.requires_grad and X.is_contiguous() and \
+        (residual is None or (residual.shape == orig_shape and not residual.requires_grad and residual.is_contiguous()))
     x2 = X if flat else X.contiguous().view(-1, n)
     code = dtype_code(x2, "X")
     if weight.dtype != x2.dtype:
@@ -36,8 +36,7 @@ def skip_rmsnorm(X, residual, weight, eps=1e-5):
         r2 = residual if flat else residual.contiguous().view(-1, n)
     check(
         lib().b2l_skip_rmsnorm(
-            y.data_ptr(), x2.data_ptr(), ptr(r2), w.data_ptr(), x2.shape[0], n, x2.stride(0),
-            r2.stride(0) if r2 is not None else 0, y.stride(0), float(eps), code, stream_handle(),
+            y.data_ptr(), x2.data_ptr(), ptr(r2), w.data_ptr(), x2.shape[0], n, n, n, n, float(eps), code, stream_handle(),
         )
     )
     if flat:
@@ -61,10 +60,10 @@ def skip_rmsnorm_quant_int8(X, residual, weight, eps=1e-5):
     require_cuda(X, residual, weight)
     orig_shape = X.shape
     n = orig_shape[-1]
-    # matrices go through as they are (unless the results would inherit a requires_grad)
-    flat = is_rows(X) and not X.requires_grad and X.is_contiguous() and \
-        (residual is None or (residual.shape == orig_shape and is_rows(residual) and not residual.requires_grad and
-                              residual.is_contiguous()))
+    # matrices go through as they are (unless the results would inherit a requires_grad); all rows follow one another, whatever
+    # stride a single one claims
+    flat = len(orig_shape) == 2 and not X.requires_grad and X.is_contiguous() and \
+        (residual is None or (residual.shape == orig_shape and not residual.requires_grad and residual.is_contiguous()))
     x2 = X if flat else X.contiguous().view(-1, n)
     code = dtype_code(x2, "X")
     if weight.dtype != x2.dtype:
@@ -81,8 +80,8 @@ def skip_rmsnorm_quant_int8(X, residual, weight, eps=1e-5):
     s = torch.empty((x2.shape[0],), dtype=torch.float32, device=x2.device)
     check(
         lib().b2l_skip_rmsnorm_quant_int8(
-            q.data_ptr(), s.data_ptr(), x2.data_ptr(), ptr(r2), w.data_ptr(), x2.shape[0], n, x2.stride(0),
-            r2.stride(0) if r2 is not None else 0, q.stride(0), float(eps), code, stream_handle(),
+            q.data_ptr(), s.data_ptr(), x2.data_ptr(), ptr(r2), w.data_ptr(), x2.shape[0], n, n, n, n, float(eps), code,
+            stream_handle(),
         )
     )
     return q, s, (r2.view(orig_shape) if r2 is not None else x2.view(orig_shape))

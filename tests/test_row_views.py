@@ -24,22 +24,23 @@ VIEWS = [row_of_wide, transposed_column]
 
 
 @pytest.mark.parametrize("view", VIEWS)
-def test_as_rows_gives_a_single_row_its_own_length_as_stride(view):
-    from lite_llama_b200.kernels._common import as_rows
+def test_a_single_row_gets_its_own_length_as_stride(view):
+    from lite_llama_b200.kernels._common import as_rows, own_rows
 
     x = view("cpu")
-    assert x.is_contiguous() and x.stride(0) != K_DIM
-    a = as_rows(x)
+    assert x.is_contiguous() and x.stride(0) != K_DIM           # so contiguous() alone changes nothing
+    a = own_rows(as_rows(x))
     assert a.stride() == x.reshape(-1, K_DIM).stride() == (K_DIM, 1) and a.data_ptr() == x.data_ptr()
 
 
 def test_as_rows_passes_matrices_through():
-    from lite_llama_b200.kernels._common import as_rows
+    from lite_llama_b200.kernels._common import as_rows, own_rows
 
     for t in (torch.zeros(4, 64), torch.zeros(4, 67)[:, :64], torch.zeros(1, 64)):
         assert as_rows(t) is t
     assert as_rows(torch.zeros(2, 3, 64)).shape == (6, 64) and as_rows(torch.zeros(64)).shape == (1, 64)
     assert as_rows(torch.zeros(0, 64)).shape == (0, 64)
+    assert own_rows(torch.zeros(4, 67)[:, :64]).stride() == (64, 1) and own_rows(torch.zeros(0, 64)).shape == (0, 64)
 
 
 def calls():
