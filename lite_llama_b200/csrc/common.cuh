@@ -102,6 +102,14 @@ __device__ __forceinline__ void stg_128(void* p, const uint4& v) {
   *reinterpret_cast<uint4*>(p) = v;
 }
 
+// Index data that an earlier kernel of the chain wrote: an ordinary (coherent, cached) load that the compiler can neither
+// turn into a load of constant data (__ldg) nor move above the wait for that kernel.
+__device__ __forceinline__ int32_t ld_upstream(const int32_t* p) {
+  int32_t v;
+  asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+
 // Index loads that accept both int32 and int64 device vectors
 // (reference callers pass either).
 __device__ __forceinline__ int64_t load_index(const void* p, int64_t i, int width) {
@@ -221,14 +229,8 @@ __device__ __forceinline__ unsigned long long b2l_globaltimer() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-// A source that defines B2L_HANG_NORETURN before this header tells the compiler that the call does not come back: nothing is
-// live across it, so a barrier wait does not force the caller's registers into the callee-saved half (ptxas could not
-// allocate a thread with 128 accumulators and a returning call in its wait loops).
-#ifdef B2L_HANG_NORETURN
-[[noreturn]]
-#endif
-static __device__ __noinline__ void b2l_hang_trap(uint32_t bar_addr, uint32_t parity, unsigned int file_hash, int line,
-                                                  unsigned long long waited_ns) {
+__device__ __forceinline__ void b2l_hang_record(uint32_t bar_addr, uint32_t parity, unsigned int file_hash, int line,
+                                                unsigned long long waited_ns) {
   unsigned int* rec = b2l_hang_ctl.rec;
   if (rec != nullptr && atomicCAS(&b2l_hang_ctl.taken, 0, 1) == 0) {
     rec[1] = file_hash; rec[2] = (unsigned)line;
@@ -246,12 +248,25 @@ static __device__ __noinline__ void b2l_hang_trap(uint32_t bar_addr, uint32_t pa
     }
   }
   __trap();
-#ifdef B2L_HANG_NORETURN
-  __builtin_unreachable();
-#endif
 }
+static __device__ __noinline__ void b2l_hang_trap(uint32_t bar_addr, uint32_t parity, unsigned int file_hash, int line,
+                                                  unsigned long long waited_ns) {
+  b2l_hang_record(bar_addr, parity, file_hash, line, waited_ns);
+}
+// The same, declared as not coming back: nothing is live across the call, so a barrier wait does not force the caller's registers
+// into the callee-saved half (ptxas could not allocate a thread with 128 accumulators and a returning call in its wait
+// loops).  It changes the code around every wait, for better or worse: a source sets the default for its waits
+// (B2L_HANG_NORETURN), gemm_quant.cu chooses per instantiation.
+[[noreturn]] static __device__ __noinline__ void b2l_hang_stop(uint32_t bar_addr, uint32_t parity, unsigned int file_hash,
+                                                               int line, unsigned long long waited_ns) {
+  b2l_hang_record(bar_addr, parity, file_hash, line, waited_ns);
+  __builtin_unreachable();
+}
+#ifndef B2L_HANG_NORETURN
+#define B2L_HANG_NORETURN false
+#endif
 // mode 0: try_wait + long suspend hint, 1: test_wait polling, 2: try_wait with the default suspend window
-template <int MODE>
+template <int MODE, bool NORETURN>
 __device__ __forceinline__ void b2l_wait_slow(uint64_t* bar, uint32_t parity, unsigned int file_hash, int line) {
   const unsigned long long t0 = b2l_globaltimer();
   for (;;) {
@@ -260,20 +275,26 @@ __device__ __forceinline__ void b2l_wait_slow(uint64_t* bar, uint32_t parity, un
     if (ok) return;
     const unsigned long long lim = b2l_hang_ctl.limit_ns;
     const unsigned long long dt = b2l_globaltimer() - t0;
-    if (lim != 0ull && dt > lim) b2l_hang_trap(smem_u32(bar), parity, file_hash, line, dt);
+    if (lim != 0ull && dt > lim) {
+      if (NORETURN) b2l_hang_stop(smem_u32(bar), parity, file_hash, line, dt);
+      else b2l_hang_trap(smem_u32(bar), parity, file_hash, line, dt);
+    }
   }
 }
+template <bool NORETURN = B2L_HANG_NORETURN>
 __device__ __forceinline__ void mbar_wait_at(uint64_t* bar, uint32_t parity, unsigned int file_hash, int line) {
   if (mbar_try_wait(bar, parity)) return;
-  b2l_wait_slow<0>(bar, parity, file_hash, line);
+  b2l_wait_slow<0, NORETURN>(bar, parity, file_hash, line);
 }
+template <bool NORETURN = B2L_HANG_NORETURN>
 __device__ __forceinline__ void mbar_wait_spin_at(uint64_t* bar, uint32_t parity, unsigned int file_hash, int line) {
   if (mbar_test_wait(bar, parity)) return;
-  b2l_wait_slow<1>(bar, parity, file_hash, line);
+  b2l_wait_slow<1, NORETURN>(bar, parity, file_hash, line);
 }
+template <bool NORETURN = B2L_HANG_NORETURN>
 __device__ __forceinline__ void mbar_wait_short_at(uint64_t* bar, uint32_t parity, unsigned int file_hash, int line) {
   if (mbar_try_wait_short(bar, parity)) return;
-  b2l_wait_slow<2>(bar, parity, file_hash, line);
+  b2l_wait_slow<2, NORETURN>(bar, parity, file_hash, line);
 }
 #define mbar_wait(bar, parity) mbar_wait_at((bar), (parity), b2l_file_hash(__FILE__), __LINE__)
 #define mbar_wait_spin(bar, parity) mbar_wait_spin_at((bar), (parity), b2l_file_hash(__FILE__), __LINE__)

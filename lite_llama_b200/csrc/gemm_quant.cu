@@ -93,15 +93,19 @@ struct QuantParams {
 #ifndef B2L_DQ_ORDER
 #define B2L_DQ_ORDER 0
 #endif
-template <int MODE>
+template <int MODE, bool NORETURN>
 __device__ __forceinline__ void qwait_at(uint64_t* bar, uint32_t parity, int line) {
   constexpr unsigned int fh = b2l_file_hash(__FILE__);
-  if (MODE == 1) mbar_wait_spin_at(bar, parity, fh, line);
-  else if (MODE == 2) mbar_wait_short_at(bar, parity, fh, line);
-  else mbar_wait_at(bar, parity, fh, line);
+  if (MODE == 1) mbar_wait_spin_at<NORETURN>(bar, parity, fh, line);
+  else if (MODE == 2) mbar_wait_short_at<NORETURN>(bar, parity, fh, line);
+  else mbar_wait_at<NORETURN>(bar, parity, fh, line);
 }
-#define qwait(bar, parity) qwait_at<B2L_QWAIT_MODE>((bar), (parity), __LINE__)
-#define qwait_lat(bar, parity) qwait_at<B2L_QWAIT_LAT_MODE>((bar), (parity), __LINE__)
+// Whether the watchdog's call returns (common.cuh), by measurement: int4 tiles of 64 tokens lose 3 % if it does not (28672 x
+// 4096, 64 tokens 26.0 -> 26.9 us); 8-bit weights gain 1 - 8 % (int8 with one scale per row, 16 tokens: 4096 x 14336 37.8 ->
+// 34.9, 2048 x 4096 10.2 -> 9.7), int4 tiles of 16 and 32 tokens up to 3 %.
+__host__ __device__ constexpr bool q_noreturn(int qk, int bt) { return !(qk == Q_INT4 && bt == 64); }
+#define qwait(bar, parity) qwait_at<B2L_QWAIT_MODE, q_noreturn(QK, BT)>((bar), (parity), __LINE__)
+#define qwait_lat(bar, parity) qwait_at<B2L_QWAIT_LAT_MODE, q_noreturn(QK, BT)>((bar), (parity), __LINE__)
 // B2L_TLITE (A/B builds only, tools/build_variants.py): a handful of clock stamps per CTA
 #ifdef B2L_TLITE
 #define LT(i) do { if (p.timeline) p.timeline[(size_t)blockIdx.x * 32 + (i)] = clock64(); } while (0)
@@ -601,7 +605,6 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       int rstage = mma_idx % p.x_stages;
       uint32_t rphase = (mma_idx / p.x_stages) & 1;
       for (int rb = mma_idx; rb < nrb; rb += mma_warps) {
-        const int gsub0 = rb * RW;                                       // first operand sub-block of this raw block
         qwait(&ctl->x_full[rstage], rphase);                         // activation sub-tiles (TMA)
         tc_fence_after();
         if (rb == 0 && lane == 0) LT(4);
@@ -1302,11 +1305,6 @@ static inline SplitPlan quant_plan(int qk, int64_t M, int64_t N, int64_t K, int 
   pl.splits = (pl.num_kb + pl.kb_per_split - 1) / pl.kb_per_split;
   quant_rings(qk, pl, pl.kb_per_split / rw, groups_touched(pl.kb_per_split, seg_len));
   return pl;
-}
-
-static inline int env_int(const char* name, int dflt) {
-  const char* e = getenv(name);
-  return e && e[0] ? atoi(e) : dflt;
 }
 
 template <int QK, int BT, int LAYOUT, int EPI = 0>

@@ -17,7 +17,7 @@
 // at the cost of two operand stages: int4 878, fp8 901 us.
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of
 // the accumulator per scale group, acc = fma(scale, segment, acc) in fp32 in ascending k.
-#define B2L_HANG_NORETURN       // common.cuh: 128 accumulators beside the wait loops
+#define B2L_HANG_NORETURN true   // common.cuh: 128 accumulators beside the wait loops
 #include "gemm_tc.cuh"
 #include "gemm_quant_pair.cuh"
 #include "pair.cuh"
