@@ -15,7 +15,7 @@ struct QuantPairParams {
   const int32_t* table;                              // grouped: {tiles, {expert, first row, rows} per tile}
   const int32_t* order;                              // grouped down projection: slot of every sorted row
   const __half* row_weights;                         // grouped down projection: routing weight by slot
-  int M, N, steps, seg_steps, m_tiles, n_tiles;      // filled by quant_pair_gemm
+  int M, N, steps, seg_steps, groups, m_tiles, n_tiles;      // filled by quant_pair_gemm (groups: pitch of the int4 tables)
 };
 
 // shapes the pair kernel takes and is the faster one for (see gemm_quant_pair.cu); qk: QuantKind

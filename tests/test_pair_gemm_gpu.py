@@ -222,3 +222,24 @@ def test_expert_sum_in_vectors(tokens, n, top_k, addend, dtype):
     for k in range(top_k):
         acc = acc + x[:, k].float()
     assert torch.equal(out, (acc + add.float() if addend else acc).to(dtype))
+
+
+# ---- how long one accumulation in tensor memory runs where a scale covers all of k ----
+# (m, n, k, k values per accumulation): parts of k as 148 SMs / (n / 128 x m / 64 tiles) leave them
+@pytest.mark.parametrize("m,n,k,chain", [(16, 4096, 4096, 1024), (64, 6144, 4096, 1408), (128, 4096, 4096, 2048),
+                                         (96, 4096, 14336, 7168), (192, 2048, 4096, 1408)])
+@pytest.mark.parametrize("fp8", [True, False])
+def test_per_channel_accumulations_are_no_longer_than_the_parts_of_k(m, n, k, chain, fp8):
+    """Positive values, so that the accumulator's rounding shows as a mean deviation, far above that of the rounding to fp16.
+    One addition of 16 products loses less than 2^-23 of the partial sum; over twice the chain and more it exceeds the bound
+    for int8."""
+    x = torch.rand(m, k, device="cuda").mul_(0.5).add_(0.5).half()
+    if fp8:
+        q = (torch.rand(n, k, device="cuda") * 100 + 20).to(torch.float8_e4m3fn).view(torch.uint8)
+        w = q.view(torch.float8_e4m3fn).double()
+    else:
+        q = torch.randint(1, 127, (n, k), device="cuda", dtype=torch.int8)
+        w = q.double()
+    s = torch.rand(n, 1, device="cuda") * 1e-4 + 1e-4
+    got, want = K().w8a16_matmul(x, q, s, group_n=1, group_k=k).double(), x.double() @ (w * s.double()).T
+    assert abs(((got - want) / want).mean().item()) < chain / 16 * 2.0**-23
