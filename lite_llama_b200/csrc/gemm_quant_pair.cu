@@ -70,13 +70,13 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
 // What a tile is: `mode` plain = one weight matrix; grouped = experts, one entry of the tile table per 128 rows of an
 // expert's run of the sorted activations (moe_sort, moe_routing.cu), the entries' output tiles next to one another so that
 // the pairs in flight share the activations and an expert's second entry finds the weights in L2.  The table and the slot
-// order are earlier kernels' output, and this one may be resident before they are written: read through L2 (__ldcg), never
-// as data that is constant for the kernel (__ldg).
+// order are earlier kernels' output, and this one may be resident before they are written: never read as data that is
+// constant for the kernel (__ldg).  Through L2 (__ldcg) every role paid 3 % of a small batch for it: ld_upstream.
 enum { QP_PLAIN = 0, QP_GATE_UP = 1, QP_DOWN = 2 };
 struct QpTile { int n, m0, rows, expert; };
 template <int MODE>
 __device__ __forceinline__ int qp_tiles(const QuantPairParams& p) {
-  return MODE == QP_PLAIN ? p.m_tiles * p.n_tiles : __ldcg(p.table) * p.n_tiles;
+  return MODE == QP_PLAIN ? p.m_tiles * p.n_tiles : ld_upstream(p.table) * p.n_tiles;
 }
 template <int MODE>
 __device__ __forceinline__ QpTile qp_tile(const QuantPairParams& p, int t) {
@@ -87,7 +87,7 @@ __device__ __forceinline__ QpTile qp_tile(const QuantPairParams& p, int t) {
   } else {
     const int e = t / p.n_tiles;
     o.n = t - e * p.n_tiles;
-    o.expert = __ldcg(p.table + 1 + 3 * e); o.m0 = __ldcg(p.table + 2 + 3 * e); o.rows = __ldcg(p.table + 3 + 3 * e);
+    o.expert = ld_upstream(p.table + 1 + 3 * e); o.m0 = ld_upstream(p.table + 2 + 3 * e); o.rows = ld_upstream(p.table + 3 + 3 * e);
   }
   return o;
 }
@@ -326,8 +326,8 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           const bool in = 32 * q + lane < rows;
-          slot[q] = in ? __ldcg(p.order + m0 + 32 * q + lane) : 0;
-          wt[q] = in ? __half2float(__ldcg(p.row_weights + slot[q])) : 0.f;
+          slot[q] = in ? ld_upstream(p.order + m0 + 32 * q + lane) : 0;
+          wt[q] = in ? __half2float(p.row_weights[slot[q]]) : 0.f;
         }
 #pragma unroll
         for (int j = 0; j < kHalf; ++j) {

@@ -141,10 +141,10 @@ __global__ void __launch_bounds__(256)
 moe_gather_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, const int32_t* __restrict__ order, int num_slots,
                   int top_k, int64_t x_stride, int64_t chunks) {
   pdl_prologue();
-  const int rows = __ldcg(order + num_slots);
+  const int rows = ld_upstream(order + num_slots);
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (r >= rows) return;
-  const uint4* src = x + (int64_t)(__ldcg(order + r) / top_k) * x_stride;
+  const uint4* src = x + (int64_t)(ld_upstream(order + r) / top_k) * x_stride;
   uint4* dst = out + (int64_t)r * chunks;
   for (int64_t c = threadIdx.x & 31; c < chunks; c += 32) dst[c] = __ldcg(src + c);
 }
