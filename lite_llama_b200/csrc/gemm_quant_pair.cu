@@ -458,10 +458,11 @@ static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPa
   return B2L_OK;
 }
 
-// Where the pair kernel is the faster one (both kernels measured over 72 - 4096 tokens and seven projection shapes).  A
-// wave of pair tiles takes about 1.35 times a wave of the streaming kernel's 128 x 64 tiles (6144 x 4096, one wave each:
-// 23.5 against 17.5 us) and covers four of them per pair, so the waves decide: int4, us, streaming -> pair:
-//   28672 x 4096, 72 tokens 72 -> 46, 4096 tokens 1854 -> 982; 4096 x 4096, 320 tokens 33 -> 23, but 192 tokens 17 -> 22.
+// Where the pair kernel is the faster one (both kernels measured over 72 - 512 tokens, eight projection shapes, int4 with and
+// without the activation and fp8 in blocks): as soon as the streaming kernel's 128 x 64 tiles need a second wave.  int4, us,
+// streaming -> pair: one wave, 6144 x 4096 at 128 tokens 17 / 21, 4096 x 14336 at 72 45 / 64 (at 256, 66 / 64); two, 6144 x
+// 4096 at 256 33 -> 21, 9728 x 896 at 192 (two waves of pair tiles as well) 13.8 -> 10.8; five against four, 28672 x 4096 at 192
+// 94 -> 75; at 4096 tokens 1853 -> 900.
 // One segment over all of k (a scale per output row) leaves the streaming kernel a single MMA warp; there the pair
 // kernel wins as soon as it has 16 tiles (int8, 896 x 4864, 512 tokens 27 -> 19; 320 tokens, 12 tiles: level).  That holds
 // for decode batches too (tiles of 64 tokens, six conversion stages; int8, 32 tokens: 28672 x 4096 82 -> 28, 6144 x 4096
@@ -475,7 +476,7 @@ bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k)
   const int64_t tiles = cdiv64(M, kQpTokens) * cdiv64(N, 2 * kBlockW);
   if (group_k >= K) return M > 64 ? tiles >= 16 : qk != Q_INT4 && (tiles >= 40 || (tiles >= 16 && K <= 4096));
   if (M <= 64) return false;
-  return 4 * cdiv64(cdiv64(M, 64) * cdiv64(N, kBlockW), sms) >= 5 * cdiv64(tiles, sms / 2);
+  return cdiv64(M, 64) * cdiv64(N, kBlockW) > sms;
 }
 
 // Operand stages that one accumulation in tensor memory may run over where one scale covers all of k.  A longer chain is
