@@ -23,8 +23,11 @@ def rel(got, want):
     return ((got.double() - want).norm() / want.norm()).item()
 
 
-# 129 tokens x 10240 outputs: the fewest tokens and (40 wide tiles of 256) about the fewest tiles the pair kernel takes
-EDGES = [(129, 10240, 192), (256, 10248, 64), (257, 5128, 392), (511, 5112, 1000), (1000, 4096, 520), (2049, 4104, 256)]
+# 129 tokens x 10240 outputs: the fewest tokens and (40 wide tiles of 256) about the fewest tiles the pair kernel takes.  The
+# 4104 outputs of 511 tokens run in 66 tiles of 128 outputs.  2049 x 4104 (153 wide tiles) and 700 x 6400 (150 tiles of 128)
+# give the 74 pairs a second and a third tile, the accumulators taken in turn
+EDGES = [(129, 10240, 192), (256, 10248, 64), (257, 5128, 392), (511, 5112, 1000), (1000, 4096, 520), (2049, 4104, 256),
+         (511, 4104, 392), (300, 4104, 1008), (1000, 2056, 72), (700, 6400, 136)]
 
 
 @pytest.mark.parametrize("m,n,k", EDGES)
@@ -35,10 +38,12 @@ def test_linear_pair_tiles(m, n, k, dtype, bias):
     w = torch.randn(n, k, device="cuda", dtype=dtype)
     b = torch.randn(n, device="cuda", dtype=dtype) if bias else None
     want = x.double() @ w.double().T + (b.double() if bias else 0.0)
-    assert rel(K().linear(x, w, b), want) < REL[dtype]
+    got = K().linear(x, w, b)
+    assert rel(got, want) < REL[dtype] and torch.equal(K().linear(x, w, b), got)
 
 
-@pytest.mark.parametrize("m,n,k", [(129, 10240, 192), (256, 10248, 64), (511, 5112, 1008), (2049, 4104, 256)])
+@pytest.mark.parametrize("m,n,k", [(129, 10240, 192), (256, 10248, 64), (511, 5112, 1008), (2049, 4104, 256),
+                                   (511, 4104, 400), (300, 4104, 1008), (700, 6400, 144)])
 @pytest.mark.parametrize("bias", [False, True])
 def test_int8_pair_tiles(m, n, k, bias):
     qa = torch.randint(-127, 128, (m, k), device="cuda", dtype=torch.int8)
@@ -60,8 +65,12 @@ def test_linear_forms_the_pair_kernel_does_not_take():
 
 # ---- quantised weights (csrc/gemm_quant_pair.cu): 256-row x 128-token tiles, 128 k per operand stage ----
 # m: one token over / under a tile, 64-token edge of the dispatch; n: rows past the last tile; k: an odd number of stages
-# (half a raw block is left over), one and several stages per scale group
-QUANT_EDGES = [(65, 10240, 128), (127, 10140, 384), (129, 5128, 640), (500, 2600, 256), (1000, 1300, 896)]
+# (half a raw block is left over), one and several stages per scale group.  129 x 5128: the wave rule leaves scale groups to
+# the streaming kernel and gives one scale per row to the pair kernel; 129 x 18944 is the pair kernel's either way.  From
+# 129 x 18944 on there are 148 to 304 tiles for 74 pairs: what a pair carries from one tile to the next (ring phases, stage
+# and raw-block counts of the conversion groups, accumulator in turn), and a short last tile after full ones
+QUANT_EDGES = [(65, 10240, 128), (127, 10140, 384), (129, 5128, 640), (500, 2600, 256), (1000, 1300, 896),
+               (129, 18944, 640), (1000, 9728, 896), (1153, 5128, 384), (1100, 9728, 768)]
 
 
 def int4_case(n, k, group, m):
@@ -81,8 +90,10 @@ def test_int4_pair_tiles(m, n, k, group, bias):
         pytest.skip("groups divide k")
     q, s, z, w, x = int4_case(n, k, group, m)
     b = None if bias is None else torch.randn(n, device="cuda", dtype=bias)
-    got = K().w4a16_matmul_packed(x, K().w4a16_pack(q, s, z, group_size=group), bias=b)
+    packed = K().w4a16_pack(q, s, z, group_size=group)
+    got = K().w4a16_matmul_packed(x, packed, bias=b)
     assert rel(got, x.double() @ w.T + (0.0 if b is None else b.double())) < REL[torch.float16]
+    assert torch.equal(K().w4a16_matmul_packed(x, packed, bias=b), got)
 
 
 @pytest.mark.parametrize("m,n,k", QUANT_EDGES)
@@ -132,10 +143,14 @@ def test_w8_per_channel_decode_tiles(m, n, k, fp8):
 
 # ---- routed experts (b2l_moe_sort / b2l_moe_gather / b2l_moe_pair_gemm) ----
 @pytest.mark.parametrize("fmt", ["fp8", "int8"])
-@pytest.mark.parametrize("hidden,inter,gn,gk", [(256, 128, 128, 128), (400, 208, 16, 512), (1024, 320, 64, 128)])
-def test_experts_with_runs_around_the_tile(fmt, hidden, inter, gn, gk):
-    """Runs of 0, 1, 16, 17, 32, 33, 127, 128, 129 and 300 rows; outputs and intermediate columns past the last tile."""
-    runs = [0, 1, 16, 17, 32, 33, 127, 128, 129, 300]
+@pytest.mark.parametrize("hidden,inter,gn,gk", [(256, 128, 128, 128), (400, 208, 16, 512), (1024, 320, 64, 128),
+                                                (2176, 1152, 128, 128)])
+@pytest.mark.parametrize("idle", [0, 30])
+def test_experts_with_runs_around_the_tile(fmt, hidden, inter, gn, gk, idle):
+    """Runs of 0, 1, 16, 17, 32, 33, 127, 128, 129 and 300 rows; outputs and intermediate columns past the last tile.  With 30
+    idle experts beside them the rows per expert are few enough for tiles of 64 rows.  2176 x 1152: 108 to 153 tiles for 74
+    pairs and odd stage counts, so pairs go from one expert's tile to another's."""
+    runs = [0, 1, 16, 17, 32, 33, 127, 128, 129, 300] + [0] * idle
     E, top_k = len(runs), 1
     ids = torch.cat([torch.full((n,), e) for e, n in enumerate(runs)])
     ids = ids[torch.randperm(ids.numel())].view(-1, top_k).cuda()
@@ -155,7 +170,11 @@ def test_experts_with_runs_around_the_tile(fmt, hidden, inter, gn, gk):
     w1, s1, d1 = weight(2 * inter, hidden)
     w2, s2, d2 = weight(hidden, inter)
     tw = torch.rand(T, top_k, device="cuda").half()
-    got = K().fused_moe(x, w1, w2, tw, ids, w1_scale=s1, w2_scale=s2, group_n=gn, group_k=gk)
+    def call():
+        return K().fused_moe(x, w1, w2, tw, ids, w1_scale=s1, w2_scale=s2, group_n=gn, group_k=gk)
+
+    got = call()
+    assert torch.equal(call(), got)          # the order of an expert's rows may differ, their values not
     want = torch.empty(T, hidden, dtype=torch.float64, device="cuda")
     for e in range(E):
         t = (ids[:, 0] == e).nonzero()[:, 0]
@@ -207,7 +226,8 @@ def test_quantiser_in_vectors_equals_the_scalar_one(m, k, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("tokens,n,top_k", [(1, 8, 1), (3, 2048, 8), (70, 264, 9), (5, 100, 8)])
+@pytest.mark.parametrize("tokens,n,top_k", [(1, 8, 1), (3, 2048, 8), (70, 264, 9), (5, 100, 8), (445, 8, 1),
+                                            (300, 264, 9), (120, 2048, 8), (500, 100, 8)])
 @pytest.mark.parametrize("addend", [False, True])
 def test_expert_sum_in_vectors(tokens, n, top_k, addend, dtype):
     from lite_llama_b200 import _lib
