@@ -1,8 +1,9 @@
 // W4A16 projections of small decode batches (up to 8 tokens), on the reference's tensors or the load-time repacked layout
 // (formats and reference lines: gemm_quant.cu); the same bits from both.
 //
-// Bound: HBM; what stands in the way is latency and then the issue slots of the conversion.  The streaming kernel
-// (gemm_quant.cu) passes every 16 KiB of weights through three hand-offs (TMA -> conversion warps -> tensor memory -> MMA
+// Bound: HBM; what stands in the way is latency and then the conversion (one token, 28672 x 4096: 52 % of the issue slots are
+// used, and the warps that do not issue wait for their turn or the math pipe, not for memory; profiles/pair_gemm_ncu.txt).
+// The streaming kernel (gemm_quant.cu) passes every 16 KiB of weights through three hand-offs (TMA -> conversion warps -> tensor memory -> MMA
 // warp -> epilogue warps), 0.7 us per block and SM, after 2 us of set-up, and adds up shared tiles across CTAs: 7 - 20 us for
 // projections that take 1.5 - 10 us to read.  With so few tokens the products are cheap enough for mma.sync, whose operands
 // are registers, so here a warp does everything for its weights and hands over nothing but sums:

@@ -6,13 +6,15 @@
 // 64 tokens of MMAs last 256 cycles, so its hand-offs were the critical path (430 - 500 TF/s).  Here the tile is 256
 // weight rows x 128 tokens on a pair of SMs:
 //   * 128 rows x 128 k feed 512 cycles of MMAs per SM: conversion (two groups of four warps, each its own half of the
-//     operand stages) plus the drain of one accumulator segment take ~60 % of the issue slots;
+//     operand stages) plus the drain of one accumulator segment take half of the issue slots (1024 tokens: int4 52 %, with the
+//     tensor pipe busy for 49 % of the cycles, fp8 45 and 56 %; profiles/pair_gemm_ncu.txt): what is left is waiting at hand-offs;
 //   * cta_group::2: each SM stages 64 of the 128 tokens, 48 bytes per clock and SM from L2 for int4 weights;
 //   * the operand stays in tensor memory (4 stages of 128 k = 256 columns) beside two accumulator segments of 128 columns;
 //   * a segment's buffer is handed back as soon as its 128 columns are in the registers of eight epilogue warps, before the
 //     multiply-adds: with four warps that read it in two turns the MMAs waited for the drain (977 us against 900);
 //   * the grid is persistent, rings run on across tiles.
-// Measured, 28672 x 4096 at 4096 tokens (streaming kernel -> this one): int4 1853 -> 900 us (1.07 PFLOP/s), fp8 in 128 x 128
+// Measured, 28672 x 4096 at 4096 tokens, launches by themselves (streaming kernel -> this one; 15 - 20 % more in a pass that
+// keeps the card at its power cap): int4 1853 -> 900 us (1.07 PFLOP/s), fp8 in 128 x 128
 // blocks 1748 -> 867 us, int8 per channel 3124 -> 754 us (no drain before the end of k: 1.28 PFLOP/s).  A third accumulator
 // at the cost of two operand stages: int4 878, fp8 901 us.
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of
