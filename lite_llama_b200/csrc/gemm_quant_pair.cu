@@ -73,7 +73,7 @@ __device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c
 // expert's run of the sorted activations (moe_sort, moe_routing.cu), the entries' output tiles next to one another so that
 // the pairs in flight share the activations and an expert's second entry finds the weights in L2.  The table and the slot
 // order are earlier kernels' output, and this one may be resident before they are written: never read as data that is
-// constant for the kernel (__ldg).  Through L2 (__ldcg) every role paid 3 % of a small batch for it: ld_upstream.
+// constant for the kernel (__ldg).
 enum { QP_PLAIN = 0, QP_GATE_UP = 1, QP_DOWN = 2 };
 struct QpTile { int n, m0, rows, expert; };
 template <int MODE>

@@ -136,7 +136,8 @@ moe_sort_kernel(const void* __restrict__ topk_ids, int id_width, int num_slots, 
   }
 }
 
-// out[r, :] = x[order[r] / top_k, :]; one warp per sorted row, 16-byte accesses
+// out[r, :] = x[order[r] / top_k, :]; one warp per sorted row, 16-byte accesses.  Bound by latency: four loads of a lane are
+// under way before the first store (one at a time, a layer of 8 experts of 4096 x 1792 took 60.3 us instead of 55.3 at 8 tokens)
 __global__ void __launch_bounds__(256)
 moe_gather_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, const int32_t* __restrict__ order, int num_slots,
                   int top_k, int64_t x_stride, int64_t chunks) {
@@ -146,7 +147,13 @@ moe_gather_kernel(uint4* __restrict__ out, const uint4* __restrict__ x, const in
   if (r >= rows) return;
   const uint4* src = x + (int64_t)(ld_upstream(order + r) / top_k) * x_stride;
   uint4* dst = out + (int64_t)r * chunks;
-  for (int64_t c = threadIdx.x & 31; c < chunks; c += 32) dst[c] = __ldcg(src + c);
+  for (int64_t c = threadIdx.x & 31; c < chunks; c += 128) {
+    uint4 v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) if (c + 32 * i < chunks) v[i] = __ldcg(src + c + 32 * i);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) if (c + 32 * i < chunks) dst[c + 32 * i] = v[i];
+  }
 }
 
 // One warp per token: softmax over E logits (fp32), k rounds of arg-max (lowest index wins ties),
