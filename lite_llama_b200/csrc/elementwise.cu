@@ -870,10 +870,7 @@ extern "C" int b2l_moe_sum(void* out, const void* in, const void* addend, int64_
   if (tokens == 0 || n == 0) return B2L_OK;
   dim3 grid((unsigned)cdiv64(n, 256), (unsigned)(tokens > 65535 ? 65535 : tokens));
   cudaStream_t st = (cudaStream_t)stream;
-  // Up to three blocks per SM the kernel with one column per thread is the faster one (one row for each of 7 tokens of 4096:
-  // 1.3 against 1.5 us, eight rows of 32 x 2048: 1.8 / 1.7; in 512 blocks, 32 x 4096: 2.2 / 1.9)
-  if (tokens * cdiv64(n, 256) > 3LL * b2l_num_sms() && dtype != B2L_F32 && n % 8 == 0 &&
-      ((uintptr_t)out | (uintptr_t)in | (uintptr_t)addend) % 16 == 0 &&
+  if (dtype != B2L_F32 && n % 8 == 0 && ((uintptr_t)out | (uintptr_t)in | (uintptr_t)addend) % 16 == 0 &&
       cdiv64(tokens * (n / 8), 256) < (1ll << 31)) {
     const int64_t items = tokens * (n / 8);
     const dim3 blocks((unsigned)cdiv64(items, 256));
