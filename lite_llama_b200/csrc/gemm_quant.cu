@@ -6,9 +6,9 @@
 //   int4 : qweight int32 [N, K/8], nibble j of word i = K index 8i+j; scales, zeros fp32 [N, K/g]
 //   8-bit: qweight uint8(e4m3)/int8 [N, K]; scales fp32 [ceil(N/gn), ceil(K/gk)]
 //
-// Up to 8 tokens of int4 run in gemm_quant_decode.cu, prompt-sized batches (and 8-bit weights with one scale per output row
-// at any size with enough tiles) in gemm_quant_pair.cu; this file streams the weights for what lies between, for fine scale
-// groups and for int4 zero points that are not whole numbers.
+// Up to 8 tokens of int4 run in gemm_quant_decode.cu, up to 64 tokens in gemm_quant_batch.cu, prompt-sized batches in
+// gemm_quant_pair.cu; this file streams the weights for what lies between, for scale groups that are no multiple of 128, for
+// larger batches of int4 in the reference's layout and for repacked int4 with zero points that are not whole numbers.
 //
 // Pipeline per CTA (tile orientation: gemm_tc.cuh -- 128 weight rows on the TMEM lanes, tokens on UMMA N):
 //   TMA producer     raw quantised weight tile (128 rows x 128 BYTES, 128B-swizzled) + the matching
@@ -36,6 +36,7 @@
 #include "dequant.cuh"
 #include "gemm_quant_pair.cuh"
 #include "gemm_quant_decode.cuh"
+#include "gemm_quant_batch.cuh"
 #include <type_traits>
 #include <stdlib.h>
 
@@ -1403,9 +1404,14 @@ extern "C" int b2l_debug_set_timeline(void* device_buffer) {
 }
 extern "C" int64_t b2l_quant_gemm_workspace_bytes(int kind, int64_t m, int64_t n, int64_t k, int64_t group_k) {
   if (m <= 0 || n <= 0 || k <= 0 || group_k <= 0) return 0;
-  SplitPlan pl = quant_plan(kind, m, n, k, seg_len_for(kind, k, group_k));
-  if (pl.splits <= 1) return 0;
-  return (int64_t)pl.n_tiles * pl.m_tiles * pl.splits * pl.bt * kBlockW * 4;
+  const int seg_len = seg_len_for(kind, k, group_k);
+  SplitPlan pl = quant_plan(kind, m, n, k, seg_len);
+  int64_t bytes = pl.splits <= 1 ? 0 : (int64_t)pl.n_tiles * pl.m_tiles * pl.splits * pl.bt * kBlockW * 4;
+  if (quant_batch_takes(kind, m, n, k, seg_len)) {
+    const int64_t batch = quant_batch_workspace_bytes(kind, m, n, k);
+    bytes = batch > bytes ? batch : bytes;
+  }
+  return bytes;
 }
 // Launch plan of a quantised GEMM (pure function of shapes and the SM count; no GPU work):
 // out[0..9] = {stream-K CTAs (0 = tile x split grid), workspace slots per tile, raw blocks per tile, weight-row tiles,
@@ -1437,6 +1443,14 @@ extern "C" int b2l_w4a16_matmul(void* y, const void* x, const void* qweight, con
   B2L_REQUIRE(x_row_stride % 8 == 0 && qw_row_stride % 4 == 0,
               "w4a16_matmul: row strides must be 16-byte multiples (K a multiple of 32)");
   if (m == 0) return B2L_OK;
+  if (quant_batch_wanted(Q_INT4, 0, m, n, k, group_size) && workspace_bytes >= quant_batch_workspace_bytes(Q_INT4, m, n, k)) {
+    QuantBatchParams q;
+    q.y = (__half*)y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
+    q.scales = (const float*)scales; q.s_stride_n = s_row_stride; q.s_stride_k = s_col_stride; q.zeros = (const float*)zeros;
+    q.group_n = 1;
+    q.ws = (uint32_t*)workspace;
+    return quant_batch_gemm(Q_INT4, 0, q, x, x_row_stride, qweight, qw_row_stride * 4, m, n, k, group_size, 0, (cudaStream_t)stream);
+  }
   if (quant_decode_wanted(m, k, group_size) && (uintptr_t)x % 16 == 0 && (uintptr_t)qweight % 16 == 0)
     return quant_decode_gemm(0, y, y_row_stride, x, x_row_stride, qweight, qw_row_stride, (const float*)scales,
                              (const float*)zeros, s_row_stride, s_col_stride, bias, bias_is_f32, m, n, k, group_size, 0,
@@ -1474,6 +1488,15 @@ extern "C" int b2l_w4a16_matmul_packed(void* y, const void* x, const void* qweig
   B2L_REQUIRE(epilogue == 0 || epilogue == 1, "w4a16_matmul_packed: epilogue %d (0 = none, 1 = swiglu over interleaved rows)", epilogue);
   B2L_REQUIRE(epilogue == 0 || n % 2 == 0, "w4a16_matmul_packed: the swiglu epilogue needs an even number of rows");
   if (m == 0) return B2L_OK;
+  if (zeros_foldable && quant_batch_wanted(Q_INT4, 1, m, n, k, group_size) &&
+      workspace_bytes >= quant_batch_workspace_bytes(Q_INT4, m, n, k)) {
+    QuantBatchParams q;
+    q.y = (__half*)y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
+    q.scales = (const float*)scales_packed; q.s_stride_n = q.s_stride_k = 0; q.zeros = (const float*)zeros_packed; q.group_n = 1;
+    q.ws = (uint32_t*)workspace;
+    return quant_batch_gemm(Q_INT4, 1, q, x, x_row_stride, qweight_packed, qw_row_stride * 4, m, n, k, group_size, epilogue,
+                            (cudaStream_t)stream);
+  }
   if (quant_decode_wanted(m, k, group_size) && (uintptr_t)x % 16 == 0 && (uintptr_t)qweight_packed % 16 == 0)
     return quant_decode_gemm(1, y, y_row_stride, x, x_row_stride, qweight_packed, qw_row_stride, (const float*)scales_packed,
                              (const float*)zeros_packed, 0, 0, bias, bias_is_f32, m, n, k, group_size, epilogue,
@@ -1564,6 +1587,14 @@ extern "C" int b2l_w8a16_matmul(void* y, const void* x, const void* qweight, int
   if (m == 0) return B2L_OK;
   const int qk = weight_is_fp8 ? Q_FP8 : Q_INT8;
   const int seg_len = seg_len_for(qk, k, group_k);
+  if (quant_batch_wanted(qk, 0, m, n, k, seg_len) && workspace_bytes >= quant_batch_workspace_bytes(qk, m, n, k)) {
+    QuantBatchParams q;
+    q.y = (__half*)y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
+    q.scales = (const float*)scales; q.s_stride_n = s_row_stride; q.s_stride_k = s_col_stride; q.zeros = nullptr;
+    q.group_n = (int)(group_n > n ? n : group_n);
+    q.ws = (uint32_t*)workspace;
+    return quant_batch_gemm(qk, 0, q, x, x_row_stride, qweight, qw_row_stride, m, n, k, seg_len, 0, (cudaStream_t)stream);
+  }
   if (quant_pair_wanted(qk, m, n, k, seg_len)) {
     QuantPairParams q;
     q.y = y; q.ldy = y_row_stride; q.bias = bias; q.bias_is_f32 = bias_is_f32;
