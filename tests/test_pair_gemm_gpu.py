@@ -263,3 +263,16 @@ def test_per_channel_accumulations_are_no_longer_than_the_parts_of_k(m, n, k, ch
     s = torch.rand(n, 1, device="cuda") * 1e-4 + 1e-4
     got, want = K().w8a16_matmul(x, q, s, group_n=1, group_k=k).double(), x.double() @ (w * s.double()).T
     assert abs(((got - want) / want).mean().item()) < chain / 16 * 2.0**-23
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 136, 64), (17, 1000, 256), (130, 520, 512), (300, 10248, 144), (256, 3584, 2048)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_int8_scales_in_vectors_and_alone(m, n, k, shift):
+    """Scales and bias that start on a 16-byte boundary are loaded in vectors, others one by one: the same result."""
+    qa = torch.randint(-127, 128, (m, k), device="cuda", dtype=torch.int8)
+    qw = torch.randint(-127, 128, (n, k), device="cuda", dtype=torch.int8)
+    sa, sw, b = ((torch.rand(v + 1, device="cuda") * 1e-2)[shift : shift + v] for v in (m, n, n))
+    want = (qa.double() @ qw.double().T) * sa.double()[:, None] * sw.double() + b.double()
+    got = K().smoothquant_matmul_prequant(qa, sa, qw, sw, bias=b)
+    assert rel(got, want) < REL[torch.float16]
+    assert torch.equal(got, K().smoothquant_matmul_prequant(qa, sa.clone(), qw, sw.clone(), bias=b.clone()))
