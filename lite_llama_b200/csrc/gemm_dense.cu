@@ -268,13 +268,13 @@ static int launch(const CUtensorMap& tw, const CUtensorMap& tx, const DenseParam
 }
 
 // One wave of this kernel over a short k is over before the pair kernel has set up and drained its larger tiles (us, this one
-// against pairs): bf16 129 x 5120 x 256 4.4 / 4.9, but x 640 6.3 / 5.9; int8 257 x 5120 x 256 6.7 / 10.5, 129 x 5128 x 896 7.5 /
-// 8.2, but 129 x 5120 x 2048 9.6 / 9.1.  Of 64-token tiles with so few stages several share an SM; two 128-token tiles of int8
-// on one SM are as slow as two waves (512 x 5120 x 256: 11.7 / 10.6).
-static bool one_short_wave(int kind, const SplitPlan& pl, int64_t k) {
+// against pairs): bf16 129 x 5120 x 256 4.4 / 4.9, but x 640 6.3 / 5.9; int8 300 x 5120 x 256 4.9 / 5.9, but 129 x 3584 x 896 5.6 /
+// 5.1, 129 x 2048 x 1792 9.4 / 5.9.  Of 64-token tiles with so few stages several share an SM; two 128-token tiles of int8
+// on one SM are as slow as two waves (512 x 5120 x 256).
+static bool one_short_wave(const SplitPlan& pl, int64_t k) {
   const int64_t smem = b2l_max_smem_optin() + 1024;
   const int64_t resident = pl.bt <= 64 && pl.smem_bytes + 1024 < smem ? smem / (pl.smem_bytes + 1024) : 1;
-  return (int64_t)pl.n_tiles * pl.m_tiles * pl.splits <= resident * b2l_num_sms() && k < (kind == 0 ? 512 : 2048);
+  return (int64_t)pl.n_tiles * pl.m_tiles * pl.splits <= resident * b2l_num_sms() && k < 512;
 }
 
 }  // namespace gemm
@@ -306,7 +306,7 @@ extern "C" int b2l_linear(void* y, const void* x, const void* w, const void* bia
   if (m == 0) return B2L_OK;
   const PairGemm pg{y, y_row_stride, bias, nullptr, nullptr, m, n, k, x_row_stride, w_row_stride, x, w};
   SplitPlan pl = make_plan(m, n, k, 64, 0, 1024, 4);
-  if (pair_gemm_wanted(0, pg) && !one_short_wave(0, pl, k)) return pair_gemm(0, dtype, pg, (cudaStream_t)stream);
+  if (pair_gemm_wanted(0, pg) && !one_short_wave(pl, k)) return pair_gemm(0, dtype, pg, (cudaStream_t)stream);
   DenseParams p;
   p.y = y; p.ldy = y_row_stride; p.bias = bias; p.a_scale = nullptr; p.b_scale = nullptr; p.a_vec = 0;
   p.M = (int)m; p.N = (int)n; p.splits = pl.splits; p.kb_per_split = pl.kb_per_split; p.num_kb = pl.num_kb;
@@ -342,7 +342,7 @@ extern "C" int b2l_w8a8_gemm(void* y, const void* xq, const void* wq, const void
   const PairGemm pg{y, y_row_stride, bias_f32, (const float*)a_scale, (const float*)b_scale, m, n, k, xq_row_stride,
                     wq_row_stride, xq, wq};
   SplitPlan pl = make_plan(m, n, k, 128, 0, 1024, 4);
-  if (pair_gemm_wanted(1, pg) && !one_short_wave(1, pl, k)) return pair_gemm(1, out_dtype, pg, (cudaStream_t)stream);
+  if (pair_gemm_wanted(1, pg) && !one_short_wave(pl, k)) return pair_gemm(1, out_dtype, pg, (cudaStream_t)stream);
   DenseParams p;
   p.y = y; p.ldy = y_row_stride; p.bias = bias_f32; p.a_scale = (const float*)a_scale; p.b_scale = (const float*)b_scale;
   p.a_vec = (uintptr_t)a_scale % 16 == 0;

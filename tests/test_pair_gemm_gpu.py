@@ -276,3 +276,33 @@ def test_int8_scales_in_vectors_and_alone(m, n, k, shift):
     got = K().smoothquant_matmul_prequant(qa, sa, qw, sw, bias=b)
     assert rel(got, want) < REL[torch.float16]
     assert torch.equal(got, K().smoothquant_matmul_prequant(qa, sa.clone(), qw, sw.clone(), bias=b.clone()))
+
+
+# Clusters of two and four pairs that share a tile: parts of k of unequal length, a k tail, outputs that end inside a tile, one
+# to four token tiles, tokens in the first CTA of a pair only
+SPLIT_EDGES = [(65, 896, 4872), (128, 3584, 2056), (129, 1000, 2112), (256, 3400, 4200), (700, 776, 4104), (256, 4096, 4232),
+               (500, 2056, 8200), (1000, 1800, 5208), (600, 2300, 10248)]
+
+
+@pytest.mark.parametrize("m,n,k", SPLIT_EDGES)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("bias", [False, True])
+def test_linear_split_over_a_cluster(m, n, k, dtype, bias):
+    x = torch.randn(m, k, device="cuda", dtype=dtype)
+    w = torch.randn(n, k, device="cuda", dtype=dtype) * 0.05
+    b = torch.randn(n, device="cuda", dtype=dtype) if bias else None
+    want = x.double() @ w.double().T + (b.double() if bias else 0.0)
+    got = K().linear(x, w, b)
+    assert rel(got, want) < REL[dtype] and torch.equal(K().linear(x, w, b), got)
+
+
+@pytest.mark.parametrize("m,n,k", SPLIT_EDGES)
+@pytest.mark.parametrize("bias", [False, True])
+def test_int8_split_over_a_cluster(m, n, k, bias):
+    k = (k + 15) // 16 * 16
+    qa = torch.randint(-127, 128, (m, k), device="cuda", dtype=torch.int8)
+    qw = torch.randint(-127, 128, (n, k), device="cuda", dtype=torch.int8)
+    sa, sw = torch.rand(m, device="cuda") * 1e-3, torch.rand(n, device="cuda") * 1e-2
+    b = torch.randn(n, device="cuda") if bias else None
+    want = (qa.double() @ qw.double().T) * sa.double()[:, None] * sw.double() + (b.double() if bias else 0.0)
+    assert rel(K().smoothquant_matmul_prequant(qa, sa, qw, sw, bias=b), want) < REL[torch.float16]
