@@ -19,11 +19,14 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent / "csrc"
 OUT = Path(__file__).resolve().parent / "libb200lite.so"
+FAST_SRC = CSRC / "host" / "fast_calls.cpp"
+FAST_OUT = Path(__file__).resolve().parent / "_fast.so"
 OBJ_DIR = CSRC / "build"
 
 NVCC_FLAGS = [
@@ -83,6 +86,34 @@ def linked_sources() -> set[str]:
     return set(LINK_STAMP.read_text().split())
 
 
+def build_fast(force: bool = False) -> str | None:
+    """The native form of the hot shims, built against this interpreter and this torch.  None, or why it could not be built:
+    the shims then run in Python, slower on the host and otherwise the same."""
+    try:
+        import torch
+    except ImportError as e:
+        return str(e)
+    root = Path(torch.__file__).resolve().parent
+    include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"],
+               Path(_nvcc()).resolve().parent.parent / "include"]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DBUILT_FOR_TORCH="{torch.__version__}"',
+           *(f"-I{d}" for d in include), str(FAST_SRC), "-o", str(FAST_OUT), f"-L{root / 'lib'}",
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
+    stamp = hashlib.sha256((" ".join(cmd) + sys.version).encode() + FAST_SRC.read_bytes()).hexdigest()
+    stamp_file = OBJ_DIR / "fast_calls.stamp"
+    if not force and FAST_OUT.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
+        return None
+    try:
+        res = subprocess.run(cmd, capture_output=True, text=True)
+    except OSError as e:
+        return str(e)
+    if res.returncode != 0:
+        return res.stderr
+    stamp_file.write_text(stamp)
+    return None
+
+
 def build(force: bool = False, verbose: bool = True, sources: tuple[str, ...] | None = None) -> Path:
     OBJ_DIR.mkdir(exist_ok=True)
     every = sorted(CSRC.glob("*.cu"))
@@ -94,8 +125,12 @@ def build(force: bool = False, verbose: bool = True, sources: tuple[str, ...] | 
         if wanted <= have and not force:
             wanted = have                     # a fuller library is kept (and refreshed if its sources changed)
         every = [s for s in every if s.stem in wanted]
-    with ThreadPoolExecutor(max_workers=min(8, len(every))) as pool:
+    with ThreadPoolExecutor(max_workers=min(8, len(every)) + 1) as pool:
+        fast = pool.submit(build_fast, force)
         objs = list(pool.map(lambda s: _compile(s, force), every))
+    why = fast.result()
+    if why and verbose:
+        print(f"[b200lite] {FAST_OUT.name} was not built, the shims run in Python: {why}")
     newest = max(o.stat().st_mtime for o in objs)
     stems = sorted(s.stem for s in every)
     if force or not OUT.exists() or OUT.stat().st_mtime < newest or linked_sources() != set(stems):

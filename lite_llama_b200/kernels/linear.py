@@ -8,12 +8,21 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from ._common import as_rows, check, counters, dtype_code, float_code, lib, no_grad, own_rows, ptr, require_cuda, stream_handle, unrows, weights_written, workspace
 
 
-@no_grad
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
     """``[..., K] @ [N, K].T -> [..., N]`` in ``x``'s dtype, fp32 accumulation."""
+    if bias is None:
+        out = _native.linear(x, weight)
+        if out is not None:
+            return out
+    return _linear(x, weight, bias)
+
+
+@no_grad
+def _linear(x, weight, bias):
     require_cuda(x, weight, bias)
     if x.dtype == torch.float32 or x.shape[-1] % 8 != 0:
         return linear_simt(x, weight, bias)       # exact fp32, or a K the TMA tiles cannot start on

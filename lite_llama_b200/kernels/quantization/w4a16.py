@@ -4,6 +4,7 @@ from __future__ import annotations
 
 import torch
 
+from .. import _native
 from .._common import as_rows, check, counters, current_device, lib, no_grad, own_rows, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
 
 _Q_INT4 = 0
@@ -114,7 +115,6 @@ def w4a16_pack(qweight: torch.Tensor, scales: torch.Tensor, zeros: torch.Tensor,
     return PackedW4(qp, sp, zp, n, k, int(group_size), foldable)
 
 
-@no_grad
 def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor | None = None,
                         swiglu: bool = False) -> torch.Tensor:
     """:func:`w4a16_matmul` on a :class:`PackedW4` (same result, bit for bit in the integer unpack).
@@ -122,6 +122,16 @@ def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor
     ``swiglu=True``: the packed rows are interleaved ``(gate_0, up_0, gate_1, up_1, ...)`` (see
     :func:`interleave_gate_up`) and the GEMM's epilogue applies ``silu(gate) * up``; the result is ``[..., N/2]``
     and equals ``swiglu_forward`` of the two separate projections bit for bit."""
+    if bias is None:
+        out = _native.w4a16_packed(x, packed.qweight, packed.scales, packed.zeros, packed.n, packed.k, packed.group_size,
+                                   packed.zeros_foldable, swiglu)
+        if out is not None:
+            return out
+    return _w4a16_matmul_packed(x, packed, bias, swiglu)
+
+
+@no_grad
+def _w4a16_matmul_packed(x, packed, bias, swiglu):
     if x.dtype != torch.float16:
         raise ValueError(f"w4a16 activations must be fp16, got {x.dtype}")
     require_cuda(x, bias)

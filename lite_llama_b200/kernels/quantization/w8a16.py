@@ -4,12 +4,12 @@ from __future__ import annotations
 
 import torch
 
+from .. import _native
 from .._common import as_rows, check, counters, current_device, lib, no_grad, own_rows, ptr, quant_gemm_workspace_bytes, require_cuda, stream_handle, unrows, weights_written, zeroed_workspace
 
 _Q_FP8, _Q_INT8 = 1, 2
 
 
-@no_grad
 def w8a16_matmul(
     x: torch.Tensor,
     qweight: torch.Tensor,
@@ -21,6 +21,15 @@ def w8a16_matmul(
 ) -> torch.Tensor:
     """``x @ dequant(qweight).T (+ bias)``; ``qweight [N, K]`` uint8 (fp8-e4m3 bits) or int8,
     ``scales [ceil(N/group_n), ceil(K/group_k)]`` fp32."""
+    if bias is None:
+        out = _native.w8a16(x, qweight, scales, group_n, group_k)
+        if out is not None:
+            return out
+    return _w8a16_matmul(x, qweight, scales, group_n, group_k, bias)
+
+
+@no_grad
+def _w8a16_matmul(x, qweight, scales, group_n, group_k, bias):
     is_fp8 = qweight.dtype == torch.uint8
     if not is_fp8 and qweight.dtype != torch.int8:
         raise ValueError(f"qweight must be uint8 (fp8) or int8, got {qweight.dtype}")

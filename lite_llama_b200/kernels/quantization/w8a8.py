@@ -4,13 +4,18 @@ from __future__ import annotations
 
 import torch
 
+from .. import _native
 from .._common import as_rows, check, counters, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle, unrows, weights_written, workspace
 
 
-@no_grad
 def quantize_activations_int8(a: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
     """Per-token dynamic int8 quantisation: ``scale = absmax/127``, ``q = trunc(x / scale)``
     (reference kernel: w8a8.py:35-68). Returns ``(q [M, K] int8, scales [M] fp32)``."""
+    return _native.quantize(a) or _quantize_activations_int8(a)
+
+
+@no_grad
+def _quantize_activations_int8(a):
     require_cuda(a)
     m, k = a.shape
     q = torch.empty((m, k), dtype=torch.int8, device=a.device)
@@ -24,7 +29,6 @@ def quantize_activations_int8(a: torch.Tensor) -> tuple[torch.Tensor, torch.Tens
     return q, s
 
 
-@no_grad
 def smoothquant_matmul_prequant(
     qa: torch.Tensor,
     a_scales: torch.Tensor,
@@ -37,6 +41,15 @@ def smoothquant_matmul_prequant(
     """The int8 GEMM half of :func:`smoothquant_matmul` (w8a8.py:75-130) on activations that are already
     quantised (``qa [M, K] int8``, ``a_scales [M] fp32``): ``(qa @ qweight.T) * a_scales[:, None] * weight_scales
     (+ bias)`` in ``out_dtype``."""
+    if bias is None and out_dtype in (torch.float16, torch.bfloat16):
+        out = _native.w8a8(qa, a_scales, qweight, weight_scales, out_dtype == torch.bfloat16)
+        if out is not None:
+            return out
+    return _smoothquant_matmul_prequant(qa, a_scales, qweight, weight_scales, bias, out_dtype)
+
+
+@no_grad
+def _smoothquant_matmul_prequant(qa, a_scales, qweight, weight_scales, bias, out_dtype):
     require_cuda(qa, a_scales, qweight, weight_scales, bias)
     if qa.dtype != torch.int8 or qweight.dtype != torch.int8:
         raise ValueError("smoothquant_matmul_prequant: activations and weights must be int8")

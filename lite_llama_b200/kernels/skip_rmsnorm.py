@@ -4,10 +4,10 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from ._common import check, dtype_code, lib, no_grad, ptr, require_cuda, stream_handle
 
 
-@no_grad
 def skip_rmsnorm(X, residual, weight, eps=1e-5):
     """``(Y, residual)``: ``residual += X`` in place, ``Y = rmsnorm(residual) * weight``.
 
@@ -15,6 +15,11 @@ def skip_rmsnorm(X, residual, weight, eps=1e-5):
     exactly like the reference (skip_rmsnorm.py:219,234). The last dim is normalised; any leading
     shape is accepted (the per-head q/k norm passes ``[tokens, heads, head_dim]``).
     """
+    return _native.norm(X, residual, weight, eps) or _skip_rmsnorm(X, residual, weight, eps)
+
+
+@no_grad
+def _skip_rmsnorm(X, residual, weight, eps):
     require_cuda(X, residual, weight)
     orig_shape = X.shape
     n = orig_shape[-1]
@@ -51,12 +56,19 @@ def can_fuse_int8_quant(n: int) -> bool:
     return n % 8 == 0 and n <= 16384
 
 
-@no_grad
 def skip_rmsnorm_quant_int8(X, residual, weight, eps=1e-5):
     """``skip_rmsnorm`` whose output goes straight into a SmoothQuant GEMM: returns ``(q int8 [rows, n],
     scales fp32 [rows], residual)`` -- the per-token dynamic quantisation of the (fp16-rounded) norm output
     (reference: skip_rmsnorm.py:192-234 then quantization/w8a8.py:35-68), bit-identical to calling the two ops,
     in one launch and without writing the fp16 activations."""
+    out = _native.norm_quant(X, residual, weight, eps)
+    if out is not None:
+        return *out, (X if residual is None else residual)
+    return _skip_rmsnorm_quant_int8(X, residual, weight, eps)
+
+
+@no_grad
+def _skip_rmsnorm_quant_int8(X, residual, weight, eps):
     require_cuda(X, residual, weight)
     orig_shape = X.shape
     n = orig_shape[-1]

@@ -4,11 +4,17 @@ from __future__ import annotations
 
 import torch
 
+from . import _native
 from ._common import as_rows, check, float_code, lib, no_grad, require_cuda, stream_handle, unrows
 
 
-@no_grad
 def swiglu_forward(a, b):
+    c = _native.swiglu(a, b)
+    return _swiglu_forward(a, b) if c is None else c
+
+
+@no_grad
+def _swiglu_forward(a, b):
     require_cuda(a, b)
     n_cols = a.shape[-1]
     a2, b2 = as_rows(a), as_rows(b) if b.shape[-1] == n_cols else b.reshape(-1, n_cols)
