@@ -373,6 +373,47 @@ __global__ void rope_kv_write_kernel(T* __restrict__ q, T* __restrict__ k, const
   }
 }
 
+// The same in units of 16 bytes, one unit a thread, with the token's units spread over blocks.  Bound by latency: above, a
+// decode step's thread makes seven dependent trips to L2 for a token of 32 + 8 heads of 128, here one (launches one after the
+// other in a graph, us: 1 token 3.2 -> 1.3, 32 tokens 3.9 -> 1.5, 256 8.0 -> 2.5, 2048 13.2 -> 9.0).
+template <typename T>
+__global__ void __launch_bounds__(128)
+rope_kv_write_vec_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict__ v, const T* __restrict__ cosp,
+                         const T* __restrict__ sinp, const void* __restrict__ select_index, int idx_width,
+                         T* __restrict__ pool, int seq_len, int n_qh, int n_kh, int hd, int64_t q_ts, int64_t q_hs, int64_t k_ts,
+                         int64_t k_hs, int64_t v_ts, int64_t v_hs, int64_t cs_b, int64_t cs_s, int64_t d_ts, int64_t d_hs) {
+  pdl_prologue();
+  using T2 = typename Vec2<T>::type;
+  const int tok = blockIdx.x, half = hd / 2, units = half / 8;
+  const int rot = (n_qh + n_kh) * units;
+  const int i = blockIdx.y * 128 + threadIdx.x;
+  if (i < rot) {
+    const int h = i / units, c = (i - h * units) * 8;
+    const bool is_k = h >= n_qh;
+    T* base = (is_k ? k + tok * k_ts + (int64_t)(h - n_qh) * k_hs : q + tok * q_ts + (int64_t)h * q_hs) + c;
+    const int64_t cs = (int64_t)(tok / seq_len) * cs_b + (int64_t)(tok % seq_len) * cs_s + c;
+    uint4 a = *reinterpret_cast<const uint4*>(base), b = *reinterpret_cast<const uint4*>(base + half);
+    const uint4 cv = *reinterpret_cast<const uint4*>(cosp + cs), sv = *reinterpret_cast<const uint4*>(sinp + cs);
+    const int64_t dest = is_k ? load_index(select_index, tok, idx_width) : 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      rope_pair(reinterpret_cast<T2*>(&a)[j], reinterpret_cast<T2*>(&b)[j], reinterpret_cast<const T2*>(&cv)[j],
+                reinterpret_cast<const T2*>(&sv)[j]);
+    *reinterpret_cast<uint4*>(base) = a;
+    *reinterpret_cast<uint4*>(base + half) = b;
+    if (is_k) {
+      T* row = pool + dest * d_ts + (int64_t)(h - n_qh) * d_hs + c;
+      *reinterpret_cast<uint4*>(row) = a;
+      *reinterpret_cast<uint4*>(row + half) = b;
+    }
+  } else if (i < rot + n_kh * 2 * units) {
+    const int j = i - rot, h = j / (2 * units), c = (j - h * 2 * units) * 8;
+    const uint4 val = *reinterpret_cast<const uint4*>(v + tok * v_ts + (int64_t)h * v_hs + c);
+    const int64_t dest = load_index(select_index, tok, idx_width);
+    *reinterpret_cast<uint4*>(pool + dest * d_ts + (int64_t)(n_kh + h) * d_hs + c) = val;
+  }
+}
+
 extern "C" int b2l_rope_kv_write(void* q, void* k, const void* v, const void* cos, const void* sin,
                                  const void* select_index, int index_width, void* kv_buffer, int64_t batch,
                                  int64_t seq_len, int n_qh, int n_kh, int head_dim, int64_t q_tok_stride,
@@ -392,21 +433,25 @@ extern "C" int b2l_rope_kv_write(void* q, void* k, const void* v, const void* co
   const int64_t tokens = batch * seq_len;
   if (tokens == 0) return B2L_OK;
   cudaStream_t st = (cudaStream_t)stream;
+  // whole 16-byte units in every row and half row
+  bool vec = head_dim % 16 == 0 && tokens < (1ll << 31) &&
+             ((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cos | (uintptr_t)sin | (uintptr_t)kv_buffer) % 16 == 0;
+  for (int64_t st : strides) vec = vec && st % 8 == 0;
+  const int64_t units = ((int64_t)n_qh + 3 * (int64_t)n_kh) * (head_dim / 16), parts = cdiv64(units, 128);
+  vec = vec && parts <= 65535;
   const int work = (n_qh + n_kh) * (head_dim / 4) + n_kh * (head_dim / 2);
-  const int threads = work >= 256 ? 256 : (work >= 128 ? 128 : 64);
-  if (dtype == B2L_F16)
-    b2l_launch(rope_kv_write_kernel<__half>, dim3((unsigned)tokens), dim3(threads), (size_t)0, st, (__half*)q, (__half*)k,
-               (const __half*)v, (const __half*)cos, (const __half*)sin, select_index, index_width, (__half*)kv_buffer,
-               (int)seq_len, n_qh, n_kh, head_dim, q_tok_stride, q_head_stride, k_tok_stride, k_head_stride, v_tok_stride,
-               v_head_stride, cs_batch_stride, cs_seq_stride, d_tok_stride, d_head_stride);
-  else if (dtype == B2L_BF16)
-    b2l_launch(rope_kv_write_kernel<__nv_bfloat16>, dim3((unsigned)tokens), dim3(threads), (size_t)0, st,
-               (__nv_bfloat16*)q, (__nv_bfloat16*)k, (const __nv_bfloat16*)v, (const __nv_bfloat16*)cos,
-               (const __nv_bfloat16*)sin, select_index, index_width, (__nv_bfloat16*)kv_buffer, (int)seq_len, n_qh, n_kh,
-               head_dim, q_tok_stride, q_head_stride, k_tok_stride, k_head_stride, v_tok_stride, v_head_stride,
-               cs_batch_stride, cs_seq_stride, d_tok_stride, d_head_stride);
+  const int threads = vec ? 128 : work >= 256 ? 256 : (work >= 128 ? 128 : 64);
+  const dim3 grid((unsigned)tokens, vec ? (unsigned)parts : 1);
+#define ROPE_KV(TT)                                                                                                          \
+  b2l_launch(vec ? rope_kv_write_vec_kernel<TT> : rope_kv_write_kernel<TT>, grid, dim3(threads), (size_t)0, st, (TT*)q,      \
+             (TT*)k, (const TT*)v, (const TT*)cos, (const TT*)sin, select_index, index_width, (TT*)kv_buffer, (int)seq_len,  \
+             n_qh, n_kh, head_dim, q_tok_stride, q_head_stride, k_tok_stride, k_head_stride, v_tok_stride, v_head_stride,    \
+             cs_batch_stride, cs_seq_stride, d_tok_stride, d_head_stride)
+  if (dtype == B2L_F16) ROPE_KV(__half);
+  else if (dtype == B2L_BF16) ROPE_KV(__nv_bfloat16);
   else
     B2L_UNSUPPORTED("rope_kv_write: dtype %d", dtype);
+#undef ROPE_KV
   B2L_LAUNCH_CHECK();
   return B2L_OK;
 }
