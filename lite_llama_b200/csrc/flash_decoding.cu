@@ -19,7 +19,9 @@
 //  * QK^T and PV on tensor cores with fp32 accumulation (fp16 products are exact in fp32, which
 //    keeps the reference's "fp32 product" precision, flashdecoding.py:115-120), fp32 online softmax;
 //  * split-KV sized from host-known quantities only (graph-safe); fp32 partials + log-sum-exp,
-//    merged by a second small kernel (reference stage 2, flashdecoding.py:224-313).
+//    merged by a second small kernel (reference stage 2, flashdecoding.py:224-313);
+//  * a step too small to fill the chip is bound by latency instead: its splits are the CTAs of a cluster, with as few kv
+//    heads each as still fit in one wave, and merge through one another's shared memory (FD_CLUSTER below).
 #include "common.cuh"
 
 namespace {
@@ -27,6 +29,7 @@ namespace {
 constexpr int kTT = 16;            // tokens per pipeline stage (one m16n8k16 k-step of PV)
 constexpr int kMaxConsumers = 8;
 constexpr int kMaxStages = 4;
+constexpr int kMaxCluster = 8;
 
 struct DecodeParams {
   const void* q; int64_t q_bs, q_hs;
@@ -50,7 +53,28 @@ struct DecodeParams {
 
 __host__ __device__ inline int row_pitch(int HB, int D) { return 2 * HB * D * 2 + 16; }  // +16: ldmatrix conflict-free
 
-template <typename T, int D>
+// all threads of the cluster that have not left; what each wrote to shared memory before is visible to the others after
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_smem(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_peer(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ld_peer4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// FD_CLUSTER: the grid's x is one cluster of up to kMaxCluster splits, which merge their results themselves.
+template <typename T, int D, bool FD_CLUSTER = false>
 __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_kernel(const DecodeParams p) {
   pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
   extern __shared__ __align__(128) uint8_t smem[];
@@ -66,7 +90,15 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
 
   const int64_t seq_len = load_index(p.seq_len, b, p.len_w);
   const int64_t start = (int64_t)split * p.chunk;
-  if (start >= seq_len) return;  // empty split: nothing to contribute (whole CTA exits together)
+  if (start >= seq_len) {        // empty split: nothing to contribute (whole CTA exits together)
+    if (FD_CLUSTER && split == 0) {                       // an empty row is zero
+      const int heads = p.HB * p.G;
+      for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +
+                                     (int64_t)(hblk * heads + i / (D / 2)) * p.o_hs + 2 * (i % (D / 2))) = 0u;
+    }
+    return;
+  }
   const int64_t end = (start + p.chunk < seq_len) ? start + p.chunk : seq_len;
   const int ntiles = (int)((end - start + kTT - 1) / kTT);
   const int64_t req = load_index(p.req_idx, b, p.req_w);
@@ -121,6 +153,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       }
       if (++s == p.stages) { s = 0; phase ^= 1; }
     }
+    if (FD_CLUSTER) __syncthreads();
   } else {
     // ===================== consumer warps: one (kv head, 16-query-head block) each =====================
     const int hl = warp / p.qblocks;            // kv head inside this CTA's block
@@ -236,6 +269,9 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       l_run[r2] += __shfl_xor_sync(0xffffffffu, l_run[r2], 1);
       l_run[r2] += __shfl_xor_sync(0xffffffffu, l_run[r2], 2);
     }
+    // Cluster: the partial rows go to the CTA's own shared memory, over the stages that every warp has finished with
+    float* part = reinterpret_cast<float*>(stage_base);
+    if (FD_CLUSTER) __syncthreads();
     // this warp saw every token of the split for its heads: write the result rows directly
 #pragma unroll
     for (int r2 = 0; r2 < 2; ++r2) {
@@ -243,7 +279,13 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       if (!ok) continue;
       const int head = kvh * p.G + (r2 == 0 ? hq0 : hq1);
       const float inv = 1.0f / l_run[r2];
-      if (p.splits == 1) {
+      if (FD_CLUSTER) {
+        const int local = hl * p.G + (r2 == 0 ? hq0 : hq1);
+#pragma unroll
+        for (int i = 0; i < D / 8; ++i)
+          *reinterpret_cast<float2*>(part + local * D + i * 8 + 2 * tq) = make_float2(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
+        if (tq == 0) part[p.HB * p.G * D + local] = m_run[r2] + log2f(l_run[r2]);
+      } else if (p.splits == 1) {
         T* orow = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)head * p.o_hs;
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
@@ -257,6 +299,47 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
         if (tq == 0) p.ws_lse[off] = m_run[r2] + log2f(l_run[r2]);
       }
     }
+  }
+
+  if (FD_CLUSTER) {
+    // Every CTA with tokens merges its share of the outputs, in split order like the kernel below.  (Empty splits have left; the
+    // barrier does not wait for them.)
+    __syncwarp();
+    cluster_sync_all();
+    const int nsp = (int)((seq_len + p.chunk - 1) / p.chunk) < p.splits ? (int)((seq_len + p.chunk - 1) / p.chunk) : p.splits;
+    const int heads = p.HB * p.G;
+    const uint32_t part = smem_u32(stage_base);
+    for (int i = split * blockDim.x + threadIdx.x; i < heads * (D / 4); i += nsp * blockDim.x) {
+      const int local = i / (D / 4), d = i % (D / 4) * 4;
+      float lse[kMaxCluster];
+      float4 v[kMaxCluster];
+#pragma unroll
+      for (int r = 0; r < kMaxCluster; ++r)
+        if (r < nsp) {
+          const uint32_t peer = peer_smem(part, r);
+          lse[r] = ld_peer(peer + (heads * D + local) * 4);
+          v[r] = ld_peer4(peer + (local * D + d) * 4);
+        }
+      float M = -INFINITY, L = 0.f;
+#pragma unroll
+      for (int r = 0; r < kMaxCluster; ++r)
+        if (r < nsp) M = fmaxf(M, lse[r]);
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int r = 0; r < kMaxCluster; ++r)
+        if (r < nsp) {
+          const float w = fast_exp2(lse[r] - M);
+          acc.x += w * v[r].x; acc.y += w * v[r].y; acc.z += w * v[r].z; acc.w += w * v[r].w;
+          L += w;
+        }
+      uint32_t* to = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +
+                                                 (int64_t)(hblk * heads + local) * p.o_hs + d);
+      to[0] = pack2<T>(acc.x / L, acc.y / L);
+      to[1] = pack2<T>(acc.z / L, acc.w / L);
+    }
+    __syncwarp();
+    cluster_sync_all();                 // the peers have read this CTA's rows
+    return;
   }
 
   // ---- stage 2 folded in (reference: a second kernel, flashdecoding.py:224-313): the CTA that finishes a
@@ -350,7 +433,43 @@ __global__ void flash_decode_combine_kernel(const DecodeParams p) {
   }
 }
 
-struct Plan { int splits, chunk, qblocks, HB, stages, smem; };
+struct Plan { int splits, chunk, qblocks, HB, stages, smem; bool cluster; };
+
+// ring of a block of HB kv heads: stages and bytes
+void plan_ring(Plan& pl, int D, int smem_cap) {
+  const int stage = kTT * row_pitch(pl.HB, D);
+  int stages = kMaxStages;
+  while (stages > 2 && stages * stage > smem_cap) --stages;
+  // prefer two resident CTAs per SM when a 3-deep ring fits in half the shared memory
+  if (stages * stage > smem_cap / 2 && 3 * stage <= smem_cap / 2) stages = 3;
+  pl.stages = stages;
+  pl.smem = stages * stage + 128;
+}
+
+// Steps of up to 256 tokens a row that leave most of the chip idle: one wave of clusters of eight splits, two of their CTAs to an
+// SM.  A tile costs its CTA 0.6 - 1 us (copies, and one warp's chain of products), the merge kernel 3 us, a cluster's launch and
+// barriers 2 us.  us in a graph, splits of 64 tokens and the merge kernel -> this: 8 kv heads of 128, one sequence of 200 tokens
+// 8.5 -> 6.6, of 80 7.2 -> 5.0, eight of 200 8.6 -> 7.5; 18 of 4 kv heads 8.6 -> 7.2; rows of a quarter of the bound 8.2 -> 6.1 (one
+// sequence), 6.1 - 8.2 -> 5.3 - 7.7 (4 kv heads; slower in one case of twenty, eight rows of 20 tokens under a bound of 80, 6.1 ->
+// 6.4).  Longer splits are the longer chain here (512 tokens in four tiles each 9.1 against 8.9), up to four tiles there is a single
+// split without a merge (40 tokens 5.3 against 6.0), and with one CTA to an SM the clusters of eight do not all fit (16 sequences
+// of 8 kv heads 8.7 against 13.1).
+bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles, int hb_cap, int smem_cap) {
+  if (tiles <= 4 || tiles > 2 * kMaxCluster) return false;
+  Plan c = pl;
+  c.HB = 0;
+  for (int h = hb_cap; h >= 1; --h)
+    if (Hkv % h == 0 && batch * (Hkv / h) * kMaxCluster <= b2l_num_sms()) c.HB = h;
+  if (c.HB == 0) return false;
+  plan_ring(c, D, smem_cap);
+  if (2 * c.smem > smem_cap) return false;
+  if ((int64_t)c.HB * G * (D + 1) * 4 > c.smem - 128) return false;     // the partial rows lie over the ring
+  c.splits = kMaxCluster;
+  c.chunk = (int)((tiles + kMaxCluster - 1) / kMaxCluster) * kTT;
+  c.cluster = true;
+  pl = c;
+  return true;
+}
 
 // Pure function of host-known sizes => identical inside and outside graph capture.
 Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
@@ -366,15 +485,11 @@ Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
   for (int h = 1; h <= hb_cap; ++h)
     if (Hkv % h == 0) HB = h;
   pl.HB = HB;
-  const int stage = kTT * row_pitch(HB, D);
-  int stages = kMaxStages;
-  while (stages > 2 && stages * stage > smem_cap) --stages;
-  // prefer two resident CTAs per SM when a 3-deep ring fits in half the shared memory
-  if (stages * stage > smem_cap / 2 && 3 * stage <= smem_cap / 2) stages = 3;
-  pl.stages = stages;
-  pl.smem = stages * stage + 128;
+  plan_ring(pl, D, smem_cap);
   const int64_t pairs = batch * (Hkv / HB);
   const int64_t tiles = max_len > 0 ? (max_len + kTT - 1) / kTT : 1;
+  pl.cluster = false;
+  if (plan_cluster(pl, batch, G, Hkv, D, tiles, hb_cap, smem_cap)) return pl;
   // Six CTAs per SM over all splits of the longest possible length.  max_len is only a bound: the lengths are device data, one
   // long sequence may stand among short ones, and a captured graph's bucket may be twice the longest.  One wave of larger
   // splits is faster where every length is near max_len (32 sequences of 1000 - 2000 tokens, 8 kv heads of 128: 25 splits
@@ -392,6 +507,28 @@ Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
 
 template <typename T, int D>
 int launch_decode(const DecodeParams& p, const Plan& pl, int64_t batch, cudaStream_t st) {
+  if (pl.cluster) {
+    static int configured_cluster[64] = {0};
+    auto kern = flash_decode_split_kernel<T, D, true>;
+    B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, pl.smem, configured_cluster));
+    b2l_hang_arm(st);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p.splits, (unsigned)(p.Hkv / p.HB), (unsigned)batch);
+    cfg.blockDim = dim3((p.HB * p.qblocks + 1) * 32);
+    cfg.dynamicSmemBytes = pl.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = p.splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = b2l_pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&cfg, kern, p);
+    B2L_LAUNCH_CHECK();
+    return B2L_OK;
+  }
   static int configured[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(flash_decode_split_kernel<T, D>, pl.smem, configured));
   dim3 grid((unsigned)p.splits, (unsigned)(p.Hkv / p.HB), (unsigned)batch);
@@ -415,7 +552,7 @@ extern "C" int64_t b2l_flash_decoding_workspace_bytes(int64_t batch, int num_q_h
                                                        int64_t max_seq_len) {
   if (batch <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
   Plan pl = make_plan(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
-  if (pl.splits <= 1) return 16;
+  if (pl.splits <= 1 || pl.cluster) return 16;
   return (int64_t)batch * num_q_heads * pl.splits * (head_dim + 1) * 4 + 16;
 }
 
@@ -463,7 +600,7 @@ extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache,
   p.ws_o = nullptr; p.ws_lse = nullptr;
   // the split CTAs merge their own results when the caller provides zeroed tickets (one per batch row x head block)
   p.tickets = (tickets && num_tickets >= batch * (num_kv_heads / pl.HB)) ? (int*)tickets : nullptr;
-  if (pl.splits > 1) {
+  if (pl.splits > 1 && !pl.cluster) {
     const int64_t need = b2l_flash_decoding_workspace_bytes(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
     B2L_REQUIRE(workspace && workspace_bytes >= need, "flash_decoding: workspace too small (%lld < %lld)",
                 (long long)workspace_bytes, (long long)need);
