@@ -406,18 +406,21 @@ extern "C" int b2l_moe_sort(void* order, void* table, const void* topk_ids, int 
   b2l_launch(moe_sort_kernel<HELD>, dim3(1), dim3(kSortThreads), (size_t)(BYTES), (cudaStream_t)stream, topk_ids, id_width,  \
              (int)num_slots, tile_rows, num_experts, (int32_t*)order, (int32_t*)table)
   const size_t count_bytes = (size_t)num_experts * sizeof(int);
+#define SORT_HELD(HELD)                                                                                                     \
+  static int configured[64] = {0};                                                                                          \
+  const int most = (8192 + HELD * kSortThreads) * (int)sizeof(int);       /* with the most experts that are taken */        \
+  B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(moe_sort_kernel<HELD>, most, configured));                                         \
+  SORT(HELD, count_bytes + HELD * kSortThreads * sizeof(int))
   if (num_slots <= kSortThreads) {
-    SORT(1, count_bytes + kSortThreads * sizeof(int));
+    SORT_HELD(1);
   } else if (num_slots <= 4 * kSortThreads) {
-    SORT(4, count_bytes + 4 * kSortThreads * sizeof(int));
+    SORT_HELD(4);
   } else if (num_slots <= kSortHeld * kSortThreads) {
-    static int configured[64] = {0};
-    const int bytes = (8192 + kSortHeld * kSortThreads) * (int)sizeof(int);       // the most experts that are taken
-    B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(moe_sort_kernel<kSortHeld>, bytes, configured));
-    SORT(kSortHeld, count_bytes + kSortHeld * kSortThreads * sizeof(int));
+    SORT_HELD(kSortHeld);
   } else {
     SORT(0, count_bytes);
   }
+#undef SORT_HELD
 #undef SORT
   B2L_LAUNCH_CHECK();
   return B2L_OK;
