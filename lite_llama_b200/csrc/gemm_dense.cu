@@ -1,7 +1,7 @@
 // Dense projections on tcgen05: fp16/bf16 linear (q/kv/o/gate/up/down/lm_head, the reference's
 // F.linear call sites: lite_llama/models/quantization/methods/unquantized.py:21-22,
 // lite_llama/models/base.py:489) and the int8 x int8 GEMM of SmoothQuant-W8A8
-// (lite_llama/kernels/quantization/w8a8.py:75-130).  See gemm_tc.cuh for the tile design.  Batches of more than 128 tokens
+// (lite_llama/kernels/quantization/w8a8.py:75-130).  See gemm_tc.cuh for the tile design.  Batches of more than 64 tokens
 // with enough tiles run in gemm_pair.cu.
 #include "gemm_tc.cuh"
 #include "gemm_pair.cuh"
