@@ -11,7 +11,7 @@
 //   * tokens are the MMA rows, so a thread holds consecutive outputs of one token: 16-byte shared-memory writes and
 //     one TMA store per warp and 64 outputs, clipped at the edges by the TMA unit.
 // Measured, launches by themselves (bf16, 4096 x 28672 x 4096): 974 us (988 TFLOP/s) -> 582 us (1652 TFLOP/s); int8 768 us ->
-// 298 us (3.2 POP/s); the tensor pipe is busy for 94 % of the active cycles (1024 tokens, profiles/pair_gemm_ncu.txt).  In a pass
+// 289 us (3.3 POP/s); the tensor pipe is busy for 94 % of the active cycles (1024 tokens, profiles/pair_gemm_ncu.txt).  In a pass
 // that keeps the card at its power cap they take 15 - 20 % longer: a feed-forward of 4096 tokens, 4096 x 14336, is 1200 us
 // where its launches by themselves add up to 1030.
 #include "gemm_tc.cuh"
