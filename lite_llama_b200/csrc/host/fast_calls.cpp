@@ -5,13 +5,15 @@
 //
 // Every function returns None for anything else (other dimensions, strides, types or devices, a bias, tensor subclasses,
 // wrapped or fake tensors, active torch modes): the Python shim then does what it always did, error messages included.  The
-// results are those of the Python path: same kernels, same arguments, outputs without a gradient.
+// results are those of the Python path: same kernels, same arguments, outputs without a gradient; exceptions too (torch's own
+// translation: an allocation that fails is a torch.OutOfMemoryError, which the graph captures of ModelRunner wait for).
 #include <Python.h>
 #include <ATen/ATen.h>
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
@@ -127,20 +129,13 @@ i64 quant_workspace(int kind, i64 m, i64 n, i64 k, i64 group, int device) {
   return (*seen)[s] = abi.quant_workspace(kind, m, n, k, group);
 }
 
-#define FAST_BEGIN try {
-#define FAST_END                                     \
-  }                                                  \
-  catch (const std::exception& e) {                  \
-    PyErr_SetString(PyExc_RuntimeError, e.what());   \
-    return nullptr;                                  \
-  }
 #define ARGS(n) \
   if (count != (n)) { PyErr_SetString(PyExc_TypeError, "wrong number of arguments"); return nullptr; }
 
 // (x, qweight, scales, group_n, group_k) -> y
 PyObject* w8a16(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(5)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *x = plain(a[0]), *q = plain(a[1]), *s = plain(a[2]);
   const int device = device_for(abi.w8a16, {x, q, s});
   if (device < 0 || !PyLong_CheckExact(a[3]) || !PyLong_CheckExact(a[4])) return none();
@@ -167,13 +162,13 @@ PyObject* w8a16(PyObject*, PyObject* const* a, Py_ssize_t count) {
                    bytes, tickets, num_tickets, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // (x, qweight, scales, zeros, n, k, group_size, zeros_foldable, swiglu) -> y
 PyObject* w4a16_packed(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(9)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *x = plain(a[0]), *q = plain(a[1]), *s = plain(a[2]), *z = plain(a[3]);
   const int device = device_for(abi.w4a16, {x, q, s, z});
   if (device < 0) return none();
@@ -200,13 +195,13 @@ PyObject* w4a16_packed(PyObject*, PyObject* const* a, Py_ssize_t count) {
                    tickets, num_tickets, swiglu, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // (x, weight) -> y
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(2)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
   const int device = device_for(abi.linear, {x, w});
   if (device < 0) return none();
@@ -228,13 +223,13 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
                     bytes > 0 ? ws.data_ptr() : nullptr, bytes, tickets, num_tickets, code, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // (qa, a_scales, qweight, weight_scales [N] or [N, 1], bfloat16 out) -> y
 PyObject* w8a8(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(5)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *x = plain(a[0]), *sa = plain(a[1]), *w = plain(a[2]), *sw = plain(a[3]);
   const int device = device_for(abi.w8a8, {x, sa, w, sw});
   if (device < 0) return none();
@@ -261,7 +256,7 @@ PyObject* w8a8(PyObject*, PyObject* const* a, Py_ssize_t count) {
                   bf16, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 PyObject* pair_of(at::Tensor a, at::Tensor b) {
@@ -275,7 +270,7 @@ PyObject* pair_of(at::Tensor a, at::Tensor b) {
 // (a) -> (q, scales)
 PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(1)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor* x = plain(a[0]);
   const int device = device_for(abi.quantize, {x});
   if (device < 0) return none();
@@ -291,7 +286,7 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t count) {
     rc = abi.quantize(q.data_ptr(), s.data_ptr(), x->data_ptr(), m, k, x->stride(0), k, code, stream(device));
   }
   return rc ? failed(rc) : pair_of(std::move(q), std::move(s));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // rows of the norms: contiguous matrices that the results may alias
@@ -305,7 +300,7 @@ bool norm_rows(const at::Tensor& x, PyObject* res, const at::Tensor* r, const at
 // (X, residual or None, weight, eps) -> (Y, residual or X)
 PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(4)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *x = plain(a[0]), *r = a[1] == Py_None ? nullptr : plain(a[1]), *w = plain(a[2]);
   const int device = r ? device_for(abi.norm, {x, w, r}) : device_for(abi.norm, {x, w});
   if (device < 0 || !PyFloat_CheckExact(a[3]) || !norm_rows(*x, a[1], r, *w)) return none();
@@ -324,13 +319,13 @@ PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(y)));
   PyTuple_SET_ITEM(out, 1, Py_NewRef(r ? a[1] : a[0]));
   return out;
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // (X, residual or None, weight, eps) -> (q, scales)
 PyObject* norm_quant(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(4)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *x = plain(a[0]), *r = a[1] == Py_None ? nullptr : plain(a[1]), *w = plain(a[2]);
   const int device = r ? device_for(abi.norm_quant, {x, w, r}) : device_for(abi.norm_quant, {x, w});
   if (device < 0 || !PyFloat_CheckExact(a[3]) || !norm_rows(*x, a[1], r, *w)) return none();
@@ -346,13 +341,13 @@ PyObject* norm_quant(PyObject*, PyObject* const* a, Py_ssize_t count) {
                         (float)PyFloat_AS_DOUBLE(a[3]), half_code(*x), stream(device));
   }
   return rc ? failed(rc) : pair_of(std::move(q), std::move(s));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // (a, b) -> silu(a) * b
 PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(2)
-  FAST_BEGIN
+  HANDLE_TH_ERRORS
   const at::Tensor *g = plain(a[0]), *u = plain(a[1]);
   const int device = device_for(abi.swiglu, {g, u});
   if (device < 0) return none();
@@ -367,7 +362,7 @@ PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t count) {
     rc = abi.swiglu(y.data_ptr(), g->data_ptr(), u->data_ptr(), rows, n, g->stride(0), u->stride(0), n, code, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  FAST_END
+  END_HANDLE_TH_ERRORS
 }
 
 // (addresses of the C functions in the order of `abi`, zeroed_workspace, counters)

@@ -134,3 +134,37 @@ def test_native_calls_inside_a_graph_and_on_another_stream():
     x.copy_(x2)
     graph.replay()
     assert torch.equal(out, general(x2))
+
+
+@pytest.mark.parametrize("name", ["w8a16", "w4a16", "linear", "w8a8", "quantize", "norm", "norm_quant", "swiglu"])
+def test_an_allocation_that_fails_is_an_out_of_memory_error(name):
+    """ModelRunner falls back to eager steps on this type.  The inputs are there before the allocator is closed to new segments,
+    and every result needs one of its own (more than 10 MB)."""
+    from lite_llama_b200.kernels import _native as N
+    import lite_llama_b200.kernels as K
+
+    m, n, k = 16384, 2048, 1024
+    x, w = torch.ones(m, k, device="cuda", dtype=torch.float16), torch.ones(n, k, device="cuda", dtype=torch.float16)
+    q8, xq, s = w.to(torch.int8), x.to(torch.int8), torch.ones(m, device="cuda")
+    p = K.w4a16_pack(torch.zeros(n, k // 8, device="cuda", dtype=torch.int32), s[:1].expand(n, k // 128).contiguous(),
+                     torch.zeros(n, k // 128, device="cuda"), group_size=128)
+    call = {
+        "w8a16": lambda: N.w8a16(x, q8, s[:n].view(n, 1), 1, k),
+        "w4a16": lambda: N.w4a16_packed(x, p.qweight, p.scales, p.zeros, n, k, 128, True, False),
+        "linear": lambda: N.linear(x, w),
+        "w8a8": lambda: N.w8a8(xq, s, q8, s[:n], False),
+        "quantize": lambda: N.quantize(x),
+        "norm": lambda: N.norm(x, None, w[0], 1e-5),
+        "norm_quant": lambda: N.norm_quant(x, None, w[0], 1e-5),
+        "swiglu": lambda: N.swiglu(x, x),
+    }[name]
+    assert call() is not None
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(1e-6)
+    try:
+        with pytest.raises(torch.cuda.OutOfMemoryError):
+            call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert call() is not None                                          # and nothing is left behind
