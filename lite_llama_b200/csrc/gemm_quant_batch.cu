@@ -22,7 +22,8 @@
 // groups, 21.9; four groups with one buffer 18.0), the helpers split into loaders and issuers (fewer registers for the
 // groups, 30), MMAs predicated on their lane instead of in a branch (+2 %).
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, whole zero points subtracted exactly, others (known
-// only on the device in the reference's layout) as scale * (segment - z * sum of x), acc = fma(scale, segment, acc) in fp32; the sum over k runs over every NWG-th block first, then over groups and CTAs in a fixed order.
+// only on the device in the reference's layout) as scale * (segment - z * sum of x), acc = fma(scale, segment, acc) in fp32; the sum over k runs over every NWG-th
+// block first, then over groups and CTAs in a fixed order, with all 32 bits of every partial sum (bq_partial).
 #define B2L_HANG_NORETURN true
 #include "gemm_tc.cuh"
 #include "dequant.cuh"
@@ -109,10 +110,11 @@ __device__ __forceinline__ uint4 bq_lds_128(uint32_t a) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a));
   return v;
 }
-// A partial sum travels as one word whose lowest bit says that it is there.  With that bit an infinity is the bit pattern of a
-// signalling NaN, which no arithmetic returns: it is read back as the infinity.
-__device__ __forceinline__ float bq_untag(uint32_t w) {
-  return __uint_as_float((w & 0x7FFFFFFFu) == 0x7F800001u ? w - 1u : w);
+// A partial sum travels as one word that is not zero once it is there, all 32 bits of it: +0 goes as -0, which adds the same to
+// a sum that starts at +0.
+__device__ __forceinline__ uint32_t bq_partial(float f) {
+  const uint32_t w = __float_as_uint(f);
+  return w != 0u ? w : 0x80000000u;
 }
 // CTA that owns a raw block of the linearised (tile, raw block) space; 32 bits hold total * (ctas + 1) (host)
 __host__ __device__ __forceinline__ int bq_owner(int lin, int ctas, int total) {
@@ -563,7 +565,7 @@ gemm_quant_batch_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
         } else {
           uint32_t t[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) t[e] = __float_as_uint(f[e]) | 1u;
+          for (int e = 0; e < 8; ++e) t[e] = bq_partial(f[e]);
           uint4* dst = base + slot * kSlotVec + c * kChVec;
           dst[0] = make_uint4(t[0], t[1], t[2], t[3]);
           dst[kBlockW] = make_uint4(t[4], t[5], t[6], t[7]);
@@ -584,7 +586,7 @@ gemm_quant_batch_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
             uint32_t v[SB][8];
             unsigned long long t0 = 0ull;
             for (;;) {
-              uint32_t all = 1u;
+              uint32_t least = 1u;                              // 0: a word is still missing
 #pragma unroll
               for (int u = 0; u < SB; ++u) {
                 const uint4* src = base + (s0 + u) * kSlotVec + c * kChVec;
@@ -600,8 +602,8 @@ gemm_quant_batch_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
 #pragma unroll
               for (int u = 0; u < SB; ++u)
 #pragma unroll
-                for (int e = 0; e < 8; ++e) all &= v[u][e];
-              if (all & 1u) break;
+                for (int e = 0; e < 8; ++e) least = min(least, v[u][e]);
+              if (least != 0u) break;
               const unsigned long long now = b2l_globaltimer();
               if (t0 == 0ull) t0 = now;
               const unsigned long long lim = b2l_hang_ctl.limit_ns;
@@ -614,7 +616,7 @@ gemm_quant_batch_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid
               if (s0 + u < sharers) {
                 uint4* src = base + (s0 + u) * kSlotVec + c * kChVec;
 #pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] += s0 + u == slot ? own[e] : bq_untag(v[u][e]);
+                for (int e = 0; e < 8; ++e) f[e] += s0 + u == slot ? own[e] : __uint_as_float(v[u][e]);
                 if (s0 + u != slot) src[0] = src[kBlockW] = make_uint4(0u, 0u, 0u, 0u);        // leave the workspace clean
               }
             }

@@ -109,6 +109,18 @@ def test_infinities_pass_through_shared_tiles(m):
     assert got[2].isnan().all() and got[3].isnan().all() and (got[4:] == 0).all()
 
 
+@pytest.mark.parametrize("m", [1, 16, 33, 64])
+@pytest.mark.parametrize("n,k", [(2048, 2048), (20100, 1280)])        # equal parts of a tile; parts of several tiles
+def test_partial_sums_keep_their_bits(m, n, k):
+    """Every product is a multiple of 12.5 and every sum of them below 2^17, so 32-bit sums are exact in any order, and the halves
+    of k cancel.  A partial sum that loses its last bit between CTAs leaves a remainder."""
+    q = torch.full((n, k), 100, device="cuda", dtype=torch.int8)
+    half = torch.randint(1, 16, (m, k // 2), device="cuda").half() / 2
+    x = torch.cat([half, -half.flip(1)], 1)
+    got = K().w8a16_matmul(x, q, torch.full((n, 1), 0.25, device="cuda"), group_n=1, group_k=k)
+    assert not got.any()
+
+
 def test_workspace_is_left_clean_and_a_smaller_one_takes_the_streaming_kernel():
     import lite_llama_b200.kernels._common as c
     from lite_llama_b200 import _lib
