@@ -25,6 +25,7 @@ from pathlib import Path
 
 CSRC = Path(__file__).resolve().parent / "csrc"
 OUT = Path(__file__).resolve().parent / "libb200lite.so"
+HEADER = CSRC.parents[1] / "include" / "b200_lite_kernels.h"
 FAST_SRC = CSRC / "host" / "fast_calls.cpp"
 FAST_OUT = Path(__file__).resolve().parent / "_fast.so"
 OBJ_DIR = CSRC / "build"
@@ -86,30 +87,41 @@ def linked_sources() -> set[str]:
     return set(LINK_STAMP.read_text().split())
 
 
+def fast_tag(torch_version: str) -> str:
+    """What a build of the extension is good for.  It calls the library through bare function pointers, so one of another
+    header, source, interpreter or torch must not be used: the header and the source by their contents."""
+    h = hashlib.sha256(FAST_SRC.read_bytes() + HEADER.read_bytes())
+    return f"{torch_version} {sys.version_info.major}.{sys.version_info.minor} {h.hexdigest()}"
+
+
 def build_fast(force: bool = False) -> str | None:
     """The native form of the hot shims, built against this interpreter and this torch.  None, or why it could not be built:
-    the shims then run in Python, slower on the host and otherwise the same."""
+    the shims then run in Python, slower on the host and otherwise the same (an earlier extension does not stay)."""
+    stamp_file = OBJ_DIR / "fast_calls.stamp"
     try:
         import torch
     except ImportError as e:
+        FAST_OUT.unlink(missing_ok=True)
         return str(e)
     root = Path(torch.__file__).resolve().parent
     include = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", sysconfig.get_paths()["include"],
                Path(_nvcc()).resolve().parent.parent / "include"]
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DBUILT_FOR_TORCH="{torch.__version__}"',
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DBUILT_FOR="{fast_tag(torch.__version__)}"',
            *(f"-I{d}" for d in include), str(FAST_SRC), "-o", str(FAST_OUT), f"-L{root / 'lib'}",
            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"]
     stamp = hashlib.sha256((" ".join(cmd) + sys.version).encode() + FAST_SRC.read_bytes()).hexdigest()
-    stamp_file = OBJ_DIR / "fast_calls.stamp"
     if not force and FAST_OUT.exists() and stamp_file.exists() and stamp_file.read_text() == stamp:
         return None
+    FAST_OUT.unlink(missing_ok=True)
+    stamp_file.unlink(missing_ok=True)
     try:
         res = subprocess.run(cmd, capture_output=True, text=True)
     except OSError as e:
         return str(e)
     if res.returncode != 0:
-        return res.stderr
+        FAST_OUT.unlink(missing_ok=True)
+        return res.stderr or f"{cmd[0]} returned {res.returncode}"
     stamp_file.write_text(stamp)
     return None
 

@@ -388,7 +388,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fast", nullptr, -1, methods};
 
 PyMODINIT_FUNC PyInit__fast() {
   PyObject* m = PyModule_Create(&module);
-  if (m && PyModule_AddStringConstant(m, "torch_version", BUILT_FOR_TORCH) < 0) {
+  if (m && PyModule_AddStringConstant(m, "built_for", BUILT_FOR) < 0) {
     Py_DECREF(m);
     return nullptr;
   }

@@ -1,7 +1,7 @@
 """The native form of the hot shims (csrc/host/fast_calls.cpp).
 
 Each function takes the plain form of its shim's call and returns None for every other form; the shim then goes on in Python.
-Where the extension is missing or was built for another torch, every call goes on in Python.
+Where the extension is missing or was built for another header, source, interpreter or torch, every call goes on in Python.
 """
 
 from __future__ import annotations
@@ -10,6 +10,7 @@ import ctypes
 
 import torch
 
+from ..build import fast_tag
 from . import _common
 
 # the order of the function table in fast_calls.cpp
@@ -31,9 +32,10 @@ def _python(*_args) -> None:
 def _table() -> dict:
     try:
         from .. import _fast
-    except ImportError:
+        wanted = fast_tag(torch.__version__)
+    except (ImportError, OSError):          # not built, or its source is not there to compare with
         return {}
-    if getattr(_fast, "torch_version", None) != torch.__version__:
+    if getattr(_fast, "built_for", None) != wanted:
         return {}
     _fast.init(*map(_address, _ABI), _common.zeroed_workspace, _common.counters)
     return {name: getattr(_fast, name) for name in NAMES}
