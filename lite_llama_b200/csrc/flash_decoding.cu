@@ -91,7 +91,8 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
   const int64_t seq_len = load_index(p.seq_len, b, p.len_w);
   const int64_t start = (int64_t)split * p.chunk;
   if (start >= seq_len) {        // empty split: nothing to contribute (whole CTA exits together)
-    if (FD_CLUSTER && split == 0) {                       // an empty row is zero
+    // an empty row is zero; where a second kernel merges, it says so
+    if (split == 0 && (FD_CLUSTER || p.splits == 1 || p.tickets != nullptr)) {
       const int heads = p.HB * p.G;
       for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
         *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +

@@ -9,6 +9,25 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("bound", [16, 64, 65, 256, 257, 2000])     # one split, clusters, splits with a merge of their own
+@pytest.mark.parametrize("fold", [False, True])
+def test_an_empty_row_is_zero_whatever_the_bound(bound, fold, monkeypatch):
+    import sys
+
+    import lite_llama_b200.kernels as K
+
+    monkeypatch.setattr(sys.modules["lite_llama_b200.kernels.flashdecoding"], "_FOLD", fold)
+    q = torch.randn(3, 8, 64, device="cuda", dtype=torch.float16)
+    pool = torch.randn(3 * bound, 4, 64, device="cuda", dtype=torch.float16)
+    table = torch.arange(3 * bound, device="cuda", dtype=torch.int32).view(3, bound)
+    lens = torch.tensor([bound, 0, 1], device="cuda")
+    scratch = [torch.full((3, 8, 64), float("nan"), device="cuda", dtype=torch.float16) for _ in range(8)]
+    del scratch                                                      # what the result's memory held before
+    got = K.flash_decoding(q, pool[:, :2], pool[:, 2:], 0.125, table, torch.arange(3, device="cuda"), lens, bound)
+    assert not got[1].any()
+    torch.testing.assert_close(got[2].view(2, 4, 64), pool[2 * bound, 2:, None].expand(2, 4, 64), rtol=0, atol=0)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("batch,hq,hkv,d", [(1, 32, 8, 128), (3, 14, 2, 64), (18, 28, 4, 128), (4, 8, 8, 32), (1, 40, 1, 64),
                                             (2, 6, 2, 256)])
