@@ -50,6 +50,37 @@ def test_two_tiles_per_cta(lens, hq, hk, dtype):
     assert math.sqrt(diff / norm) < (2.0**-11 if dtype == torch.float16 else 2.0**-8)
 
 
+@pytest.mark.parametrize("lens", [[200], [0, 300, 0, 129], [40 + i for i in range(70)]])
+@pytest.mark.parametrize("hq,hk", [(16, 2), (9, 3)])
+def test_a_bound_far_above_the_lengths(lens, hq, hk):
+    """The bound decides how many blocks there might be, not what comes out: the same bits as with the next larger bound whose
+    grid is as large, in about the same time."""
+    q = torch.randn(sum(lens), hq, 128, device="cuda", dtype=torch.float16)
+    k, v = torch.randn(2, sum(lens), hk, 128, device="cuda", dtype=torch.float16)
+    n = torch.tensor(lens, device="cuda", dtype=torch.int32)
+    start = (n.cumsum(0) - n).int()
+    call = lambda bound: K().flash_attention2_no_pad(q, k, v, 0.1275, start, n, bound)                      # noqa: E731
+    near = -(-150 // (hq * len(lens))) * 128 + 256
+    got, want = call(32768), call(near)
+    assert got.isfinite().all() and torch.equal(got, want)
+
+    def time(bound):
+        graph, a, b = torch.cuda.CUDAGraph(), *(torch.cuda.Event(enable_timing=True) for _ in range(2))
+        with torch.cuda.graph(graph):
+            for _ in range(20):
+                call(bound)
+        best = float("inf")
+        for _ in range(5):
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    assert time(32768) < 2 * time(near)                 # the scheduler of every CTA walked through all levels: up to 6 times
+
+
 def test_large_scores_rescale_the_sums():
     """Scores that grow along the keys by far more than the 2^8 that the running maximum may lag behind, and a row of one size."""
     d, m, h = 128, 900, 24
