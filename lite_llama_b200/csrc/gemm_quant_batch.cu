@@ -738,7 +738,9 @@ int quant_batch_gemm(int qk, int layout, QuantBatchParams& p, const void* x, int
     // the threads, whose 4-byte copies take as long as the conversion (28672 x 4096, 32 tokens: 31 us).
     BqMaps<Q_INT4, 0> tabs;
     memset(&tabs, 0, sizeof(tabs));
+    // (Rows of a tensor map lie behind one another: expanded or overlapping tables are the threads'.)
     p.quads = p.groups % 4 == 0 && (p.group_steps & (p.group_steps - 1)) == 0 && p.s_stride_k == 1 && p.s_stride_n % 4 == 0 &&
+              p.s_stride_n >= p.groups &&
               ((uintptr_t)p.scales | (uintptr_t)p.zeros) % 16 == 0;
     if (p.quads) {
       rc = b2l_make_tmap_2d(&tabs.s, p.scales, TMA_I32, (uint64_t)N, (uint64_t)p.groups, (uint64_t)p.s_stride_n * 4, kBlockW, 4, false);

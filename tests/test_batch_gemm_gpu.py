@@ -65,6 +65,22 @@ def test_int4_batches_with_zero_points_that_are_not_whole(n, k):
         assert torch.equal(K().w4a16_matmul(x64[:m], q, s, z + off, group_size=128), got), m
 
 
+@pytest.mark.parametrize("m", [9, 64])
+def test_int4_tables_of_any_stride(m):
+    """The scales and zero points of the reference's layout as views: one row for all, rows that overlap, groups along the rows,
+    rows with a gap, a start that is no multiple of 16 bytes."""
+    n, k, groups = 300, 1024, 8
+    q, s, z, _, x = int4_case(n, k, 128, m)
+    flat_s, flat_z = torch.rand(8 * n, device="cuda") * 4e-3 + 1e-3, torch.randint(0, 16, (8 * n,), device="cuda").float()
+    views = [lambda t: t[:groups].expand(n, groups), lambda t: t.as_strided((n, groups), (4, 1)),
+             lambda t: t[: n * groups].view(groups, n).t(), lambda t: t.repeat(2).as_strided((n, groups), (12, 1)),
+             lambda t: t[1:].as_strided((n, groups), (4, 1))]
+    for view in views:
+        sv, zv = view(flat_s), view(flat_z)
+        want = K().w4a16_matmul(x, q, sv.contiguous(), zv.contiguous(), group_size=128)
+        assert torch.equal(K().w4a16_matmul(x, q, sv, zv, group_size=128), want)
+
+
 @pytest.mark.parametrize("n,k", SHAPES)
 def test_int4_batches_with_activation_are_gemm_then_swiglu(n, k):
     from lite_llama_b200.kernels.quantization import interleave_gate_up
