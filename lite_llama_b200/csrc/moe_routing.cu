@@ -85,9 +85,10 @@ moe_align_kernel(const void* __restrict__ topk_ids, int id_width, int num_slots,
 // Bound: latency of one CTA.  The padded protocol above spends 28 us at 256 and 58 us at 16000 slots over 128 experts, most
 // of it in its single-thread prefix; here counts, prefix and placement are all in parallel.
 // HELD: ids that a thread keeps, with their places within the experts; the order is then put together in shared memory and
-// leaves in whole lines.  Bound by the stores of one SM otherwise, 4 bytes to a line of their own (in a graph, us: 16000 slots over
-// 128 experts 12.2 -> 7.0, 2048 over 64 3.4 -> 2.9, 256 over 128 2.3 -> 2.2; 16384 over 8, whose stores meet, 7.3 / 7.7).  0: any
-// number of slots.
+// leaves in whole lines.  Bound by the stores of one SM otherwise, 4 bytes to a line of their own.  0: any number of slots.  In a
+// graph, us, 0 -> held: 16000 slots over 128 experts 12.1 -> 7.2, 2048 over 64 3.6 -> 3.1, 256 over 128 2.6 -> 2.4.  With few
+// experts the stores meet in a line: 4096 over 8 3.6 / 3.7, 8192 over 16 4.8 / 5.8, 16384 over 8 7.1 / 8.0.  16 ids a thread cost 5 us
+// however many there are: 4097 over 32 4.5 / 5.1, over 128 5.1 / 5.2, but 8192 over 32 6.1 / 5.6.
 constexpr int kSortThreads = 1024, kSortHeld = 16;
 template <int HELD>
 __global__ void __launch_bounds__(kSortThreads)
@@ -411,11 +412,12 @@ extern "C" int b2l_moe_sort(void* order, void* table, const void* topk_ids, int 
   const int most = (8192 + HELD * kSortThreads) * (int)sizeof(int);       /* with the most experts that are taken */        \
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(moe_sort_kernel<HELD>, most, configured));                                         \
   SORT(HELD, count_bytes + HELD * kSortThreads * sizeof(int))
+  const bool few = num_experts < 32;
   if (num_slots <= kSortThreads) {
     SORT_HELD(1);
-  } else if (num_slots <= 4 * kSortThreads) {
+  } else if (num_slots <= (few ? 2 : 4) * kSortThreads) {
     SORT_HELD(4);
-  } else if (num_slots <= kSortHeld * kSortThreads) {
+  } else if (!few && num_slots > 6 * kSortThreads && num_slots <= kSortHeld * kSortThreads) {
     SORT_HELD(kSortHeld);
   } else {
     SORT(0, count_bytes);
