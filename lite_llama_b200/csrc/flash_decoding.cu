@@ -73,6 +73,48 @@ __device__ __forceinline__ float4 ld_peer4(uint32_t addr) {
   return v;
 }
 
+// The splits of a row and head block, left by the CTAs of a cluster in their own shared memory (rows, then statistics), added up
+// in split order like in the kernels below.  Every CTA takes its share of the outputs, also those whose split is empty: where
+// those left before, two of eight CTAs made four trips through shared memory for 32 heads (4 kv heads, 16 rows of 20 tokens under
+// a bound of 80: 7.4 us, the merge kernel 7.0, now 5.5).
+template <typename T, int D>
+__device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t part, int64_t seq_len) {
+  const int split = blockIdx.x, heads = p.HB * p.G;
+  __syncwarp();
+  cluster_sync_all();
+  const int nsp = (int)((seq_len + p.chunk - 1) / p.chunk) < p.splits ? (int)((seq_len + p.chunk - 1) / p.chunk) : p.splits;
+  for (int i = split * blockDim.x + threadIdx.x; i < heads * (D / 4); i += p.splits * blockDim.x) {
+    const int local = i / (D / 4), d = i % (D / 4) * 4;
+    float lse[kMaxCluster];
+    float4 v[kMaxCluster];
+#pragma unroll
+    for (int r = 0; r < kMaxCluster; ++r)
+      if (r < nsp) {
+        const uint32_t peer = peer_smem(part, r);
+        lse[r] = ld_peer(peer + (heads * D + local) * 4);
+        v[r] = ld_peer4(peer + (local * D + d) * 4);
+      }
+    float M = -INFINITY, L = 0.f;
+#pragma unroll
+    for (int r = 0; r < kMaxCluster; ++r)
+      if (r < nsp) M = fmaxf(M, lse[r]);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int r = 0; r < kMaxCluster; ++r)
+      if (r < nsp) {
+        const float w = fast_exp2(lse[r] - M);
+        acc.x += w * v[r].x; acc.y += w * v[r].y; acc.z += w * v[r].z; acc.w += w * v[r].w;
+        L += w;
+      }
+    uint32_t* to = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)blockIdx.z * p.o_bs +
+                                               (int64_t)(blockIdx.y * heads + local) * p.o_hs + d);
+    to[0] = pack2<T>(acc.x / L, acc.y / L);
+    to[1] = pack2<T>(acc.z / L, acc.w / L);
+  }
+  __syncwarp();
+  cluster_sync_all();                 // the peers have read this CTA's rows
+}
+
 // FD_CLUSTER: the grid's x is one cluster of up to kMaxCluster splits, which merge their results themselves.
 template <typename T, int D, bool FD_CLUSTER = false>
 __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_kernel(const DecodeParams p) {
@@ -90,15 +132,19 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
 
   const int64_t seq_len = load_index(p.seq_len, b, p.len_w);
   const int64_t start = (int64_t)split * p.chunk;
-  if (start >= seq_len) {        // empty split: nothing to contribute (whole CTA exits together)
-    // an empty row is zero; where a second kernel merges, it says so
-    if (split == 0 && (FD_CLUSTER || p.splits == 1 || p.tickets != nullptr)) {
+  // a row of one split has nothing to merge
+  const bool alone = FD_CLUSTER ? seq_len <= p.chunk : p.splits == 1;
+  if (start >= seq_len) {        // empty split: nothing to contribute
+    if (FD_CLUSTER && !alone) {
+      cluster_merge<T, D>(p, smem_u32(stage_base), seq_len);
+    } else if (split == 0 && (FD_CLUSTER || p.splits == 1 || p.tickets != nullptr)) {
+      // an empty row is zero; where a second kernel merges, it says so
       const int heads = p.HB * p.G;
       for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
         *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +
                                      (int64_t)(hblk * heads + i / (D / 2)) * p.o_hs + 2 * (i % (D / 2))) = 0u;
     }
-    return;
+    return;                      // the whole CTA together
   }
   const int64_t end = (start + p.chunk < seq_len) ? start + p.chunk : seq_len;
   const int ntiles = (int)((end - start + kTT - 1) / kTT);
@@ -280,13 +326,13 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       if (!ok) continue;
       const int head = kvh * p.G + (r2 == 0 ? hq0 : hq1);
       const float inv = 1.0f / l_run[r2];
-      if (FD_CLUSTER) {
+      if (FD_CLUSTER && !alone) {
         const int local = hl * p.G + (r2 == 0 ? hq0 : hq1);
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
           *reinterpret_cast<float2*>(part + local * D + i * 8 + 2 * tq) = make_float2(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
         if (tq == 0) part[p.HB * p.G * D + local] = m_run[r2] + log2f(l_run[r2]);
-      } else if (p.splits == 1) {
+      } else if (alone) {
         T* orow = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)head * p.o_hs;
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
@@ -303,43 +349,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
   }
 
   if (FD_CLUSTER) {
-    // Every CTA with tokens merges its share of the outputs, in split order like the kernel below.  (Empty splits have left; the
-    // barrier does not wait for them.)
-    __syncwarp();
-    cluster_sync_all();
-    const int nsp = (int)((seq_len + p.chunk - 1) / p.chunk) < p.splits ? (int)((seq_len + p.chunk - 1) / p.chunk) : p.splits;
-    const int heads = p.HB * p.G;
-    const uint32_t part = smem_u32(stage_base);
-    for (int i = split * blockDim.x + threadIdx.x; i < heads * (D / 4); i += nsp * blockDim.x) {
-      const int local = i / (D / 4), d = i % (D / 4) * 4;
-      float lse[kMaxCluster];
-      float4 v[kMaxCluster];
-#pragma unroll
-      for (int r = 0; r < kMaxCluster; ++r)
-        if (r < nsp) {
-          const uint32_t peer = peer_smem(part, r);
-          lse[r] = ld_peer(peer + (heads * D + local) * 4);
-          v[r] = ld_peer4(peer + (local * D + d) * 4);
-        }
-      float M = -INFINITY, L = 0.f;
-#pragma unroll
-      for (int r = 0; r < kMaxCluster; ++r)
-        if (r < nsp) M = fmaxf(M, lse[r]);
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int r = 0; r < kMaxCluster; ++r)
-        if (r < nsp) {
-          const float w = fast_exp2(lse[r] - M);
-          acc.x += w * v[r].x; acc.y += w * v[r].y; acc.z += w * v[r].z; acc.w += w * v[r].w;
-          L += w;
-        }
-      uint32_t* to = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +
-                                                 (int64_t)(hblk * heads + local) * p.o_hs + d);
-      to[0] = pack2<T>(acc.x / L, acc.y / L);
-      to[1] = pack2<T>(acc.z / L, acc.w / L);
-    }
-    __syncwarp();
-    cluster_sync_all();                 // the peers have read this CTA's rows
+    if (!alone) cluster_merge<T, D>(p, smem_u32(stage_base), seq_len);
     return;
   }
 
@@ -450,11 +460,12 @@ void plan_ring(Plan& pl, int D, int smem_cap) {
 // Steps of up to 256 tokens a row that leave most of the chip idle: one wave of clusters of eight splits, two of their CTAs to an
 // SM.  A tile costs its CTA 0.6 - 1 us (copies, and one warp's chain of products), the merge kernel 3 us, a cluster's launch and
 // barriers 2 us.  us in a graph, splits of 64 tokens and the merge kernel -> this: 8 kv heads of 128, one sequence of 200 tokens
-// 8.5 -> 6.6, of 80 7.2 -> 5.0, eight of 200 8.6 -> 7.5; 18 of 4 kv heads 8.6 -> 7.2; rows of a quarter of the bound 8.2 -> 6.1 (one
-// sequence), 6.1 - 8.2 -> 5.3 - 7.7 (4 kv heads; slower in one case of twenty, eight rows of 20 tokens under a bound of 80, 6.1 ->
-// 6.4).  Longer splits are the longer chain here (512 tokens in four tiles each 9.1 against 8.9), up to four tiles there is a single
-// split without a merge (40 tokens 5.3 against 6.0), and with one CTA to an SM the clusters of eight do not all fit (16 sequences
-// of 8 kv heads 8.7 against 13.1).
+// 8.6 -> 6.7, of 80 7.6 -> 5.2, eight of 200 8.8 -> 7.7; 16 of 4 kv heads 8.6 -> 7.4; mixed lengths under that bound 8.6 -> 6.7, 9.2 ->
+// 7.4 and 9.4 -> 6.8; rows of a quarter of the bound 8.4 -> 6.3, 8.7 -> 7.1 and 8.8 -> 6.5; of one tile, under 65, 5.1 - 5.9 -> 3.6 - 4.0.
+// None of 540 mixtures (1 - 16 sequences, bounds of 65 - 256, six head layouts) is slower.
+// Longer splits are the longer chain here (512 tokens in four tiles each 9.1 against 8.9), up to four tiles there is a single
+// split without a merge, and with one CTA to an SM the clusters of eight do not all fit (16 sequences of 8 kv heads 8.7 against
+// 13.1).
 bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles, int hb_cap, int smem_cap) {
   if (tiles <= 4 || tiles > 2 * kMaxCluster) return false;
   Plan c = pl;
