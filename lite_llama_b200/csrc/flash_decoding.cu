@@ -21,7 +21,7 @@
 //  * split-KV sized from host-known quantities only (graph-safe); fp32 partials + log-sum-exp,
 //    merged by a second small kernel (reference stage 2, flashdecoding.py:224-313);
 //  * a step too small to fill the chip is bound by latency instead: its splits are the CTAs of a cluster, with as few kv
-//    heads each as still fit in one wave, and merge through one another's shared memory (FD_CLUSTER below).
+//    heads each as still fit in one wave, and merge through one another's shared memory (cluster_merge below).
 #include "common.cuh"
 
 namespace {
@@ -115,8 +115,11 @@ __device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t pa
   cluster_sync_all();                 // the peers have read this CTA's rows
 }
 
-// FD_CLUSTER: the grid's x is one cluster of up to kMaxCluster splits, which merge their results themselves.
-template <typename T, int D, bool FD_CLUSTER = false>
+// Who merges the splits of a row: a second kernel; nobody (a single split), or the last CTA (tickets); the CTAs of a cluster,
+// which are the grid's x, up to kMaxCluster splits.  The second form does the first one's work as well; its code for the rest costs
+// 0.2 - 0.3 us of 16 - 51, except with heads of 256, whose sums do not fit into registers and spill less in it (4 %).
+enum { FD_SPLITS, FD_WHOLE, FD_CLUSTER };
+template <typename T, int D, int FORM>
 __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_kernel(const DecodeParams p) {
   pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
   extern __shared__ __align__(128) uint8_t smem[];
@@ -133,12 +136,11 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
   const int64_t seq_len = load_index(p.seq_len, b, p.len_w);
   const int64_t start = (int64_t)split * p.chunk;
   // a row of one split has nothing to merge
-  const bool alone = FD_CLUSTER ? seq_len <= p.chunk : p.splits == 1;
+  const bool alone = FORM == FD_CLUSTER ? seq_len <= p.chunk : FORM == FD_WHOLE && p.splits == 1;
   if (start >= seq_len) {        // empty split: nothing to contribute
-    if (FD_CLUSTER && !alone) {
+    if (FORM == FD_CLUSTER && !alone) {
       cluster_merge<T, D>(p, smem_u32(stage_base), seq_len);
-    } else if (split == 0 && (FD_CLUSTER || p.splits == 1 || p.tickets != nullptr)) {
-      // an empty row is zero; where a second kernel merges, it says so
+    } else if (FORM != FD_SPLITS && split == 0) {     // an empty row is zero
       const int heads = p.HB * p.G;
       for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
         *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +
@@ -200,7 +202,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       }
       if (++s == p.stages) { s = 0; phase ^= 1; }
     }
-    if (FD_CLUSTER) __syncthreads();
+    if (FORM == FD_CLUSTER) __syncthreads();
   } else {
     // ===================== consumer warps: one (kv head, 16-query-head block) each =====================
     const int hl = warp / p.qblocks;            // kv head inside this CTA's block
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
     }
     // Cluster: the partial rows go to the CTA's own shared memory, over the stages that every warp has finished with
     float* part = reinterpret_cast<float*>(stage_base);
-    if (FD_CLUSTER) __syncthreads();
+    if (FORM == FD_CLUSTER) __syncthreads();
     // this warp saw every token of the split for its heads: write the result rows directly
 #pragma unroll
     for (int r2 = 0; r2 < 2; ++r2) {
@@ -326,7 +328,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       if (!ok) continue;
       const int head = kvh * p.G + (r2 == 0 ? hq0 : hq1);
       const float inv = 1.0f / l_run[r2];
-      if (FD_CLUSTER && !alone) {
+      if (FORM == FD_CLUSTER && !alone) {
         const int local = hl * p.G + (r2 == 0 ? hq0 : hq1);
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
@@ -348,7 +350,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
     }
   }
 
-  if (FD_CLUSTER) {
+  if (FORM == FD_CLUSTER) {
     if (!alone) cluster_merge<T, D>(p, smem_u32(stage_base), seq_len);
     return;
   }
@@ -356,7 +358,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
   // ---- stage 2 folded in (reference: a second kernel, flashdecoding.py:224-313): the CTA that finishes a
   // (batch row, kv-head block) LAST merges its splits.  Deterministic: the merge always runs over all splits in index
   // order, whoever executes it.  The ticket resets itself, so graph replays start clean. ----
-  if (p.splits > 1 && p.tickets != nullptr) {
+  if (FORM == FD_WHOLE && p.splits > 1 && p.tickets != nullptr) {
     __shared__ int s_last;
     __threadfence();
     __syncthreads();
@@ -521,7 +523,7 @@ template <typename T, int D>
 int launch_decode(const DecodeParams& p, const Plan& pl, int64_t batch, cudaStream_t st) {
   if (pl.cluster) {
     static int configured_cluster[64] = {0};
-    auto kern = flash_decode_split_kernel<T, D, true>;
+    auto kern = flash_decode_split_kernel<T, D, FD_CLUSTER>;
     B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, pl.smem, configured_cluster));
     b2l_hang_arm(st);
     cudaLaunchConfig_t cfg = {};
@@ -541,13 +543,16 @@ int launch_decode(const DecodeParams& p, const Plan& pl, int64_t batch, cudaStre
     B2L_LAUNCH_CHECK();
     return B2L_OK;
   }
-  static int configured[64] = {0};
-  B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(flash_decode_split_kernel<T, D>, pl.smem, configured));
+  const bool merge = p.splits > 1 && p.tickets == nullptr;
+  static int configured[2][64] = {{0}};
+  constexpr int kSplits = D < 256 ? FD_SPLITS : FD_WHOLE;
+  auto kern = merge ? flash_decode_split_kernel<T, D, kSplits> : flash_decode_split_kernel<T, D, FD_WHOLE>;
+  B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, pl.smem, configured[merge && D < 256]));     // one record per kernel
   dim3 grid((unsigned)p.splits, (unsigned)(p.Hkv / p.HB), (unsigned)batch);
   const int threads = (p.HB * p.qblocks + 1) * 32;
-  b2l_launch(flash_decode_split_kernel<T, D>, dim3(grid), dim3(threads), (size_t)(pl.smem), st, p);
+  b2l_launch(kern, dim3(grid), dim3(threads), (size_t)(pl.smem), st, p);
   B2L_LAUNCH_CHECK();
-  if (p.splits > 1 && p.tickets == nullptr) {
+  if (merge) {
     dim3 g2((unsigned)batch, (unsigned)p.Hq);
     // up to nine blocks per SM the merge waits for its rows, beyond that the shorter kernel is the faster one (kv heads of 128,
     // up to 2000 tokens: 24 x 32 heads 44.0 against 40.7 us, 48 x 28 heads 31.7 / 30.6; 64 x 32 heads, 1000 of 4096 59.4 / 60.9)
