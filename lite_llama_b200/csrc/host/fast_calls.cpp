@@ -129,13 +129,21 @@ i64 quant_workspace(int kind, i64 m, i64 n, i64 k, i64 group, int device) {
   return (*seen)[s] = abi.quant_workspace(kind, m, n, k, group);
 }
 
+// Torch's translation of exceptions, without the buffer for warnings of HANDLE_TH_ERRORS: nothing here warns.
+#define FAST_BEGIN try {
+#define FAST_END                                                      \
+  }                                                                   \
+  catch (...) {                                                       \
+    torch::translate_exception_to_python(std::current_exception());   \
+    return nullptr;                                                   \
+  }
 #define ARGS(n) \
   if (count != (n)) { PyErr_SetString(PyExc_TypeError, "wrong number of arguments"); return nullptr; }
 
 // (x, qweight, scales, group_n, group_k) -> y
 PyObject* w8a16(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(5)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *x = plain(a[0]), *q = plain(a[1]), *s = plain(a[2]);
   const int device = device_for(abi.w8a16, {x, q, s});
   if (device < 0 || !PyLong_CheckExact(a[3]) || !PyLong_CheckExact(a[4])) return none();
@@ -162,13 +170,13 @@ PyObject* w8a16(PyObject*, PyObject* const* a, Py_ssize_t count) {
                    bytes, tickets, num_tickets, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // (x, qweight, scales, zeros, n, k, group_size, zeros_foldable, swiglu) -> y
 PyObject* w4a16_packed(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(9)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *x = plain(a[0]), *q = plain(a[1]), *s = plain(a[2]), *z = plain(a[3]);
   const int device = device_for(abi.w4a16, {x, q, s, z});
   if (device < 0) return none();
@@ -195,13 +203,13 @@ PyObject* w4a16_packed(PyObject*, PyObject* const* a, Py_ssize_t count) {
                    tickets, num_tickets, swiglu, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // (x, weight) -> y
 PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(2)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *x = plain(a[0]), *w = plain(a[1]);
   const int device = device_for(abi.linear, {x, w});
   if (device < 0) return none();
@@ -223,13 +231,13 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t count) {
                     bytes > 0 ? ws.data_ptr() : nullptr, bytes, tickets, num_tickets, code, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // (qa, a_scales, qweight, weight_scales [N] or [N, 1], bfloat16 out) -> y
 PyObject* w8a8(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(5)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *x = plain(a[0]), *sa = plain(a[1]), *w = plain(a[2]), *sw = plain(a[3]);
   const int device = device_for(abi.w8a8, {x, sa, w, sw});
   if (device < 0) return none();
@@ -256,7 +264,7 @@ PyObject* w8a8(PyObject*, PyObject* const* a, Py_ssize_t count) {
                   bf16, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 PyObject* pair_of(at::Tensor a, at::Tensor b) {
@@ -270,7 +278,7 @@ PyObject* pair_of(at::Tensor a, at::Tensor b) {
 // (a) -> (q, scales)
 PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(1)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor* x = plain(a[0]);
   const int device = device_for(abi.quantize, {x});
   if (device < 0) return none();
@@ -286,7 +294,7 @@ PyObject* quantize(PyObject*, PyObject* const* a, Py_ssize_t count) {
     rc = abi.quantize(q.data_ptr(), s.data_ptr(), x->data_ptr(), m, k, x->stride(0), k, code, stream(device));
   }
   return rc ? failed(rc) : pair_of(std::move(q), std::move(s));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // rows of the norms: contiguous matrices that the results may alias
@@ -300,7 +308,7 @@ bool norm_rows(const at::Tensor& x, PyObject* res, const at::Tensor* r, const at
 // (X, residual or None, weight, eps) -> (Y, residual or X)
 PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(4)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *x = plain(a[0]), *r = a[1] == Py_None ? nullptr : plain(a[1]), *w = plain(a[2]);
   const int device = r ? device_for(abi.norm, {x, w, r}) : device_for(abi.norm, {x, w});
   if (device < 0 || !PyFloat_CheckExact(a[3]) || !norm_rows(*x, a[1], r, *w)) return none();
@@ -319,13 +327,13 @@ PyObject* norm(PyObject*, PyObject* const* a, Py_ssize_t count) {
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(std::move(y)));
   PyTuple_SET_ITEM(out, 1, Py_NewRef(r ? a[1] : a[0]));
   return out;
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // (X, residual or None, weight, eps) -> (q, scales)
 PyObject* norm_quant(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(4)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *x = plain(a[0]), *r = a[1] == Py_None ? nullptr : plain(a[1]), *w = plain(a[2]);
   const int device = r ? device_for(abi.norm_quant, {x, w, r}) : device_for(abi.norm_quant, {x, w});
   if (device < 0 || !PyFloat_CheckExact(a[3]) || !norm_rows(*x, a[1], r, *w)) return none();
@@ -341,13 +349,13 @@ PyObject* norm_quant(PyObject*, PyObject* const* a, Py_ssize_t count) {
                         (float)PyFloat_AS_DOUBLE(a[3]), half_code(*x), stream(device));
   }
   return rc ? failed(rc) : pair_of(std::move(q), std::move(s));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // (a, b) -> silu(a) * b
 PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t count) {
   ARGS(2)
-  HANDLE_TH_ERRORS
+  FAST_BEGIN
   const at::Tensor *g = plain(a[0]), *u = plain(a[1]);
   const int device = device_for(abi.swiglu, {g, u});
   if (device < 0) return none();
@@ -362,7 +370,7 @@ PyObject* swiglu(PyObject*, PyObject* const* a, Py_ssize_t count) {
     rc = abi.swiglu(y.data_ptr(), g->data_ptr(), u->data_ptr(), rows, n, g->stride(0), u->stride(0), n, code, stream(device));
   }
   return rc ? failed(rc) : THPVariable_Wrap(std::move(y));
-  END_HANDLE_TH_ERRORS
+  FAST_END
 }
 
 // (addresses of the C functions in the order of `abi`, zeroed_workspace, counters)
