@@ -466,10 +466,11 @@ static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPa
 // 4096 at 256 33 -> 21, 9728 x 896 at 192 (two waves of pair tiles as well) 13.8 -> 10.8; five against four, 28672 x 4096 at 192
 // 94 -> 75; at 4096 tokens 1853 -> 900.
 // One segment over all of k (a scale per output row) leaves the streaming kernel a single MMA warp; there the pair
-// kernel wins as soon as it has 16 tiles (int8, 896 x 4864, 512 tokens 27 -> 19; 320 tokens, 12 tiles: level).  That holds
-// for decode batches too (tiles of 64 tokens, six conversion stages; int8, 32 tokens: 28672 x 4096 82 -> 28, 6144 x 4096
-// 18.7 -> 14.5, 4096 x 4096 16.1 -> 14.5) unless k is long and few pairs have work, where the split of k wins (4096 x 14336,
-// 16 tiles: 37 against 45).
+// kernel wins as soon as it has 16 tiles (int8, 896 x 4864, 512 tokens 27 -> 19; 320 tokens, 12 tiles: level).
+// Up to 64 tokens (tiles of 64, six conversion stages) the batch kernel is asked first and faster (gemm_quant_batch.cu).  What
+// it leaves: 49 - 64 tokens with more weight tiles than SMs (28672 x 4096, int8: 26 here, 28 there), which are more than 40 tiles
+// of this kernel, and callers without its workspace, which this kernel does not need.  For those, against the streaming kernel
+// (int8, 32 tokens): 28672 x 4096 82 -> 28, 4096 x 4096 16.1 -> 14.5, but 4096 x 14336 (long k, 16 tiles) 37 / 45.
 bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k) {
   // segments of whole operand stages, or one segment over all of K
   if (group_k % kQpStepK != 0 && group_k < K) return false;

@@ -126,7 +126,7 @@ def test_w8_pair_tiles(m, n, k, fmt):
 
 
 @pytest.mark.parametrize("m", [1, 31, 33, 64])
-@pytest.mark.parametrize("n,k", [(10140, 528), (4096, 4096)])
+@pytest.mark.parametrize("n,k", [(10140, 528), (4096, 4096), (19210, 528)])      # 64 tokens of the last: the pair kernel's tiles
 @pytest.mark.parametrize("fp8", [True, False])
 def test_w8_per_channel_decode_tiles(m, n, k, fp8):
     x = torch.randn(m, k, device="cuda", dtype=torch.float16)
