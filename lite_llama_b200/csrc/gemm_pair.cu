@@ -484,12 +484,13 @@ static int pair_bn(int64_t m_tiles, int64_t N, int pairs) {
   return w128 * 132 < w256 * 100 ? 128 : 256;
 }
 
-// How many pairs share a tile: as many as still fit in one wave of clusters (a B200 holds 15 of eight CTAs, 33 of four), where
-// the parts of k outweigh the sum at their end.  us, whichever kernel had the call -> split: 4 pairs, 256 x 3584 x 18944 bf16
-// 69 -> 33, int8 38 -> 19.5; 96 tokens (half of the rows are padding) 40 -> 30 and 26 -> 18.5; 192 x 1024 x 2048 11.2 -> 8.8 and
-// 11.0 -> 7.8; 2 pairs, 256 x 4096 x 14336 53 -> 39 and 30 -> 24, 512 x 2048 x 4096 18 -> 16 and 13.4 -> 11.9.  Not: 192 x 3328 x
-// 1024 bf16 7.2 / 8.9, 512 x 2048 x 768 6.9 / 8.4, 1024 x 2048 x 4096 int8 12.5 / 13.4 (64 tiles of 128 outputs fill the pairs),
-// 384 x 512 x 8192 bf16 14.8 / 16.0 (four tiles: the one-SM kernel splits k further).
+// How many pairs share a tile: four or two where all clusters are in one wave and the parts of k outweigh the sum at their end.
+// us, whichever kernel had the call -> split: 4 pairs, 256 x 3584 x 18944 bf16 69 -> 33, int8 38 -> 19.5; 96 tokens (half of the
+// rows are padding) 40 -> 30 and 26 -> 18.5; 192 x 1024 x 2048 11.2 -> 8.8 and 11.0 -> 7.8; 2 pairs, 256 x 4096 x 14336 53 -> 39 and
+// 30 -> 24, 512 x 2048 x 4096 18 -> 16 and 13.4 -> 11.9.  Not: 192 x 3328 x 1024 bf16 7.2 / 8.9, 512 x 2048 x 768 6.9 / 8.4, 1024 x 2048 x
+// 4096 int8 12.5 / 13.4 (64 tiles of 128 outputs fill the pairs), 384 x 512 x 8192 bf16 14.8 / 16.0 (four tiles: the one-SM kernel
+// splits k further).  The limits in tiles stay below what a whole B200 holds at once, 15 clusters of eight CTAs and 33 of four;
+// a part with fewer SMs may hold fewer, so below 132 nothing is shared.
 static int pair_splits(int kind, const PairGemm& g) {
   const int64_t tiles = cdiv64(g.M, 2 * kPairRows) * cdiv64(g.N, 256), kb = cdiv64(g.K, kind == 0 ? 64 : 128);
   if (b2l_num_sms() < 132 || g.M <= kPairRows / 2) return 1;

@@ -16,6 +16,9 @@
 //   * a tile's groups meet in tensor memory, where a row is the same lane for all of them: each group sums up some tokens.
 //   * a tile shared by several CTAs is split evenly where possible, and every sharer then adds up its part of the tokens
 //     (bq_plan): with one CTA reading all partial sums of 64 tokens, a 4096 x 4096 projection ended with 4 us of trips to L2.
+//     The sharers then wait for one another, so all CTAs of a launch have to be resident at the same time: the grid is at most
+//     one CTA per SM, and the calls of a device follow one another on one stream, as the workspace and the tickets that they have in
+//     common demand in any case (kernels/_common.py).
 //   * conversion starts before the previous kernel has ended (weights are static); only activations and results wait for it.
 // Measured against the kernels that had these calls: quant_batch_wanted below.  Tried and not kept: both halves of a segment
 // handed to the MMAs one by one (28672 x 4096, int4, 32 tokens 30 us), accumulators or operands in two buffers (three

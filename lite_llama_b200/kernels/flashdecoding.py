@@ -23,7 +23,8 @@ def flash_decoding(
     Args mirror the reference: ``q [B, Hq, D]``; ``k_cache``/``v_cache`` ``[max_tokens, Hkv, D]``
     (usually strided views of one ``[max_tokens, 2*Hkv, D]`` pool); ``qk_scale = 1/sqrt(D)``;
     ``b_req_tokens_table [max_requests, max_seq_len]`` int32; ``b_req_idx``/``b_seq_len`` ``[B]``
-    int32 or int64; ``max_actual_seq_len`` a Python int (sizes the split grid; graph-safe).
+    int32 or int64; ``max_actual_seq_len`` a Python int (sizes the split grid; graph-safe).  The result of a row of length 0
+    is zero.
     """
     require_cuda(q, k_cache, v_cache, b_req_tokens_table, b_req_idx, b_seq_len)
     assert q.shape[-1] == k_cache.shape[-1] == v_cache.shape[-1]

@@ -121,7 +121,11 @@ def w4a16_matmul_packed(x: torch.Tensor, packed: PackedW4, *, bias: torch.Tensor
 
     ``swiglu=True``: the packed rows are interleaved ``(gate_0, up_0, gate_1, up_1, ...)`` (see
     :func:`interleave_gate_up`) and the GEMM's epilogue applies ``silu(gate) * up``; the result is ``[..., N/2]``
-    and equals ``swiglu_forward`` of the two separate projections bit for bit."""
+    and equals ``swiglu_forward`` of the two halves of the same product without ``swiglu``, bit for bit.
+
+    Both layouts give the same bits while the same kernel takes them: up to 48 tokens, and up to 64 where there are no more tiles
+    of 128 weight rows than SMs, with whole zero points.  Beyond that, and with other zero points (but in the kernel of up
+    to 8 tokens), the sums over k may run in another order."""
     if bias is None:
         out = _native.w4a16_packed(x, packed.qweight, packed.scales, packed.zeros, packed.n, packed.k, packed.group_size,
                                    packed.zeros_foldable, swiglu)
