@@ -142,24 +142,29 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     constexpr int CH = 16;
     T* y = reinterpret_cast<T*>(p.y);
 
-    // int8: activation scales of CH tokens (the same address in every lane), requested before the sums they go with are waited
-    // for: one load per token behind them took 3.5 us of a projection (96 tokens, 18944 x 3584: 19.3 -> 16.0)
+    // int8: the scales are requested before the sums they go with are waited for: one load per token behind them took 3.5 us of a
+    // projection (96 tokens, 18944 x 3584: 19.3 -> 16.0).  Activation scales of CH tokens are four loads with the same address in
+    // every lane, or, in a chunk that is not full, one load whose lanes pass on a token each.
     float sa[KIND == 1 ? CH : 1];
-    // (the weight scale too, from 64 tokens on: with fewer the early request costs more, 1024 x 896 3.3 -> 3.5 us)
-    const float sb = KIND == 1 && BT >= 64 && n < p.N ? p.b_scale[n] : 0.f;
-    bool ahead = false;
+    float sb = 0.f;
+    bool full = false;
     auto scales = [&](int col0) {
+      if (KIND != 1) return;
       const int m0 = m_tile * BT + col0;
-      ahead = KIND == 1 && p.a_vec && m0 + CH <= p.M;
-      if (ahead) {
+      if (col0 == 0) sb = p.b_scale[n < p.N ? n : p.N - 1];
+      full = p.a_vec && m0 + CH <= p.M;
+      if (full) {
 #pragma unroll
         for (int j = 0; j < CH; j += 4) {
           const float4 f = *reinterpret_cast<const float4*>(p.a_scale + m0 + j);
           sa[KIND == 1 ? j : 0] = f.x; sa[KIND == 1 ? j + 1 : 0] = f.y; sa[KIND == 1 ? j + 2 : 0] = f.z; sa[KIND == 1 ? j + 3 : 0] = f.w;
         }
+      } else {
+        const int m = m0 + (lane & (CH - 1));
+        sa[0] = p.a_scale[m < p.M ? m : p.M - 1];
       }
     };
-    auto finish_as = [&](int col0, const uint32_t (&v)[CH], auto ahead) {
+    auto finish_as = [&](int col0, const uint32_t (&v)[CH]) {
       if (n >= p.N) return;
 #pragma unroll
       for (int j = 0; j < CH; ++j) {
@@ -171,7 +176,7 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             if (p.bias) r += to_f32(reinterpret_cast<const T*>(p.bias)[n]);
           } else {
             // w8a8.py:117-123: acc.float * a_scale[m] * b_scale[n] (+ bias)
-            r = (float)(int)v[j] * (decltype(ahead)::value ? sa[KIND == 1 ? j : 0] : p.a_scale[m]) * (BT >= 64 ? sb : p.b_scale[n]);
+            r = (float)(int)v[j] * sa[KIND == 1 ? j : 0] * sb;
             if (p.bias) r += reinterpret_cast<const float*>(p.bias)[n];
           }
           y[(int64_t)m * p.ldy + n] = from_f32<T>(r);
@@ -179,8 +184,12 @@ gemm_swapab_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     };
     auto finish = [&](int col0, const uint32_t (&v)[CH]) {
-      if (ahead) finish_as(col0, v, std::true_type{});
-      else finish_as(col0, v, std::false_type{});
+      if (KIND == 1 && !full) {
+        const float mine = sa[0];
+#pragma unroll
+        for (int j = 0; j < CH; ++j) sa[KIND == 1 ? j : 0] = __shfl_sync(0xffffffffu, mine, j);
+      }
+      finish_as(col0, v);
     };
 
     if (p.splits == 1) {

@@ -265,7 +265,8 @@ def test_per_channel_accumulations_are_no_longer_than_the_parts_of_k(m, n, k, ch
     assert abs(((got - want) / want).mean().item()) < chain / 16 * 2.0**-23
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 136, 64), (17, 1000, 256), (130, 520, 512), (300, 10248, 144), (256, 3584, 2048)])
+@pytest.mark.parametrize("m,n,k", [(1, 136, 64), (17, 1000, 256), (130, 520, 512), (300, 10248, 144), (256, 3584, 2048),
+                                   (7, 1000, 256), (33, 520, 4096), (65, 9736, 896), (97, 9736, 128)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_int8_scales_in_vectors_and_alone(m, n, k, shift):
     """Scales and bias that start on a 16-byte boundary are loaded in vectors, others one by one: the same result."""
