@@ -83,7 +83,7 @@ struct QuantParams {
 };
 // Wait flavour of the hand-off barriers (0: try_wait with the long suspend hint, 1: test_wait polling, 2: try_wait
 // with the default suspend window).  B2L_QWAIT_MODE covers every wait, B2L_QWAIT_LAT_MODE the latency-critical
-// ones (operand stage full / free, accumulator full): A/B builds, see tools/build_variants.py.
+// ones (operand stage full / free, accumulator full): for A/B builds.
 #ifndef B2L_QWAIT_MODE
 #define B2L_QWAIT_MODE 0
 #endif
@@ -107,14 +107,14 @@ __device__ __forceinline__ void qwait_at(uint64_t* bar, uint32_t parity, int lin
 __host__ __device__ constexpr bool q_noreturn(int qk, int bt) { return !(qk == Q_INT4 && bt == 64); }
 #define qwait(bar, parity) qwait_at<B2L_QWAIT_MODE, q_noreturn(QK, BT)>((bar), (parity), __LINE__)
 #define qwait_lat(bar, parity) qwait_at<B2L_QWAIT_LAT_MODE, q_noreturn(QK, BT)>((bar), (parity), __LINE__)
-// B2L_TLITE (A/B builds only, tools/build_variants.py): a handful of clock stamps per CTA
+// B2L_TLITE (A/B builds only): a handful of clock stamps per CTA
 #ifdef B2L_TLITE
 #define LT(i) do { if (p.timeline) p.timeline[(size_t)blockIdx.x * 32 + (i)] = clock64(); } while (0)
 #else
 #define LT(i) do {} while (0)
 #endif
 
-static long long* g_timeline = nullptr;   // set through b2l_debug_set_timeline (tools/tlite.py)
+static long long* g_timeline = nullptr;   // set through b2l_debug_set_timeline
 
 struct __align__(8) QControl {
   uint64_t w_full[kMaxRawStages];
@@ -215,7 +215,7 @@ __device__ __forceinline__ void st_release_smem(int* p, int v) {
 // MMA issue of one full raw block whose K range holds whole segments of SPS sub-blocks each (scale group divides the
 // raw block): one operand stage (two sub-blocks, 8 MMA steps) per elected-lane block, every offset a compile-time
 // constant.  The issuing warp shares its scheduler with two dequant warps and gets an issue slot every ~4-6
-// cycles, so its instruction count -- not the tensor pipe (16 cycles per MMA at 32 tokens: tools/mma_rate.cu) --
+// cycles, so its instruction count -- not the tensor pipe (16 cycles per MMA at 32 tokens) --
 // sets the pace of the accumulator hand-offs: ~25 instructions per sub-block here against ~90 in a rolled loop
 // with run-time stage arithmetic (700 cycles per segment on the device timeline, profiles/).
 // Operand-ring slot of operand stage `sp` (0 .. SUBST-1) of raw block `rb`.  The ring is split into two halves of
@@ -871,7 +871,7 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         // other slots once all 512 threads are free (end of the kernel), clearing the words behind it: the workspace
         // is all-zero between launches (contract of the C ABI, like the ticket counters).  Ticket protocol before:
         // fence + atomic (two L2 round trips) on every sharer, then up to two serial tile reductions on whoever came
-        // last -- 3 to 5 us on the grid's critical path (per-CTA stamps, profiles/r2n_tlite*.txt).  All
+        // last -- 3 to 5 us on the grid's critical path (per-CTA stamps).  All
         // sk_ctas <= #SM CTAs are co-resident, so waiting for a sharer cannot dead-lock.
         uint32_t* base32 = p.ws + (size_t)pc.n_tile * slots_per_tile * (BT * kBlockW);
         if (slot != 0) {
@@ -963,7 +963,7 @@ gemm_quant_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       // a refill that found its weights in L2 could land in the stage first (rows are written in order, so the
       // lowest rows of a tile were the ones hit).  Found by tests/test_kernels_gpu.py::
       // test_w4a16_streamk_back_to_back_launches_are_isolated at 33-64 tokens: ~10 % of the launches over a long-K
-      // shape had one or a few output columns off by one scale group's contribution (tools/nondet_probe.py).
+      // shape had one or a few output columns off by one scale group's contribution.
       if (warp == 0 && lane == 0 && rb == 0) LT(8);
       // one operand sub-stage per 64-element sub-block; the "sub-block ready" arrive of sub-block s is issued
       // after the conversion of s+1, so tcgen05.wait::st never waits for a store that was just issued
