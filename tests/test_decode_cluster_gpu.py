@@ -39,7 +39,7 @@ def test_cluster_splits(bound, batch, hq, hkv, d, dtype):
     lens = torch.randint(1, bound + 1, (batch,), generator=gen)
     lens[0] = bound
     if batch > 2:
-        lens[1], lens[2] = (0 if bound > 64 else 5), 1          # (a single split leaves an empty row as it is)
+        lens[1], lens[2] = 0, 1
     q = torch.randn(batch, hq, d, generator=gen).to(dtype).cuda()
     pool = torch.randn(batch * bound + 5, 2 * hkv, d, generator=gen).to(dtype).cuda()
     table = torch.randperm(batch * bound, generator=gen).int().view(batch, bound).cuda() + 5
