@@ -30,6 +30,7 @@ constexpr int kTT = 16;            // tokens per pipeline stage (one m16n8k16 k-
 constexpr int kMaxConsumers = 8;
 constexpr int kMaxStages = 4;
 constexpr int kMaxCluster = 8;
+constexpr int kStagesAt = 128;     // bytes of shared memory before the stages: their barriers
 
 struct DecodeParams {
   const void* q; int64_t q_bs, q_hs;
@@ -75,14 +76,15 @@ __device__ __forceinline__ float4 ld_peer4(uint32_t addr) {
 
 // The splits of a row and head block, left by the CTAs of a cluster in their own shared memory (rows, then statistics), added up
 // in split order like in the kernels below.  Every CTA takes its share of the outputs, also those whose split is empty: where
-// those left before, two of eight CTAs made four trips through shared memory for 32 heads (4 kv heads, 16 rows of 20 tokens under
-// a bound of 80: 7.4 us, the merge kernel 7.0, now 5.5).
+// those left before, one or two of eight CTAs made four to eight trips through shared memory for 32 heads (4 kv heads, 16 rows of
+// 16 tokens under a bound of 65 8.6 us, of 20 under 80 7.4; merge kernel 5.9 and 6.9; now 5.3 and 5.4).  A way of its own for rows of
+// one split took 4.0, and all others 0.2 - 0.6 longer: these steps are short enough for the size of their code to count.
 template <typename T, int D>
-__device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t part, int64_t seq_len) {
+__device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t part, int len) {
   const int split = blockIdx.x, heads = p.HB * p.G;
   __syncwarp();
   cluster_sync_all();
-  const int nsp = (int)((seq_len + p.chunk - 1) / p.chunk) < p.splits ? (int)((seq_len + p.chunk - 1) / p.chunk) : p.splits;
+  const int nsp = (int)((unsigned)(len + p.chunk - 1) / (unsigned)p.chunk);
   for (int i = split * blockDim.x + threadIdx.x; i < heads * (D / 4); i += p.splits * blockDim.x) {
     const int local = i / (D / 4), d = i % (D / 4) * 4;
     float lse[kMaxCluster];
@@ -119,13 +121,12 @@ __device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t pa
 // which are the grid's x, up to kMaxCluster splits.  The second form does the first one's work as well; its code for the rest costs
 // 0.2 - 0.3 us of 16 - 51, except with heads of 256, whose sums do not fit into registers and spill less in it (4 %).
 enum { FD_SPLITS, FD_WHOLE, FD_CLUSTER };
+// one split with tokens
 template <typename T, int D, int FORM>
-__global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_kernel(const DecodeParams p) {
-  pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
-  extern __shared__ __align__(128) uint8_t smem[];
+__device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* smem, int64_t seq_len, int64_t start) {
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);   // [kMaxStages]
   uint64_t* empty_bar = full_bar + kMaxStages;              // [kMaxStages]
-  uint8_t* stage_base = smem + 128;
+  uint8_t* stage_base = smem + kStagesAt;
 
   const int split = blockIdx.x;
   const int hblk = blockIdx.y;
@@ -133,21 +134,6 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nconsumers = p.HB * p.qblocks;      // blockDim.x == (nconsumers + 1) * 32
 
-  const int64_t seq_len = load_index(p.seq_len, b, p.len_w);
-  const int64_t start = (int64_t)split * p.chunk;
-  // a row of one split has nothing to merge
-  const bool alone = FORM == FD_CLUSTER ? seq_len <= p.chunk : FORM == FD_WHOLE && p.splits == 1;
-  if (start >= seq_len) {        // empty split: nothing to contribute
-    if (FORM == FD_CLUSTER && !alone) {
-      cluster_merge<T, D>(p, smem_u32(stage_base), seq_len);
-    } else if (FORM != FD_SPLITS && split == 0) {     // an empty row is zero
-      const int heads = p.HB * p.G;
-      for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
-        *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs +
-                                     (int64_t)(hblk * heads + i / (D / 2)) * p.o_hs + 2 * (i % (D / 2))) = 0u;
-    }
-    return;                      // the whole CTA together
-  }
   const int64_t end = (start + p.chunk < seq_len) ? start + p.chunk : seq_len;
   const int ntiles = (int)((end - start + kTT - 1) / kTT);
   const int64_t req = load_index(p.req_idx, b, p.req_w);
@@ -328,13 +314,13 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       if (!ok) continue;
       const int head = kvh * p.G + (r2 == 0 ? hq0 : hq1);
       const float inv = 1.0f / l_run[r2];
-      if (FORM == FD_CLUSTER && !alone) {
+      if (FORM == FD_CLUSTER) {
         const int local = hl * p.G + (r2 == 0 ? hq0 : hq1);
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
           *reinterpret_cast<float2*>(part + local * D + i * 8 + 2 * tq) = make_float2(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
         if (tq == 0) part[p.HB * p.G * D + local] = m_run[r2] + log2f(l_run[r2]);
-      } else if (alone) {
+      } else if (FORM == FD_WHOLE && p.splits == 1) {
         T* orow = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)head * p.o_hs;
 #pragma unroll
         for (int i = 0; i < D / 8; ++i)
@@ -348,11 +334,6 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
         if (tq == 0) p.ws_lse[off] = m_run[r2] + log2f(l_run[r2]);
       }
     }
-  }
-
-  if (FORM == FD_CLUSTER) {
-    if (!alone) cluster_merge<T, D>(p, smem_u32(stage_base), seq_len);
-    return;
   }
 
   // ---- stage 2 folded in (reference: a second kernel, flashdecoding.py:224-313): the CTA that finishes a
@@ -390,6 +371,25 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
       }
     }
   }
+}
+
+template <typename T, int D, int FORM>
+__global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_kernel(const DecodeParams p) {
+  pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
+  extern __shared__ __align__(128) uint8_t smem[];
+  const int64_t seq_len = load_index(p.seq_len, blockIdx.z, p.len_w);
+  const int64_t start = (int64_t)blockIdx.x * p.chunk;
+  const int most = p.chunk * kMaxCluster;                   // FD_CLUSTER: tokens that its kMaxCluster splits hold
+  const int len = seq_len < most ? (int)seq_len : most;
+  if (start < seq_len) {
+    decode_split<T, D, FORM>(p, smem, seq_len, start);
+  } else if (FORM != FD_SPLITS && blockIdx.x == 0) {        // an empty row is zero; other empty splits have nothing to contribute
+    const int heads = p.HB * p.G;
+    for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
+      *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)blockIdx.z * p.o_bs +
+                                   (int64_t)(blockIdx.y * heads + i / (D / 2)) * p.o_hs + 2 * (i % (D / 2))) = 0u;
+  }
+  if (FORM == FD_CLUSTER && len > 0) cluster_merge<T, D>(p, smem_u32(smem + kStagesAt), len);
 }
 
 // Stage 2: log-sum-exp merge of the per-split partials (reference: flashdecoding.py:224-313).
@@ -462,8 +462,8 @@ void plan_ring(Plan& pl, int D, int smem_cap) {
 // Steps of up to 256 tokens a row that leave most of the chip idle: one wave of clusters of eight splits, two of their CTAs to an
 // SM.  A tile costs its CTA 0.6 - 1 us (copies, and one warp's chain of products), the merge kernel 3 us, a cluster's launch and
 // barriers 2 us.  us in a graph, splits of 64 tokens and the merge kernel -> this: 8 kv heads of 128, one sequence of 200 tokens
-// 8.6 -> 6.7, of 80 7.6 -> 5.2, eight of 200 8.8 -> 7.7; 16 of 4 kv heads 8.6 -> 7.4; mixed lengths under that bound 8.6 -> 6.7, 9.2 ->
-// 7.4 and 9.4 -> 6.8; rows of a quarter of the bound 8.4 -> 6.3, 8.7 -> 7.1 and 8.8 -> 6.5; of one tile, under 65, 5.1 - 5.9 -> 3.6 - 4.0.
+// 8.6 -> 6.6, of 80 7.5 -> 5.1, eight of 200 8.8 -> 7.7; 16 of 4 kv heads 8.6 -> 7.4; mixed lengths under that bound 8.6 -> 6.6, 9.2 ->
+// 7.3 and 9.4 -> 6.8; rows of a quarter of the bound 8.4 -> 6.2, 8.7 -> 7.1 and 8.9 -> 6.5; of one tile, under 65, 5.1 - 5.9 -> 4.9 - 5.5.
 // None of 540 mixtures (1 - 16 sequences, bounds of 65 - 256, six head layouts) is slower.
 // Longer splits are the longer chain here (512 tokens in four tiles each 9.1 against 8.9), up to four tiles there is a single
 // split without a merge, and with one CTA to an SM the clusters of eight do not all fit (16 sequences of 8 kv heads 8.7 against
