@@ -16,7 +16,8 @@
 // Measured, 28672 x 4096 at 4096 tokens, launches by themselves (streaming kernel -> this one; 15 - 20 % more in a pass that
 // keeps the card at its power cap): int4 1853 -> 900 us (1.07 PFLOP/s), fp8 in 128 x 128
 // blocks 1748 -> 867 us, int8 per channel 3124 -> 754 us (no drain before the end of k: 1.28 PFLOP/s).  A third accumulator
-// at the cost of two operand stages: int4 878, fp8 901 us.
+// at the cost of two operand stages: int4 878, fp8 901 us.  Sizes of that order are now taken by the kernel of 256 tokens per
+// tile (gemm_quant_wide.cu).
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of
 // the accumulator per scale group, acc = fma(scale, segment, acc) in fp32 in ascending k.
 #define B2L_HANG_NORETURN true   // common.cuh: 128 accumulators beside the wait loops
@@ -53,21 +54,6 @@ struct __align__(8) QpControl {
   uint32_t tmem_base;
 };
 static_assert(sizeof(QpControl) <= 1024, "control block too large");
-
-__device__ __forceinline__ uint64_t pack_f32x2(float a, float b) {
-  uint64_t r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ void unpack_f32x2(uint64_t v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-// two IEEE fused multiply-adds in one instruction
-__device__ __forceinline__ uint64_t fma_f32x2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t r;
-  asm volatile("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 // What a tile is: `mode` plain = one weight matrix; grouped = experts, one entry of the tile table per 128 rows of an
 // expert's run of the sorted activations (moe_sort, moe_routing.cu), the entries' output tiles next to one another so that
@@ -516,6 +502,7 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
   if (rc != B2L_OK) return rc;
   rc = b2l_make_tmap_2d(&tx, x, TMA_F16, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, kQpTokens / 2, 64, true);
   if (rc != B2L_OK) return rc;
+  if (quant_wide_wanted(qk, M, N)) return quant_wide_gemm(qk, p, tw, tx, swiglu, st);
   if (qk == Q_INT4) return swiglu ? launch_qp<Q_INT4, 1>(tw, tx, p, grid, st) : launch_qp<Q_INT4, 0>(tw, tx, p, grid, st);
   if (M <= 64)
     return qk == Q_FP8 ? launch_qp<Q_FP8, 0, QP_PLAIN, 64>(tw, tx, p, grid, st) : launch_qp<Q_INT8, 0, QP_PLAIN, 64>(tw, tx, p, grid, st);

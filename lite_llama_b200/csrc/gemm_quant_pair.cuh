@@ -16,12 +16,16 @@ struct QuantPairParams {
   const int32_t* order;                              // grouped down projection: slot of every sorted row
   const __half* row_weights;                         // grouped down projection: routing weight by slot
   int M, N, steps, seg_steps, groups, m_tiles, n_tiles;      // filled by quant_pair_gemm (groups: pitch of the int4 tables)
+  int tiles, split_from, vec;                        // wide tiles: their number, the first that is cut in two, y in 8-byte stores
 };
 
 // shapes the pair kernel takes and is the faster one for (see gemm_quant_pair.cu); qk: QuantKind
 bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k);
 int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, const void* w, int64_t w_stride_bytes,
                     int64_t M, int64_t N, int64_t K, int64_t group_k, int swiglu, cudaStream_t st);
+// the same with 256 tokens per tile (gemm_quant_wide.cu); boxes of the tensor maps: 128 weight rows, 64 tokens
+bool quant_wide_wanted(int qk, int64_t M, int64_t N);
+int quant_wide_gemm(int qk, QuantPairParams& p, const CUtensorMap& tw, const CUtensorMap& tx, int swiglu, cudaStream_t st);
 
 // The two products of a routed SwiGLU layer over activations sorted by expert (moe_routing.cu: b2l_moe_sort, b2l_moe_gather).
 struct MoePairGemm {

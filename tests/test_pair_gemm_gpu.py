@@ -307,3 +307,34 @@ def test_int8_split_over_a_cluster(m, n, k, bias):
     b = torch.randn(n, device="cuda") if bias else None
     want = (qa.double() @ qw.double().T) * sa.double()[:, None] * sw.double() + (b.double() if bias else 0.0)
     assert rel(K().smoothquant_matmul_prequant(qa, sa, qw, sw, bias=b), want) < REL[torch.float16]
+
+
+# ---- 256 tokens per tile (csrc/gemm_quant_wide.cu) ----
+# 74 pairs: whole waves; a last wave cut in two, its second parts empty or short; a last tile of one half between tiles of two
+# (the accumulators' turn shifts by an odd number of segments); rows of y that no 8-byte store fits; an odd number of steps
+WIDE_EDGES = [(300, 18944, 384), (513, 12800, 640), (1000, 9734, 128), (769, 9734, 384), (640, 18688, 896), (1537, 3330, 1152)]
+
+
+@pytest.mark.parametrize("m,n,k", WIDE_EDGES)
+@pytest.mark.parametrize("group", [128, 384])
+def test_int4_wide_tiles(m, n, k, group):
+    if k % group:
+        pytest.skip("groups divide k")
+    q, s, z, w, x = int4_case(n, k, group, m)
+    b = torch.randn(n, device="cuda")
+    packed = K().w4a16_pack(q, s, z, group_size=group)
+    got = K().w4a16_matmul_packed(x, packed, bias=b)
+    assert rel(got, x.double() @ w.T + b.double()) < REL[torch.float16]
+    if n > 148 * 64:    # a row's sums do not depend on its tile: the same bits from the kernel of 128 tokens per tile
+        assert torch.equal(K().w4a16_matmul_packed(x[:128], packed, bias=b), got[:128])
+
+
+@pytest.mark.parametrize("m,n,k", WIDE_EDGES)
+def test_int4_wide_swiglu_is_gemm_then_swiglu(m, n, k):
+    test_int4_pair_swiglu_is_gemm_then_swiglu(m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", WIDE_EDGES)
+@pytest.mark.parametrize("fmt", ["fp8_block", "fp8_channel", "int8_channel", "int8_group_n"])
+def test_w8_wide_tiles(m, n, k, fmt):
+    test_w8_pair_tiles(m, n, k, fmt)
