@@ -6,18 +6,21 @@
 // 64 tokens of MMAs last 256 cycles, so its hand-offs were the critical path (430 - 500 TF/s).  Here the tile is 256
 // weight rows x 128 tokens on a pair of SMs:
 //   * 128 rows x 128 k feed 512 cycles of MMAs per SM: conversion (two groups of four warps, each its own half of the
-//     operand stages) plus the drain of one accumulator segment take half of the issue slots (1024 tokens: int4 52 %, with the
-//     tensor pipe busy for 49 % of the cycles, fp8 45 and 56 %; profiles/pair_gemm_ncu.txt): what is left is waiting at hand-offs;
+//     operand stages) plus the drain of one accumulator segment take half of the issue slots: what was left was waiting at
+//     hand-offs, most of all for the one issuing warp and for the trip of an accumulator (gemm_quant_wide.cu), so there are two
+//     issuers and three or four accumulators where every 128 k are a segment of their own;
 //   * cta_group::2: each SM stages 64 of the 128 tokens, 48 bytes per clock and SM from L2 for int4 weights;
-//   * the operand stays in tensor memory (4 stages of 128 k = 256 columns) beside two accumulator segments of 128 columns;
-//   * a segment's buffer is handed back as soon as its 128 columns are in the registers of eight epilogue warps, before the
+//   * the operand stays in tensor memory beside the accumulators;
+//   * a segment's buffer is handed back as soon as its columns are in the registers of eight epilogue warps, before the last
 //     multiply-adds: with four warps that read it in two turns the MMAs waited for the drain (977 us against 900);
 //   * the grid is persistent, rings run on across tiles.
 // Measured, 28672 x 4096 at 4096 tokens, launches by themselves (streaming kernel -> this one; 15 - 20 % more in a pass that
 // keeps the card at its power cap): int4 1853 -> 900 us (1.07 PFLOP/s), fp8 in 128 x 128
 // blocks 1748 -> 867 us, int8 per channel 3124 -> 754 us (no drain before the end of k: 1.28 PFLOP/s).  A third accumulator
 // at the cost of two operand stages: int4 878, fp8 901 us.  Sizes of that order are now taken by the kernel of 256 tokens per
-// tile (gemm_quant_wide.cu).
+// tile (gemm_quant_wide.cu).  One issuer and two accumulators -> two and three or four, us: int4 28672 x 4096 with the
+// activation at 128 tokens 42.7 -> 36.8, 4096 x 14336 at 512 63 -> 54, fp8 in blocks 4096 x 4096 at 512 19.3 -> 17.1; experts (128 of
+// 2048 x 768, fp8, top 8) gate|up and down at 2000 tokens 173 + 153 -> 135 + 126, at 32 69 + 46 -> 58 + 33.
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of
 // the accumulator per scale group, acc = fma(scale, segment, acc) in fp32 in ascending k.
 #define B2L_HANG_NORETURN true   // common.cuh: 128 accumulators beside the wait loops
@@ -25,32 +28,36 @@
 #include "gemm_quant_pair.cuh"
 #include "pair.cuh"
 #include "dequant.cuh"
+#include "gemm_quant_out.cuh"
 
 namespace gemm {
 
 constexpr int kQpThreads = 20 * 32;
-constexpr int kQpWStages = 6, kQpXStages = 6, kQpMaxOp = 6;
+constexpr int kQpWStages = 6, kQpXStages = 6, kQpMaxAcc = 4, kQpMaxOp = 8;
 constexpr int kQpTokens = 128;                              // per pair tile; each CTA stages half
-// Operand stages that fit beside the two accumulator segments of a tile of NT tokens.  With few tokens the MMAs are short and
-// the trip conversion -> leader -> MMA -> both CTAs is what a stage waits for: three stages per conversion group instead of
-// two.
-__host__ __device__ constexpr int qp_op_stages(int nt) { return nt == kQpTokens ? 4 : 6; }
-constexpr int kQpStepK = 128;                               // k per operand stage
+// Accumulators and operand steps that share tensor memory, for tiles of NT tokens.  Where every step of 128 k is a segment of
+// its own, the trip of an accumulator (commit, wake-up, loads of the epilogue, arrival, issue: about 1000 cycles, the MMAs of a
+// step 512 or 300) asks for three or four, and two issuing warps take turns.  CHAIN (longer segments): an accumulator's MMAs
+// follow one another, so one warp issues them, and what a step waits for is its conversion: two accumulators, more steps.
+__host__ __device__ constexpr int qp_accs(int nt, bool chain) { return chain ? 2 : nt == kQpTokens ? 3 : 4; }
+__host__ __device__ constexpr int qp_op_steps(int nt, bool chain) { return (512 - qp_accs(nt, chain) * nt) / 64; }
+constexpr int kQpStepK = 128;                               // k per operand step; without CHAIN handed over and back in stages of 64
 constexpr int kQpXSub = kQpTokens / 2 * kStageKBytes;       // 64 tokens x 64 k
 constexpr int kQpXBytes = 2 * kQpXSub;
-constexpr int kQpSmem = 1024 + 1024 + kQpWStages * kABytes + kQpXStages * kQpXBytes;
+constexpr int kQpMeta = 8 * 64 * 8;                         // down projection: {slot, routing weight} of the epilogue warps' rows
+constexpr int kQpSmem = 1024 + 1024 + kQpWStages * kABytes + kQpXStages * kQpXBytes + kQpMeta;
 constexpr int kQpBand = 16;
-constexpr int kQpEpi0 = 8, kQpWProd = 16, kQpXProd = 17, kQpMma = 18;   // eight conversion, eight epilogue warps
+constexpr int kQpEpi0 = 8, kQpWProd = 16, kQpXProd = 17, kQpMma = 18;   // eight conversion, eight epilogue warps, two issuers
 
 struct __align__(8) QpControl {
   uint64_t w_full[kQpWStages];      // own: a raw weight block has landed
   uint64_t w_empty[kQpWStages];     // own: its words have been converted (4 warp arrivals per operand stage in it)
   uint64_t x_full[kQpXStages];      // leader: both CTAs' token halves have landed
   uint64_t x_empty[kQpXStages];     // both: the MMAs that read them have retired
-  uint64_t op_full[kQpMaxOp];    // leader: both CTAs' converted rows are in tensor memory (8 warp arrivals)
-  uint64_t op_empty[kQpMaxOp];   // both
-  uint64_t acc_full[2];             // both: a segment is complete
-  uint64_t acc_empty[2];            // leader: both CTAs' epilogue warps have read it (16 warp arrivals)
+  uint64_t op_full[kQpMaxOp];       // leader: both CTAs' converted rows are in tensor memory (8 warp arrivals)
+  uint64_t op_empty[kQpMaxOp];      // both
+  uint64_t acc_full[kQpMaxAcc];     // both: a segment is complete
+  uint64_t acc_empty[kQpMaxAcc];    // leader: both CTAs' epilogue warps have read it (16 warp arrivals)
   uint32_t tmem_base;
 };
 static_assert(sizeof(QpControl) <= 1024, "control block too large");
@@ -87,7 +94,7 @@ __device__ __forceinline__ int qp_tile_n(int rows_left) {
   return n < NT ? n : NT;
 }
 
-template <int QK, int EPI, int MODE, int NT>
+template <int QK, int EPI, int MODE, int NT, bool CHAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kQpThreads, 1)
 gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                        const QuantPairParams p) {
@@ -97,7 +104,8 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   uint8_t* w_ring = smem + 1024;
   uint8_t* x_ring = w_ring + kQpWStages * kABytes;
   constexpr int kHalf = NT / 2;                            // tokens per epilogue warp
-  constexpr int kAccCols = NT, kOpCol0 = 2 * NT, kOpStages = qp_op_stages(NT);
+  constexpr int kAccs = qp_accs(NT, CHAIN), kOpSteps = qp_op_steps(NT, CHAIN), kOpCol0 = kAccs * NT;
+  constexpr int kSub = CHAIN ? 1 : 2, kOpStages = kSub * kOpSteps;      // stages per operand step
   // (plain mode with NT 64 is launched for up to 64 tokens only: one row of tiles)
   constexpr int kStepsPerRaw = QK == Q_INT4 ? 2 : 1;       // a raw block is 128 rows x 128 bytes
 
@@ -122,7 +130,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       mbar_init(&ctl->op_full[s], 8);
       mbar_init(&ctl->op_empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < kAccs; ++s) {
       mbar_init(&ctl->acc_full[s], 1);
       mbar_init(&ctl->acc_empty[s], 16);
     }
@@ -138,9 +146,11 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
 
-  // registers per lane: five warpgroups x 96 at launch = 2 x 80 + 2 x 136 + 48
+  // registers per lane: five warpgroups x 96 at launch = 2 x 80 + 2 x 136 + 48 = 2 x 80 + 2 x 128 + 64 = 2 x 88 + 2 x 112 + 80
+  constexpr bool kTall = NT == kQpTokens;
+  constexpr int kRegsEpi = CHAIN ? 136 : kTall ? 128 : 112, kRegsConv = CHAIN ? 80 : kTall ? 80 : 88, kRegsRest = CHAIN ? 48 : kTall ? 64 : 80;
   if (warp >= kQpWProd) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 48;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsRest));
     if (warp == kQpWProd) {
       // ===================== raw weight blocks of this CTA's 128 rows =====================
       PipeState ws(kQpWStages);
@@ -204,52 +214,82 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         mbar_wait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
         xs.advance();
       }
-    } else if (warp == kQpMma && rank == 0) {
-      // ===================== MMA issuer (leader) =====================
+    } else if (rank == 0 && (warp == kQpMma || !CHAIN)) {
+      // ===================== MMA issuers (leader) =====================
+      // Waits, 8 MMAs and commits of a step take a warp some 800 cycles, so two take turns where every step is a segment of its
+      // own.  An operand stage and a slot of X are then always the same one's (both rings have an even number of steps), and of
+      // an accumulator, whose turns alternate, the trip before the last one is over: the one after it was waited for at this
+      // issuer's last step.
+      static_assert(kOpSteps % 2 == 0 && kQpXStages % 2 == 0, "rings and issuers");
       const uint64_t x_desc0 = umma_desc_sw128_kmajor(smem_u32(x_ring));
-      PipeState xs(kQpXStages), os(kOpStages);
-      int seg = 0;
+      PipeState xs(kQpXStages), os(kOpSteps), as(kAccs);
+      int turn = warp - kQpMma;                            // 0: the next step is this issuer's
       for (int t = pair; t < tiles; t += pairs) {
         const QpTile pt = qp_tile<MODE>(p, t);
         const uint32_t idesc = umma_idesc(1u, 0u, 0u, 0u, 0u, 2 * kBlockW, (uint32_t)qp_tile_n<NT>(pt.rows));
         int in_seg = 0;
         for (int s = 0; s < steps; ++s) {
-          const int buf = seg & 1;
-          if (in_seg == 0) mbar_wait(&ctl->acc_empty[buf], ((seg >> 1) & 1) ^ 1);
-          mbar_wait(&ctl->x_full[xs.stage], xs.phase);
-          mbar_wait(&ctl->op_full[os.stage], os.phase);
-          tc_fence_after();
-          const bool last = in_seg + 1 == p.seg_steps || s + 1 == steps;
-          if (elect_one()) {
-            const uint32_t a = tmem_base + kOpCol0 + os.stage * 64;
+          const bool last = !CHAIN || in_seg + 1 == p.seg_steps || s + 1 == steps;
+          if (CHAIN || turn == 0) {
+            const uint32_t acc = tmem_base + as.stage * NT, a = tmem_base + kOpCol0 + os.stage * 64;
             const uint64_t b = x_desc0 + (uint64_t)((xs.stage * kQpXBytes) >> 4);
+            if (CHAIN && in_seg == 0) mbar_wait(&ctl->acc_empty[as.stage], as.phase ^ 1);
+            mbar_wait(&ctl->x_full[xs.stage], xs.phase);
+            mbar_wait(&ctl->op_full[kSub * os.stage], os.phase);
+            if (!CHAIN) mbar_wait(&ctl->acc_empty[as.stage], as.phase ^ 1);
+            tc_fence_after();
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              umma_pair_ts(tmem_base + buf * kAccCols, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)),
-                           idesc, (in_seg | k) != 0 ? 1u : 0u);
-            tc_commit_pair(&ctl->op_empty[os.stage]);
-            tc_commit_pair(&ctl->x_empty[xs.stage]);
-            if (last) tc_commit_pair(&ctl->acc_full[buf]);
+            for (int h = 0; h < kSub; ++h) {
+              if (h == 1) {
+                mbar_wait(&ctl->op_full[kSub * os.stage + 1], os.phase);
+                tc_fence_after();
+              }
+              if (elect_one()) {
+#pragma unroll
+                for (int k = h * 4; k < (CHAIN ? 8 : h * 4 + 4); ++k)
+                  umma_pair_ts(acc, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)), idesc,
+                               (in_seg | k) != 0 ? 1u : 0u);
+                tc_commit_pair(&ctl->op_empty[kSub * os.stage + h]);
+                if (h == kSub - 1) {
+                  if (last) tc_commit_pair(&ctl->acc_full[as.stage]);
+                  tc_commit_pair(&ctl->x_empty[xs.stage]);   // the last one: the X producers wait for it before they leave
+                }
+              }
+              __syncwarp();
+            }
           }
-          __syncwarp();
-          if (last) { ++seg; in_seg = 0; } else { ++in_seg; }
+          if (!CHAIN) turn ^= 1;
+          if (last) { as.advance(); in_seg = 0; } else { ++in_seg; }
           xs.advance();
           os.advance();
         }
       }
     }
   } else if (warp >= kQpEpi0) {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsEpi));
     // ===================== epilogue: one thread per weight row and token half =====================
     const int quad = warp & 3, half = (warp - kQpEpi0) >> 2;
     const int row = quad * 32 + lane;
     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + half * kHalf;
-    const uint32_t empty0 = leader_addr(&ctl->acc_empty[0]), empty1 = leader_addr(&ctl->acc_empty[1]);
+    const uint32_t empty0 = leader_addr(&ctl->acc_empty[0]);
     const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
+    uint8_t* meta = x_ring + kQpXStages * kQpXBytes + (warp - kQpEpi0) * 64 * 8;
     pdl_wait_prior();               // y may still be read upstream
-    int seg = 0;
+    PipeState as(kAccs);
     for (int t = pair; t < tiles; t += pairs) {
       const QpTile pt = qp_tile<MODE>(p, t);
+      if (MODE == QP_DOWN) {
+        // slots and routing weights of this warp's rows: asked for now, two trips to L2 at the tile's end otherwise
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kHalf / 32; ++q) {
+          const int r = half * kHalf + 32 * q + lane;
+          const int slot = r < pt.rows ? ld_upstream(p.order + pt.m0 + r) : 0;
+          reinterpret_cast<float*>(meta)[32 * q + lane] = r < pt.rows ? __half2float(p.row_weights[slot]) : 0.f;
+          reinterpret_cast<int*>(meta + 256)[32 * q + lane] = slot;
+        }
+        __syncwarp();
+      }
       const int n_tile = pt.n * 2 + (int)rank;
       // weight row of this thread, and for the gate / up rows the output that the pair (lane, lane + 16) forms
       const int out = pt.n * kBlockW + (int)rank * (kBlockW / 2) + quad * 16 + (lane & 15);
@@ -263,71 +303,68 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 #pragma unroll
       for (int j = 0; j < kHalf / 2; ++j) acc[j] = 0ull;
       float sc = __ldg(sp);
-      for (int g = 0; g < nseg; ++g, ++seg) {
-        const int buf = seg & 1;
+      for (int g = 0; g < nseg; ++g) {
         const uint64_t s2 = pack_f32x2(sc, sc);
         if (g + 1 < nseg) sc = __ldg(sp + (int64_t)(g + 1) * p.s_stride_k);
-        mbar_wait(&ctl->acc_full[buf], (seg >> 1) & 1);
+        mbar_wait(&ctl->acc_full[as.stage], as.phase);
         tc_fence_after();
-        uint32_t v[kHalf];
-        tmem_ld_32x32b_x32(taddr + buf * kAccCols, *reinterpret_cast<uint32_t(*)[32]>(v));
-        if (kHalf == 64) tmem_ld_32x32b_x32(taddr + buf * kAccCols + 32, *reinterpret_cast<uint32_t(*)[32]>(v + (kHalf - 32)));
-        tc_wait_ld();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(buf ? empty1 : empty0);     // in registers: the segment's buffer may be refilled
 #pragma unroll
-        for (int j = 0; j < kHalf / 2; ++j) {
-          const uint64_t pv = pack_f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1]));
-          acc[j] = fma_f32x2(s2, pv, acc[j]);
+        for (int c = 0; c < kHalf; c += (CHAIN ? kHalf : 32)) {
+          uint32_t v[CHAIN ? kHalf : 32];
+          tmem_ld_32x32b_x32(taddr + as.stage * NT + c, *reinterpret_cast<uint32_t(*)[32]>(v));
+          if (CHAIN && kHalf == 64) tmem_ld_32x32b_x32(taddr + as.stage * NT + c + 32, *reinterpret_cast<uint32_t(*)[32]>(v + (CHAIN ? kHalf - 32 : 0)));
+          tc_wait_ld();
+          if (CHAIN || c + 32 == kHalf) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(empty0 + as.stage * 8);     // in registers: the segment's buffer may be refilled
+          }
+#pragma unroll
+          for (int j = 0; j < (CHAIN ? kHalf / 2 : 16); ++j)
+            acc[c / 2 + j] = fma_f32x2(s2, pack_f32x2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), acc[c / 2 + j]);
         }
+        as.advance();
       }
-      // ---- the tile's results: a warp writes 32 consecutive outputs of one token at a time ----
+      // ---- the tile's results ----
       float bv = 0.f;
       if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
       const int m0 = pt.m0 + half * kHalf;
       const int rows = pt.rows - half * kHalf;
+      if (rows <= 0) continue;                               // uniform over the warp
       __half* y = reinterpret_cast<__half*>(p.y);
+      constexpr bool kFewRows = NT < kQpTokens;              // an early end costs the large tiles 5 % (registers)
       if (MODE == QP_GATE_UP) {
-        // like the fused activation below, with the pair 16 lanes apart
+        // like store_swiglu, with the pair 16 lanes apart and no further exchange (92.8 against 94.1 us for 64 experts of 190 rows)
         const bool high = lane >> 4;
         __half* yp = y + (int64_t)(m0 + (high ? 1 : 0)) * p.ldy + out;
 #pragma unroll
         for (int j = 0; j < kHalf / 2; ++j) {
+          if (kFewRows && 2 * j >= rows) break;
           float a, b;
           unpack_f32x2(acc[j], a, b);
-          a = __half2float(__float2half_rn(a));
-          b = __half2float(__float2half_rn(b));
-          const float other = __shfl_xor_sync(0xffffffffu, high ? a : b, 16);
-          const float gate = high ? other : a, up = high ? b : other;
-          if (n_ok && 2 * j + (high ? 1 : 0) < rows) *yp = __float2half_rn(silu_q(gate) * up);
+          const float o = swiglu_h2(exchange_pair<16>(pack2<__half>(a, b), lane));
+          if (n_ok && 2 * j + (high ? 1 : 0) < rows) *yp = __float2half_rn(o);
           yp += 2 * p.ldy;
         }
-        continue;
-      }
-      if (MODE == QP_DOWN) {
-        // rows go back to their slots, times the routing weight in fp32 before the rounding (fused_moe.py:201-205);
-        // lane l keeps the slots and weights of rows l and l + 32 of this half
-        int slot[2];
-        float wt[2];
+      } else if (MODE == QP_DOWN) {
+        // rows go back to their slots, times the routing weight in fp32 before the rounding (fused_moe.py:201-205); in stores of
+        // four outputs: 64 experts of 190 rows 84 us, of one 95
+        const int col = n_tile * kBlockW + quad * 32 + (lane & ~3);
 #pragma unroll
-        for (int q = 0; q < 2; ++q) {
-          const bool in = 32 * q + lane < rows;
-          slot[q] = in ? ld_upstream(p.order + m0 + 32 * q + lane) : 0;
-          wt[q] = in ? __half2float(p.row_weights[slot[q]]) : 0.f;
+        for (int j = 0; j < kHalf / 2; j += 2) {
+          if (kFewRows && 2 * j >= rows) break;
+          const float4 w = *reinterpret_cast<const float4*>(meta + 8 * j);
+          float f[4];
+          unpack_f32x2(acc[j], f[0], f[1]);
+          unpack_f32x2(acc[j + 1], f[2], f[3]);
+          const uint2 v = exchange4(pack2<__half>(f[0] * w.x, f[1] * w.y), pack2<__half>(f[2] * w.z, f[3] * w.w), lane);
+          const int r = 2 * j + (lane & 3);
+          if (r < rows) store4(y + (int64_t)reinterpret_cast<const int*>(meta + 256)[r] * p.ldy + col, v, p.N - col, p.vec);
         }
-#pragma unroll
-        for (int j = 0; j < kHalf; ++j) {
-          float v[2];
-          unpack_f32x2(acc[j / 2], v[0], v[1]);
-          const int to = __shfl_sync(0xffffffffu, slot[j / 32], j % 32);
-          const float w = __shfl_sync(0xffffffffu, wt[j / 32], j % 32);
-          if (n_ok && j < rows) y[(int64_t)to * p.ldy + n] = __float2half_rn(v[j & 1] * w);
-        }
-        continue;
-      }
-      if (EPI == 0) {
+      } else if (EPI == 0) {
+        // (stores of two bytes: with few tiles per pair the exchanges of store_rows cost more than they save, 256 x 4096 x
+        // 4096 int8 14.6 against 15.4 us)
         __half* yp = y + (int64_t)m0 * p.ldy + n;
         if (n_ok) {
 #pragma unroll
@@ -340,33 +377,19 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           }
         }
       } else {
-        // SiLU(gate) * up over (gate_i, up_i) row pairs, both rounded to fp16 first (gemm_quant.cu).  Of two tokens the
-        // even lane forms the first result and the odd lane the second: one exchange for both.
-        const bool odd = lane & 1;
-        __half* yp = y + (int64_t)(m0 + (odd ? 1 : 0)) * p.ldy + (n >> 1);
-#pragma unroll
-        for (int j = 0; j < kHalf / 2; ++j) {
-          float a, b;
-          unpack_f32x2(acc[j], a, b);
-          a = __half2float(__float2half_rn(a + bv));
-          b = __half2float(__float2half_rn(b + bv));
-          const float other = __shfl_xor_sync(0xffffffffu, odd ? a : b, 1);
-          const float gate = odd ? other : a, up = odd ? b : other;
-          if (n_ok && 2 * j + (odd ? 1 : 0) < rows) *yp = __float2half_rn(silu_q(gate) * up);
-          yp += 2 * p.ldy;
-        }
+        store_swiglu<kHalf / 2>(acc, y, p.ldy, m0, rows, (n_tile * kBlockW + quad * 32) >> 1, p.N >> 1, bv, lane, p.vec);
       }
     }
   } else {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsConv));
     // ===================== conversion: one thread per weight row, the two groups take alternate operand stages ==========
-    // Stage i of the CTA's running count belongs to group i & 1, so every op_empty barrier is waited on by one group
+    // Step i of the CTA's running count belongs to group i & 1, so every op_empty barrier is waited on by one group
     // that has seen all of its phases.
     const int group = warp >> 2, quad = warp & 3;
     const int row = quad * 32 + lane, rx = row & 7;
     const uint32_t dst0 = tmem_base + ((uint32_t)(quad * 32) << 16) + kOpCol0;
-    constexpr int kOwn = kOpStages / 2;                     // stages of this group: group, group + 2, ...
-    const uint32_t full0 = leader_addr(&ctl->op_full[group]);
+    constexpr int kOwn = kOpSteps / 2;                      // operand steps of this group: group, group + 2, ...
+    const uint32_t full0 = leader_addr(&ctl->op_full[0]);
     int own = 0;
     uint32_t own_phase = 0;
     int i0 = 0;                                             // running stage count at the tile's first step
@@ -392,38 +415,54 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         const int rs = raw % kQpWStages;
         mbar_wait(&ctl->w_full[rs], (raw / kQpWStages) & 1);
         const uint8_t* src = w_ring + (size_t)rs * kABytes + row * 128;
-        const int stage = group + 2 * own;
-        mbar_wait(&ctl->op_empty[stage], own_phase ^ 1);
-        tc_fence_after();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           constexpr int kChunks = QK == Q_INT4 ? 2 : 4;     // 16-byte chunks of the row per 64 k
+          const int stage = kSub * (group + 2 * own) + (CHAIN ? 0 : h);
           const int c0 = (QK == Q_INT4 ? (k & 1) * 4 : 0) + h * kChunks;
+          if (CHAIN && h == 0) {
+            mbar_wait(&ctl->op_empty[stage], own_phase ^ 1);
+            tc_fence_after();
+          }
           uint4 w[kChunks];
 #pragma unroll
           for (int c = 0; c < kChunks; ++c) w[c] = lds_128(src + (((c0 + c) ^ rx) << 4));
-          uint32_t vals[32];
+          constexpr int kParts = CHAIN ? 1 : 2;             // 64 or 32 k at a time: 32 or 16 columns
 #pragma unroll
-          for (int c = 0; c < kChunks; ++c) {
-            const uint32_t ws[4] = {w[c].x, w[c].y, w[c].z, w[c].w};
+          for (int q = 0; q < kParts; ++q) {
+            uint32_t vals[32 / kParts];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (QK == Q_INT4) dequant_int4_packed(ws[j], add_lo, add_hi, vals + (QK == Q_INT4 ? 16 * c + 4 * j : 0));
-              else dequant_w8_word(ws[j], QK == Q_FP8, vals + (QK == Q_INT4 ? 0 : 8 * c + 2 * j));
+            for (int c = 0; c < kChunks / kParts; ++c) {
+              const uint4 v = w[q * (kChunks / kParts) + c];
+              const uint32_t ws[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                if (QK == Q_INT4) dequant_int4_packed(ws[j], add_lo, add_hi, vals + (QK == Q_INT4 ? 16 * c + 4 * j : 0));
+                else dequant_w8_word(ws[j], QK == Q_FP8, vals + (QK == Q_INT4 ? 0 : 8 * c + 2 * j));
+              }
+            }
+            if (!CHAIN && q == 0) {
+              mbar_wait(&ctl->op_empty[stage], own_phase ^ 1);
+              tc_fence_after();
+            }
+            const uint32_t dst = dst0 + (group + 2 * own) * 64 + h * 32 + q * 16;
+            if constexpr (CHAIN) tmem_st_32x32b_x32(dst, vals);
+            else tmem_st_32x32b_x16(dst, vals);
+          }
+          if (CHAIN && h == 0) continue;
+          if (h == 1) {
+            // the raw words have all been converted: the block may be refilled (an odd last step speaks for both halves)
+            __syncwarp();
+            if (lane == 0) {
+              mbar_arrive(&ctl->w_empty[rs]);
+              if (QK == Q_INT4 && k + 1 == steps && (k & 1) == 0) mbar_arrive(&ctl->w_empty[rs]);
             }
           }
-          tmem_st_32x32b_x32(dst0 + stage * 64 + h * 32, vals);
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(full0 + stage * 8);   // barriers are 8 bytes apart
         }
-        // the raw words have all been converted: the block may be refilled (an odd last step speaks for both halves)
-        __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(&ctl->w_empty[rs]);
-          if (QK == Q_INT4 && k + 1 == steps && (k & 1) == 0) mbar_arrive(&ctl->w_empty[rs]);
-        }
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(full0 + own * 16);   // barriers are 8 bytes apart
         if (++own == kOwn) { own = 0; own_phase ^= 1; }
       }
       i0 += steps;
@@ -436,14 +475,20 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   if (warp == kQpMma) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int QK, int EPI, int MODE = QP_PLAIN, int NT = kQpTokens>
-static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
-  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE, NT>;
+template <int QK, int EPI, int MODE, int NT, bool CHAIN>
+static int launch_qp_form(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
+  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE, NT, CHAIN>;
   static int configured[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, kQpSmem, configured));
   b2l_launch(kern, dim3((unsigned)grid), dim3(kQpThreads), (size_t)kQpSmem, st, tw, tx, p);
   B2L_LAUNCH_CHECK();
   return B2L_OK;
+}
+
+template <int QK, int EPI, int MODE = QP_PLAIN, int NT = kQpTokens>
+static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
+  return p.seg_steps == 1 ? launch_qp_form<QK, EPI, MODE, NT, false>(tw, tx, p, grid, st)
+                          : launch_qp_form<QK, EPI, MODE, NT, true>(tw, tx, p, grid, st);
 }
 
 // Where the pair kernel is the faster one (both kernels measured over 72 - 512 tokens, eight projection shapes, int4 with and
@@ -491,6 +536,7 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
     p.seg_steps = qp_chain_steps(M, N, K);
     p.s_stride_k = 0;
   }
+  p.vec = p.ldy % 4 == 0 && (uintptr_t)p.y % 8 == 0;
   p.m_tiles = (int)cdiv64(M, kQpTokens);
   p.n_tiles = (int)cdiv64(N, 2 * kBlockW);
   const int64_t tiles = (int64_t)p.m_tiles * p.n_tiles;
@@ -524,6 +570,7 @@ static int grouped(int qk, const MoePairGemm& g, cudaStream_t st) {
   p.steps = (int)cdiv64(g.K, kQpStepK);
   p.groups = 0;
   p.seg_steps = g.group_k >= g.K ? p.steps : (int)(g.group_k / kQpStepK);
+  p.vec = p.ldy % 4 == 0 && (uintptr_t)p.y % 8 == 0;
   p.m_tiles = 0;
   p.n_tiles = (int)cdiv64(g.N, 2 * kBlockW);
   const int64_t most = (int64_t)g.max_tiles * p.n_tiles;

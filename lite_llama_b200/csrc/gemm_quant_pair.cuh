@@ -16,7 +16,8 @@ struct QuantPairParams {
   const int32_t* order;                              // grouped down projection: slot of every sorted row
   const __half* row_weights;                         // grouped down projection: routing weight by slot
   int M, N, steps, seg_steps, groups, m_tiles, n_tiles;      // filled by quant_pair_gemm (groups: pitch of the int4 tables)
-  int tiles, split_from, vec;                        // wide tiles: their number, the first that is cut in two, y in 8-byte stores
+  int vec;                                           // y in stores of four outputs
+  int tiles, split_from;                             // wide tiles: their number, and the first that is cut in two
 };
 
 // shapes the pair kernel takes and is the faster one for (see gemm_quant_pair.cu); qk: QuantKind

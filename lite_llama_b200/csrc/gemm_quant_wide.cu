@@ -24,6 +24,7 @@
 #include "gemm_quant_pair.cuh"
 #include "pair.cuh"
 #include "dequant.cuh"
+#include "gemm_quant_out.cuh"
 
 namespace gemm {
 
@@ -75,19 +76,6 @@ __device__ __forceinline__ QwTile qw_tile(const QuantPairParams& p, int t) {
 __device__ __forceinline__ int qw_half_n(int rows_left) {
   const int n = (rows_left + 31) & ~31;
   return n < kQwHalf ? n : kQwHalf;
-}
-
-// four neighbouring outputs of a token, `left` of them in range
-__device__ __forceinline__ void qw_store4(__half* dst, uint32_t lo, uint32_t hi, int left, int vec) {
-  if (vec && left >= 4) {
-    *reinterpret_cast<uint2*>(dst) = make_uint2(lo, hi);
-  } else {
-    const uint32_t v[2] = {lo, hi};
-    const __half* f = reinterpret_cast<const __half*>(v);
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (i < left) dst[i] = f[i];
-  }
 }
 
 template <int QK, int EPI>
@@ -304,57 +292,13 @@ gemm_quant_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
       __half* y = reinterpret_cast<__half*>(p.y);
-      const uint32_t sel1 = lane & 1 ? 0x3276u : 0x5410u, sel2 = lane & 2 ? 0x3276u : 0x5410u;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int m0 = pt.m0 + h * kQwHalf + part * 64;
         const int rows = h < pt.halves ? pt.rows - h * kQwHalf - part * 64 : 0;
         if (rows <= 0) continue;
-        if (EPI == 0) {
-          // four tokens: lane l leaves with token l & 3 and the outputs of lanes l & ~3 .. l | 3
-          const int col = n_tile * kBlockW + quad * 32 + (lane & ~3);
-          __half* yp = y + (int64_t)(m0 + (lane & 3)) * p.ldy + col;
-#pragma unroll
-          for (int j = 0; j < 32; j += 2) {
-            float f[4];
-            unpack_f32x2(acc[h][j], f[0], f[1]);
-            unpack_f32x2(acc[h][j + 1], f[2], f[3]);
-            const uint32_t p0 = pack2<__half>(f[0] + bv, f[1] + bv), p1 = pack2<__half>(f[2] + bv, f[3] + bv);
-            const uint32_t a0 = __byte_perm(p0, __shfl_xor_sync(0xffffffffu, p0, 1), sel1);
-            const uint32_t a1 = __byte_perm(p1, __shfl_xor_sync(0xffffffffu, p1, 1), sel1);
-            const uint32_t r = __shfl_xor_sync(0xffffffffu, lane & 2 ? a0 : a1, 2);
-            if (2 * j + (lane & 3) < rows) qw_store4(yp, lane & 2 ? r : a0, lane & 2 ? a1 : r, p.N - col, p.vec);
-            yp += 4 * p.ldy;
-          }
-        } else {
-          // SiLU(gate) * up over (gate_i, up_i) row pairs, both rounded to fp16 first (gemm_quant.cu).  Eight tokens: lane l
-          // leaves with token l & 7 and the four outputs of lanes l & ~7 .. l | 7
-          const int col = (n_tile * kBlockW + quad * 32 + (lane & ~7)) >> 1;
-          __half* yp = y + (int64_t)(m0 + (lane & 7)) * p.ldy + col;
-#pragma unroll
-          for (int j = 0; j < 32; j += 4) {
-            uint32_t d[2];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-              float o[2];
-#pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                // of two tokens the even lane forms the first result and the odd lane the second
-                float f[2];
-                unpack_f32x2(acc[h][j + 2 * u + q], f[0], f[1]);
-                const uint32_t own = pack2<__half>(f[0] + bv, f[1] + bv);
-                const uint32_t gu = __byte_perm(own, __shfl_xor_sync(0xffffffffu, own, 1), sel1);
-                const float2 g2 = __half22float2(*reinterpret_cast<const __half2*>(&gu));
-                o[q] = silu_q(g2.x) * g2.y;
-              }
-              const uint32_t c = pack2<__half>(o[0], o[1]);
-              d[u] = __byte_perm(c, __shfl_xor_sync(0xffffffffu, c, 2), sel2);
-            }
-            const uint32_t r = __shfl_xor_sync(0xffffffffu, lane & 4 ? d[0] : d[1], 4);
-            if (2 * j + (lane & 7) < rows) qw_store4(yp, lane & 4 ? r : d[0], lane & 4 ? d[1] : r, p.N / 2 - col, p.vec);
-            yp += 8 * p.ldy;
-          }
-        }
+        if (EPI == 0) store_rows<32>(acc[h], y, p.ldy, m0, rows, n_tile * kBlockW + quad * 32, p.N, bv, lane, p.vec);
+        else store_swiglu<32>(acc[h], y, p.ldy, m0, rows, (n_tile * kBlockW + quad * 32) >> 1, p.N >> 1, bv, lane, p.vec);
       }
     }
   } else {
@@ -472,7 +416,6 @@ int quant_wide_gemm(int qk, QuantPairParams& p, const CUtensorMap& tw, const CUt
   const int tiles = p.m_tiles * p.n_tiles;
   p.split_from = qw_split(tiles, pairs) ? tiles - tiles % pairs : tiles;
   p.tiles = tiles + (tiles - p.split_from);
-  p.vec = p.ldy % 4 == 0 && (uintptr_t)p.y % 8 == 0;
   const int grid = 2 * (p.tiles < pairs ? p.tiles : pairs);
   if (qk == Q_INT4) return swiglu ? launch_qw<Q_INT4, 1>(tw, tx, p, grid, st) : launch_qw<Q_INT4, 0>(tw, tx, p, grid, st);
   return qk == Q_FP8 ? launch_qw<Q_FP8, 0>(tw, tx, p, grid, st) : launch_qw<Q_INT8, 0>(tw, tx, p, grid, st);
