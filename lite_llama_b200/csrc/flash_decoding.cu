@@ -19,7 +19,8 @@
 //  * QK^T and PV on tensor cores with fp32 accumulation (fp16 products are exact in fp32, which
 //    keeps the reference's "fp32 product" precision, flashdecoding.py:115-120), fp32 online softmax;
 //  * split-KV sized from host-known quantities only (graph-safe); fp32 partials + log-sum-exp,
-//    merged by a second small kernel (reference stage 2, flashdecoding.py:224-313);
+//    merged by a second small kernel (reference stage 2, flashdecoding.py:224-313); large steps: shares of the work that there
+//    is, whatever rows it belongs to (flash_decode_shares_kernel);
 //  * a step too small to fill the chip is bound by latency instead: its splits are the CTAs of a cluster, with as few kv
 //    heads each as still fit in one wave, and merge through one another's shared memory (cluster_merge below).
 #include "common.cuh"
@@ -49,6 +50,9 @@ struct DecodeParams {
   int stages;
   int chunk;      // tokens per split (multiple of kTT)
   int splits;
+  int batch;
+  int2* ws_info;  // shares: first and last CTA of every (kv-head block, batch row); ws_o [head of a block, slots, D]
+  int slots;      // two per CTA
   float scale_log2;
 };
 
@@ -116,6 +120,135 @@ __device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t pa
   __syncwarp();
   cluster_sync_all();                 // the peers have read this CTA's rows
 }
+
+// One consumer warp's work: 16 query heads (fewer: rows of zeros) of one kv head, its tiles of kTT tokens in turn.
+template <typename T, int D>
+struct Consumer {
+  uint32_t qf[D / 16][4];             // A operand, m16 x k16 per step; rows = query heads of this KV group
+  float o[D / 8][4];
+  float m_run[2], l_run[2];
+  bool v0, v1;                        // rows g and g + 8 exist
+
+  __device__ __forceinline__ void begin(const DecodeParams& p, int b, int kvh, int hq0, int hq1, int tq) {
+    v0 = hq0 < p.G;
+    v1 = hq1 < p.G;
+    const T* qb = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_bs;
+    const T* q0 = qb + (int64_t)(kvh * p.G + (v0 ? hq0 : 0)) * p.q_hs;
+    const T* q1 = qb + (int64_t)(kvh * p.G + (v1 ? hq1 : 0)) * p.q_hs;
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      const int c = kk * 16 + 2 * tq;
+      qf[kk][0] = v0 ? *reinterpret_cast<const uint32_t*>(q0 + c) : 0u;
+      qf[kk][1] = v1 ? *reinterpret_cast<const uint32_t*>(q1 + c) : 0u;
+      qf[kk][2] = v0 ? *reinterpret_cast<const uint32_t*>(q0 + c + 8) : 0u;
+      qf[kk][3] = v1 ? *reinterpret_cast<const uint32_t*>(q1 + c + 8) : 0u;
+    }
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+    m_run[0] = m_run[1] = -INFINITY;
+    l_run[0] = l_run[1] = 0.f;
+  }
+  // the tile at shared address sb, tokens tbase .. of which those before `end` count; ka, va: ldmatrix lane addresses.
+  // REST: what the probabilities lose as 16-bit operands is multiplied as well.  Of every split the largest probability is 1, which
+  // loses nothing, so rows in few parts would end 2 - 5 % further from the exact result than rows in many; with it they end closer.
+  template <bool REST>
+  __device__ __forceinline__ void tile(const DecodeParams& p, uint32_t sb, uint32_t ka, uint32_t va, int64_t tbase, int64_t end, int tq) {
+    // ---- S = Q K^T  (16 heads x 16 tokens) ----
+    float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t bf[4];
+      ldmatrix_x4(bf, sb + ka + kk * 32);
+      mma_m16n8k16<T>(sc[0], qf[kk], bf[0], bf[1]);
+      mma_m16n8k16<T>(sc[1], qf[kk], bf[2], bf[3]);
+    }
+    // ---- scale, mask, online softmax (log2 domain) ----
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int64_t pos = tbase + j * 8 + 2 * tq + (e & 1);
+        float v = sc[j][e] * p.scale_log2;
+        v = pos < end ? v : -INFINITY;
+        sc[j][e] = v;
+        mx[e >> 1] = fmaxf(mx[e >> 1], v);
+      }
+    }
+    float alpha[2], base[2];
+#pragma unroll
+    for (int r2 = 0; r2 < 2; ++r2) {
+      mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 1));
+      mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 2));
+      const float mnew = fmaxf(m_run[r2], mx[r2]);
+      base[r2] = mnew == -INFINITY ? 0.f : mnew;   // avoid (-inf) - (-inf)
+      alpha[r2] = fast_exp2(m_run[r2] - base[r2]);
+      m_run[r2] = mnew;
+    }
+    float ps[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float pv = fast_exp2(sc[j][e] - base[e >> 1]);
+        sc[j][e] = pv;
+        ps[e >> 1] += pv;
+      }
+    }
+    l_run[0] = l_run[0] * alpha[0] + ps[0];
+    l_run[1] = l_run[1] * alpha[1] + ps[1];
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i) {
+      o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
+      o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+    }
+    // ---- O += P V  (P: 16 heads x 16 tokens as the A operand) ----
+    uint32_t pf[4];
+    pf[0] = pack2<T>(sc[0][0], sc[0][1]);
+    pf[1] = pack2<T>(sc[0][2], sc[0][3]);
+    pf[2] = pack2<T>(sc[1][0], sc[1][1]);
+    pf[3] = pack2<T>(sc[1][2], sc[1][3]);
+    uint32_t rest[4];
+    if (REST) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const typename Vec2<T>::type h = *reinterpret_cast<const typename Vec2<T>::type*>(&pf[i]);
+        rest[i] = pack2<T>(sc[i >> 1][2 * (i & 1)] - to_f32(h.x), sc[i >> 1][2 * (i & 1) + 1] - to_f32(h.y));
+      }
+    }
+#pragma unroll
+    for (int dn = 0; dn < D / 16; ++dn) {
+      uint32_t bf[4];
+      ldmatrix_x4_trans(bf, sb + va + dn * 32);
+      mma_m16n8k16<T>(o[2 * dn], pf, bf[0], bf[1]);
+      mma_m16n8k16<T>(o[2 * dn + 1], pf, bf[2], bf[3]);
+      if (REST) {
+        mma_m16n8k16<T>(o[2 * dn], rest, bf[0], bf[1]);
+        mma_m16n8k16<T>(o[2 * dn + 1], rest, bf[2], bf[3]);
+      }
+    }
+  }
+  // quad-reduce the row sums (each lane only summed its own 4 columns per tile)
+  __device__ __forceinline__ void sum_rows() {
+#pragma unroll
+    for (int r2 = 0; r2 < 2; ++r2) {
+      l_run[r2] += __shfl_xor_sync(0xffffffffu, l_run[r2], 1);
+      l_run[r2] += __shfl_xor_sync(0xffffffffu, l_run[r2], 2);
+    }
+  }
+  // rows r2 (0: head hq0, 1: hq1) as 16-bit results or as fp32 partial rows
+  __device__ __forceinline__ void store_out(const DecodeParams& p, int r2, int b, int head, float inv, int tq) const {
+    T* orow = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)head * p.o_hs;
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i)
+      *reinterpret_cast<uint32_t*>(orow + i * 8 + 2 * tq) = pack2<T>(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
+  }
+  __device__ __forceinline__ void store_part(float* orow, int r2, float inv, int tq) const {
+#pragma unroll
+    for (int i = 0; i < D / 8; ++i)
+      *reinterpret_cast<float2*>(orow + i * 8 + 2 * tq) = make_float2(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
+  }
+};
 
 // Who merges the splits of a row: a second kernel; nobody (a single split), or the last CTA (tickets); the CTAs of a cluster,
 // which are the grid's x, up to kMaxCluster splits.  The second form does the first one's work as well; its code for the rest costs
@@ -195,28 +328,9 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
     const int qblk = warp % p.qblocks;
     const int kvh = hblk * p.HB + hl;
     const int g = lane >> 2, tq = lane & 3;
-    // Q fragments (A operand, m16 x k16 per step); rows = query heads of this KV group.
-    uint32_t qf[D / 16][4];
     const int hq0 = qblk * 16 + g, hq1 = hq0 + 8;
-    const bool v0 = hq0 < p.G, v1 = hq1 < p.G;
-    {
-      const T* qb = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_bs;
-      const T* q0 = qb + (int64_t)(kvh * p.G + (v0 ? hq0 : 0)) * p.q_hs;
-      const T* q1 = qb + (int64_t)(kvh * p.G + (v1 ? hq1 : 0)) * p.q_hs;
-#pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        const int c = kk * 16 + 2 * tq;
-        qf[kk][0] = v0 ? *reinterpret_cast<const uint32_t*>(q0 + c) : 0u;
-        qf[kk][1] = v1 ? *reinterpret_cast<const uint32_t*>(q1 + c) : 0u;
-        qf[kk][2] = v0 ? *reinterpret_cast<const uint32_t*>(q0 + c + 8) : 0u;
-        qf[kk][3] = v1 ? *reinterpret_cast<const uint32_t*>(q1 + c + 8) : 0u;
-      }
-    }
-    float o[D / 8][4];
-#pragma unroll
-    for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    float m_run[2] = {-INFINITY, -INFINITY};
-    float l_run[2] = {0.f, 0.f};
+    Consumer<T, D> c;
+    c.begin(p, b, kvh, hq0, hq1, tq);
 
     const uint32_t k_off = hl * HEAD_BYTES;
     const uint32_t v_off = (p.HB + hl) * HEAD_BYTES;
@@ -230,108 +344,32 @@ __device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* sme
       mbar_wait(&full_bar[s], phase);
       const uint32_t sb = smem_u32(stage_base + s * stage_bytes);
 
-      // ---- S = Q K^T  (16 heads x 16 tokens) ----
-      float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t bf[4];
-        ldmatrix_x4(bf, sb + ka + kk * 32);
-        mma_m16n8k16<T>(sc[0], qf[kk], bf[0], bf[1]);
-        mma_m16n8k16<T>(sc[1], qf[kk], bf[2], bf[3]);
-      }
-      // ---- scale, mask, online softmax (log2 domain) ----
-      const int64_t tbase = start + (int64_t)t * kTT;
-      float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int64_t pos = tbase + j * 8 + 2 * tq + (e & 1);
-          float v = sc[j][e] * p.scale_log2;
-          v = pos < end ? v : -INFINITY;
-          sc[j][e] = v;
-          mx[e >> 1] = fmaxf(mx[e >> 1], v);
-        }
-      }
-      float alpha[2], base[2];
-#pragma unroll
-      for (int r2 = 0; r2 < 2; ++r2) {
-        mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 1));
-        mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 2));
-        const float mnew = fmaxf(m_run[r2], mx[r2]);
-        base[r2] = mnew == -INFINITY ? 0.f : mnew;   // avoid (-inf) - (-inf)
-        alpha[r2] = fast_exp2(m_run[r2] - base[r2]);
-        m_run[r2] = mnew;
-      }
-      float ps[2] = {0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float pv = fast_exp2(sc[j][e] - base[e >> 1]);
-          sc[j][e] = pv;
-          ps[e >> 1] += pv;
-        }
-      }
-      l_run[0] = l_run[0] * alpha[0] + ps[0];
-      l_run[1] = l_run[1] * alpha[1] + ps[1];
-#pragma unroll
-      for (int i = 0; i < D / 8; ++i) {
-        o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-        o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
-      }
-      // ---- O += P V  (P: 16 heads x 16 tokens as the A operand) ----
-      uint32_t pf[4];
-      pf[0] = pack2<T>(sc[0][0], sc[0][1]);
-      pf[1] = pack2<T>(sc[0][2], sc[0][3]);
-      pf[2] = pack2<T>(sc[1][0], sc[1][1]);
-      pf[3] = pack2<T>(sc[1][2], sc[1][3]);
-#pragma unroll
-      for (int dn = 0; dn < D / 16; ++dn) {
-        uint32_t bf[4];
-        ldmatrix_x4_trans(bf, sb + va + dn * 32);
-        mma_m16n8k16<T>(o[2 * dn], pf, bf[0], bf[1]);
-        mma_m16n8k16<T>(o[2 * dn + 1], pf, bf[2], bf[3]);
-      }
+      c.template tile<false>(p, sb, ka, va, start + (int64_t)t * kTT, end, tq);
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty_bar[s]);
       if (++s == p.stages) { s = 0; phase ^= 1; }
     }
 
-    // quad-reduce the row sums (each lane only summed its own 4 columns per tile)
-#pragma unroll
-    for (int r2 = 0; r2 < 2; ++r2) {
-      l_run[r2] += __shfl_xor_sync(0xffffffffu, l_run[r2], 1);
-      l_run[r2] += __shfl_xor_sync(0xffffffffu, l_run[r2], 2);
-    }
+    c.sum_rows();
     // Cluster: the partial rows go to the CTA's own shared memory, over the stages that every warp has finished with
     float* part = reinterpret_cast<float*>(stage_base);
     if (FORM == FD_CLUSTER) __syncthreads();
     // this warp saw every token of the split for its heads: write the result rows directly
 #pragma unroll
     for (int r2 = 0; r2 < 2; ++r2) {
-      const bool ok = r2 == 0 ? v0 : v1;
-      if (!ok) continue;
+      if (!(r2 == 0 ? c.v0 : c.v1)) continue;
       const int head = kvh * p.G + (r2 == 0 ? hq0 : hq1);
-      const float inv = 1.0f / l_run[r2];
+      const float inv = 1.0f / c.l_run[r2];
       if (FORM == FD_CLUSTER) {
         const int local = hl * p.G + (r2 == 0 ? hq0 : hq1);
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i)
-          *reinterpret_cast<float2*>(part + local * D + i * 8 + 2 * tq) = make_float2(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
-        if (tq == 0) part[p.HB * p.G * D + local] = m_run[r2] + log2f(l_run[r2]);
+        c.store_part(part + local * D, r2, inv, tq);
+        if (tq == 0) part[p.HB * p.G * D + local] = c.m_run[r2] + log2f(c.l_run[r2]);
       } else if (FORM == FD_WHOLE && p.splits == 1) {
-        T* orow = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)head * p.o_hs;
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i)
-          *reinterpret_cast<uint32_t*>(orow + i * 8 + 2 * tq) = pack2<T>(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
+        c.store_out(p, r2, b, head, inv, tq);
       } else {
         const int64_t off = ((int64_t)b * p.Hq + head) * p.splits + split;
-        float* orow = p.ws_o + off * D;
-#pragma unroll
-        for (int i = 0; i < D / 8; ++i)
-          *reinterpret_cast<float2*>(orow + i * 8 + 2 * tq) = make_float2(o[i][2 * r2] * inv, o[i][2 * r2 + 1] * inv);
-        if (tq == 0) p.ws_lse[off] = m_run[r2] + log2f(l_run[r2]);
+        c.store_part(p.ws_o + off * D, r2, inv, tq);
+        if (tq == 0) p.ws_lse[off] = c.m_run[r2] + log2f(c.l_run[r2]);
       }
     }
   }
@@ -446,7 +484,323 @@ __global__ void flash_decode_combine_kernel(const DecodeParams p) {
   }
 }
 
-struct Plan { int splits, chunk, qblocks, HB, stages, smem; bool cluster; };
+// Shares.  The lengths are device data, so a grid of (split, row) CTAs cut for the longest possible length spends six waves
+// of short CTAs on a batch that would fill the chip once, each with the start of its ring (25 splits of 80 tokens per row, 32
+// sequences of 1000 - 2000 tokens: 44 us of 30 at the rate of a copy), and larger splits lose where most rows are short.  Here every
+// CTA adds up the lengths and takes its part of the work there is:
+//   * little of it (as many items of up to kItemMax tiles, of one row each, as CTAs, or fewer): an item each;
+//   * else an equal share of all tiles of all rows, whatever rows they belong to: one wave, one ring that runs on from row
+//     to row.
+// A CTA that covers a row whole writes its result; else the row's parts go to the workspace (each CTA has at most two: of a row
+// that began before it, and of one that ends after it), and the owner of a row's first tile notes its first and last CTA for
+// the merge.
+constexpr int kShareRows = 1024, kItemMax = 8;
+// tiles per item of a row: at least four of a longer one, whose merge would ask for its parts in several turns
+__device__ __forceinline__ int item_tiles(int tiles, int q) { return q < 4 && tiles > 16 ? 4 : q; }
+// units of a row: items, or (q = 0) tiles
+__device__ __forceinline__ int share_units(int tiles, int q) {
+  if (q == 0) return tiles;
+  const int n = item_tiles(tiles, q);
+  return (unsigned)(tiles + n - 1) / (unsigned)n;
+}
+// the smallest items that there are CTAs for in any case (a row has at most one that is not full), or four tiles where they fit
+__device__ __forceinline__ int share_pick(int tiles, int fours, int rows, int grid) {
+  const int room = grid - rows;
+  int q = 0;
+  if (room > 0 && tiles <= kItemMax * room) q = (unsigned)(tiles + room - 1) / (unsigned)room;
+  if (q == 0 || q > 4) return fours <= grid ? 4 : q;
+  return q < 2 ? 2 : q;
+}
+struct RowPart { int b, blk, first, last, tiles, cta_last; };   // tiles first .. last - 1 of a row of `tiles`; its last CTA
+
+// the parts of rows that a CTA works on, in turn
+struct ShareWalk {
+  const int* prefix;
+  int batch, all, t, hi, b, blk, ctas, total, items;
+  // prefix: items (of the `items_` scheme) or, with 0, tiles of the rows before, [batch + 1]
+  __device__ __forceinline__ ShareWalk(const int* prefix_, int items_, int batch_, int nblk, int cta, int grid)
+      : prefix(prefix_), batch(batch_), items(items_) {
+    all = prefix[batch];                          // of one kv-head block
+    total = all * nblk;
+    ctas = items ? total : grid;
+    t = cta < ctas ? (items ? cta : (int)((unsigned long long)cta * (unsigned)total / (unsigned)ctas)) : 0;
+    hi = cta < ctas ? (items ? cta + 1 : (int)((unsigned long long)(cta + 1) * (unsigned)total / (unsigned)ctas)) : 0;
+    b = blk = 0;
+    if (t >= hi) return;
+    blk = (unsigned)t / (unsigned)all;
+    const int rem = t - blk * all;
+    // the last row that begins at or before rem (empty rows have nothing): 32 at a time, the whole warp
+    const int lane = threadIdx.x & 31;
+    for (int step = batch > 32 ? 32 : 1;; step = 1) {
+      const int at = b + lane * step;
+      b += step * (__popc(__ballot_sync(0xffffffffu, at < batch && prefix[at] <= rem)) - 1);
+      if (step == 1) break;
+    }
+  }
+  __device__ __forceinline__ bool next(const int* lens, RowPart& r) {
+    while (t < hi) {
+      const int begin = blk * all + prefix[b], end = blk * all + prefix[b + 1], from = t - begin;
+      r.b = b;
+      r.blk = blk;
+      if (++b == batch) { b = 0; ++blk; }
+      if (end <= t) continue;                     // an empty row
+      t = end < hi ? end : hi;
+      if (items) {
+        r.tiles = (lens[r.b] + kTT - 1) / kTT;
+        const int q = item_tiles(r.tiles, items);
+        r.first = from * q;
+        r.last = r.first + q < r.tiles ? r.first + q : r.tiles;
+        r.cta_last = end - 1;
+      } else {
+        r.tiles = end - begin;
+        r.first = from;
+        r.last = t - begin;
+        r.cta_last = r.last == r.tiles ? 0 : (int)(((unsigned long long)end * (unsigned)ctas - 1u) / (unsigned)total);   // 0: this one
+      }
+      return true;
+    }
+    return false;
+  }
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_kernel(const DecodeParams p) {
+  pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ int warp_sum[3][kMaxConsumers + 1];
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);   // [kMaxStages]
+  uint64_t* empty_bar = full_bar + kMaxStages;              // [kMaxStages]
+  uint8_t* stage_base = smem + kStagesAt;
+  const int PITCH = row_pitch(p.HB, D), stage_bytes = kTT * PITCH;
+  constexpr uint32_t HEAD_BYTES = D * 2;
+  int* prefix = reinterpret_cast<int*>(stage_base + p.stages * stage_bytes);    // [batch + 1]
+  int* lens = prefix + p.batch + 1;                                             // [batch]
+  int* reqs = lens + p.batch;                                                   // [batch]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int nconsumers = p.HB * p.qblocks;      // blockDim.x == (nconsumers + 1) * 32
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < p.stages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], nconsumers);
+    }
+    mbar_fence_init();
+  }
+  // ---- tiles of all rows, and the units of the rows before each ----
+  const int most = p.chunk * p.splits;          // tokens of a row that the call's bound lets count
+  const int nblk = p.Hkv / p.HB, grid = (int)gridDim.x;
+  auto load_row = [&](int r) {                  // tiles
+    const int64_t n = load_index(p.seq_len, r, p.len_w);
+    reqs[r] = (int)load_index(p.req_idx, r, p.req_w);
+    const int len = n > most ? most : n > 0 ? (int)n : 0;
+    lens[r] = len;
+    return (len + kTT - 1) / kTT;
+  };
+  auto scan = [&](int v) {                      // inclusive, over the warp
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, v, o);
+      if (lane >= o) v += x;
+    }
+    return v;
+  };
+  int items;
+  if (p.batch <= 128) {
+    // every warp for itself (the same values go to the same places): one barrier in all, and small steps feel each
+    const int per = (p.batch + 31) / 32, r_lo = lane * per;
+    const int r_hi = r_lo + per < p.batch ? r_lo + per : p.batch;
+    int own = 0, fours = 0, units = 0;
+    for (int r = r_lo; r < r_hi; ++r) {
+      const int tiles = load_row(r);
+      own += tiles;
+      fours += (tiles + 3) >> 2;
+    }
+    items = share_pick(nblk * __reduce_add_sync(0xffffffffu, own), nblk * __reduce_add_sync(0xffffffffu, fours), nblk * p.batch, grid);
+    for (int r = r_lo; r < r_hi; ++r) units += share_units((lens[r] + kTT - 1) / kTT, items);
+    int at = scan(units) - units;
+    for (int r = r_lo; r < r_hi; ++r) {
+      at += share_units((lens[r] + kTT - 1) / kTT, items);
+      prefix[r + 1] = at;
+    }
+    if (lane == 0) prefix[0] = 0;
+  } else {
+    // a thread owns neighbouring rows
+    const int per = (p.batch + blockDim.x - 1) / blockDim.x, r_lo = threadIdx.x * per;
+    const int r_hi = r_lo + per < p.batch ? r_lo + per : p.batch;
+    int own = 0, fours = 0, all = 0, all_fours = 0;
+    for (int r = r_lo; r < r_hi; ++r) {
+      const int tiles = load_row(r);
+      own += tiles;
+      fours += (tiles + 3) >> 2;
+    }
+    own = __reduce_add_sync(0xffffffffu, own);
+    fours = __reduce_add_sync(0xffffffffu, fours);
+    if (lane == 0) {
+      warp_sum[0][warp] = own;
+      warp_sum[2][warp] = fours;
+    }
+    __syncthreads();
+    for (int w = 0; w <= nconsumers; ++w) {
+      all += warp_sum[0][w];
+      all_fours += warp_sum[2][w];
+    }
+    items = share_pick(nblk * all, nblk * all_fours, nblk * p.batch, grid);
+    own = 0;
+    for (int r = r_lo; r < r_hi; ++r) own += share_units((lens[r] + kTT - 1) / kTT, items);
+    const int upto = scan(own);
+    if (lane == 31) warp_sum[1][warp] = upto;
+    __syncthreads();
+    int at = upto - own;
+    for (int w = 0; w < warp; ++w) at += warp_sum[1][w];
+    for (int r = r_lo; r < r_hi; ++r) {
+      prefix[r] = at;
+      at += share_units((lens[r] + kTT - 1) / kTT, items);
+    }
+    if (r_lo < p.batch && r_hi == p.batch) prefix[p.batch] = at;
+  }
+  __syncthreads();
+
+  const int cta = blockIdx.x;
+  for (int b = cta; b < p.batch; b += gridDim.x)            // an empty row is zero
+    if (lens[b] == 0)
+      for (int i = threadIdx.x; i < p.Hq * (D / 2); i += blockDim.x)
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)(i / (D / 2)) * p.o_hs + 2 * (i % (D / 2))) = 0u;
+
+  ShareWalk walk(prefix, items, p.batch, nblk, cta, grid);
+  RowPart r;
+  int s = 0;
+  uint32_t phase = 0;
+  if (warp == nconsumers) {
+    // ===================== producer warp: gather token rows through the table =====================
+    const int tok = lane & 15;          // token of the tile this lane serves
+    const int half = lane >> 4;         // lanes 16..31 take the V side in modes 1/2
+    const uint32_t side_bytes = p.HB * HEAD_BYTES;
+    // table entry of this lane's token: padded rows duplicate a valid row (finite data, masked later)
+    auto entry = [&](const RowPart& at, int tile) {
+      int pos = tile * kTT + tok;
+      pos = pos < lens[at.b] ? pos : lens[at.b] - 1;
+      return p.table[(int64_t)reqs[at.b] * p.tab_bs + (int64_t)pos * p.tab_ss];
+    };
+    bool more = walk.next(lens, r);
+    int tile = more ? r.first : 0;
+    int64_t row_next = more ? entry(r, tile) : 0;
+    while (more) {
+      const int64_t row = row_next;
+      const RowPart at = r;
+      const bool begins = tile == 0;
+      // the next tile's entry is on its way while this one waits for its stage
+      if (++tile == at.last) {
+        more = walk.next(lens, r);
+        tile = more ? r.first : 0;
+      }
+      if (more) row_next = entry(r, tile);
+      const char* kbase = reinterpret_cast<const char*>(p.k) + (int64_t)at.blk * p.HB * p.k_hs * 2;
+      const char* vbase = reinterpret_cast<const char*>(p.v) + (int64_t)at.blk * p.HB * p.v_hs * 2;
+      mbar_wait(&empty_bar[s], phase ^ 1);
+      if (lane == 0) mbar_arrive_expect_tx(&full_bar[s], (uint32_t)kTT * 2u * side_bytes);
+      __syncwarp();
+      uint8_t* dst = stage_base + s * stage_bytes + tok * PITCH;
+      if (p.copy_mode == 0) {
+        if (half == 0) bulk_g2s(dst, kbase + row * p.k_ts * 2, 2u * side_bytes, &full_bar[s]);
+      } else if (p.copy_mode == 1) {
+        if (half == 0) bulk_g2s(dst, kbase + row * p.k_ts * 2, side_bytes, &full_bar[s]);
+        else bulk_g2s(dst + side_bytes, vbase + row * p.v_ts * 2, side_bytes, &full_bar[s]);
+      } else {
+        const char* src = half == 0 ? kbase + row * p.k_ts * 2 : vbase + row * p.v_ts * 2;
+        const int64_t hs = (half == 0 ? p.k_hs : p.v_hs) * 2;
+        for (int h = 0; h < p.HB; ++h)
+          bulk_g2s(dst + half * side_bytes + h * HEAD_BYTES, src + h * hs, HEAD_BYTES, &full_bar[s]);
+      }
+      if (begins && lane == 0) p.ws_info[at.blk * p.batch + at.b] = make_int2(cta, at.last == at.tiles ? cta : at.cta_last);
+      if (++s == p.stages) { s = 0; phase ^= 1; }
+    }
+  } else {
+    // ===================== consumer warps: one (kv head, 16-query-head block) each =====================
+    const int hl = warp / p.qblocks;            // kv head inside the block
+    const int qblk = warp % p.qblocks;
+    const int g = lane >> 2, tq = lane & 3;
+    const int hq0 = qblk * 16 + g, hq1 = hq0 + 8;
+    const uint32_t k_off = hl * HEAD_BYTES;
+    const uint32_t v_off = (p.HB + hl) * HEAD_BYTES;
+    const int mj = lane >> 3, r8 = lane & 7;
+    // ldmatrix lane addresses (relative to the stage base)
+    const uint32_t ka = ((mj >> 1) * 8 + r8) * PITCH + k_off + (mj & 1) * 16;
+    const uint32_t va = ((mj & 1) * 8 + r8) * PITCH + v_off + (mj >> 1) * 16;
+    Consumer<T, D> c;
+    while (walk.next(lens, r)) {
+      const int kvh = r.blk * p.HB + hl;
+      const int64_t end = lens[r.b];
+      c.begin(p, r.b, kvh, hq0, hq1, tq);
+      for (int t = r.first; t < r.last; ++t) {
+        mbar_wait(&full_bar[s], phase);
+        c.template tile<true>(p, smem_u32(stage_base + s * stage_bytes), ka, va, (int64_t)t * kTT, end, tq);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty_bar[s]);
+        if (++s == p.stages) { s = 0; phase ^= 1; }
+      }
+      c.sum_rows();
+      const bool whole = r.first == 0 && r.last == r.tiles;
+#pragma unroll
+      for (int r2 = 0; r2 < 2; ++r2) {
+        if (!(r2 == 0 ? c.v0 : c.v1)) continue;
+        const int hq = r2 == 0 ? hq0 : hq1;
+        const float inv = 1.0f / c.l_run[r2];
+        if (whole) {
+          c.store_out(p, r2, r.b, kvh * p.G + hq, inv, tq);
+        } else {
+          const int64_t off = (int64_t)(hl * p.G + hq) * p.slots + 2 * cta + (r.first == 0 ? 1 : 0);
+          c.store_part(p.ws_o + off * D, r2, inv, tq);
+          if (tq == 0) p.ws_lse[off] = c.m_run[r2] + log2f(c.l_run[r2]);
+        }
+      }
+    }
+  }
+}
+
+// Merge of the rows that several shares met in, in token order.  Bound by latency: the statistics of up to 32 parts are read side by
+// side, and eight partial rows are requested before the first is added.
+template <typename T, int D>
+__global__ void flash_decode_shares_merge_kernel(const DecodeParams p) {
+  pdl_prologue();
+  const int b = blockIdx.x, head = blockIdx.y, heads = p.HB * p.G, blk = head / heads, local = head - blk * heads;
+  const int2 who = __ldcg(p.ws_info + blk * p.batch + b);   // (of an empty row: an earlier call's)
+  const int64_t len = load_index(p.seq_len, b, p.len_w);
+  const int n = who.y - who.x + 1;
+  if (len <= 0 || n < 2) return;                            // zeros, or written by its only CTA
+  auto part = [&](int i) { return (int64_t)local * p.slots + (i == 0 ? 2 * who.x + 1 : 2 * (who.x + i)); };
+  const int lane = threadIdx.x & 31;
+  const int d = threadIdx.x;                                // blockDim.x == D
+  auto ask = [&](float (&v)[8], int from) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = from + i < n ? __ldcg(p.ws_o + part(from + i) * D + d) : 0.f;
+  };
+  // the first rows are asked for along with the statistics
+  float first[8];
+  const float lse0 = lane < n ? __ldcg(p.ws_lse + part(lane)) : -INFINITY;
+  ask(first, 0);
+  float M = lse0;
+  for (int i = lane + 32; i < n; i += 32) M = fmaxf(M, __ldcg(p.ws_lse + part(i)));
+  M = warp_reduce_max(M);
+  float acc = 0.f, L = 0.f;
+  float mine = fast_exp2(lse0 - M);                         // lanes beyond n: 0
+  auto add = [&](const float (&v)[8], int from) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float w = __shfl_sync(0xffffffffu, mine, (from + i) & 31);
+      if (from + i < n) { acc += w * v[i]; L += w; }
+    }
+  };
+  add(first, 0);
+  for (int from = 8; from < n; from += 8) {
+    if (from % 32 == 0) mine = from + lane < n ? fast_exp2(__ldcg(p.ws_lse + part(from + lane)) - M) : 0.f;
+    float v[8];
+    ask(v, from);
+    add(v, from);
+  }
+  reinterpret_cast<T*>(p.out)[(int64_t)b * p.o_bs + (int64_t)head * p.o_hs + d] = from_f32<T>(acc / L);
+}
+
+struct Plan { int splits, chunk, qblocks, HB, stages, smem; bool cluster; int share_grid, share_smem; };   // share_grid 0: not the shares' kernel
 
 // ring of a block of HB kv heads: stages and bytes
 void plan_ring(Plan& pl, int D, int smem_cap) {
@@ -485,6 +839,20 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
   return true;
 }
 
+// Steps that would take several waves of CTAs of which an SM holds one, whose ring of large stages starts anew with each.  us in a
+// graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 35.8 -> 29.8, of 500 - 1000 27.2 -> 23.5, of
+// 1000 - 2000 50.5 -> 40.6, 256 of 200 58.5 -> 50.0; 32 kv heads, 32 of 250 - 480 54 -> 45.  The lengths are not known here: a step far
+// below its bound pays up to 1.5 us for adding them up (one of 1000 among 31 of 50 11.0 -> 12.5, 32 of 200 11.3 -> 12.1; from 20 tiles
+// per SM on level or faster but for one of 5400 among 7 of 270, 17.6 -> 18.2).  Below 13 tiles per SM, and where an SM holds several
+// CTAs, the splits stay: 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
+void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int smem_cap) {
+  if (pl.splits < 2 || batch > kShareRows || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 30)) return;
+  pl.share_smem = pl.smem + (int)(3 * batch + 1) * 4;
+  if (pl.share_smem > smem_cap) return;
+  if (2 * pl.smem <= smem_cap || batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * b2l_num_sms()) return;
+  pl.share_grid = b2l_num_sms();
+}
+
 // Pure function of host-known sizes => identical inside and outside graph capture.
 Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
   Plan pl;
@@ -503,6 +871,7 @@ Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
   const int64_t pairs = batch * (Hkv / HB);
   const int64_t tiles = max_len > 0 ? (max_len + kTT - 1) / kTT : 1;
   pl.cluster = false;
+  pl.share_grid = 0;
   if (plan_cluster(pl, batch, G, Hkv, D, tiles, hb_cap, smem_cap)) return pl;
   // Six CTAs per SM over all splits of the longest possible length.  max_len is only a bound: the lengths are device data, one
   // long sequence may stand among short ones, and a captured graph's bucket may be twice the longest.  One wave of larger
@@ -516,7 +885,12 @@ Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
   const int64_t tiles_per = (tiles + splits - 1) / splits;
   pl.splits = (int)((tiles + tiles_per - 1) / tiles_per);
   pl.chunk = (int)(tiles_per * kTT);
+  plan_shares(pl, batch, Hkv, D, tiles, smem_cap);
   return pl;
+}
+int64_t share_bytes(const Plan& pl, int64_t batch, int G, int Hkv, int D) {
+  if (pl.share_grid == 0) return 0;
+  return (batch * (Hkv / pl.HB) * 8 + 15) / 16 * 16 + 2ll * pl.share_grid * pl.HB * G * (D + 1) * 4 + 16;
 }
 
 template <typename T, int D>
@@ -542,6 +916,18 @@ int launch_decode(const DecodeParams& p, const Plan& pl, int64_t batch, cudaStre
     cudaLaunchKernelEx(&cfg, kern, p);
     B2L_LAUNCH_CHECK();
     return B2L_OK;
+  }
+  if constexpr (D <= 128) {
+    if (p.ws_info != nullptr) {
+      static int configured_shares[64] = {0};
+      auto kern = flash_decode_shares_kernel<T, D>;
+      B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, pl.share_smem, configured_shares));
+      b2l_launch(kern, dim3((unsigned)pl.share_grid), dim3((p.HB * p.qblocks + 1) * 32), (size_t)pl.share_smem, st, p);
+      B2L_LAUNCH_CHECK();
+      b2l_launch(flash_decode_shares_merge_kernel<T, D>, dim3((unsigned)batch, (unsigned)p.Hq), dim3(D), (size_t)0, st, p);
+      B2L_LAUNCH_CHECK();
+      return B2L_OK;
+    }
   }
   const bool merge = p.splits > 1 && p.tickets == nullptr;
   static int configured[2][64] = {{0}};
@@ -570,7 +956,9 @@ extern "C" int64_t b2l_flash_decoding_workspace_bytes(int64_t batch, int num_q_h
   if (batch <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
   Plan pl = make_plan(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
   if (pl.splits <= 1 || pl.cluster) return 16;
-  return (int64_t)batch * num_q_heads * pl.splits * (head_dim + 1) * 4 + 16;
+  const int64_t split_bytes = (int64_t)batch * num_q_heads * pl.splits * (head_dim + 1) * 4 + 16;
+  const int64_t shares = share_bytes(pl, batch, num_q_heads / num_kv_heads, num_kv_heads, head_dim);
+  return shares > split_bytes ? shares : split_bytes;
 }
 
 extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache, const void* v_cache,
@@ -614,7 +1002,8 @@ extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache,
   const bool fused_run = heads_packed && pl.HB == num_kv_heads && k_token_stride == v_token_stride &&
                          (const char*)v_cache == (const char*)k_cache + (int64_t)num_kv_heads * head_dim * 2;
   p.copy_mode = fused_run ? 0 : (heads_packed ? 1 : 2);
-  p.ws_o = nullptr; p.ws_lse = nullptr;
+  p.ws_o = nullptr; p.ws_lse = nullptr; p.ws_info = nullptr;
+  p.batch = (int)batch;
   // the split CTAs merge their own results when the caller provides zeroed tickets (one per batch row x head block)
   p.tickets = (tickets && num_tickets >= batch * (num_kv_heads / pl.HB)) ? (int*)tickets : nullptr;
   if (pl.splits > 1 && !pl.cluster) {
@@ -622,8 +1011,15 @@ extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache,
     B2L_REQUIRE(workspace && workspace_bytes >= need, "flash_decoding: workspace too small (%lld < %lld)",
                 (long long)workspace_bytes, (long long)need);
     B2L_REQUIRE((uintptr_t)workspace % 16 == 0, "flash_decoding: workspace must be 16-byte aligned");
-    p.ws_o = (float*)workspace;
-    p.ws_lse = p.ws_o + (int64_t)batch * num_q_heads * pl.splits * head_dim;
+    if (pl.share_grid != 0 && p.tickets == nullptr) {
+      p.ws_info = (int2*)workspace;
+      p.slots = 2 * pl.share_grid;
+      p.ws_o = (float*)((char*)workspace + (batch * (num_kv_heads / pl.HB) * 8 + 15) / 16 * 16);
+      p.ws_lse = p.ws_o + 2ll * pl.share_grid * pl.HB * p.G * head_dim;
+    } else {
+      p.ws_o = (float*)workspace;
+      p.ws_lse = p.ws_o + (int64_t)batch * num_q_heads * pl.splits * head_dim;
+    }
   }
   cudaStream_t st = (cudaStream_t)stream;
 #define DISPATCH_D(TT)                                                    \
