@@ -17,10 +17,12 @@
 //     subtracted exactly in the conversion, others as scale * (sum - z * xsum).  (Nibbles as fp16 subnormals, with the zero point applied to the sums, need 5 instead of 9
 //     instructions per word and measured the same: 15.4 us against 16.3 us for 28672 x 4096, 5.5 against 5.0 us for 6144 x
 //     4096, so the exact form stays.)
-//   * after a chunk of up to 4 strips the warps add up their sums through shared memory in warp order (deterministic); the
-//     next chunk's weights are on their way meanwhile.
+//   * after a chunk of strips the warps add up their sums through shared memory in warp order (deterministic); the next
+//     chunk's weights are on their way meanwhile, and the other warps go on to them while some add (a second barrier right after
+//     the sums: 28672 x 4096, one token 18.1 us instead of 17.1).
 // Measured, one token, streaming kernel -> this one: 4096 x 4096 7.0 -> 3.7 us, 6144 x 4096 8.3 -> 5.0, 28672 x 4096 19.6 ->
-// 16.3, 4096 x 14336 12.9 -> 9.6.
+// 15.0, 4096 x 14336 12.9 -> 9.6.  Copies by TMA (one lane instead of address arithmetic in all): 0.3 us slower to start, 4096 x
+// 14336 at eight tokens 13.1 -> 15.5.
 #include "common.cuh"
 #include "dequant.cuh"
 #include "gemm_quant_decode.cuh"
@@ -32,7 +34,11 @@ namespace {
 constexpr int kDecWarps = 16, kDecThreads = kDecWarps * 32;
 constexpr int kDecSlice = 256, kDecBlocks = kDecSlice / 128;       // k per slice, 128-k blocks in it
 constexpr int kDecUnit = kDecBlocks * (1024 + 128);                // a strip's slice: words, then {16 scales, 16 zeros} per block
-constexpr int kDecDepth = 4, kDecChunk = 4;
+// CHUNK: strips whose sums a thread holds at a time; the warps meet once per chunk.  With twelve strips to a CTA or more, chunks of
+// seven and a ring that is a strip shorter to make room for them (28672 x 4096, one / eight tokens, us: chunks of four 17.1 and 18.8,
+// of seven 16.4 and 17.9); with one or two, chunks of two leave registers (4096 x 14336, eight tokens 13.7 -> 12.7); chunks of seven for
+// few strips cost 5 - 10 % (6144 x 4096, eight tokens 7.0 / 7.3).
+__host__ __device__ constexpr int dec_depth(int chunk) { return chunk > 4 ? 3 : 4; }
 
 struct DecParams {
   __half* y; int64_t ldy;
@@ -58,12 +64,13 @@ __device__ __forceinline__ void mma_f16_zero(float (&d)[4], const uint32_t (&a)[
 
 // WHOLE: the packer has seen that every zero point is an integer in [0, 1023] (the test costs 10 % where it has to be made:
 // 28672 x 4096, one token 17.9 against 16.3 us)
-template <int LAYOUT, int EPI, bool WHOLE>
+template <int LAYOUT, int EPI, bool WHOLE, int CHUNK>
 __global__ void __launch_bounds__(kDecThreads, 1)
 gemm_quant_decode_kernel(const DecParams p) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;              // MMA fragment coordinates
+  constexpr int kDecDepth = dec_depth(CHUNK);
   uint8_t* ring = smem + warp * kDecDepth * kDecUnit;
   float4* red = reinterpret_cast<float4*>(smem + kDecWarps * kDecDepth * kDecUnit);   // [strip][warp][lane]
   pdl_launch_dependents();
@@ -71,7 +78,7 @@ gemm_quant_decode_kernel(const DecParams p) {
   const int s_hi = (int)((int64_t)(blockIdx.x + 1) * p.strips / gridDim.x);
 
   // chunks of equal size
-  const int chunks = (s_hi - s_lo + kDecChunk - 1) / kDecChunk;
+  const int chunks = (s_hi - s_lo + CHUNK - 1) / CHUNK;
   const int step = chunks > 0 ? (s_hi - s_lo + chunks - 1) / chunks : 1;
   const int slices = p.K / kDecSlice;
   const int mine = slices > warp ? (slices - warp - 1) / kDecWarps + 1 : 0;      // this warp's slices
@@ -117,9 +124,9 @@ gemm_quant_decode_kernel(const DecParams p) {
   float xs[kDecBlocks][2];                            // sum of the block's activations, tokens 2t and 2t + 1
   for (int chunk = s_lo; chunk < s_hi; chunk += step) {
     const int in_chunk = s_hi - chunk < step ? s_hi - chunk : step;
-    float acc[kDecChunk][4];
+    float acc[CHUNK][4];
 #pragma unroll
-    for (int r = 0; r < kDecChunk; ++r)
+    for (int r = 0; r < CHUNK; ++r)
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
     for (int sl = 0; sl < mine; ++sl) {
@@ -149,7 +156,7 @@ gemm_quant_decode_kernel(const DecParams p) {
         }
       }
 #pragma unroll
-      for (int r = 0; r < kDecChunk; ++r) {
+      for (int r = 0; r < CHUNK; ++r) {
         if (r < in_chunk) {
           issue();
           asm volatile("cp.async.wait_group %0;" ::"n"(kDecDepth - 1) : "memory");
@@ -198,8 +205,9 @@ gemm_quant_decode_kernel(const DecParams p) {
       }
     }
     // ---- sums of the 16 warps, in warp order ----
+    if (chunk != s_lo) __syncthreads();               // the last chunk's have been read
 #pragma unroll
-    for (int r = 0; r < kDecChunk; ++r)
+    for (int r = 0; r < CHUNK; ++r)
       if (r < in_chunk) red[(r * kDecWarps + warp) * 32 + lane] = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
     __syncthreads();
     if (warp < in_chunk) {                            // warp r stores strip r; lane is the fragment's
@@ -227,22 +235,28 @@ gemm_quant_decode_kernel(const DecParams p) {
         }
       }
     }
-    __syncthreads();
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <int LAYOUT, int EPI, bool WHOLE>
-int launch_dec(const DecParams& p, cudaStream_t st) {
-  constexpr int smem = kDecWarps * kDecDepth * kDecUnit + kDecChunk * kDecWarps * 32 * 16;
+template <int LAYOUT, int EPI, bool WHOLE, int CHUNK>
+int launch_dec_chunk(const DecParams& p, cudaStream_t st) {
+  constexpr int smem = kDecWarps * dec_depth(CHUNK) * kDecUnit + CHUNK * kDecWarps * 32 * 16;
   static_assert(smem <= 227 * 1024, "shared memory");
-  auto kern = gemm_quant_decode_kernel<LAYOUT, EPI, WHOLE>;
+  auto kern = gemm_quant_decode_kernel<LAYOUT, EPI, WHOLE, CHUNK>;
   static int configured[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, smem, configured));
   const int sms = b2l_num_sms();
   b2l_launch(kern, dim3((unsigned)(p.strips < sms ? p.strips : sms)), dim3(kDecThreads), (size_t)smem, st, p);
   B2L_LAUNCH_CHECK();
   return B2L_OK;
+}
+template <int LAYOUT, int EPI, bool WHOLE>
+int launch_dec(const DecParams& p, cudaStream_t st) {
+  const int sms = b2l_num_sms();
+  if (p.strips <= 2 * sms) return launch_dec_chunk<LAYOUT, EPI, WHOLE, 2>(p, st);
+  if (LAYOUT == 1 && p.strips >= 12 * sms) return launch_dec_chunk<LAYOUT, EPI, WHOLE, 7>(p, st);
+  return launch_dec_chunk<LAYOUT, EPI, WHOLE, 4>(p, st);
 }
 
 }  // namespace
