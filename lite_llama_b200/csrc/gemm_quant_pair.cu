@@ -41,7 +41,7 @@ constexpr int kQpTokens = 128;                              // per pair tile; ea
 // follow one another, so one warp issues them, and what a step waits for is its conversion: two accumulators, more steps.
 __host__ __device__ constexpr int qp_accs(int nt, bool chain) { return chain ? 2 : nt == kQpTokens ? 3 : 4; }
 __host__ __device__ constexpr int qp_op_steps(int nt, bool chain) { return (512 - qp_accs(nt, chain) * nt) / 64; }
-constexpr int kQpStepK = 128;                               // k per operand step; without CHAIN handed over and back in stages of 64
+constexpr int kQpStepK = 128;                               // k per operand step; handed over and back in stages of 64 where there are two steps of it
 constexpr int kQpXSub = kQpTokens / 2 * kStageKBytes;       // 64 tokens x 64 k
 constexpr int kQpXBytes = 2 * kQpXSub;
 constexpr int kQpMeta = 8 * 64 * 8;                         // down projection: {slot, routing weight} of the epilogue warps' rows
@@ -105,7 +105,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   uint8_t* x_ring = w_ring + kQpWStages * kABytes;
   constexpr int kHalf = NT / 2;                            // tokens per epilogue warp
   constexpr int kAccs = qp_accs(NT, CHAIN), kOpSteps = qp_op_steps(NT, CHAIN), kOpCol0 = kAccs * NT;
-  constexpr int kSub = CHAIN ? 1 : 2, kOpStages = kSub * kOpSteps;      // stages per operand step
+  constexpr int kSub = CHAIN || NT != kQpTokens ? 1 : 2, kOpStages = kSub * kOpSteps;      // stages per operand step
   // (plain mode with NT 64 is launched for up to 64 tokens only: one row of tiles)
   constexpr int kStepsPerRaw = QK == Q_INT4 ? 2 : 1;       // a raw block is 128 rows x 128 bytes
 
@@ -246,7 +246,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
               }
               if (elect_one()) {
 #pragma unroll
-                for (int k = h * 4; k < (CHAIN ? 8 : h * 4 + 4); ++k)
+                for (int k = h * 4; k < (kSub == 1 ? 8 : h * 4 + 4); ++k)
                   umma_pair_ts(acc, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)), idesc,
                                (in_seg | k) != 0 ? 1u : 0u);
                 tc_commit_pair(&ctl->op_empty[kSub * os.stage + h]);
@@ -276,19 +276,43 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     uint8_t* meta = x_ring + kQpXStages * kQpXBytes + (warp - kQpEpi0) * 64 * 8;
     pdl_wait_prior();               // y may still be read upstream
     PipeState as(kAccs);
+    // down projection: slots and routing weights of a tile's rows; one trip to L2 behind the other, they took 1600 of 10300 cycles
+    // at the start of each tile of 128 rows, so they are asked for during the tile before
+    constexpr bool kAhead = MODE == QP_DOWN && NT == kQpTokens;     // (with few rows a tile's end does not last: 34.2 against 35.0 us)
+    constexpr int kQ = MODE == QP_DOWN ? kHalf / 32 : 1;
+    int slot[kQ];
+    float weight[kQ];
+    auto ask_slots = [&](int t) {
+      const QpTile pt = qp_tile<MODE>(p, t);
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        const int r = half * kHalf + 32 * q + lane;
+        slot[q] = r < pt.rows ? ld_upstream(p.order + pt.m0 + r) : -1;
+      }
+    };
+    auto ask_weights = [&]() {
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) weight[q] = slot[q] >= 0 ? __half2float(p.row_weights[slot[q]]) : 0.f;
+    };
+    if (kAhead && pair < tiles) {
+      ask_slots(pair);
+      ask_weights();
+    }
     for (int t = pair; t < tiles; t += pairs) {
       const QpTile pt = qp_tile<MODE>(p, t);
       if (MODE == QP_DOWN) {
-        // slots and routing weights of this warp's rows: asked for now, two trips to L2 at the tile's end otherwise
-        __syncwarp();
-#pragma unroll
-        for (int q = 0; q < kHalf / 32; ++q) {
-          const int r = half * kHalf + 32 * q + lane;
-          const int slot = r < pt.rows ? ld_upstream(p.order + pt.m0 + r) : 0;
-          reinterpret_cast<float*>(meta)[32 * q + lane] = r < pt.rows ? __half2float(p.row_weights[slot]) : 0.f;
-          reinterpret_cast<int*>(meta + 256)[32 * q + lane] = slot;
+        if (!kAhead) {
+          ask_slots(t);
+          ask_weights();
         }
         __syncwarp();
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          reinterpret_cast<float*>(meta)[32 * q + lane] = weight[q];
+          reinterpret_cast<int*>(meta + 256)[32 * q + lane] = slot[q];
+        }
+        __syncwarp();
+        if (kAhead && t + pairs < tiles) ask_slots(t + pairs);
       }
       const int n_tile = pt.n * 2 + (int)rank;
       // weight row of this thread, and for the gate / up rows the output that the pair (lane, lane + 16) forms
@@ -326,6 +350,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
         as.advance();
       }
       // ---- the tile's results ----
+      if (kAhead && t + pairs < tiles) ask_weights();
       float bv = 0.f;
       if (n_ok && p.bias) bv = p.bias_is_f32 ? reinterpret_cast<const float*>(p.bias)[n]
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
@@ -418,7 +443,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           constexpr int kChunks = QK == Q_INT4 ? 2 : 4;     // 16-byte chunks of the row per 64 k
-          const int stage = kSub * (group + 2 * own) + (CHAIN ? 0 : h);
+          const int stage = kSub * (group + 2 * own) + (kSub == 1 ? 0 : h);
           const int c0 = (QK == Q_INT4 ? (k & 1) * 4 : 0) + h * kChunks;
           if (CHAIN && h == 0) {
             mbar_wait(&ctl->op_empty[stage], own_phase ^ 1);
@@ -441,7 +466,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
                 else dequant_w8_word(ws[j], QK == Q_FP8, vals + (QK == Q_INT4 ? 0 : 8 * c + 2 * j));
               }
             }
-            if (!CHAIN && q == 0) {
+            if (!CHAIN && q == 0 && (h == 0 || kSub == 2)) {
               mbar_wait(&ctl->op_empty[stage], own_phase ^ 1);
               tc_fence_after();
             }
@@ -449,7 +474,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
             if constexpr (CHAIN) tmem_st_32x32b_x32(dst, vals);
             else tmem_st_32x32b_x16(dst, vals);
           }
-          if (CHAIN && h == 0) continue;
+          if (kSub == 1 && h == 0) continue;
           if (h == 1) {
             // the raw words have all been converted: the block may be refilled (an odd last step speaks for both halves)
             __syncwarp();
