@@ -839,18 +839,22 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
   return true;
 }
 
-// Steps that would take several waves of CTAs of which an SM holds one, whose ring of large stages starts anew with each.  us in a
-// graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 35.8 -> 29.8, of 500 - 1000 27.2 -> 23.5, of
-// 1000 - 2000 50.5 -> 40.6, 256 of 200 58.5 -> 50.0; 32 kv heads, 32 of 250 - 480 54 -> 45.  The lengths are not known here: a step far
-// below its bound pays up to 1.5 us for adding them up (one of 1000 among 31 of 50 11.0 -> 12.5, 32 of 200 11.3 -> 12.1; from 20 tiles
-// per SM on level or faster but for one of 5400 among 7 of 270, 17.6 -> 18.2).  Below 13 tiles per SM, and where an SM holds several
-// CTAs, the splits stay: 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
+// Steps that would take several waves of CTAs of which an SM holds one or two, whose rings of large stages start anew with each.
+// us in a graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 35.8 -> 29.8, of 500 - 1000 27.2 ->
+// 24.0, of 1000 - 2000 50.4 -> 41.0, 256 of 200 58.5 -> 50.5; 32 kv heads, 32 of 250 - 480 54 -> 45; 4 kv heads, 32 of 1000 - 2000 30.0 ->
+// 25.2, 64 of 1000 35.1 -> 30.9, 128 of 2000 105 -> 94.  The lengths are not known here: a step far below its bound pays up to 1.7 us for
+// adding them up (8 kv heads, one of 1000 among 31 of 50 11.0 -> 12.5, 32 of 200 11.3 -> 12.1; 4 kv heads, 32 of 40 under 2000 8.8 -> 9.8;
+// with 20 tiles per SM and more mostly level or faster).  Below 13 tiles per CTA, or with more CTAs to an SM, the splits stay: 8 kv
+// heads 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
 void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int smem_cap) {
   if (pl.splits < 2 || batch > kShareRows || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 30)) return;
   pl.share_smem = pl.smem + (int)(3 * batch + 1) * 4;
   if (pl.share_smem > smem_cap) return;
-  if (2 * pl.smem <= smem_cap || batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * b2l_num_sms()) return;
-  pl.share_grid = b2l_num_sms();
+  const int per_sm = (smem_cap + 256) / (pl.share_smem + 1024);
+  if (per_sm > 2) return;
+  const int grid = b2l_num_sms() * (per_sm > 1 ? per_sm : 1);
+  if (batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * grid) return;
+  pl.share_grid = grid;
 }
 
 // Pure function of host-known sizes => identical inside and outside graph capture.
