@@ -63,7 +63,9 @@ static inline SplitPlan make_plan(int64_t M, int64_t N, int64_t K, int k_elems_p
   // with SMALLER token tiles before resorting to split-K -- a split of a 256-token tile moves 128 KiB of fp32
   // partials per CTA through the workspace, which cost more than the GEMM (measured 57 us vs 34 us for the
   // reference's Triton kernel on this shape, profiles/r2c_triton_vs_b200.md).
-  while (pl.bt > 64 && (int64_t)pl.n_tiles * cdiv64(M, pl.bt) < sms) pl.bt /= 2;
+  // Not where that makes a second wave out of the first, which streams the weights twice (65 - 128 tokens, us: bf16 16384 x 4096 44 -
+  // 46 -> 27 - 29, 9728 x 896 13.0 -> 10.3, int8 12288 x 3584 20 -> 14).
+  while (pl.bt > 64 && (int64_t)pl.n_tiles * cdiv64(M, pl.bt) < sms && (int64_t)pl.n_tiles * cdiv64(M, pl.bt / 2) <= sms) pl.bt /= 2;
   pl.m_tiles = (int)cdiv64(M, pl.bt);
   pl.num_kb = (int)cdiv64(K, k_elems_per_stage);
   const int tiles = pl.n_tiles * pl.m_tiles;
@@ -75,6 +77,14 @@ static inline SplitPlan make_plan(int64_t M, int64_t N, int64_t K, int k_elems_p
     if (splits > max_splits) splits = max_splits;
     if (splits > 32) splits = 32;
     if (splits < 1) splits = 1;
+    // The last CTA of a tile adds up the parts, four splits and 16 tokens a trip to L2: with many tokens and splits that takes
+    // longer than the stream itself (64 tokens, 896 x 4864, bf16, 19 splits: 12 of 18.9 us).  In 1/100 us, per SM 75 bytes per ns.
+    const int stage = kABytes + pl.bt * kStageKBytes;
+    auto cost = [&](int s) { return (pl.num_kb + s - 1) / s * (stage / 750) + (s > 1 ? 100 + (s + 3) / 4 * (pl.bt / 16) * 55 : 0); };
+    int best = splits;
+    for (int s = splits - 1; s >= 2; --s)
+      if (cost(s) < cost(best)) best = s;
+    if (cost(best) * 100 < cost(splits) * 85) splits = best;
   }
   pl.kb_per_split = (pl.num_kb + splits - 1) / splits;
   pl.splits = (pl.num_kb + pl.kb_per_split - 1) / pl.kb_per_split;

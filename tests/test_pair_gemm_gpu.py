@@ -338,3 +338,19 @@ def test_int4_wide_swiglu_is_gemm_then_swiglu(m, n, k):
 @pytest.mark.parametrize("fmt", ["fp8_block", "fp8_channel", "int8_channel", "int8_group_n"])
 def test_w8_wide_tiles(m, n, k, fmt):
     test_w8_pair_tiles(m, n, k, fmt)
+
+
+# ---- one-SM kernel (csrc/gemm_dense.cu): 128-token tiles where 64-token tiles would need a second wave (75 - 148 weight tiles), and
+# fewer splits of k than there are SMs for where the last CTA of a tile would add up too many
+PLAN_EDGES = [(65, 9728, 896), (128, 18944, 192), (100, 9600, 320), (16, 128, 4096), (64, 896, 4864), (33, 512, 8192), (200, 256, 2048)]
+
+
+@pytest.mark.parametrize("m,n,k", PLAN_EDGES)
+def test_linear_token_tiles_and_splits(m, n, k):
+    for dtype in (torch.float16, torch.bfloat16):
+        test_linear_pair_tiles(m, n, k, dtype, True)
+
+
+@pytest.mark.parametrize("m,n,k", PLAN_EDGES)
+def test_int8_token_tiles_and_splits(m, n, k):
+    test_int8_pair_tiles(m, n, k, True)
