@@ -259,23 +259,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 // consecutive, and CTA s adds up columns [s BN / S, ...) of its rows over the S CTAs of its rank parity, in order of s.
 // Measured: pair_splits below.
 // ---------------------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ uint4 ld_cluster_128(uint32_t a) {
-  uint4 v;
-  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
-  return v;
-}
-// one arrival in both CTAs of the pair whose even rank is `first`
-__device__ __forceinline__ void tc_commit_pair_at(uint64_t* bar, uint32_t first) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-      ::"r"(smem_u32(bar)), "h"((uint16_t)(3u << first)) : "memory");
-}
-
 template <int KIND, typename T, int BN, int S>
 __global__ void __cluster_dims__(2 * S, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_split_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,

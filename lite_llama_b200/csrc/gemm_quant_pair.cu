@@ -94,8 +94,8 @@ __device__ __forceinline__ int qp_tile_n(int rows_left) {
   return n < NT ? n : NT;
 }
 
-template <int QK, int EPI, int MODE, int NT, bool CHAIN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kQpThreads, 1)
+template <int QK, int EPI, int MODE, int NT, bool CHAIN, int S>
+__global__ void __cluster_dims__(2 * S, 1, 1) __launch_bounds__(kQpThreads, 1)
 gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                        const QuantPairParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -110,11 +110,18 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
   constexpr int kStepsPerRaw = QK == Q_INT4 ? 2 : 1;       // a raw block is 128 rows x 128 bytes
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = pair_rank();
-  const int pairs = gridDim.x >> 1, pair = blockIdx.x >> 1;
+  // S > 1: S pairs share a tile and run over a part of k each (one tile per cluster)
+  const uint32_t first = S > 1 ? pair_rank() & ~1u : 0u, rank = pair_rank() - first;
+  const int pairs = gridDim.x / (2 * S), pair = blockIdx.x / (2 * S);
+  auto lead = [&](const void* q) { return S > 1 ? cluster_addr(q, first) : leader_addr(q); };
+  auto commit = [&](uint64_t* bar) {
+    if (S > 1) tc_commit_pair_at(bar, first);
+    else tc_commit_pair(bar);
+  };
   if (MODE != QP_PLAIN) pdl_wait_prior();                  // the tile table is an earlier kernel's output
   const int tiles = qp_tiles<MODE>(p);
-  const int steps = p.steps;                               // operand stages per tile
+  const int step0 = S > 1 ? (int)(first / 2) * p.split_steps : 0;
+  const int steps = S > 1 && p.steps - step0 > p.split_steps ? p.split_steps : p.steps - step0;      // operand steps of this pair
   if (threadIdx.x == kQpWProd * 32) {
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
@@ -164,7 +171,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           if (elect_one()) {
             mbar_arrive_expect_tx(&ctl->w_full[ws.stage], kABytes);
             uint8_t* dst = w_ring + (size_t)ws.stage * kABytes;
-            const int col = rb * (QK == Q_INT4 ? 32 : 128);
+            const int col = (step0 / kStepsPerRaw + rb) * (QK == Q_INT4 ? 32 : 128);
             if (MODE == QP_GATE_UP) {
               // 16 gate rows, the 16 up rows of the same outputs, 16 gate rows ...: a warp then holds both
 #pragma unroll
@@ -191,11 +198,11 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
           mbar_wait(&ctl->x_empty[xs.stage], xs.phase ^ 1);
           if (elect_one()) {
             uint8_t* dst = x_ring + (size_t)xs.stage * kQpXBytes;
-            const uint32_t bar = leader_addr(&ctl->x_full[xs.stage]);
+            const uint32_t bar = lead(&ctl->x_full[xs.stage]);
             if (MODE == QP_PLAIN) {
               if (rank == 0) mbar_arrive_expect_tx(&ctl->x_full[xs.stage], 2 * kQpXBytes);
-              tma_load_2d_pair(dst, &tmap_x, s * kQpStepK, row, bar, kEvictNormal);
-              tma_load_2d_pair(dst + kQpXSub, &tmap_x, s * kQpStepK + 64, row, bar, kEvictNormal);
+              tma_load_2d_pair(dst, &tmap_x, (step0 + s) * kQpStepK, row, bar, kEvictNormal);
+              tma_load_2d_pair(dst + kQpXSub, &tmap_x, (step0 + s) * kQpStepK + 64, row, bar, kEvictNormal);
             } else {
               // an expert may have two rows: only the 16-row boxes that are read
               if (rank == 0) mbar_arrive_expect_tx(&ctl->x_full[xs.stage], 2 * 2 * half * kStageKBytes);
@@ -249,10 +256,10 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
                 for (int k = h * 4; k < (kSub == 1 ? 8 : h * 4 + 4); ++k)
                   umma_pair_ts(acc, a + 8 * k, b + (uint64_t)((k >> 2) * (kQpXSub >> 4) + 2 * (k & 3)), idesc,
                                (in_seg | k) != 0 ? 1u : 0u);
-                tc_commit_pair(&ctl->op_empty[kSub * os.stage + h]);
+                commit(&ctl->op_empty[kSub * os.stage + h]);
                 if (h == kSub - 1) {
-                  if (last) tc_commit_pair(&ctl->acc_full[as.stage]);
-                  tc_commit_pair(&ctl->x_empty[xs.stage]);   // the last one: the X producers wait for it before they leave
+                  if (last) commit(&ctl->acc_full[as.stage]);
+                  commit(&ctl->x_empty[xs.stage]);   // the last one: the X producers wait for it before they leave
                 }
               }
               __syncwarp();
@@ -271,7 +278,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     const int quad = warp & 3, half = (warp - kQpEpi0) >> 2;
     const int row = quad * 32 + lane;
     const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + half * kHalf;
-    const uint32_t empty0 = leader_addr(&ctl->acc_empty[0]);
+    const uint32_t empty0 = lead(&ctl->acc_empty[0]);
     const int nseg = (steps + p.seg_steps - 1) / p.seg_steps;
     uint8_t* meta = x_ring + kQpXStages * kQpXBytes + (warp - kQpEpi0) * 64 * 8;
     pdl_wait_prior();               // y may still be read upstream
@@ -326,6 +333,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       uint64_t acc[kHalf / 2];
 #pragma unroll
       for (int j = 0; j < kHalf / 2; ++j) acc[j] = 0ull;
+      if (S > 1) sp += (int64_t)(step0 / p.seg_steps) * p.s_stride_k;
       float sc = __ldg(sp);
       for (int g = 0; g < nseg; ++g) {
         const uint64_t s2 = pack_f32x2(sc, sc);
@@ -356,8 +364,50 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
                                              : __half2float(reinterpret_cast<const __half*>(p.bias)[n]);
       const int m0 = pt.m0 + half * kHalf;
       const int rows = pt.rows - half * kHalf;
-      if (rows <= 0) continue;                               // uniform over the warp
+      if (S == 1 && rows <= 0) continue;                     // uniform over the warp
       __half* y = reinterpret_cast<__half*>(p.y);
+      if constexpr (S > 1) {
+        // The pairs' sums meet in shared memory (over the rings: the last segment's products have read them), [token / 4][row][4], and
+        // each pair adds up every S-th four tokens of its rows, in order of k.
+        uint8_t* sums = w_ring + (size_t)row * 16;
+#pragma unroll
+        for (int j = 0; j < kHalf / 2; j += 2) {
+          float f[4];
+          unpack_f32x2(acc[j], f[0], f[1]);
+          unpack_f32x2(acc[j + 1], f[2], f[3]);
+          *reinterpret_cast<float4*>(sums + (size_t)(half * (kHalf / 4) + j / 2) * (kBlockW * 16)) = make_float4(f[0], f[1], f[2], f[3]);
+        }
+        __syncwarp();
+        pair_sync();
+        const int left = pt.rows < NT ? pt.rows : NT;
+#pragma unroll 2
+        for (int q = (int)(first / 2) + S * half; 4 * q < left; q += 2 * S) {
+          uint4 part[S];
+#pragma unroll
+          for (int u = 0; u < S; ++u) part[u] = ld_cluster_128(cluster_addr(sums + (size_t)q * (kBlockW * 16), 2u * u + rank));
+          float f[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+          for (int u = 0; u < S; ++u) {
+            f[0] += __uint_as_float(part[u].x);
+            f[1] += __uint_as_float(part[u].y);
+            f[2] += __uint_as_float(part[u].z);
+            f[3] += __uint_as_float(part[u].w);
+          }
+          const int m = pt.m0 + 4 * q;
+          if (EPI == 0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (n_ok && 4 * q + e < left) y[(int64_t)(m + e) * p.ldy + n] = __float2half_rn(f[e] + bv);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; e += 2) {
+              const float o = swiglu_h2(exchange_pair<1>(pack2<__half>(f[e] + bv, f[e + 1] + bv), lane));
+              if (n_ok && 4 * q + e + (lane & 1) < left) y[(int64_t)(m + e + (lane & 1)) * p.ldy + (n >> 1)] = __float2half_rn(o);
+            }
+          }
+        }
+        continue;
+      }
       constexpr bool kFewRows = NT < kQpTokens;              // an early end costs the large tiles 5 % (registers)
       if (MODE == QP_GATE_UP) {
         // like store_swiglu, with the pair 16 lanes apart and no further exchange (92.8 against 94.1 us for 64 experts of 190 rows)
@@ -414,7 +464,7 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     const int row = quad * 32 + lane, rx = row & 7;
     const uint32_t dst0 = tmem_base + ((uint32_t)(quad * 32) << 16) + kOpCol0;
     constexpr int kOwn = kOpSteps / 2;                      // operand steps of this group: group, group + 2, ...
-    const uint32_t full0 = leader_addr(&ctl->op_full[0]);
+    const uint32_t full0 = lead(&ctl->op_full[0]);
     int own = 0;
     uint32_t own_phase = 0;
     int i0 = 0;                                             // running stage count at the tile's first step
@@ -427,14 +477,14 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
       if (QK == Q_INT4) {
         const int n_tile = qp_tile<MODE>(p, t).n * 2 + (int)rank;
         zp = p.zeros + ((int64_t)(n_tile * kBlockW < p.N ? n_tile : 0) * p.groups) * kBlockW + row;
-        if (k < steps) z = __ldg(zp + (int64_t)(k / p.seg_steps) * p.s_stride_k);
+        if (k < steps) z = __ldg(zp + (int64_t)((step0 + k) / p.seg_steps) * p.s_stride_k);
       }
       for (; k < steps; k += 2) {
         __half2 add_lo, add_hi;
         if (QK == Q_INT4) {
           add_lo = __float2half2_rn(-1024.f - z);
           add_hi = __float2half2_rn(-64.f - z);
-          if (k + 2 < steps) z = __ldg(zp + (int64_t)((k + 2) / p.seg_steps) * p.s_stride_k);
+          if (k + 2 < steps) z = __ldg(zp + (int64_t)((step0 + k + 2) / p.seg_steps) * p.s_stride_k);
         }
         const int raw = raw0 + (QK == Q_INT4 ? k >> 1 : k);
         const int rs = raw % kQpWStages;
@@ -495,14 +545,18 @@ gemm_quant_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     }
   }
 
+  if (S > 1 && (warp < kQpEpi0 || warp >= kQpWProd)) {
+    __syncwarp();
+    pair_sync();                    // the epilogue's: sums in place
+  }
   tc_fence_before();
-  pair_sync();                      // the peer's MMAs, commits and arrivals are over
+  pair_sync();                      // the peer's MMAs, commits and arrivals are over, its sums have been read
   if (warp == kQpMma) tmem_dealloc_pair(tmem_base, 512);
 }
 
-template <int QK, int EPI, int MODE, int NT, bool CHAIN>
+template <int QK, int EPI, int MODE, int NT, bool CHAIN, int S = 1>
 static int launch_qp_form(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, int grid, cudaStream_t st) {
-  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE, NT, CHAIN>;
+  auto kern = gemm_quant_pair_kernel<QK, EPI, MODE, NT, CHAIN, S>;
   static int configured[64] = {0};
   B2L_CUDA_CHECK(b2l_ensure_dynamic_smem(kern, kQpSmem, configured));
   b2l_launch(kern, dim3((unsigned)grid), dim3(kQpThreads), (size_t)kQpSmem, st, tw, tx, p);
@@ -516,7 +570,41 @@ static int launch_qp(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPa
                           : launch_qp_form<QK, EPI, MODE, NT, true>(tw, tx, p, grid, st);
 }
 
-// Where the pair kernel is the faster one (both kernels measured over 72 - 512 tokens, eight projection shapes, int4 with and
+template <int QK, int EPI, int S>
+static int launch_qp_split(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParams& p, cudaStream_t st) {
+  const int grid = p.m_tiles * p.n_tiles * 2 * S;
+  return p.seg_steps == 1 ? launch_qp_form<QK, EPI, QP_PLAIN, kQpTokens, false, S>(tw, tx, p, grid, st)
+                          : launch_qp_form<QK, EPI, QP_PLAIN, kQpTokens, true, S>(tw, tx, p, grid, st);
+}
+
+// Pairs that share a tile, and the steps of each: whole raw blocks and scale groups.  A pair takes ~870 cycles a step however few of
+// the SMs have a tile, so few tiles are shared by as many pairs as a whole B200 holds at once: 15 clusters of eight CTAs, 22 of six, 33
+// of four.  Set-up, exchange and the larger cluster cost ~3 us, and what else would run decides from which k on they pay (us, else ->
+// shared, int4 in groups of 128 / fp8 in blocks / int8 per row):
+//   * grouped scales where the streaming kernel shares k as well (up to half the SMs have a tile), and one scale per row with too few
+//     tiles for the plain pair form: from 8 steps on.  2048 x 1024 at 128 tokens 8.8 / 8.4 / 10.5 -> 6.7 / 6.5 / 6.5, 896 x 4864 at 256
+//     13.8 / 14.0 / 17.7 -> 10.0 / 9.4 / 9.6, 4096 x 14336 at 128 (three pairs a tile) 46 / 40 / 45 -> 23 / 21 / 22
+//   * where that is one wave without shares: from 18 steps on with three pairs (5632 x 2048 at 128 tokens, 16 steps: 10.1 / 9.8 / 9.3
+//     -> 10.0 / 9.7 / 9.8; 5376 x 2304, 18 steps: 10.8 / 10.4 / 10.0 -> 9.9 / 9.7 / 9.8), from 24 with two (2048 x 2048 at 384: 10.0 /
+//     9.8 / 9.3 -> 10.2 / 10.0 / 10.0; 4096 x 3072 at 256, 24 steps: 13.5 / 13.4 / 12.7 -> 13.0 / 12.3 / 12.4; 4096 x 14336 at 256:
+//     66 / 59 / 45 -> 32 / 30 / 30)
+// The same for the form with the activation, whose result is the plain form's to the bit (5632 x 2048 at 65 tokens 13.6 -> 9.1).  Sums
+// in order of k, in fp32; error against 64 bits of seven shapes as before, up to 0.05 % smaller per row (shorter accumulations).
+static int qp_splits(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k, int64_t* part) {
+  const int64_t tiles = cdiv64(M, kQpTokens) * cdiv64(N, 2 * kBlockW), steps = cdiv64(K, kQpStepK), sms = b2l_num_sms();
+  if (M <= 64 || sms < 132) return 1;
+  const bool one_part = group_k >= K ? tiles >= 16 : cdiv64(M, 64) * cdiv64(N, kBlockW) > sms / 2;
+  int64_t unit = group_k >= K ? 1 : group_k / kQpStepK;
+  if (qk == Q_INT4 && unit % 2 != 0) unit *= 2;
+  for (int s = 4; s > 1; --s) {
+    if (tiles > (s == 4 ? 15 : s == 3 ? 22 : 33) || steps < (!one_part ? 8 : s == 2 ? 24 : 18)) continue;
+    *part = cdiv64(cdiv64(steps, s), unit) * unit;
+    if ((s - 1) * *part < steps) return s;
+  }
+  return 1;
+}
+
+// Where the pair kernel is the faster one: with shared tiles as above, else (both kernels measured over 72 - 512 tokens, eight projection shapes, int4 with and
 // without the activation and fp8 in blocks): as soon as the streaming kernel's 128 x 64 tiles need a second wave.  int4, us,
 // streaming -> pair: one wave, 6144 x 4096 at 128 tokens 17 / 21, 4096 x 14336 at 72 45 / 64 (at 256, 66 / 64); two, 6144 x
 // 4096 at 256 33 -> 21, 9728 x 896 at 192 (two waves of pair tiles as well) 13.8 -> 10.8; five against four, 28672 x 4096 at 192
@@ -533,6 +621,8 @@ bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k)
   if (qk == Q_INT4 && K % kQpStepK != 0) return false;      // the packed tables are read per 128 k
   const int64_t sms = b2l_num_sms();
   const int64_t tiles = cdiv64(M, kQpTokens) * cdiv64(N, 2 * kBlockW);
+  int64_t part;
+  if (qp_splits(qk, M, N, K, group_k, &part) > 1) return true;
   if (group_k >= K) return M > 64 ? tiles >= 16 : qk != Q_INT4 && (tiles >= 40 || (tiles >= 16 && K <= 4096));
   if (M <= 64) return false;
   return cdiv64(M, 64) * cdiv64(N, kBlockW) > sms;
@@ -574,6 +664,17 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
   rc = b2l_make_tmap_2d(&tx, x, TMA_F16, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, kQpTokens / 2, 64, true);
   if (rc != B2L_OK) return rc;
   if (quant_wide_wanted(qk, M, N)) return quant_wide_gemm(qk, p, tw, tx, swiglu, st);
+  int64_t part = 0;
+  const int splits = qp_splits(qk, M, N, K, group_k, &part);
+  p.split_steps = (int)part;
+#define QP_SPLIT(QK, EPI)                                      \
+  (splits == 4 ? launch_qp_split<QK, EPI, 4>(tw, tx, p, st)    \
+               : splits == 3 ? launch_qp_split<QK, EPI, 3>(tw, tx, p, st) : launch_qp_split<QK, EPI, 2>(tw, tx, p, st))
+  if (splits > 1) {
+    if (qk == Q_INT4) return swiglu ? QP_SPLIT(Q_INT4, 1) : QP_SPLIT(Q_INT4, 0);
+    return qk == Q_FP8 ? QP_SPLIT(Q_FP8, 0) : QP_SPLIT(Q_INT8, 0);
+  }
+#undef QP_SPLIT
   if (qk == Q_INT4) return swiglu ? launch_qp<Q_INT4, 1>(tw, tx, p, grid, st) : launch_qp<Q_INT4, 0>(tw, tx, p, grid, st);
   if (M <= 64)
     return qk == Q_FP8 ? launch_qp<Q_FP8, 0, QP_PLAIN, 64>(tw, tx, p, grid, st) : launch_qp<Q_INT8, 0, QP_PLAIN, 64>(tw, tx, p, grid, st);

@@ -17,6 +17,7 @@ struct QuantPairParams {
   const __half* row_weights;                         // grouped down projection: routing weight by slot
   int M, N, steps, seg_steps, groups, m_tiles, n_tiles;      // filled by quant_pair_gemm (groups: pitch of the int4 tables)
   int vec;                                           // y in stores of four outputs
+  int split_steps;                                   // a tile shared by several pairs: steps of each
   int tiles, split_from;                             // wide tiles: their number, and the first that is cut in two
 };
 

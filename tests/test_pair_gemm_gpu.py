@@ -354,3 +354,27 @@ def test_linear_token_tiles_and_splits(m, n, k):
 @pytest.mark.parametrize("m,n,k", PLAN_EDGES)
 def test_int8_token_tiles_and_splits(m, n, k):
     test_int8_pair_tiles(m, n, k, True)
+
+
+# ---- several pairs on a tile (csrc/gemm_quant_pair.cu): four up to 14 tiles, two up to 32; the last part shorter, a k that no four
+# parts share, tokens that end within the four a thread stores, a tile of one half (64 tokens) or less
+SPLIT_EDGES = [(65, 2560, 2176), (129, 1302, 4864), (100, 8192, 1152), (200, 4096, 1408), (500, 1730, 2048), (67, 256, 16384),
+               (257, 2600, 1024)]
+
+
+@pytest.mark.parametrize("m,n,k", SPLIT_EDGES)
+@pytest.mark.parametrize("group", [128, 256, 0])
+@pytest.mark.parametrize("bias", [None, torch.float16, torch.float32])
+def test_int4_shared_tiles(m, n, k, group, bias):
+    test_int4_pair_tiles(m, n, k, group or k, bias)
+
+
+@pytest.mark.parametrize("m,n,k", SPLIT_EDGES)
+def test_int4_shared_swiglu_is_gemm_then_swiglu(m, n, k):
+    test_int4_pair_swiglu_is_gemm_then_swiglu(m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", SPLIT_EDGES + [(300, 1000, 2000)])
+@pytest.mark.parametrize("fmt", ["fp8_block", "fp8_channel", "int8_channel", "int8_group_n"])
+def test_w8_shared_tiles(m, n, k, fmt):
+    test_w8_pair_tiles(m, n, k, fmt)
