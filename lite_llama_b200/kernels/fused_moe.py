@@ -89,8 +89,11 @@ def _moe_gemm(a, w, c, scale, kind, topk_weights, sorted_ids, expert_ids, num_po
 
 def _pair_tile(slots: int, num_experts: int) -> int:
     """Rows of a tile of the pair GEMMs (csrc/gemm_quant_pair.cu): 64 leave room for more conversion stages, 128 convert an
-    expert's weights once for twice the rows.  The line is where an expert's run rarely exceeds 64 rows."""
-    return 64 if slots <= 32 * num_experts else 128
+    expert's weights once for twice the rows.  Where the line lies: up to 48 rows per expert on average 64 is the faster one
+    however the rows fall (128 experts of 2048 x 768 fp8, top 8, us for 128 -> 64 rows: 40 each 186 -> 153, 48 each 197 -> 168,
+    between 10 and 370 of them 197 -> 179; 8 experts of 4096 x 2048, 48 each 64 -> 58); from 52 on it depends on how many
+    experts exceed 64 (8 experts, two of them over: 64 -> 75), at 64 level, beyond 128 wins (80 each 210 / 273)."""
+    return 64 if slots <= 48 * num_experts else 128
 
 
 def _pair_gemm_takes(kind: int, hidden: int, intermediate: int, group_k: int, w1: torch.Tensor, w2: torch.Tensor) -> bool:

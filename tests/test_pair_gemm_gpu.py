@@ -378,3 +378,9 @@ def test_int4_shared_swiglu_is_gemm_then_swiglu(m, n, k):
 @pytest.mark.parametrize("fmt", ["fp8_block", "fp8_channel", "int8_channel", "int8_group_n"])
 def test_w8_shared_tiles(m, n, k, fmt):
     test_w8_pair_tiles(m, n, k, fmt)
+
+
+@pytest.mark.parametrize("idle", [5, 7])      # 52 and 46 rows per expert: either side of the line between tiles of 128 and 64 rows
+@pytest.mark.parametrize("fmt", ["fp8", "int8"])
+def test_experts_either_side_of_the_smaller_tile(fmt, idle):
+    test_experts_with_runs_around_the_tile(fmt, 1024, 384, 128, 128, idle)
