@@ -604,8 +604,8 @@ static int qp_splits(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k, i
   return 1;
 }
 
-// Where the pair kernel is the faster one: with shared tiles as above, else (both kernels measured over 72 - 512 tokens, eight projection shapes, int4 with and
-// without the activation and fp8 in blocks): as soon as the streaming kernel's 128 x 64 tiles need a second wave.  int4, us,
+// Where the pair kernel is the faster one: with shared tiles as above, else (both kernels measured over 72 - 512 tokens, eight
+// projection shapes, int4 with and without the activation and fp8 in blocks) as soon as the streaming kernel's 128 x 64 tiles need a second wave.  int4, us,
 // streaming -> pair: one wave, 6144 x 4096 at 128 tokens 17 / 21, 4096 x 14336 at 72 45 / 64 (at 256, 66 / 64); two, 6144 x
 // 4096 at 256 33 -> 21, 9728 x 896 at 192 (two waves of pair tiles as well) 13.8 -> 10.8; five against four, 28672 x 4096 at 192
 // 94 -> 75; at 4096 tokens 1853 -> 900.
