@@ -55,6 +55,7 @@ struct DecodeParams {
 // apart: with these the calls of the other kernels cost the host 0.36 us more (16 bytes; 8.3 -> 8.7 us a call through ctypes)
 struct ShareParams : DecodeParams {
   int2* ws_info;  // first and last CTA of every (kv-head block, batch row); ws_o [head of a block, slots, D]
+  int* ws_cut;    // 1: rows are cut in splits after all, ws_o [B, Hq, splits, D]
   int batch;
   int slots;      // two per CTA
 };
@@ -259,20 +260,17 @@ struct Consumer {
 enum { FD_SPLITS, FD_WHOLE, FD_CLUSTER };
 // one split with tokens
 template <typename T, int D, int FORM>
-__device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* smem, int64_t seq_len, int64_t start) {
+__device__ __forceinline__ void decode_split(const DecodeParams& p, uint8_t* smem, int64_t seq_len, int64_t start, int split, int hblk,
+                                             int b, int64_t req) {
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);   // [kMaxStages]
   uint64_t* empty_bar = full_bar + kMaxStages;              // [kMaxStages]
   uint8_t* stage_base = smem + kStagesAt;
 
-  const int split = blockIdx.x;
-  const int hblk = blockIdx.y;
-  const int b = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nconsumers = p.HB * p.qblocks;      // blockDim.x == (nconsumers + 1) * 32
 
   const int64_t end = (start + p.chunk < seq_len) ? start + p.chunk : seq_len;
   const int ntiles = (int)((end - start + kTT - 1) / kTT);
-  const int64_t req = load_index(p.req_idx, b, p.req_w);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.stages; ++s) {
@@ -423,7 +421,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_split_k
   const int most = p.chunk * kMaxCluster;                   // FD_CLUSTER: tokens that its kMaxCluster splits hold
   const int len = seq_len < most ? (int)seq_len : most;
   if (start < seq_len) {
-    decode_split<T, D, FORM>(p, smem, seq_len, start);
+    decode_split<T, D, FORM>(p, smem, seq_len, start, blockIdx.x, blockIdx.y, blockIdx.z, load_index(p.req_idx, blockIdx.z, p.req_w));
   } else if (FORM != FD_SPLITS && blockIdx.x == 0) {        // an empty row is zero; other empty splits have nothing to contribute
     const int heads = p.HB * p.G;
     for (int i = threadIdx.x; i < heads * (D / 2); i += blockDim.x)
@@ -491,46 +489,25 @@ __global__ void flash_decode_combine_kernel(const DecodeParams p) {
 // of short CTAs on a batch that would fill the chip once, each with the start of its ring (25 splits of 80 tokens per row, 32
 // sequences of 1000 - 2000 tokens: 44 us of 30 at the rate of a copy), and larger splits lose where most rows are short.  Here every
 // CTA adds up the lengths and takes its part of the work there is:
-//   * little of it (as many items of up to kItemMax tiles, of one row each, as CTAs, or fewer): an item each;
+//   * no more splits with tokens than CTAs: a split each, as in the grid of splits, and with its result;
 //   * else an equal share of all tiles of all rows, whatever rows they belong to: one wave, one ring that runs on from row
-//     to row.
-// A CTA that covers a row whole writes its result; else the row's parts go to the workspace (each CTA has at most two: of a row
-// that began before it, and of one that ends after it), and the owner of a row's first tile notes its first and last CTA for
-// the merge.
-constexpr int kShareRows = 1024, kItemMax = 8;
-// tiles per item of a row: at least four of a longer one, whose merge would ask for its parts in several turns
-__device__ __forceinline__ int item_tiles(int tiles, int q) { return q < 4 && tiles > 16 ? 4 : q; }
-// units of a row: items, or (q = 0) tiles
-__device__ __forceinline__ int share_units(int tiles, int q) {
-  if (q == 0) return tiles;
-  const int n = item_tiles(tiles, q);
-  return (unsigned)(tiles + n - 1) / (unsigned)n;
-}
-// the smallest items that there are CTAs for in any case (a row has at most one that is not full), or four tiles where they fit
-__device__ __forceinline__ int share_pick(int tiles, int fours, int rows, int grid) {
-  const int room = grid - rows;
-  int q = 0;
-  if (room > 0 && tiles <= kItemMax * room) q = (unsigned)(tiles + room - 1) / (unsigned)room;
-  if (q == 0 || q > 4) return fours <= grid ? 4 : q;
-  return q < 2 ? 2 : q;
-}
+//     to row.  A CTA that covers a row whole writes its result; else the row's parts go to the workspace (each CTA has at most
+//     two: of a row that began before it, and of one that ends after it), and the owner of a row's first tile notes its first
+//     and last CTA for the merge.  A row's bits then depend on where the shares part it, hence on the other rows' lengths.
 struct RowPart { int b, blk, first, last, tiles, cta_last; };   // tiles first .. last - 1 of a row of `tiles`; its last CTA
 
 // the parts of rows that a CTA works on, in turn
 struct ShareWalk {
-  const int* prefix;
-  int batch, all, t, hi, b, blk, ctas, total, items;
-  // prefix: items (of the `items_` scheme) or, with 0, tiles of the rows before, [batch + 1]
-  __device__ __forceinline__ ShareWalk(const int* prefix_, int items_, int batch_, int nblk, int cta, int grid)
-      : prefix(prefix_), batch(batch_), items(items_) {
+  const int* prefix;                              // tiles of the rows before, [batch + 1]
+  int batch, all, t, hi, b, blk, grid, total;
+  __device__ __forceinline__ ShareWalk(const int* prefix_, int batch_, int nblk, int cta, int grid_)
+      : prefix(prefix_), batch(batch_), grid(grid_) {
     all = prefix[batch];                          // of one kv-head block
     total = all * nblk;
-    ctas = items ? total : grid;
-    t = cta < ctas ? (items ? cta : (int)((unsigned long long)cta * (unsigned)total / (unsigned)ctas)) : 0;
-    hi = cta < ctas ? (items ? cta + 1 : (int)((unsigned long long)(cta + 1) * (unsigned)total / (unsigned)ctas)) : 0;
-    b = blk = 0;
-    if (t >= hi) return;
+    t = (int)((unsigned long long)cta * (unsigned)total / (unsigned)grid);
+    hi = (int)((unsigned long long)(cta + 1) * (unsigned)total / (unsigned)grid);
     blk = (unsigned)t / (unsigned)all;
+    b = 0;
     const int rem = t - blk * all;
     // the last row that begins at or before rem (empty rows have nothing): 32 at a time, the whole warp
     const int lane = threadIdx.x & 31;
@@ -540,7 +517,7 @@ struct ShareWalk {
       if (step == 1) break;
     }
   }
-  __device__ __forceinline__ bool next(const int* lens, RowPart& r) {
+  __device__ __forceinline__ bool next(RowPart& r) {
     while (t < hi) {
       const int begin = blk * all + prefix[b], end = blk * all + prefix[b + 1], from = t - begin;
       r.b = b;
@@ -548,18 +525,10 @@ struct ShareWalk {
       if (++b == batch) { b = 0; ++blk; }
       if (end <= t) continue;                     // an empty row
       t = end < hi ? end : hi;
-      if (items) {
-        r.tiles = (lens[r.b] + kTT - 1) / kTT;
-        const int q = item_tiles(r.tiles, items);
-        r.first = from * q;
-        r.last = r.first + q < r.tiles ? r.first + q : r.tiles;
-        r.cta_last = end - 1;
-      } else {
-        r.tiles = end - begin;
-        r.first = from;
-        r.last = t - begin;
-        r.cta_last = r.last == r.tiles ? 0 : (int)(((unsigned long long)end * (unsigned)ctas - 1u) / (unsigned)total);   // 0: this one
-      }
+      r.tiles = end - begin;
+      r.first = from;
+      r.last = t - begin;
+      r.cta_last = r.last == r.tiles ? 0 : (int)(((unsigned long long)end * (unsigned)grid - 1u) / (unsigned)total);   // 0: this one
       return true;
     }
     return false;
@@ -570,7 +539,8 @@ template <typename T, int D>
 __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_kernel(const ShareParams p) {
   pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ int warp_sum[3][kMaxConsumers + 1];
+  __shared__ int warp_sum[2][kMaxConsumers + 1];
+  __shared__ int found[2];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem);   // [kMaxStages]
   uint64_t* empty_bar = full_bar + kMaxStages;              // [kMaxStages]
   uint8_t* stage_base = smem + kStagesAt;
@@ -581,95 +551,73 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_
   int* reqs = lens + p.batch;                                                   // [batch]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nconsumers = p.HB * p.qblocks;      // blockDim.x == (nconsumers + 1) * 32
+  const int nblk = p.Hkv / p.HB, grid = (int)gridDim.x, cta = blockIdx.x;
 
+  // ---- splits with tokens; a thread owns neighbouring rows ----
+  const int most = p.chunk * p.splits;          // tokens of a row that the call's bound lets count
+  const int per = (p.batch + blockDim.x - 1) / blockDim.x, r_lo = threadIdx.x * per;
+  const int r_hi = r_lo + per < p.batch ? r_lo + per : p.batch;
+  auto units = [](int len, int tokens) { return (int)((unsigned)(len + tokens - 1) / (unsigned)tokens); };
+  // of the rows before this thread's, and of all rows
+  auto sum_before = [&](int own, int* sums, int& all) {
+    int upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += x;
+    }
+    if (lane == 31) sums[warp] = upto;
+    __syncthreads();
+    const int of_warp = lane <= nconsumers ? sums[lane] : 0;
+    all = __reduce_add_sync(0xffffffffu, of_warp);
+    return upto - own + (int)__reduce_add_sync(0xffffffffu, lane < warp ? of_warp : 0);
+  };
+  int own = 0, all;
+#pragma unroll 1
+  for (int r = r_lo; r < r_hi; ++r) {
+    const int64_t n = load_index(p.seq_len, r, p.len_w);
+    reqs[r] = (int)load_index(p.req_idx, r, p.req_w);
+    lens[r] = n > most ? most : n > 0 ? (int)n : 0;
+    own += units(lens[r], p.chunk);
+  }
+  int at = sum_before(own, warp_sum[0], all);
+  if (cta == 0 && threadIdx.x == 0) *p.ws_cut = nblk * all <= grid;
+  if (nblk * all <= grid) {
+    if (cta >= nblk * all) return;
+    const int hblk = nblk == 1 ? 0 : (unsigned)cta / (unsigned)all;
+    int split = cta - hblk * all - at;          // of this thread's rows
+    if (split >= 0 && split < own) {
+      int r = r_lo;
+      for (int n; r + 1 < r_hi && split >= (n = units(lens[r], p.chunk)); ++r) split -= n;
+      found[0] = r;
+      found[1] = split;
+    }
+    __syncthreads();
+    const int b = found[0];
+    split = found[1];
+    decode_split<T, D, FD_SPLITS>(p, smem, lens[b], (int64_t)split * p.chunk, split, hblk, b, reqs[b]);
+    return;
+  }
+
+  // ---- tiles of the rows before each ----
+  own = 0;
+  for (int r = r_lo; r < r_hi; ++r) own += units(lens[r], kTT);
+  at = sum_before(own, warp_sum[1], all);
+  for (int r = r_lo; r < r_hi; ++r) {
+    prefix[r] = at;
+    at += units(lens[r], kTT);
+  }
   if (threadIdx.x == 0) {
+    prefix[p.batch] = all;
     for (int s = 0; s < p.stages; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], nconsumers);
     }
     mbar_fence_init();
   }
-  // ---- tiles of all rows, and the units of the rows before each ----
-  const int most = p.chunk * p.splits;          // tokens of a row that the call's bound lets count
-  const int nblk = p.Hkv / p.HB, grid = (int)gridDim.x;
-  auto load_row = [&](int r) {                  // tiles
-    const int64_t n = load_index(p.seq_len, r, p.len_w);
-    reqs[r] = (int)load_index(p.req_idx, r, p.req_w);
-    const int len = n > most ? most : n > 0 ? (int)n : 0;
-    lens[r] = len;
-    return (len + kTT - 1) / kTT;
-  };
-  auto scan = [&](int v) {                      // inclusive, over the warp
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += x;
-    }
-    return v;
-  };
-  int items;
-  if (p.batch <= 128) {
-    // every warp for itself (the same values go to the same places): one barrier in all, and small steps feel each
-    const int per = (p.batch + 31) / 32, r_lo = lane * per;
-    const int r_hi = r_lo + per < p.batch ? r_lo + per : p.batch;
-    int own = 0, fours = 0, units = 0;
-    for (int r = r_lo; r < r_hi; ++r) {
-      const int tiles = load_row(r);
-      own += tiles;
-      fours += (tiles + 3) >> 2;
-    }
-    items = share_pick(nblk * __reduce_add_sync(0xffffffffu, own), nblk * __reduce_add_sync(0xffffffffu, fours), nblk * p.batch, grid);
-    for (int r = r_lo; r < r_hi; ++r) units += share_units((lens[r] + kTT - 1) / kTT, items);
-    int at = scan(units) - units;
-    for (int r = r_lo; r < r_hi; ++r) {
-      at += share_units((lens[r] + kTT - 1) / kTT, items);
-      prefix[r + 1] = at;
-    }
-    if (lane == 0) prefix[0] = 0;
-  } else {
-    // a thread owns neighbouring rows
-    const int per = (p.batch + blockDim.x - 1) / blockDim.x, r_lo = threadIdx.x * per;
-    const int r_hi = r_lo + per < p.batch ? r_lo + per : p.batch;
-    int own = 0, fours = 0, all = 0, all_fours = 0;
-    for (int r = r_lo; r < r_hi; ++r) {
-      const int tiles = load_row(r);
-      own += tiles;
-      fours += (tiles + 3) >> 2;
-    }
-    own = __reduce_add_sync(0xffffffffu, own);
-    fours = __reduce_add_sync(0xffffffffu, fours);
-    if (lane == 0) {
-      warp_sum[0][warp] = own;
-      warp_sum[2][warp] = fours;
-    }
-    __syncthreads();
-    for (int w = 0; w <= nconsumers; ++w) {
-      all += warp_sum[0][w];
-      all_fours += warp_sum[2][w];
-    }
-    items = share_pick(nblk * all, nblk * all_fours, nblk * p.batch, grid);
-    own = 0;
-    for (int r = r_lo; r < r_hi; ++r) own += share_units((lens[r] + kTT - 1) / kTT, items);
-    const int upto = scan(own);
-    if (lane == 31) warp_sum[1][warp] = upto;
-    __syncthreads();
-    int at = upto - own;
-    for (int w = 0; w < warp; ++w) at += warp_sum[1][w];
-    for (int r = r_lo; r < r_hi; ++r) {
-      prefix[r] = at;
-      at += share_units((lens[r] + kTT - 1) / kTT, items);
-    }
-    if (r_lo < p.batch && r_hi == p.batch) prefix[p.batch] = at;
-  }
   __syncthreads();
 
-  const int cta = blockIdx.x;
-  for (int b = cta; b < p.batch; b += gridDim.x)            // an empty row is zero
-    if (lens[b] == 0)
-      for (int i = threadIdx.x; i < p.Hq * (D / 2); i += blockDim.x)
-        *reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)(i / (D / 2)) * p.o_hs + 2 * (i % (D / 2))) = 0u;
-
-  ShareWalk walk(prefix, items, p.batch, nblk, cta, grid);
+  ShareWalk walk(prefix, p.batch, nblk, cta, grid);
   RowPart r;
   int s = 0;
   uint32_t phase = 0;
@@ -684,7 +632,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_
       pos = pos < lens[at.b] ? pos : lens[at.b] - 1;
       return p.table[(int64_t)reqs[at.b] * p.tab_bs + (int64_t)pos * p.tab_ss];
     };
-    bool more = walk.next(lens, r);
+    bool more = walk.next(r);
     int tile = more ? r.first : 0;
     int64_t row_next = more ? entry(r, tile) : 0;
     while (more) {
@@ -693,7 +641,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_
       const bool begins = tile == 0;
       // the next tile's entry is on its way while this one waits for its stage
       if (++tile == at.last) {
-        more = walk.next(lens, r);
+        more = walk.next(r);
         tile = more ? r.first : 0;
       }
       if (more) row_next = entry(r, tile);
@@ -730,7 +678,7 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_
     const uint32_t ka = ((mj >> 1) * 8 + r8) * PITCH + k_off + (mj & 1) * 16;
     const uint32_t va = ((mj & 1) * 8 + r8) * PITCH + v_off + (mj >> 1) * 16;
     Consumer<T, D> c;
-    while (walk.next(lens, r)) {
+    while (walk.next(r)) {
       const int kvh = r.blk * p.HB + hl;
       const int64_t end = lens[r.b];
       c.begin(p, r.b, kvh, hq0, hq1, tq);
@@ -760,17 +708,33 @@ __global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_
   }
 }
 
-// Merge of the rows that several shares met in, in token order.  Bound by latency: the statistics of up to 32 parts are read side by
+// Merge of the rows that several CTAs met in, in token order.  Bound by latency: the statistics of up to 32 parts are read side by
 // side, and eight partial rows are requested before the first is added.
 template <typename T, int D>
 __global__ void flash_decode_shares_merge_kernel(const ShareParams p) {
   pdl_prologue();
   const int b = blockIdx.x, head = blockIdx.y, heads = p.HB * p.G, blk = head / heads, local = head - blk * heads;
-  const int2 who = __ldcg(p.ws_info + blk * p.batch + b);   // (of an empty row: an earlier call's)
+  const int2 who = __ldcg(p.ws_info + blk * p.batch + b);   // of shares (else, and of an empty row: an earlier call's)
+  const bool splits = __ldcg(p.ws_cut) != 0;
   const int64_t len = load_index(p.seq_len, b, p.len_w);
-  const int n = who.y - who.x + 1;
-  if (len <= 0 || n < 2) return;                            // zeros, or written by its only CTA
-  auto part = [&](int i) { return (int64_t)local * p.slots + (i == 0 ? 2 * who.x + 1 : 2 * (who.x + i)); };
+  T* out = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_bs + (int64_t)head * p.o_hs + threadIdx.x;
+  if (len <= 0) {
+    *out = from_f32<T>(0.f);
+    return;
+  }
+  int n = who.y - who.x + 1;
+  if (splits) {
+    const int64_t all = (len + p.chunk - 1) / p.chunk;
+    n = all < p.splits ? (int)all : p.splits;
+  } else if (n < 2) {
+    return;                                                 // written by its only CTA
+  }
+  const int64_t base = splits ? ((int64_t)b * p.Hq + head) * p.splits : (int64_t)local * p.slots + 2 * who.x;
+  auto part = [&](int i) { return base + (splits ? i : i == 0 ? 1 : 2 * i); };
+  if (n == 1) {                                             // most rows of a step far below its bound
+    *out = from_f32<T>(__ldcg(p.ws_o + base * D + threadIdx.x));
+    return;
+  }
   const int lane = threadIdx.x & 31;
   const int d = threadIdx.x;                                // blockDim.x == D
   auto ask = [&](float (&v)[8], int from) {
@@ -800,7 +764,7 @@ __global__ void flash_decode_shares_merge_kernel(const ShareParams p) {
     ask(v, from);
     add(v, from);
   }
-  reinterpret_cast<T*>(p.out)[(int64_t)b * p.o_bs + (int64_t)head * p.o_hs + d] = from_f32<T>(acc / L);
+  *out = from_f32<T>(acc / L);
 }
 
 struct Plan { int splits, chunk, qblocks, HB, stages, smem; bool cluster; int share_grid, share_smem; };   // share_grid 0: not the shares' kernel
@@ -843,14 +807,15 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
 }
 
 // Steps that would take several waves of CTAs of which an SM holds one or two, whose rings of large stages start anew with each.
-// us in a graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 35.8 -> 29.8, of 500 - 1000 27.2 ->
-// 24.0, of 1000 - 2000 50.4 -> 41.0, 256 of 200 58.5 -> 50.5; 32 kv heads, 32 of 250 - 480 54 -> 45; 4 kv heads, 32 of 1000 - 2000 30.0 ->
-// 25.2, 64 of 1000 35.1 -> 30.9, 128 of 2000 105 -> 94.  The lengths are not known here: a step far below its bound pays up to 1.7 us for
-// adding them up (8 kv heads, one of 1000 among 31 of 50 11.0 -> 12.5, 32 of 200 11.3 -> 12.1; 4 kv heads, 32 of 40 under 2000 8.8 -> 9.8;
-// with 20 tiles per SM and more mostly level or faster).  Below 13 tiles per CTA, or with more CTAs to an SM, the splits stay: 8 kv
-// heads 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
+// us in a graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 35.8 -> 29.7, of 500 - 1000 27.0 ->
+// 23.6, of 1000 - 2000 50.6 -> 40.8, 256 of 200 58.7 -> 50.2; 32 kv heads, 64 of 250 - 500 94 -> 84; 4 kv heads, 32 of 1000 - 2000 29.8 ->
+// 24.8, 64 of 1000 35.1 -> 31.1.  The lengths are not known here.  Far below the bound the splits that have tokens go to a CTA each,
+// which is level or faster in most (8 kv heads, one of 1000 among 31 of 50 11.1 -> 10.5, 32 of 200 11.3 -> 11.0; 4 kv heads, 32 of 40 under
+// 2000 8.7 -> 8.9; 32 kv heads, one of 1600 under 8000 13.1 -> 12.3; slowest: 8 of 800 under 4000 11.1 -> 11.9, 4 kv heads, one of 2000
+// among 31 of 100 12.3 -> 13.3).  Below 13 tiles per CTA, or with more CTAs to an SM, the splits stay: 8 kv heads 32 x 480 16.7 against
+// 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
 void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int smem_cap) {
-  if (pl.splits < 2 || batch > kShareRows || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 30)) return;
+  if (pl.splits < 2 || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 26)) return;
   pl.share_smem = pl.smem + (int)(3 * batch + 1) * 4;
   if (pl.share_smem > smem_cap) return;
   const int per_sm = (smem_cap + 256) / (pl.share_smem + 1024);
@@ -895,9 +860,14 @@ Plan make_plan(int64_t batch, int Hq, int Hkv, int D, int64_t max_len) {
   plan_shares(pl, batch, Hkv, D, tiles, smem_cap);
   return pl;
 }
-int64_t share_bytes(const Plan& pl, int64_t batch, int G, int Hkv, int D) {
-  if (pl.share_grid == 0) return 0;
-  return (batch * (Hkv / pl.HB) * 8 + 15) / 16 * 16 + 2ll * pl.share_grid * pl.HB * G * (D + 1) * 4 + 16;
+int64_t split_rows(const Plan& pl, int64_t batch, int Hq) { return batch * Hq * pl.splits; }
+// partial rows of either cut, and behind them the notes
+int64_t share_rows(const Plan& pl, int64_t batch, int Hq, int Hkv) {
+  const int64_t shares = 2ll * pl.share_grid * (Hq / Hkv) * pl.HB, splits = split_rows(pl, batch, Hq);
+  return shares > splits ? shares : splits;
+}
+int64_t share_bytes(const Plan& pl, int64_t batch, int Hq, int Hkv, int D) {
+  return share_rows(pl, batch, Hq, Hkv) * (D + 1) * 4 + 8 + batch * (Hkv / pl.HB) * 8 + 16;
 }
 
 template <typename T, int D>
@@ -958,14 +928,26 @@ int launch_decode(const ShareParams& p, const Plan& pl, int64_t batch, cudaStrea
 
 }  // namespace
 
+// What a call does with these sizes, for tests and tools (no GPU work): out[0..4] = {form: 0 a grid of splits, 1 clusters, 2 shares;
+// splits per row; tokens per split; CTAs of the shares' grid; blocks of kv heads}
+extern "C" int b2l_flash_decoding_plan(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t max_seq_len, int* out) {
+  B2L_REQUIRE(out && batch > 0 && num_q_heads > 0 && num_kv_heads > 0 && num_q_heads % num_kv_heads == 0, "flash_decoding_plan: bad arguments");
+  const Plan pl = make_plan(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
+  out[0] = pl.cluster ? 1 : pl.share_grid != 0 ? 2 : 0;
+  out[1] = pl.splits;
+  out[2] = pl.chunk;
+  out[3] = pl.share_grid;
+  out[4] = num_kv_heads / pl.HB;
+  return B2L_OK;
+}
+
 extern "C" int64_t b2l_flash_decoding_workspace_bytes(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim,
                                                        int64_t max_seq_len) {
   if (batch <= 0 || num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads != 0) return 0;
   Plan pl = make_plan(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
   if (pl.splits <= 1 || pl.cluster) return 16;
-  const int64_t split_bytes = (int64_t)batch * num_q_heads * pl.splits * (head_dim + 1) * 4 + 16;
-  const int64_t shares = share_bytes(pl, batch, num_q_heads / num_kv_heads, num_kv_heads, head_dim);
-  return shares > split_bytes ? shares : split_bytes;
+  if (pl.share_grid != 0) return share_bytes(pl, batch, num_q_heads, num_kv_heads, head_dim);
+  return split_rows(pl, batch, num_q_heads) * (head_dim + 1) * 4 + 16;
 }
 
 extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache, const void* v_cache,
@@ -1014,18 +996,19 @@ extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache,
   // the split CTAs merge their own results when the caller provides zeroed tickets (one per batch row x head block)
   p.tickets = (tickets && num_tickets >= batch * (num_kv_heads / pl.HB)) ? (int*)tickets : nullptr;
   if (pl.splits > 1 && !pl.cluster) {
+    const int64_t rows = split_rows(pl, batch, num_q_heads);
     const int64_t need = b2l_flash_decoding_workspace_bytes(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
     B2L_REQUIRE(workspace && workspace_bytes >= need, "flash_decoding: workspace too small (%lld < %lld)",
                 (long long)workspace_bytes, (long long)need);
     B2L_REQUIRE((uintptr_t)workspace % 16 == 0, "flash_decoding: workspace must be 16-byte aligned");
+    p.ws_o = (float*)workspace;
+    p.ws_lse = p.ws_o + rows * head_dim;
     if (pl.share_grid != 0 && p.tickets == nullptr) {
-      p.ws_info = (int2*)workspace;
+      const int64_t most = share_rows(pl, batch, num_q_heads, num_kv_heads);
       p.slots = 2 * pl.share_grid;
-      p.ws_o = (float*)((char*)workspace + (batch * (num_kv_heads / pl.HB) * 8 + 15) / 16 * 16);
-      p.ws_lse = p.ws_o + 2ll * pl.share_grid * pl.HB * p.G * head_dim;
-    } else {
-      p.ws_o = (float*)workspace;
-      p.ws_lse = p.ws_o + (int64_t)batch * num_q_heads * pl.splits * head_dim;
+      p.ws_lse = p.ws_o + most * head_dim;
+      p.ws_info = (int2*)(p.ws_lse + (most + 1) / 2 * 2);
+      p.ws_cut = (int*)(p.ws_info + batch * (num_kv_heads / pl.HB));
     }
   }
   cudaStream_t st = (cudaStream_t)stream;
