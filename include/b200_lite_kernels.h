@@ -108,8 +108,9 @@ int b2l_update_kv_index(void* table, const void* b_req_idx, int req_width, const
 int64_t b2l_flash_decoding_workspace_bytes(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim,
                                            int64_t max_seq_len);
 /* launch plan of a call, for tests and tools (no GPU work): out[5] = {form (0 a grid of splits, 1 clusters, 2 shares),
- * splits per row, tokens per split, CTAs of the shares' grid, blocks of kv heads}. */
-int b2l_flash_decoding_plan(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t max_seq_len, int* out);
+ * splits per row, tokens per split, CTAs of the shares' grid, blocks of kv heads}.  The trailing argument is unused. */
+int b2l_flash_decoding_plan(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t max_seq_len, int* out,
+                            void* reserved);
 int b2l_flash_decoding(void* out, const void* q, const void* k_cache, const void* v_cache,
                        const void* b_req_tokens_table, const void* b_req_idx, int req_idx_width,
                        const void* b_seq_len, int seq_len_width, int64_t batch, int num_q_heads, int num_kv_heads,

@@ -930,7 +930,8 @@ int launch_decode(const ShareParams& p, const Plan& pl, int64_t batch, cudaStrea
 
 // What a call does with these sizes, for tests and tools (no GPU work): out[0..4] = {form: 0 a grid of splits, 1 clusters, 2 shares;
 // splits per row; tokens per split; CTAs of the shares' grid; blocks of kv heads}
-extern "C" int b2l_flash_decoding_plan(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t max_seq_len, int* out) {
+extern "C" int b2l_flash_decoding_plan(int64_t batch, int num_q_heads, int num_kv_heads, int head_dim, int64_t max_seq_len, int* out,
+                                       void* /*reserved*/) {
   B2L_REQUIRE(out && batch > 0 && num_q_heads > 0 && num_kv_heads > 0 && num_q_heads % num_kv_heads == 0, "flash_decoding_plan: bad arguments");
   const Plan pl = make_plan(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
   out[0] = pl.cluster ? 1 : pl.share_grid != 0 ? 2 : 0;

@@ -42,7 +42,7 @@ class Plan(NamedTuple):
 
 def plan(batch: int, heads: int, kv_heads: int, d: int, longest: int) -> Plan:
     out = (ctypes.c_int * 5)()
-    _lib.check(_lib.load().b2l_flash_decoding_plan(batch, heads, kv_heads, d, longest, out))
+    _lib.check(_lib.load().b2l_flash_decoding_plan(batch, heads, kv_heads, d, longest, out, None))
     return Plan(*out)
 
 
