@@ -31,6 +31,7 @@ constexpr int kTT = 16;            // tokens per pipeline stage (one m16n8k16 k-
 constexpr int kMaxConsumers = 8;
 constexpr int kMaxStages = 4;
 constexpr int kMaxCluster = 8;
+constexpr float kNear = 4.f;       // Consumer::tile
 constexpr int kStagesAt = 128;     // bytes of shared memory before the stages: their barriers
 
 struct DecodeParams {
@@ -130,7 +131,8 @@ template <typename T, int D>
 struct Consumer {
   uint32_t qf[D / 16][4];             // A operand, m16 x k16 per step; rows = query heads of this KV group
   float o[D / 8][4];
-  float m_run[2], l_run[2];
+  float m_run[2], l_run[2];           // what the sums are relative to (log2), and the sums of the probabilities
+  float top[2];                       // largest score so far
   bool v0, v1;                        // rows g and g + 8 exist
 
   __device__ __forceinline__ void begin(const DecodeParams& p, int b, int kvh, int hq0, int hq1, int tq) {
@@ -149,13 +151,15 @@ struct Consumer {
     }
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    m_run[0] = m_run[1] = -INFINITY;
+    m_run[0] = m_run[1] = top[0] = top[1] = -INFINITY;
     l_run[0] = l_run[1] = 0.f;
   }
   // the tile at shared address sb, tokens tbase .. of which those before `end` count; ka, va: ldmatrix lane addresses.
-  // REST: what the probabilities lose as 16-bit operands is multiplied as well.  Of every split the largest probability is 1, which
-  // loses nothing, so rows in few parts would end 2 - 5 % further from the exact result than rows in many; with it they end closer.
-  template <bool REST>
+  // NEAR: probabilities relative to the largest score of the tile, not of all tiles so far, unless that is more than kNear (in log2)
+  // above.  The largest of each tile is then 1, which loses nothing as a 16-bit operand; with one such in a whole part, rows in few
+  // parts end 2 - 5 % further from the exact result than rows in many.  (The rest of each probability as an operand of its own does
+  // better still, but 0 and what is below 0 turn an infinite value into NaN.)  Sums grow by up to 2^kNear.
+  template <bool NEAR>
   __device__ __forceinline__ void tile(const DecodeParams& p, uint32_t sb, uint32_t ka, uint32_t va, int64_t tbase, int64_t end, int tq) {
     // ---- S = Q K^T  (16 heads x 16 tokens) ----
     float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -184,7 +188,8 @@ struct Consumer {
     for (int r2 = 0; r2 < 2; ++r2) {
       mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 1));
       mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 2));
-      const float mnew = fmaxf(m_run[r2], mx[r2]);
+      top[r2] = fmaxf(top[r2], mx[r2]);
+      const float mnew = NEAR ? fmaxf(mx[r2], top[r2] - kNear) : top[r2];
       base[r2] = mnew == -INFINITY ? 0.f : mnew;   // avoid (-inf) - (-inf)
       alpha[r2] = fast_exp2(m_run[r2] - base[r2]);
       m_run[r2] = mnew;
@@ -212,24 +217,12 @@ struct Consumer {
     pf[1] = pack2<T>(sc[0][2], sc[0][3]);
     pf[2] = pack2<T>(sc[1][0], sc[1][1]);
     pf[3] = pack2<T>(sc[1][2], sc[1][3]);
-    uint32_t rest[4];
-    if (REST) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const typename Vec2<T>::type h = *reinterpret_cast<const typename Vec2<T>::type*>(&pf[i]);
-        rest[i] = pack2<T>(sc[i >> 1][2 * (i & 1)] - to_f32(h.x), sc[i >> 1][2 * (i & 1) + 1] - to_f32(h.y));
-      }
-    }
 #pragma unroll
     for (int dn = 0; dn < D / 16; ++dn) {
       uint32_t bf[4];
       ldmatrix_x4_trans(bf, sb + va + dn * 32);
       mma_m16n8k16<T>(o[2 * dn], pf, bf[0], bf[1]);
       mma_m16n8k16<T>(o[2 * dn + 1], pf, bf[2], bf[3]);
-      if (REST) {
-        mma_m16n8k16<T>(o[2 * dn], rest, bf[0], bf[1]);
-        mma_m16n8k16<T>(o[2 * dn + 1], rest, bf[2], bf[3]);
-      }
     }
   }
   // quad-reduce the row sums (each lane only summed its own 4 columns per tile)

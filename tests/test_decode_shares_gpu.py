@@ -123,3 +123,28 @@ def test_rows_do_not_depend_on_the_others_where_the_splits_fit(heads, kv_heads, 
         assert torch.equal(got, run(*data, lens, bound))
     finally:
         F._FOLD = False
+
+
+@pytest.mark.parametrize("heads,kv_heads,d", HEADS)
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kind", ["full", "few"])
+def test_infinite_values_stay_infinite(heads, kv_heads, d, dtype, kind):
+    """Every probability is one that 16 bits hold, so an infinite value makes its column infinite, and only infinite values of both
+    signs make it NaN; the other columns do not notice."""
+    batch, bound = 32, 2000
+    q, k, v, table, order = inputs(batch, bound, heads, kv_heads, d, dtype)
+    q = q * 0.1
+    lens = lengths(kind, batch, bound)
+    for b, n in enumerate(lens):
+        tokens = table[order[b], torch.randint(0, n - 1, (3,), device="cuda")].long()   # (a last one also stands for those beyond the row)
+        v[tokens, b % kv_heads, b % 7] = math.inf
+        v[tokens, b % kv_heads, b % 7 + 8] = -math.inf
+        if b % 2 and n > 1:
+            v[table[order[b], 0].long(), b % kv_heads, b % 7 + 16] = math.inf
+            v[table[order[b], n - 1].long(), b % kv_heads, b % 7 + 16] = -math.inf
+    assert plan(batch, heads, kv_heads, d, bound).form == SHARES
+    got, want = run(q, k, v, table, order, lens, bound), exact(q, k, v, table, order, lens)
+    assert torch.equal(got.isinf(), want.isinf()) and torch.equal(got.isnan(), want.isnan()) and want.isinf().any()
+    assert torch.equal(got[got.isinf()].double(), want[want.isinf()])
+    ok = want.isfinite()
+    assert ((got[ok].double() - want[ok]).norm() / want[ok].norm()).item() < (2.0**-10 if dtype is torch.float16 else 2.0**-7)
