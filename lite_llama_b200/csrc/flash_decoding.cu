@@ -811,11 +811,15 @@ void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int sme
   if (pl.splits < 2 || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 26)) return;
   pl.share_smem = pl.smem + (int)(3 * batch + 1) * 4;
   if (pl.share_smem > smem_cap) return;
-  const int per_sm = (smem_cap + 256) / (pl.share_smem + 1024);
+  int per_sm = (smem_cap + 256) / (pl.share_smem + 1024);
   if (per_sm > 2) return;
-  const int grid = b2l_num_sms() * (per_sm > 1 ? per_sm : 1);
-  if (batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * grid) return;
-  pl.share_grid = grid;
+  if (per_sm < 1) per_sm = 1;
+  if (batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * per_sm * b2l_num_sms()) return;
+  // One wave: by registers, too (151, 96 and 72 a thread, handed out in eights), an SM may hold one CTA only, of heads of 128 with two
+  // warps of query heads to a kv head (4 kv heads, 20 query heads each, 32 of 1000 - 2000 tokens, splits 52.9 us, shares in two waves
+  // 46.4, in one 39.2).
+  if (per_sm == 2 && 2 * (pl.HB * pl.qblocks + 1) * 32 * (D == 128 ? 152 : D == 64 ? 96 : 72) > 65536) per_sm = 1;
+  pl.share_grid = per_sm * b2l_num_sms();
 }
 
 // Pure function of host-known sizes => identical inside and outside graph capture.

@@ -46,12 +46,14 @@ def plan(batch: int, heads: int, kv_heads: int, d: int, longest: int) -> Plan:
     return Plan(*out)
 
 
-# on 148 SMs: 13 tiles of 16 tokens per CTA (six with several blocks of kv heads), with one or two CTAs to an SM and two splits or more
+# on 148 SMs: 13 tiles of 16 tokens per CTA (six with several blocks of kv heads), with one or two CTAs to an SM by shared memory and
+# two splits or more; as many CTAs as fit at once, by registers as well (nine warps of heads of 128: one to an SM)
 @pytest.mark.parametrize("batch,heads,kv_heads,d,longest,form,grid", [
     (1, 32, 8, 128, 200, CLUSTER, 0), (1, 32, 8, 128, 2000, SPLITS, 0), (32, 32, 8, 128, 480, SPLITS, 0),
     (32, 32, 8, 128, 1000, SHARES, 148), (887, 32, 8, 128, 200, SHARES, 148), (888, 32, 8, 128, 200, SPLITS, 0),
     (32, 28, 4, 128, 2000, SHARES, 296), (32, 14, 2, 64, 2000, SPLITS, 0), (8, 32, 32, 128, 600, SHARES, 148),
-    (64, 16, 8, 256, 2000, SPLITS, 0),
+    (64, 16, 8, 256, 2000, SPLITS, 0), (32, 80, 4, 128, 2000, SHARES, 148), (32, 64, 4, 128, 2000, SHARES, 296),
+    (16, 80, 4, 128, 2000, SPLITS, 0), (64, 64, 16, 64, 2000, SHARES, 296),
 ])
 def test_form(batch, heads, kv_heads, d, longest, form, grid):
     p = plan(batch, heads, kv_heads, d, longest)
