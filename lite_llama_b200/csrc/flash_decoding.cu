@@ -994,14 +994,14 @@ extern "C" int b2l_flash_decoding(void* out, const void* q, const void* k_cache,
   // the split CTAs merge their own results when the caller provides zeroed tickets (one per batch row x head block)
   p.tickets = (tickets && num_tickets >= batch * (num_kv_heads / pl.HB)) ? (int*)tickets : nullptr;
   if (pl.splits > 1 && !pl.cluster) {
-    const int64_t rows = split_rows(pl, batch, num_q_heads);
-    const int64_t need = b2l_flash_decoding_workspace_bytes(batch, num_q_heads, num_kv_heads, head_dim, max_seq_len);
+    // (room for the splits alone is enough, with its own formula or an earlier one's: the shares then stay out)
+    const int64_t rows = split_rows(pl, batch, num_q_heads), need = rows * (head_dim + 1) * 4 + 16;
     B2L_REQUIRE(workspace && workspace_bytes >= need, "flash_decoding: workspace too small (%lld < %lld)",
                 (long long)workspace_bytes, (long long)need);
     B2L_REQUIRE((uintptr_t)workspace % 16 == 0, "flash_decoding: workspace must be 16-byte aligned");
     p.ws_o = (float*)workspace;
     p.ws_lse = p.ws_o + rows * head_dim;
-    if (pl.share_grid != 0 && p.tickets == nullptr) {
+    if (pl.share_grid != 0 && p.tickets == nullptr && workspace_bytes >= share_bytes(pl, batch, num_q_heads, num_kv_heads, head_dim)) {
       const int64_t most = share_rows(pl, batch, num_q_heads, num_kv_heads);
       p.slots = 2 * pl.share_grid;
       p.ws_lse = p.ws_o + most * head_dim;

@@ -148,3 +148,29 @@ def test_infinite_values_stay_infinite(heads, kv_heads, d, dtype, kind):
     assert torch.equal(got[got.isinf()].double(), want[want.isinf()])
     ok = want.isfinite()
     assert ((got[ok].double() - want[ok]).norm() / want[ok].norm()).item() < (2.0**-10 if dtype is torch.float16 else 2.0**-7)
+
+
+@pytest.mark.parametrize("heads,kv_heads,d", HEADS)
+def test_a_workspace_for_the_splits_alone_is_enough(heads, kv_heads, d):
+    """A caller of the C entry may have sized it for [batch, heads, splits] partial rows and their statistics."""
+    from lite_llama_b200 import _lib
+
+    batch, bound = 32, 2000
+    q, k, v, table, order = inputs(batch, bound, heads, kv_heads, d, torch.float16)
+    lens, order, out = torch.full((batch,), bound, device="cuda").int(), order.int(), torch.empty_like(q)
+    p = plan(batch, heads, kv_heads, d, bound)
+    nbytes = batch * heads * p.splits * (d + 1) * 4 + 16
+    ws = torch.empty(nbytes + 64, dtype=torch.uint8, device="cuda")
+    ws[nbytes:] = 7
+
+    def call(size):
+        return _lib.load().b2l_flash_decoding(
+            out.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), table.data_ptr(), order.data_ptr(), 4, lens.data_ptr(), 4, batch,
+            heads, kv_heads, d, bound, d**-0.5, q.stride(0), q.stride(1), k.stride(0), k.stride(1), v.stride(0), v.stride(1),
+            table.stride(0), 1, out.stride(0), out.stride(1), ws.data_ptr(), size, None, 0, 0, torch.cuda.current_stream().cuda_stream)
+
+    assert p.form == SHARES and call(nbytes - 1) != 0
+    _lib.check(call(nbytes))
+    want = exact(q, k, v, table, order, [bound] * batch)
+    assert ((out.double() - want).norm() / want.norm()).item() < 2.0**-10
+    assert (ws[nbytes:] == 7).all()
