@@ -25,6 +25,10 @@ def flash_decoding(
     ``b_req_tokens_table [max_requests, max_seq_len]`` int32; ``b_req_idx``/``b_seq_len`` ``[B]``
     int32 or int64; ``max_actual_seq_len`` a Python int (sizes the split grid; graph-safe).  The result of a row of length 0
     is zero.
+
+    The same arguments give the same bits.  Where a row's tokens are parted for the sum follows from batch, heads and
+    ``max_actual_seq_len``; in large steps (csrc/flash_decoding.cu: shares, with more splits that have tokens than CTAs) also from
+    the lengths of the other rows, so a sequence's last bits may change there with what stands beside it.
     """
     require_cuda(q, k_cache, v_cache, b_req_tokens_table, b_req_idx, b_seq_len)
     assert q.shape[-1] == k_cache.shape[-1] == v_cache.shape[-1]
