@@ -34,6 +34,7 @@ struct SplitPlan {
   int num_kb;         // k-blocks in total
   int splits;
   int kb_per_split;
+  int seg_kb;         // k-blocks that one accumulation runs over
   int stages;
   int x_stages;       // quantised GEMMs: depth of the separate activation ring
   int smem_bytes;
@@ -69,7 +70,7 @@ static inline SplitPlan make_plan(int64_t M, int64_t N, int64_t K, int k_elems_p
   pl.m_tiles = (int)cdiv64(M, pl.bt);
   pl.num_kb = (int)cdiv64(K, k_elems_per_stage);
   const int tiles = pl.n_tiles * pl.m_tiles;
-  int splits = 1;
+  int splits = 1, seg = pl.num_kb;
   if (tiles < sms) {
     splits = sms / tiles;
     int max_splits = pl.num_kb / min_kb_per_split;
@@ -77,16 +78,22 @@ static inline SplitPlan make_plan(int64_t M, int64_t N, int64_t K, int k_elems_p
     if (splits > max_splits) splits = max_splits;
     if (splits > 32) splits = 32;
     if (splits < 1) splits = 1;
+    seg = (pl.num_kb + splits - 1) / splits;
     // The last CTA of a tile adds up the parts, four splits and 16 tokens a trip to L2: with many tokens and splits that takes
     // longer than the stream itself (64 tokens, 896 x 4864, bf16, 19 splits: 12 of 18.9 us).  In 1/100 us, per SM 75 bytes per ns.
-    const int stage = kABytes + pl.bt * kStageKBytes;
-    auto cost = [&](int s) { return (pl.num_kb + s - 1) / s * (stage / 750) + (s > 1 ? 100 + (s + 3) / 4 * (pl.bt / 16) * 55 : 0); };
+    // A part of a sum of floats then holds several of the segments that had a CTA each, and adds them up as those would (gemm_dense.cu).
+    const int stage = kABytes + pl.bt * kStageKBytes, unit = k_elems_per_stage == 64 ? seg : 1;
+    const int units = (pl.num_kb + unit - 1) / unit;
+    auto cost = [&](int s) { return (units + s - 1) / s * unit * (stage / 750) + (s > 1 ? 100 + (s + 3) / 4 * (pl.bt / 16) * 55 : 0); };
     int best = splits;
     for (int s = splits - 1; s >= 2; --s)
       if (cost(s) < cost(best)) best = s;
     if (cost(best) * 100 < cost(splits) * 85) splits = best;
+    pl.kb_per_split = (units + splits - 1) / splits * unit;
+  } else {
+    pl.kb_per_split = pl.num_kb;
   }
-  pl.kb_per_split = (pl.num_kb + splits - 1) / splits;
+  pl.seg_kb = seg < pl.kb_per_split ? seg : pl.kb_per_split;
   pl.splits = (pl.num_kb + pl.kb_per_split - 1) / pl.kb_per_split;
   const int stage_bytes = kABytes + pl.bt * kStageKBytes + extra_stage_bytes;
   int budget = b2l_max_smem_optin() - fixed_bytes - 1024 /*alignment slack*/;

@@ -265,6 +265,21 @@ def test_per_channel_accumulations_are_no_longer_than_the_parts_of_k(m, n, k, ch
     assert abs(((got - want) / want).mean().item()) < chain / 16 * 2.0**-23
 
 
+# parts of k that had a CTA each (four blocks of 64 on 148 SMs) and now share one: two, three, four of them, the last part shorter
+@pytest.mark.parametrize("m,n,k", [(64, 896, 4864), (33, 512, 8192), (64, 512, 8192), (17, 896, 4864), (48, 1000, 2104), (16, 344, 5360)])
+def test_linear_accumulates_no_longer_than_the_parts_of_k(m, n, k):
+    """Positive values: one addition of 16 products cuts off less than 2^-23 of the partial sum, over 256 k (16 additions) half of
+    16 * 2^-23 on average.  The mean over eight inputs leaves 5e-7 of the rounding to fp16; over 640 k and more the bound is missed
+    by half and more."""
+    dev = 0.0
+    for _ in range(8):
+        x = torch.rand(m, k, device="cuda").mul_(0.5).add_(0.5).half()
+        w = (torch.rand(n, k, device="cuda") + 0.1).half()
+        want = x.double() @ w.double().T
+        dev += ((K().linear(x, w).double() - want) / want).mean().item() / 8
+    assert abs(dev) < 16 * 2.0**-23
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 136, 64), (17, 1000, 256), (130, 520, 512), (300, 10248, 144), (256, 3584, 2048),
                                    (7, 1000, 256), (33, 520, 4096), (65, 9736, 896), (97, 9736, 128)])
 @pytest.mark.parametrize("shift", [0, 1])
