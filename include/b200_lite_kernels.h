@@ -151,6 +151,10 @@ int b2l_argmax_rows(void* out_index_i64, const void* x, int64_t rows, int64_t n,
  * (lite_llama/models/quantization/methods/unquantized.py:21-22, lite_llama/models/base.py:489). */
 int64_t b2l_linear_workspace_bytes(int64_t m, int64_t n, int64_t k, int elem_bytes);
 int64_t b2l_linear_num_counters(int64_t m, int64_t n);
+/* launch plan of a projection with plain rows, 16-bit or int8 operands, for tests and tools (no GPU work): out[5] = {SM pairs
+ * instead of the one-SM kernel; tokens per tile, parts of k, k-blocks per part and per accumulation of the latter}.  The trailing
+ * argument is unused. */
+int b2l_linear_plan(int64_t m, int64_t n, int64_t k, int elem_bytes, int* out, void* reserved);
 int b2l_linear(void* y, const void* x, const void* w, const void* bias, int64_t m, int64_t n, int64_t k,
                int64_t x_row_stride, int64_t w_row_stride, int64_t y_row_stride, void* workspace,
                int64_t workspace_bytes, void* counters, int64_t num_counters, int dtype, void* stream);

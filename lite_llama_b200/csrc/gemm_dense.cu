@@ -361,6 +361,20 @@ extern "C" int64_t b2l_linear_num_counters(int64_t m, int64_t n) {
   return cdiv64(n, kBlockW) * cdiv64(m, bt);
 }
 
+// What a call with plain rows does, for tests and tools (no GPU work): out[0..4] = {SM pairs (gemm_pair.cu) instead of this kernel;
+// tokens per tile, parts of k, blocks of k per part and per accumulation of this kernel}
+extern "C" int b2l_linear_plan(int64_t m, int64_t n, int64_t k, int elem_bytes, int* out, void* /*reserved*/) {
+  B2L_REQUIRE(out && m > 0 && n > 0 && k > 0 && (elem_bytes == 1 || elem_bytes == 2), "linear_plan: bad arguments");
+  const SplitPlan pl = make_plan(m, n, k, elem_bytes == 1 ? 128 : 64, 0, 1024, 4);
+  const PairGemm pg{nullptr, n, nullptr, nullptr, nullptr, m, n, k, k, k, nullptr, nullptr};
+  out[0] = pair_gemm_wanted(elem_bytes == 1 ? 1 : 0, pg) && !one_short_wave(pl, k);
+  out[1] = pl.bt;
+  out[2] = pl.splits;
+  out[3] = pl.kb_per_split;
+  out[4] = elem_bytes == 1 ? pl.kb_per_split : pl.seg_kb;
+  return B2L_OK;
+}
+
 extern "C" int b2l_linear(void* y, const void* x, const void* w, const void* bias, int64_t m, int64_t n, int64_t k,
                           int64_t x_row_stride, int64_t w_row_stride, int64_t y_row_stride, void* workspace,
                           int64_t workspace_bytes, void* counters, int64_t num_counters, int dtype, void* stream) {

@@ -65,8 +65,16 @@ static inline SplitPlan make_plan(int64_t M, int64_t N, int64_t K, int k_elems_p
   // partials per CTA through the workspace, which cost more than the GEMM (measured 57 us vs 34 us for the
   // reference's Triton kernel on this shape, profiles/r2c_triton_vs_b200.md).
   // Not where that makes a second wave out of the first, which streams the weights twice (65 - 128 tokens, us: bf16 16384 x 4096 44 -
-  // 46 -> 27 - 29, 9728 x 896 13.0 -> 10.3, int8 12288 x 3584 20 -> 14).
-  while (pl.bt > 64 && (int64_t)pl.n_tiles * cdiv64(M, pl.bt) < sms && (int64_t)pl.n_tiles * cdiv64(M, pl.bt / 2) <= sms) pl.bt /= 2;
+  // 46 -> 27 - 29, 9728 x 896 13.0 -> 10.3, int8 12288 x 3584 20 -> 14).  With a short k several of the smaller tiles share an SM, and
+  // beyond 128 tokens it is not this kernel that the larger ones compete with (gemm_dense.cu: one_short_wave): 257 x 4864 x 128 bf16
+  // 4.4, with larger tiles 7.4, int8 400 x 4864 x 256 6.1 / 11.6, but 65 x 14336 x 256 bf16 8.8 / 7.1.
+  auto tiles_of = [&](int bt) { return (int64_t)pl.n_tiles * cdiv64(M, bt); };
+  auto resident = [&](int bt) {
+    const int64_t stages = cdiv64(K, k_elems_per_stage) + 1, smem = stages * (kABytes + bt * kStageKBytes + extra_stage_bytes) + fixed_bytes + 2048;
+    return smem < b2l_max_smem_optin() + 1024 ? (b2l_max_smem_optin() + 1024) / smem : 1;
+  };
+  while (pl.bt > 64 && tiles_of(pl.bt) < sms &&
+         ((M > 128 && K < 512) || tiles_of(pl.bt / 2) <= resident(pl.bt / 2) * sms)) pl.bt /= 2;
   pl.m_tiles = (int)cdiv64(M, pl.bt);
   pl.num_kb = (int)cdiv64(K, k_elems_per_stage);
   const int tiles = pl.n_tiles * pl.m_tiles;
