@@ -167,6 +167,10 @@ int64_t b2l_quant_gemm_num_counters(int64_t m, int64_t n);
  * grid), workspace slots per tile, raw blocks per tile, weight-row tiles, splits, k-blocks per split, weight ring
  * depth, activation ring depth, shared-memory bytes, scale-table columns}.  The trailing argument is unused. */
 int b2l_quant_gemm_plan(int kind, int64_t m, int64_t n, int64_t k, int64_t group_k, int* out, void* reserved);
+/* kernel that takes a quantised GEMM on the repacked layout (int4: whole zero points), for tests and tools (no GPU work): out[2] =
+ * {0 streaming, 1 decode, 2 batch, 3 SM pairs, 4 SM pairs with 256 tokens per tile; pairs that share a tile}.  The trailing argument
+ * is unused. */
+int b2l_quant_gemm_form(int kind, int64_t m, int64_t n, int64_t k, int64_t group_k, int swiglu, int* out, void* reserved);
 int b2l_w4a16_matmul(void* y, const void* x, const void* qweight, const void* scales, const void* zeros,
                      const void* bias, int bias_is_f32, int64_t m, int64_t n, int64_t k, int group_size,
                      int64_t x_row_stride, int64_t qw_row_stride, int64_t s_row_stride, int64_t s_col_stride,

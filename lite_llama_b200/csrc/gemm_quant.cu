@@ -1424,6 +1424,22 @@ extern "C" int b2l_quant_gemm_plan(int kind, int64_t m, int64_t n, int64_t k, in
   return B2L_OK;
 }
 
+// Which kernel takes a quantised GEMM on the repacked layout (int4: whole zero points), with the workspace that it asks for; for tests
+// and tools, no GPU work.  out[0]: 0 streaming, 1 decode, 2 batch, 3 SM pairs, 4 SM pairs with 256 tokens per tile; out[1]: pairs that
+// share a tile.
+extern "C" int b2l_quant_gemm_form(int kind, int64_t m, int64_t n, int64_t k, int64_t group_k, int swiglu, int* out, void* /*reserved*/) {
+  B2L_REQUIRE(out && kind >= Q_INT4 && kind <= Q_INT8 && m > 0 && n > 0 && k > 0 && group_k > 0, "quant_gemm_form: bad arguments");
+  const int64_t seg = seg_len_for(kind, k, group_k);
+  out[0] = out[1] = 0;
+  if (quant_batch_wanted(kind, kind == Q_INT4 ? 1 : 0, m, n, k, seg)) out[0] = 2;
+  else if (kind == Q_INT4 && quant_decode_wanted(m, k, seg)) out[0] = 1;
+  else if (const int pairs = quant_pair_form(kind, m, n, k, seg, swiglu)) {
+    out[0] = pairs < 0 ? 4 : 3;
+    out[1] = pairs < 0 ? 1 : pairs;
+  }
+  return B2L_OK;
+}
+
 extern "C" int64_t b2l_quant_gemm_num_counters(int64_t m, int64_t n) {
   if (m <= 0 || n <= 0) return 0;
   return cdiv64(n, kBlockW) * cdiv64(m, pick_bt(m > 64 ? 64 : m));

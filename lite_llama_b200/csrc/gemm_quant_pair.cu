@@ -639,6 +639,18 @@ static int qp_chain_steps(int64_t M, int64_t N, int64_t K) {
   return (int)cdiv64(steps, parts);
 }
 
+// steps of 128 k that one scale covers, or one accumulation where a scale covers all of k
+static int qp_seg_steps(int64_t M, int64_t N, int64_t K, int64_t group_k) {
+  return group_k >= K ? qp_chain_steps(M, N, K) : (int)(group_k / kQpStepK);
+}
+
+int quant_pair_form(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k, int swiglu) {
+  if (!quant_pair_wanted(qk, M, N, K, group_k)) return 0;
+  if (quant_wide_wanted(qk, M, N, cdiv64(K, kQpStepK), qp_seg_steps(M, N, K, group_k), swiglu)) return -1;
+  int64_t part;
+  return qp_splits(qk, M, N, K, group_k, &part);
+}
+
 int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, const void* w, int64_t w_stride_bytes,
                     int64_t M, int64_t N, int64_t K, int64_t group_k, int swiglu, cudaStream_t st) {
   const int pairs = b2l_num_sms() / 2;
@@ -646,11 +658,8 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
   p.steps = (int)cdiv64(K, kQpStepK);
   p.groups = group_k >= K ? 1 : (int)(K / group_k);
   if (qk == Q_INT4) p.s_stride_k = kBlockW;
-  p.seg_steps = (int)(group_k / kQpStepK);
-  if (group_k >= K) {
-    p.seg_steps = qp_chain_steps(M, N, K);
-    p.s_stride_k = 0;
-  }
+  p.seg_steps = qp_seg_steps(M, N, K, group_k);
+  if (group_k >= K) p.s_stride_k = 0;
   p.vec = p.ldy % 4 == 0 && (uintptr_t)p.y % 8 == 0;
   p.m_tiles = (int)cdiv64(M, kQpTokens);
   p.n_tiles = (int)cdiv64(N, 2 * kBlockW);
@@ -663,7 +672,7 @@ int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, cons
   if (rc != B2L_OK) return rc;
   rc = b2l_make_tmap_2d(&tx, x, TMA_F16, (uint64_t)M, (uint64_t)K, (uint64_t)ldx * 2, kQpTokens / 2, 64, true);
   if (rc != B2L_OK) return rc;
-  if (quant_wide_wanted(qk, M, N)) return quant_wide_gemm(qk, p, tw, tx, swiglu, st);
+  if (quant_wide_wanted(qk, M, N, p.steps, p.seg_steps, swiglu)) return quant_wide_gemm(qk, p, tw, tx, swiglu, st);
   int64_t part = 0;
   const int splits = qp_splits(qk, M, N, K, group_k, &part);
   p.split_steps = (int)part;

@@ -23,10 +23,12 @@ struct QuantPairParams {
 
 // shapes the pair kernel takes and is the faster one for (see gemm_quant_pair.cu); qk: QuantKind
 bool quant_pair_wanted(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k);
+// pairs that share a tile, -1: tiles of 256 tokens, 0: not wanted
+int quant_pair_form(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k, int swiglu);
 int quant_pair_gemm(int qk, QuantPairParams& p, const void* x, int64_t ldx, const void* w, int64_t w_stride_bytes,
                     int64_t M, int64_t N, int64_t K, int64_t group_k, int swiglu, cudaStream_t st);
 // the same with 256 tokens per tile (gemm_quant_wide.cu); boxes of the tensor maps: 128 weight rows, 64 tokens
-bool quant_wide_wanted(int qk, int64_t M, int64_t N);
+bool quant_wide_wanted(int qk, int64_t M, int64_t N, int64_t steps, int64_t seg_steps, int swiglu);
 int quant_wide_gemm(int qk, QuantPairParams& p, const CUtensorMap& tw, const CUtensorMap& tx, int swiglu, cudaStream_t st);
 
 // The two products of a routed SwiGLU layer over activations sorted by expert (moe_routing.cu: b2l_moe_sort, b2l_moe_gather).

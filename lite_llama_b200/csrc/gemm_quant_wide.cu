@@ -394,19 +394,28 @@ int launch_qw(const CUtensorMap& tw, const CUtensorMap& tx, const QuantPairParam
 // Tiles of a last wave that leaves half of the pairs idle or more are cut in two.
 static bool qw_split(int64_t tiles, int64_t pairs) { return tiles % pairs * 2 <= pairs; }
 
-// Where it is the faster one, counted in waves of the kernel with 128 tokens per tile: a wave of wide tiles takes 1.4 - 1.5 of
-// its waves with int4 weights and 1.6 - 1.8 with 8-bit ones (whose narrow form loses less at hand-offs), one of tiles cut in two
-// 1.25 and 1.3 - 1.5 (one issuer, one conversion group).  Measured over 100 - 3000 tokens and seven projections, us, narrow ->
-// wide: int4, 6144 x 4096 at 384 tokens 22 / 29 (one wave either way), at 512 38 -> 31 (two against one), 28672 x 4096 at 384
-// 106 / 105 (five; three and a cut one), at 1024 294 -> 219; fp8 in blocks, 6144 x 4096 at 512 35 -> 32, at 1024 52 / 54 (three; one
-// and a cut one).
-bool quant_wide_wanted(int qk, int64_t M, int64_t N) {
-  if (M <= kQwHalf) return false;
+// Where it is the faster one.  Both kernels' times are waves x (steps of 128 k x time per step + set-up and end of a tile) + start, with
+// a wave of tiles cut in two beside full ones; the ends of a wide tile take longer and nothing covers them, so a short k keeps the tiles
+// of 128 tokens.  The ratios below (hundredths of a step of the kernel of 128 tokens) are fitted to both kernels over 81 - 366 sizes of
+// 129 - 8192 tokens per kind; the choice is within 3 % of the faster one but in 3 of 285, 1 of 81 and 12 of 366.  us, 128 tokens per tile /
+// this: int4 in groups of 128, 1024 x 9728 x 896 31.4 / 34.5, 1664 x 4096 x 14336 (a wave and a cut one) 181 / 198, 1024 x 4096 x 14336
+// 112 / 102, 4096 x 28672 x 4096 937 / 841; one scale per row, int8, 1024 x 9728 x 896 20.7 / 22.2, 2048 x 28672 x 4096 459 / 353.  8-bit weights
+// in groups of 128, whose two issuers leave it nothing to gain, stay there (fp8 in blocks, 2048 x 28672 x 4096 435 / 468, 1664 x 4096 x
+// 14336 167 / 209).  With the activation the end of a tile is the heavier one in both: by waves alone (1024 x 9728 x 896 29.3 / 27.6, 2048 x
+// 28672 x 4096 494 / 427; within 3 % of the faster in 128 of 128).
+bool quant_wide_wanted(int qk, int64_t M, int64_t N, int64_t steps, int64_t seg_steps, int swiglu) {
+  if (M <= kQwHalf || (qk != Q_INT4 && seg_steps == 1)) return false;
   const int64_t pairs = b2l_num_sms() / 2, n_tiles = cdiv64(N, 2 * kBlockW);
   const int64_t wide = cdiv64(M, 2 * kQwHalf) * n_tiles, waves = cdiv64(cdiv64(M, kQwHalf) * n_tiles, pairs);
   const bool cut = wide % pairs != 0 && qw_split(wide, pairs);
   const int64_t full = cut ? wide / pairs : cdiv64(wide, pairs);
-  return full * (qk == Q_INT4 ? 150 : 175) + (cut ? (qk == Q_INT4 ? 127 : 140) : 0) < 100 * waves;
+  if (waves < 2) return false;
+  if (swiglu && seg_steps == 1) return full * 150 + (cut ? 127 : 0) < 100 * waves;
+  struct Cost { int step, tile, cut_step, cut_tile, start, narrow_tile, narrow_start; };
+  constexpr Cost kGroups{173, 240, 141, -17, 1221, 39, 953}, kLong{143, 381, 134, -195, 2109, 12, 1688}, kRow8{153, 5, 140, -273, 2810, -59, 1939};
+  const Cost c = qk != Q_INT4 ? kRow8 : seg_steps == 1 ? kGroups : kLong;
+  const int64_t narrow = waves * (100 * steps + c.narrow_tile) + c.narrow_start;
+  return full * (c.step * steps + c.tile) + (cut ? c.cut_step * steps + c.cut_tile : 0) + c.start < narrow * (qk != Q_INT4 ? 98 : 100) / 100;
 }
 
 // p: filled by quant_pair_gemm but for the tiles

@@ -8,6 +8,8 @@ from __future__ import annotations
 import pytest
 import torch
 
+from test_quant_form_cpu import FP8, INT4, INT8, SHARED_TILES, WIDE, WIDE_TILES, form
+
 pytestmark = [pytest.mark.gpu, pytest.mark.timeout(180)]
 
 REL = {torch.float16: 2.0**-11, torch.bfloat16: 2.0**-8}
@@ -324,9 +326,8 @@ def test_int8_split_over_a_cluster(m, n, k, bias):
     assert rel(K().smoothquant_matmul_prequant(qa, sa, qw, sw, bias=b), want) < REL[torch.float16]
 
 
-# ---- 256 tokens per tile (csrc/gemm_quant_wide.cu) ----
-# 74 pairs: whole waves; a last wave cut in two, its second parts empty or short; a last tile of one half between tiles of two
-# (the accumulators' turn shifts by an odd number of segments); rows of y that no 8-byte store fits; an odd number of steps
+# ---- 256 tokens per tile (csrc/gemm_quant_wide.cu): WIDE_TILES reach it, the others lie around its line (the form with the activation
+# takes most of them) ----
 WIDE_EDGES = [(300, 18944, 384), (513, 12800, 640), (1000, 9734, 128), (769, 9734, 384), (640, 18688, 896), (1537, 3330, 1152)]
 
 
@@ -355,6 +356,27 @@ def test_w8_wide_tiles(m, n, k, fmt):
     test_w8_pair_tiles(m, n, k, fmt)
 
 
+@pytest.mark.parametrize("m,n,k", WIDE_TILES)
+@pytest.mark.parametrize("group", [128, 384])
+def test_int4_tiles_of_256_tokens(m, n, k, group):
+    if k % group == 0:
+        assert form(INT4, m, n, k, group)[0] == WIDE
+    test_int4_wide_tiles(m, n, k, group)
+
+
+@pytest.mark.parametrize("m,n,k", WIDE_TILES)
+def test_int4_swiglu_tiles_of_256_tokens(m, n, k):
+    assert form(INT4, m, n, k, 128, True)[0] == WIDE
+    test_int4_pair_swiglu_is_gemm_then_swiglu(m, n, k)
+
+
+@pytest.mark.parametrize("m,n,k", WIDE_TILES)
+@pytest.mark.parametrize("fmt", ["fp8_channel", "int8_channel", "int8_group_n"])
+def test_w8_tiles_of_256_tokens(m, n, k, fmt):
+    assert form(FP8 if fmt.startswith("fp8") else INT8, m, n, k, k)[0] == WIDE
+    test_w8_pair_tiles(m, n, k, fmt)
+
+
 # ---- one-SM kernel (csrc/gemm_dense.cu): 128-token tiles where 64-token tiles would need a second wave (75 - 148 weight tiles), and
 # fewer splits of k than there are SMs for where the last CTA of a tile would add up too many
 PLAN_EDGES = [(65, 9728, 896), (128, 18944, 192), (100, 9600, 320), (16, 128, 4096), (64, 896, 4864), (33, 512, 8192), (200, 256, 2048)]
@@ -371,10 +393,9 @@ def test_int8_token_tiles_and_splits(m, n, k):
     test_int8_pair_tiles(m, n, k, True)
 
 
-# ---- several pairs on a tile (csrc/gemm_quant_pair.cu): four up to 14 tiles, two up to 32; the last part shorter, a k that no four
-# parts share, tokens that end within the four a thread stores, a tile of one half (64 tokens) or less
-SPLIT_EDGES = [(65, 2560, 2176), (129, 1302, 4864), (100, 8192, 1152), (200, 4096, 1408), (500, 1730, 2048), (67, 256, 16384),
-               (257, 2600, 1024)]
+# ---- several pairs on a tile (csrc/gemm_quant_pair.cu): four up to 15 tiles, three up to 22, two up to 33, by steps of k; and sizes
+# that the rule leaves to a pair each or to the streaming kernel
+SPLIT_EDGES = list(SHARED_TILES) + [(100, 8192, 1152), (200, 4096, 1408), (500, 1730, 2048), (257, 2600, 1024)]
 
 
 @pytest.mark.parametrize("m,n,k", SPLIT_EDGES)
