@@ -588,6 +588,8 @@ static int launch_qp_split(const CUtensorMap& tw, const CUtensorMap& tx, const Q
 //     -> 10.0 / 9.7 / 9.8; 5376 x 2304, 18 steps: 10.8 / 10.4 / 10.0 -> 9.9 / 9.7 / 9.8), from 24 with two (2048 x 2048 at 384: 10.0 /
 //     9.8 / 9.3 -> 10.2 / 10.0 / 10.0; 4096 x 3072 at 256, 24 steps: 13.5 / 13.4 / 12.7 -> 13.0 / 12.3 / 12.4; 4096 x 14336 at 256:
 //     66 / 59 / 45 -> 32 / 30 / 30)
+//   * a single weight tile leaves half of each pair to padding, and then two pairs are too few against the streaming kernel's parts
+//     (2821 x 128 x 8192, 23 tiles: 17.7 / 17.7 against 21.4 / 19.1).
 // The same for the form with the activation, whose result is the plain form's to the bit (5632 x 2048 at 65 tokens 13.6 -> 9.1).  Sums
 // in order of k, in fp32; error against 64 bits of seven shapes as before, up to 0.05 % smaller per row (shorter accumulations).
 static int qp_splits(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k, int64_t* part) {
@@ -598,6 +600,7 @@ static int qp_splits(int qk, int64_t M, int64_t N, int64_t K, int64_t group_k, i
   if (qk == Q_INT4 && unit % 2 != 0) unit *= 2;
   for (int s = 4; s > 1; --s) {
     if (tiles > (s == 4 ? 15 : s == 3 ? 22 : 33) || steps < (!one_part ? 8 : s == 2 ? 24 : 18)) continue;
+    if (s == 2 && !one_part && N <= kBlockW) continue;
     *part = cdiv64(cdiv64(steps, s), unit) * unit;
     if ((s - 1) * *part < steps) return s;
   }

@@ -50,6 +50,8 @@ def test_shared_tiles(m, n, k):
 @pytest.mark.parametrize("kind,m,n,k,group,swiglu,kernel", [
     (INT4, 8, 4096, 4096, 128, False, DECODE), (INT4, 64, 4096, 4096, 128, False, BATCH), (FP8, 33, 4096, 4096, 128, False, BATCH),
     (INT4, 72, 4096, 14336, 192, False, STREAMING), (INT4, 72, 12800, 4096, 128, False, PAIRS),
+    # one weight tile: half of a pair is padding
+    (INT4, 2821, 128, 8192, 128, False, STREAMING), (FP8, 2821, 64, 8192, 128, False, STREAMING), (INT4, 2000, 128, 8192, 128, False, PAIRS),
     # a short k, whose end of a tile nothing covers, and fewer waves in all
     (INT4, 1024, 9728, 896, 128, False, PAIRS), (INT4, 1024, 9728, 896, 128, True, WIDE), (INT4, 1081, 2776, 384, 128, False, PAIRS),
     (FP8, 1410, 2088, 576, 576, False, PAIRS), (INT8, 463, 24408, 256, 256, False, PAIRS), (INT4, 1146, 20984, 256, 128, False, PAIRS),
