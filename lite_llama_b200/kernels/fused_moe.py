@@ -87,13 +87,16 @@ def _moe_gemm(a, w, c, scale, kind, topk_weights, sorted_ids, expert_ids, num_po
     )
 
 
-def _pair_tile(slots: int, num_experts: int) -> int:
+def _pair_tile(slots: int, num_experts: int, group_k: int) -> int:
     """Rows of a tile of the pair GEMMs (csrc/gemm_quant_pair.cu): 64 leave room for more conversion stages, 128 convert an
-    expert's weights once for twice the rows.  Where the line lies: up to 48 rows per expert on average 64 is the faster one
-    however the rows fall (128 experts of 2048 x 768 fp8, top 8, us for 128 -> 64 rows: 40 each 186 -> 153, 48 each 197 -> 168,
-    between 10 and 370 of them 197 -> 179; 8 experts of 4096 x 2048, 48 each 64 -> 58); from 52 on it depends on how many
-    experts exceed 64 (8 experts, two of them over: 64 -> 75), at 64 level, beyond 128 wins (80 each 210 / 273)."""
-    return 64 if slots <= 48 * num_experts else 128
+    expert's weights once for twice the rows.  Where the line lies, in rows per expert on average: scale groups of 128, 48 (128
+    experts of 2048 x 768 fp8, top 8, us for 128 -> 64 rows: 40 each 186 -> 153, 48 each 197 -> 168, between 10 and 370 of them 197 ->
+    179; 8 experts of 4096 x 2048, 48 each 64 -> 58); from 52 on it depends on how many experts exceed 64 (8 experts, two of them
+    over: 64 -> 75), at 64 level, beyond 128 wins (80 each 210 / 273).  Where the same few experts get all rows 64 is slower from 33
+    on (768 tokens, 8 of 128 experts, gate|up 59 / 62; 132 tokens, 2 of 8, 21.4 / 25.0).  Longer groups and one scale per row, whose
+    tiles of 64 rows have one issuing warp as well, 32 (gate|up and down, 128 -> 64 rows: 128 experts, 48 each 84 -> 92, 8 experts
+    of 4096 x 14336, 48 each 177 -> 211 and 124 -> 171)."""
+    return 64 if slots <= (48 if group_k == 128 else 32) * num_experts else 128
 
 
 def _pair_gemm_takes(kind: int, hidden: int, intermediate: int, group_k: int, w1: torch.Tensor, w2: torch.Tensor) -> bool:
@@ -115,7 +118,7 @@ def _fused_moe_pair(x, w1, w2, flat_weights, topk_ids, w1_scale, w2_scale, kind,
         ids = ids.to(torch.int64)
     ids = ids.contiguous()
     L, dev, st = lib(), x.device, stream_handle()
-    tile = _pair_tile(slots, num_experts)
+    tile = _pair_tile(slots, num_experts, group_k)
     max_tiles = L.b2l_moe_sort_max_tiles(slots, tile, num_experts)
     order = torch.empty(slots + 1, dtype=torch.int32, device=dev)
     table = torch.empty(1 + 3 * max_tiles, dtype=torch.int32, device=dev)

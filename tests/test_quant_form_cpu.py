@@ -60,3 +60,10 @@ def test_shared_tiles(m, n, k):
 ])
 def test_kernel(kind, m, n, k, group, swiglu, kernel):
     assert form(kind, m, n, k, group, swiglu)[0] == kernel
+
+
+@pytest.mark.parametrize("rows,group,tile", [(32, 128, 64), (48, 128, 64), (49, 128, 128), (32, 256, 64), (33, 256, 128), (33, 4096, 128)])
+def test_rows_of_an_expert_tile(rows, group, tile):
+    from lite_llama_b200.kernels.fused_moe import _pair_tile
+
+    assert _pair_tile(rows * 16, 16, group) == tile
