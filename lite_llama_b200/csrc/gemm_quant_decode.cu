@@ -255,7 +255,8 @@ template <int LAYOUT, int EPI, bool WHOLE>
 int launch_dec(const DecParams& p, cudaStream_t st) {
   const int sms = b2l_num_sms();
   if (p.strips <= 2 * sms) return launch_dec_chunk<LAYOUT, EPI, WHOLE, 2>(p, st);
-  if (LAYOUT == 1 && p.strips >= 12 * sms) return launch_dec_chunk<LAYOUT, EPI, WHOLE, 7>(p, st);
+  if constexpr (LAYOUT == 1)
+    if (p.strips >= 12 * sms) return launch_dec_chunk<LAYOUT, EPI, WHOLE, 7>(p, st);
   return launch_dec_chunk<LAYOUT, EPI, WHOLE, 4>(p, st);
 }
 

@@ -177,8 +177,10 @@ gemm_quant_wide_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_
     } else if (rank == 0) {
       // ===================== MMA issuers (leader), one per half =====================
       // A tile of one half is the first one's alone; the other one waits for its end, so that neither waits for a barrier that
-      // is two phases behind.  (A ring slot of X was the other half's nine items ago, at most four steps: the operand stage's
-      // barrier, waited for first, says that it was issued.)
+      // is two phases behind.  A slot of X may have been the other half's: its last use is kQwXStages items back, at least four steps
+      // (more behind tiles of one half).  The operand stage, waited for first, was handed back two steps ago by both issuers, so both
+      // are past that use, and the slot's barrier is at most one phase behind.
+      static_assert((kQwXStages - 1) / 2 >= kQwOpStages / 2, "a slot of X is used again after the operand stages have gone round");
       const uint64_t x_desc0 = umma_desc_sw128_kmajor(smem_u32(x_ring));
       PipeState xs(kQwXStages), os(kQwOpStages), as(kQwAcc);
       const int h = warp - kQwMma;
