@@ -3,7 +3,7 @@
 //
 // Replaces lite_llama/kernels/flashattention2_nopad.py:45-231 for the shapes the decoder uses (D = 128, heads packed
 // inside a token row); same contract as flash_attention_nopad.cu, which stays the path for other head sizes.
-// The mma.sync kernel measured twice the reference's time at these shapes (profiles/r2c_triton_vs_b200.md); this
+// The mma.sync kernel measured twice the reference's time at these shapes; this
 // kernel is the B200-native one.
 //
 // One CTA = 128 query rows of one (sequence, q head), 192 threads:

@@ -15,13 +15,13 @@
 //     MMAs and 16 bytes of an activation row are its B fragments of two: the activations of a slice stay in registers.
 //   * one chain of 8 MMAs per 128 k, scaled into the fp32 sum like the other kernels' segments; whole zero points are
 //     subtracted exactly in the conversion, others as scale * (sum - z * xsum).  (Nibbles as fp16 subnormals, with the zero point applied to the sums, need 5 instead of 9
-//     instructions per word and measured the same: 15.4 us against 16.3 us for 28672 x 4096, 5.5 against 5.0 us for 6144 x
-//     4096, so the exact form stays.)
+//     instructions per word and measured the same, in chunks of four: 15.4 us against 16.3 us for 28672 x 4096, 5.5 against 5.0
+//     us for 6144 x 4096, so the exact form stays.)
 //   * after a chunk of strips the warps add up their sums through shared memory in warp order (deterministic); the next
 //     chunk's weights are on their way meanwhile, and the other warps go on to them while some add (a second barrier right after
-//     the sums: 28672 x 4096, one token 18.1 us instead of 17.1).
-// Measured, one token, streaming kernel -> this one: 4096 x 4096 7.0 -> 3.7 us, 6144 x 4096 8.3 -> 5.0, 28672 x 4096 19.6 ->
-// 15.0, 4096 x 14336 12.9 -> 9.6.  Copies by TMA (one lane instead of address arithmetic in all): 0.3 us slower to start, 4096 x
+//     the sums costs 6 % of 28672 x 4096).
+// Measured, one token, repacked layout, no activation, weights from memory, launches in a row, streaming kernel -> this one: 4096 x 4096
+// 7.0 -> 4.4 us, 6144 x 4096 8.3 -> 5.6, 28672 x 4096 19.6 -> 15.9 (with the activation 16.1), 4096 x 14336 12.9 -> 9.8.  Copies by TMA (one lane instead of address arithmetic in all): 0.3 us slower to start, 4096 x
 // 14336 at eight tokens 13.1 -> 15.5.
 #include "common.cuh"
 #include "dequant.cuh"
@@ -35,9 +35,9 @@ constexpr int kDecWarps = 16, kDecThreads = kDecWarps * 32;
 constexpr int kDecSlice = 256, kDecBlocks = kDecSlice / 128;       // k per slice, 128-k blocks in it
 constexpr int kDecUnit = kDecBlocks * (1024 + 128);                // a strip's slice: words, then {16 scales, 16 zeros} per block
 // CHUNK: strips whose sums a thread holds at a time; the warps meet once per chunk.  With twelve strips to a CTA or more, chunks of
-// seven and a ring that is a strip shorter to make room for them (28672 x 4096, one / eight tokens, us: chunks of four 17.1 and 18.8,
-// of seven 16.4 and 17.9); with one or two, chunks of two leave registers (4096 x 14336, eight tokens 13.7 -> 12.7); chunks of seven for
-// few strips cost 5 - 10 % (6144 x 4096, eight tokens 7.0 / 7.3).
+// seven and a ring that is a strip shorter to make room for them (28672 x 4096, one / eight tokens, us: chunks of four 16.9 and 17.7,
+// of seven 15.9 and 17.2, with the activation 17.6 and 19.1, 16.1 and 17.4); with one or two, chunks of two leave registers (4096 x 14336,
+// eight tokens 13.1 -> 12.5); chunks of seven for few strips cost 5 - 10 % (6144 x 4096, eight tokens 7.0 / 7.3).
 __host__ __device__ constexpr int dec_depth(int chunk) { return chunk > 4 ? 3 : 4; }
 
 struct DecParams {
@@ -63,7 +63,7 @@ __device__ __forceinline__ void mma_f16_zero(float (&d)[4], const uint32_t (&a)[
 }
 
 // WHOLE: the packer has seen that every zero point is an integer in [0, 1023] (the test costs 10 % where it has to be made:
-// 28672 x 4096, one token 17.9 against 16.3 us)
+// 28672 x 4096, one token, chunks of four, 17.9 against 16.3 us)
 template <int LAYOUT, int EPI, bool WHOLE, int CHUNK>
 __global__ void __launch_bounds__(kDecThreads, 1)
 gemm_quant_decode_kernel(const DecParams p) {

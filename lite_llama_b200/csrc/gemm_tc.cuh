@@ -63,7 +63,7 @@ static inline SplitPlan make_plan(int64_t M, int64_t N, int64_t K, int k_elems_p
   // Medium token counts with few weight-row tiles (e.g. 256 x 4608 x 3584: 36 tiles of 128 x 256): fill the SMs
   // with SMALLER token tiles before resorting to split-K -- a split of a 256-token tile moves 128 KiB of fp32
   // partials per CTA through the workspace, which cost more than the GEMM (measured 57 us vs 34 us for the
-  // reference's Triton kernel on this shape, profiles/r2c_triton_vs_b200.md).
+  // reference's Triton kernel on this shape).
   // Not where that makes a second wave out of the first, which streams the weights twice (65 - 128 tokens, us: bf16 16384 x 4096 44 -
   // 46 -> 27 - 29, 9728 x 896 13.0 -> 10.3, int8 12288 x 3584 20 -> 14).  With a short k several of the smaller tiles share an SM, and
   // beyond 128 tokens it is not this kernel that the larger ones compete with (gemm_dense.cu: one_short_wave): 257 x 4864 x 128 bf16

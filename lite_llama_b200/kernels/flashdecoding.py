@@ -10,7 +10,7 @@ import torch
 from ._common import check, counters, dtype_code, index_width, lib, no_grad, ptr, require_cuda, stream_handle, workspace
 
 # Folding the split-KV merge into the last-arriving split CTA (tickets) removes a launch but measured SLOWER at decode
-# sizes (24.8 us vs 11.3 + ~3 us: one CTA merges 4096 outputs serially at L2 latency, profiles/r2f_*): off by default.
+# sizes (24.8 us vs 11.3 + ~3 us: one CTA merges 4096 outputs serially at L2 latency): off by default.
 _FOLD = os.environ.get("B2L_FD_FOLD", "0") != "0"
 
 
