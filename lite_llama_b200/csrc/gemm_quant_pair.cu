@@ -18,7 +18,7 @@
 // keeps the card at its power cap): int4 1853 -> 900 us (1.07 PFLOP/s), fp8 in 128 x 128
 // blocks 1748 -> 867 us, int8 per channel 3124 -> 754 us (no drain before the end of k: 1.28 PFLOP/s).  A third accumulator
 // at the cost of two operand stages: int4 878, fp8 901 us.  Sizes of that order are now taken by the kernel of 256 tokens per
-// tile (gemm_quant_wide.cu).  One issuer and two accumulators -> two and three or four, us: int4 28672 x 4096 with the
+// tile (gemm_quant_wide.cu), but for 8-bit weights in groups of 128 (fp8 in blocks 872 us in launches in a row, with 256 tokens 910).  One issuer and two accumulators -> two and three or four, us: int4 28672 x 4096 with the
 // activation at 128 tokens 42.7 -> 36.8, 4096 x 14336 at 512 63 -> 54, fp8 in blocks 4096 x 4096 at 512 19.3 -> 17.1; experts (128 of
 // 2048 x 768, fp8, top 8) gate|up and down at 2000 tokens 173 + 153 -> 135 + 126, at 32 69 + 46 -> 58 + 33.
 // Numerics are the streaming kernel's: unscaled integer / e4m3 operands, zero points subtracted exactly, one segment of

@@ -14,11 +14,13 @@
 //   * at the end of a tile lanes exchange values for stores of four outputs: 64 or 32 bytes of a token per store kept the
 //     accumulators waiting for 9000 cycles of a 33000-cycle tile (4096 k, with the activation);
 //   * tiles of a last wave that leaves half of the pairs idle or more are cut in two.
-// The roles' registers decide: with 48 registers the issuers spill in their loop (28672 x 4096 at 2048 tokens, int4: 502 us
-// instead of 402).
+// The roles' registers decide: with 48 registers for the issuers 28672 x 4096 at 2048 tokens, int4, takes 502 us instead of 402
+// (with 72, 20 - 40 bytes of spills are left in all roles together).
 // Measured, us, 128 tokens per tile -> this kernel, launches in a row: 28672 x 4096 with the activation, int4, 4000 tokens 1198
-// -> 815 (1.15 PFLOP/s), 2048 tokens 578 -> 409; 4096 x 14336, 2048 tokens, int4 291 -> 215, fp8 in blocks 276 -> 232, int8 per
-// channel 242 -> 194.  The same bits.
+// -> 815 (1.15 PFLOP/s), 2048 tokens 578 -> 409; 4096 x 14336, 2048 tokens, int4 291 -> 215, int8 with one scale per row 242 -> 194.
+// The same bits.  (With two issuers of its own the kernel of 128 tokens per tile takes 494 and 236 us for the second and the third of
+// these, and stays the faster one for a short k and for 8-bit weights in groups of 128: quant_wide_wanted.)  Int4, 2048 x 28672 x 4096:
+// the tensor pipe active 64 % of the cycles, with one scale per row 92 % (profiles/pairs_and_shares_ncu.txt).
 #define B2L_HANG_NORETURN true   // common.cuh: 128 accumulators beside the wait loops
 #include "gemm_tc.cuh"
 #include "gemm_quant_pair.cuh"
