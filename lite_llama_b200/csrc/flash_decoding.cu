@@ -24,6 +24,7 @@
 //  * a step too small to fill the chip is bound by latency instead: its splits are the CTAs of a cluster, with as few kv
 //    heads each as still fit in one wave, and merge through one another's shared memory (cluster_merge below).
 #include "common.cuh"
+#include <type_traits>
 
 namespace {
 
@@ -31,7 +32,6 @@ constexpr int kTT = 16;            // tokens per pipeline stage (one m16n8k16 k-
 constexpr int kMaxConsumers = 8;
 constexpr int kMaxStages = 4;
 constexpr int kMaxCluster = 8;
-constexpr float kNear = 4.f;       // Consumer::tile
 constexpr int kStagesAt = 128;     // bytes of shared memory before the stages: their barriers
 
 struct DecodeParams {
@@ -126,13 +126,21 @@ __device__ __forceinline__ void cluster_merge(const DecodeParams& p, uint32_t pa
   cluster_sync_all();                 // the peers have read this CTA's rows
 }
 
+// two values of which those that are not finite become 0
+template <typename T>
+__device__ __forceinline__ uint32_t finite2(uint32_t v) {
+  typename Vec2<T>::type x = *reinterpret_cast<const typename Vec2<T>::type*>(&v), largest;
+  const uint32_t most = std::is_same<T, __half>::value ? 0x7bff7bffu : 0x7f7f7f7fu;
+  largest = *reinterpret_cast<const typename Vec2<T>::type*>(&most);
+  return v & __hle2_mask(__habs2(x), largest);
+}
+
 // One consumer warp's work: 16 query heads (fewer: rows of zeros) of one kv head, its tiles of kTT tokens in turn.
 template <typename T, int D>
 struct Consumer {
   uint32_t qf[D / 16][4];             // A operand, m16 x k16 per step; rows = query heads of this KV group
   float o[D / 8][4];
-  float m_run[2], l_run[2];           // what the sums are relative to (log2), and the sums of the probabilities
-  float top[2];                       // largest score so far
+  float m_run[2], l_run[2];
   bool v0, v1;                        // rows g and g + 8 exist
 
   __device__ __forceinline__ void begin(const DecodeParams& p, int b, int kvh, int hq0, int hq1, int tq) {
@@ -151,15 +159,14 @@ struct Consumer {
     }
 #pragma unroll
     for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-    m_run[0] = m_run[1] = top[0] = top[1] = -INFINITY;
+    m_run[0] = m_run[1] = -INFINITY;
     l_run[0] = l_run[1] = 0.f;
   }
   // the tile at shared address sb, tokens tbase .. of which those before `end` count; ka, va: ldmatrix lane addresses.
-  // NEAR: probabilities relative to the largest score of the tile, not of all tiles so far, unless that is more than kNear (in log2)
-  // above.  The largest of each tile is then 1, which loses nothing as a 16-bit operand; with one such in a whole part, rows in few
-  // parts end 2 - 5 % further from the exact result than rows in many.  (The rest of each probability as an operand of its own does
-  // better still, but 0 and what is below 0 turn an infinite value into NaN.)  Sums grow by up to 2^kNear.
-  template <bool NEAR>
+  // REST: what the probabilities lose as 16-bit operands is multiplied as well.  Of every split the largest probability is 1, which
+  // loses nothing, so rows in few parts would end 2 - 5 % further from the exact result than rows in many; with it they end 19 %
+  // closer.  That rest is 0 or negative for most, and 0 x inf and inf - inf are NaN, so it leaves out values that are not finite.
+  template <bool REST>
   __device__ __forceinline__ void tile(const DecodeParams& p, uint32_t sb, uint32_t ka, uint32_t va, int64_t tbase, int64_t end, int tq) {
     // ---- S = Q K^T  (16 heads x 16 tokens) ----
     float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
@@ -188,8 +195,7 @@ struct Consumer {
     for (int r2 = 0; r2 < 2; ++r2) {
       mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 1));
       mx[r2] = fmaxf(mx[r2], __shfl_xor_sync(0xffffffffu, mx[r2], 2));
-      top[r2] = fmaxf(top[r2], mx[r2]);
-      const float mnew = NEAR ? fmaxf(mx[r2], top[r2] - kNear) : top[r2];
+      const float mnew = fmaxf(m_run[r2], mx[r2]);
       base[r2] = mnew == -INFINITY ? 0.f : mnew;   // avoid (-inf) - (-inf)
       alpha[r2] = fast_exp2(m_run[r2] - base[r2]);
       m_run[r2] = mnew;
@@ -217,12 +223,26 @@ struct Consumer {
     pf[1] = pack2<T>(sc[0][2], sc[0][3]);
     pf[2] = pack2<T>(sc[1][0], sc[1][1]);
     pf[3] = pack2<T>(sc[1][2], sc[1][3]);
+    uint32_t rest[4];
+    if (REST) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const typename Vec2<T>::type h = *reinterpret_cast<const typename Vec2<T>::type*>(&pf[i]);
+        rest[i] = pack2<T>(sc[i >> 1][2 * (i & 1)] - to_f32(h.x), sc[i >> 1][2 * (i & 1) + 1] - to_f32(h.y));
+      }
+    }
 #pragma unroll
     for (int dn = 0; dn < D / 16; ++dn) {
       uint32_t bf[4];
       ldmatrix_x4_trans(bf, sb + va + dn * 32);
       mma_m16n8k16<T>(o[2 * dn], pf, bf[0], bf[1]);
       mma_m16n8k16<T>(o[2 * dn + 1], pf, bf[2], bf[3]);
+      if (REST) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bf[i] = finite2<T>(bf[i]);
+        mma_m16n8k16<T>(o[2 * dn], rest, bf[0], bf[1]);
+        mma_m16n8k16<T>(o[2 * dn + 1], rest, bf[2], bf[3]);
+      }
     }
   }
   // quad-reduce the row sums (each lane only summed its own 4 columns per tile)
@@ -800,13 +820,14 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
 }
 
 // Steps that would take several waves of CTAs of which an SM holds one or two, whose rings of large stages start anew with each.
-// us in a graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 35.8 -> 29.7, of 500 - 1000 27.0 ->
-// 23.6, of 1000 - 2000 50.6 -> 40.8, 256 of 200 58.7 -> 50.2; 32 kv heads, 64 of 250 - 500 94 -> 84; 4 kv heads, 32 of 1000 - 2000 29.8 ->
-// 24.8, 64 of 1000 35.1 -> 31.1.  The lengths are not known here.  Far below the bound the splits that have tokens go to a CTA each,
-// which is level or faster in most (8 kv heads, one of 1000 among 31 of 50 11.1 -> 10.5, 32 of 200 11.3 -> 11.0; 4 kv heads, 32 of 40 under
-// 2000 8.7 -> 8.9; 32 kv heads, one of 1600 under 8000 13.1 -> 12.3; slowest: 8 of 800 under 4000 11.1 -> 11.9, 4 kv heads, one of 2000
-// among 31 of 100 12.3 -> 13.3).  Below 13 tiles per CTA, or with more CTAs to an SM, the splits stay: 8 kv heads 32 x 480 16.7 against
-// 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
+// us in a graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 36.1 -> 30.3, of 500 - 1000 27.2 ->
+// 24.7, of 1000 - 2000 50.7 -> 41.5, 256 of 200 59.1 -> 50.5; 4 kv heads, 32 of 1000 - 2000 29.9 -> 25.8, 64 of 1000 35.4 -> 31.6; 32 kv
+// heads of one query head each, whose warps have the most to do per byte, 64 of 250 - 500 94.9 -> 88.4, of 1000 205 -> 214.  The lengths
+// are not known here.  Far below the bound the splits that have tokens go to a CTA each, which is level or faster in most (8 kv heads, one
+// of 1000 among 31 of 50 11.1 -> 10.4, 32 of 200 11.4 -> 11.2; 4 kv heads, 32 of 40 under 2000 8.7 -> 9.1; slowest: 4 kv heads, one of
+// 2000 among 31 of 100 12.3 -> 13.0, 32 kv heads, one of 1600 under 8000 13.2 -> 15.4).  Below 13 tiles per CTA, or with more CTAs to an SM,
+// the splits stay: 8 kv heads 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000
+// 13.2 / 20.
 void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int smem_cap) {
   if (pl.splits < 2 || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 26)) return;
   pl.share_smem = pl.smem + (int)(3 * batch + 1) * 4;
@@ -815,10 +836,10 @@ void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int sme
   if (per_sm > 2) return;
   if (per_sm < 1) per_sm = 1;
   if (batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * per_sm * b2l_num_sms()) return;
-  // One wave: by registers, too (151, 96 and 72 a thread, handed out in eights), an SM may hold one CTA only, of heads of 128 with two
-  // warps of query heads to a kv head (4 kv heads, 20 query heads each, 32 of 1000 - 2000 tokens, splits 52.9 us, shares in two waves
-  // 46.4, in one 39.2).
-  if (per_sm == 2 && 2 * (pl.HB * pl.qblocks + 1) * 32 * (D == 128 ? 152 : D == 64 ? 96 : 72) > 65536) per_sm = 1;
+  // One wave: by registers, too (168, 96 and 72 a thread), an SM may hold one CTA only, of heads of 128 with two
+  // warps of query heads to a kv head (4 kv heads, 20 query heads each, 32 of 1000 - 2000 tokens, splits 53.5 us, shares in two waves
+  // 46.4, in one 41.4).
+  if (per_sm == 2 && 2 * (pl.HB * pl.qblocks + 1) * 32 * (D == 128 ? 168 : D == 64 ? 96 : 72) > 65536) per_sm = 1;
   pl.share_grid = per_sm * b2l_num_sms();
 }
 
