@@ -174,3 +174,27 @@ def test_a_workspace_for_the_splits_alone_is_enough(heads, kv_heads, d):
     want = exact(q, k, v, table, order, [bound] * batch)
     assert ((out.double() - want).norm() / want.norm()).item() < 2.0**-10
     assert (ws[nbytes:] == 7).all()
+
+
+def test_a_captured_step_follows_the_lengths():
+    """One graph, replayed with lengths whose splits fit the CTAs and with others, in turn: nothing of a replay is left for the next."""
+    batch, bound, heads, kv_heads, d = 32, 2000, 32, 8, 128
+    data = inputs(batch, bound, heads, kv_heads, d, torch.float16)
+    lens = torch.full((batch,), bound, device="cuda").int()
+    import lite_llama_b200.kernels as K
+
+    q, k, v, table, order = data
+    call = lambda: K.flash_decoding(q, k, v, d**-0.5, table, order.int(), lens, bound)  # noqa: E731
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        call()
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    for kind in ("full", "few", "ragged", "one long", "none", "holes", "few", "full"):
+        want = lengths(kind, batch, bound)
+        lens.copy_(torch.tensor(want).int())
+        graph.replay()
+        assert torch.equal(out, run(*data, want, bound))
