@@ -212,10 +212,14 @@ struct Consumer {
     }
     l_run[0] = l_run[0] * alpha[0] + ps[0];
     l_run[1] = l_run[1] * alpha[1] + ps[1];
+    // (most tiles do not raise the largest score; what REST saves here pays for the values that it leaves out: 32 kv heads of one query
+    // head each, 64 rows of 250 - 500 88.4 -> 84.8 us)
+    if (!REST || __any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i) {
-      o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
-      o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+      for (int i = 0; i < D / 8; ++i) {
+        o[i][0] *= alpha[0]; o[i][1] *= alpha[0];
+        o[i][2] *= alpha[1]; o[i][3] *= alpha[1];
+      }
     }
     // ---- O += P V  (P: 16 heads x 16 tokens as the A operand) ----
     uint32_t pf[4];
@@ -822,7 +826,7 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
 // Steps that would take several waves of CTAs of which an SM holds one or two, whose rings of large stages start anew with each.
 // us in a graph, split and merge kernel -> shares: 8 kv heads of 128, 32 sequences of 1000 tokens 36.1 -> 30.3, of 500 - 1000 27.2 ->
 // 24.7, of 1000 - 2000 50.7 -> 41.5, 256 of 200 59.1 -> 50.5; 4 kv heads, 32 of 1000 - 2000 29.9 -> 25.8, 64 of 1000 35.4 -> 31.6; 32 kv
-// heads of one query head each, whose warps have the most to do per byte, 64 of 250 - 500 94.9 -> 88.4, of 1000 205 -> 214.  The lengths
+// heads of one query head each, whose warps have the most to do per byte, 64 of 250 - 500 94.9 -> 84.8, of 1000 205 -> 204.  The lengths
 // are not known here.  Far below the bound the splits that have tokens go to a CTA each, which is level or faster in most (8 kv heads, one
 // of 1000 among 31 of 50 11.1 -> 10.4, 32 of 200 11.4 -> 11.2; 4 kv heads, 32 of 40 under 2000 8.7 -> 9.1; slowest: 4 kv heads, one of
 // 2000 among 31 of 100 12.3 -> 13.0, 32 kv heads, one of 1600 under 8000 13.2 -> 15.4).  Below 13 tiles per CTA, or with more CTAs to an SM,
