@@ -552,8 +552,12 @@ struct ShareWalk {
   }
 };
 
+// Registers of a thread: what plan_shares counts with.  Left to itself the compiler takes 168 with heads of 128, beside which fewer blocks
+// of the merge kernel wait on the SM (32 kv heads, one of 1600 tokens under 8000 15.4 us instead of 12.5, four of 400 12.5 / 11.3).
+__host__ __device__ constexpr int share_regs(int D) { return D == 128 ? 152 : D == 64 ? 96 : 72; }
+
 template <typename T, int D>
-__global__ void __launch_bounds__((kMaxConsumers + 1) * 32) flash_decode_shares_kernel(const ShareParams p) {
+__global__ void __maxnreg__(share_regs(D)) flash_decode_shares_kernel(const ShareParams p) {
   pdl_prologue();   // everything below reads what earlier kernels of the step wrote (q, KV rows, lengths, table)
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int warp_sum[2][kMaxConsumers + 1];
@@ -828,8 +832,8 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
 // 24.7, of 1000 - 2000 50.7 -> 41.5, 256 of 200 59.1 -> 50.5; 4 kv heads, 32 of 1000 - 2000 29.9 -> 25.8, 64 of 1000 35.4 -> 31.6; 32 kv
 // heads of one query head each, whose warps have the most to do per byte, 64 of 250 - 500 94.9 -> 84.8, of 1000 205 -> 204.  The lengths
 // are not known here.  Far below the bound the splits that have tokens go to a CTA each, which is level or faster in most (8 kv heads, one
-// of 1000 among 31 of 50 11.1 -> 10.4, 32 of 200 11.4 -> 11.2; 4 kv heads, 32 of 40 under 2000 8.7 -> 9.1; slowest: 4 kv heads, one of
-// 2000 among 31 of 100 12.3 -> 13.0, 32 kv heads, one of 1600 under 8000 13.2 -> 15.4).  Below 13 tiles per CTA, or with more CTAs to an SM,
+// of 1000 among 31 of 50 11.1 -> 10.5, 32 of 200 11.3 -> 11.1; 4 kv heads, 32 of 40 under 2000 8.7 -> 9.1; 32 kv heads, one of 1600 under
+// 8000 13.1 -> 12.5; slowest: 8 kv heads, 8 of 800 under 4000 11.1 -> 12.0, 4 kv heads, one of 2000 among 31 of 100 12.3 -> 13.4).  Below 13 tiles per CTA, or with more CTAs to an SM,
 // the splits stay: 8 kv heads 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000
 // 13.2 / 20.
 void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int smem_cap) {
@@ -840,10 +844,10 @@ void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int sme
   if (per_sm > 2) return;
   if (per_sm < 1) per_sm = 1;
   if (batch * tiles * (Hkv / pl.HB) < (Hkv > pl.HB ? 6ll : 13ll) * per_sm * b2l_num_sms()) return;
-  // One wave: by registers, too (168, 96 and 72 a thread), an SM may hold one CTA only, of heads of 128 with two
+  // One wave: by registers, too, an SM may hold one CTA only, of heads of 128 with two
   // warps of query heads to a kv head (4 kv heads, 20 query heads each, 32 of 1000 - 2000 tokens, splits 53.5 us, shares in two waves
   // 46.4, in one 41.4).
-  if (per_sm == 2 && 2 * (pl.HB * pl.qblocks + 1) * 32 * (D == 128 ? 168 : D == 64 ? 96 : 72) > 65536) per_sm = 1;
+  if (per_sm == 2 && 2 * (pl.HB * pl.qblocks + 1) * 32 * share_regs(D) > 65536) per_sm = 1;
   pl.share_grid = per_sm * b2l_num_sms();
 }
 
