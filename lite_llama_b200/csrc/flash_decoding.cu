@@ -833,9 +833,9 @@ bool plan_cluster(Plan& pl, int64_t batch, int G, int Hkv, int D, int64_t tiles,
 // heads of one query head each, whose warps have the most to do per byte, 64 of 250 - 500 94.9 -> 84.8, of 1000 205 -> 204.  The lengths
 // are not known here.  Far below the bound the splits that have tokens go to a CTA each, which is level or faster in most (8 kv heads, one
 // of 1000 among 31 of 50 11.1 -> 10.5, 32 of 200 11.3 -> 11.1; 4 kv heads, 32 of 40 under 2000 8.7 -> 9.1; 32 kv heads, one of 1600 under
-// 8000 13.1 -> 12.5; slowest: 8 kv heads, 8 of 800 under 4000 11.1 -> 12.0, 4 kv heads, one of 2000 among 31 of 100 12.3 -> 13.4).  Below 13 tiles per CTA, or with more CTAs to an SM,
-// the splits stay: 8 kv heads 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8, 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000
-// 13.2 / 20.
+// 8000 13.1 -> 12.5; slowest: 8 kv heads, 8 of 800 under 4000 11.1 -> 12.0, 4 kv heads, one of 2000 among 31 of 100 12.3 -> 13.4).
+// Below 13 tiles per CTA, or with more CTAs to an SM, the splits stay: 8 kv heads 32 x 480 16.7 against 16.2, but 64 x 256 16.7 / 17.8,
+// 128 x 128 18.1 / 20.6; 2 kv heads of 64, 32 x 2000 13.2 / 20.
 void plan_shares(Plan& pl, int64_t batch, int Hkv, int D, int64_t tiles, int smem_cap) {
   if (pl.splits < 2 || D > 128 || batch * tiles * (Hkv / pl.HB) >= (1ll << 26)) return;
   pl.share_smem = pl.smem + (int)(3 * batch + 1) * 4;
