@@ -70,8 +70,8 @@ def splits_fit(batch, heads, kv_heads, d, bound, lens) -> bool:
     return sum(-(-n // p.tokens) for n in lens) * p.blocks <= p.grid
 
 
-def check(batch, bound, lens, heads, kv_heads, d, dtype, wide=False, layout="pool"):
-    assert plan(batch, heads, kv_heads, d, bound).form == SHARES
+def check(batch, bound, lens, heads, kv_heads, d, dtype, wide=False, layout="pool", shares=True):
+    assert not shares or plan(batch, heads, kv_heads, d, bound).form == SHARES
     data = inputs(batch, bound, heads, kv_heads, d, dtype, layout)
     got = run(*data, lens, bound, wide)
     assert torch.equal(got, run(*data, lens, bound, wide))
@@ -90,6 +90,19 @@ def test_shares_of_any_lengths(heads, kv_heads, d, kind, dtype):
         if batch * bound * kv_heads > 1 << 20:
             bound //= 2
         check(batch, bound, lengths(kind, batch, bound), heads, kv_heads, d, dtype, batch == 32, "two" if batch == 100 else "pool")
+
+
+@pytest.mark.parametrize("heads,kv_heads,d", HEADS[:4])
+@pytest.mark.parametrize("kind", ["full", "ragged", "fifth", "few", "one long", "holes", "none"])
+def test_lengths_around_the_line_of_the_shares(heads, kv_heads, d, kind):
+    for batch, bound in ((8, 4001), (32, 1000), (100, 460), (130, 250)):
+        lens = lengths(kind, batch, bound)
+        check(batch, bound, lens, heads, kv_heads, d, torch.float16, batch == 32, "two" if batch == 100 else "pool", shares=False)
+
+
+def test_rows_of_a_single_split_in_bf16():
+    check(1024, 33, lengths("ragged", 1024, 33), 32, 8, 128, torch.bfloat16, shares=False)
+    check(1024, 65, lengths("holes", 1024, 65), 32, 8, 128, torch.bfloat16, True, shares=False)
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
